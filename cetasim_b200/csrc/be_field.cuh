@@ -18,16 +18,14 @@ namespace cg {
 
 // BassettiErskine1 for sx > sy.  posx/posy signs are restored at the end as
 // in Bunch.cpp:161-169 (note: "<= 0" flips, so x = 0 gives -0 * F).
-template <bool LowLat = false>
 CG_HD void bassetti_erskine(double posx, double posy, double sx, double sy,
                             double* fx, double* fy) {
   double ax = fabs(posx), ay = fabs(posy);
   double sigma = sqrt(2.0 * (sx * sx) - 2.0 * (sy * sy));
   double r = sy / sx;
   double coeff = -1.0 * sqrt(kPi) / sigma;
-  cplx w1 = LowLat ? w_quadrant1_lowlat(ax / sigma, ay / sigma) : w_quadrant1(ax / sigma, ay / sigma);
-  cplx w2 = LowLat ? w_quadrant1_lowlat(r * ax / sigma, ay / sigma / r)
-                   : w_quadrant1(r * ax / sigma, ay / sigma / r);
+  cplx w1 = w_quadrant1(ax / sigma, ay / sigma);
+  cplx w2 = w_quadrant1(r * ax / sigma, ay / sigma / r);
   double tx = ax / sx, ty = ay / sy;
   double z3 = -(tx * tx) / 2.0 - (ty * ty) / 2.0;
   double w3 = -exp(z3);
@@ -50,18 +48,16 @@ CG_HD void gaussian_round_field(double posx, double posy, double sx, double* fx,
   *fy = -posy / r2 * g;
 }
 
-// The dispatch of MPBunch.cpp:1128-1146 / 1179-1197.  LowLat selects the
-// latency-optimised w(z) (Estrin form) for the sequential ion chain.
-template <bool LowLat = false>
+// The dispatch of MPBunch.cpp:1128-1146 / 1179-1197.
 CG_HD void gaussian_field(double posx, double posy, double sx, double sy,
                           double* fx, double* fy) {
   if (fabs(posx / sx) + fabs(posy / sy) < 1.0e-5) {
     *fx = 0.0;
     *fy = 0.0;
   } else if ((sx - sy) / sy > 1.e-4) {
-    bassetti_erskine<LowLat>(posx, posy, sx, sy, fx, fy);
+    bassetti_erskine(posx, posy, sx, sy, fx, fy);
   } else if ((sx - sy) / sy < -1.e-4) {
-    bassetti_erskine<LowLat>(posy, posx, sy, sx, fy, fx);
+    bassetti_erskine(posy, posx, sy, sx, fy, fx);
   } else {
     gaussian_round_field(posx, posy, sx, fx, fy);
   }
@@ -121,7 +117,7 @@ CG_HD void field_zargs(const FieldPrep& p, double posx, double posy, double* z1r
 CG_HD double field_gauss(const FieldPrep& p, double posx, double posy) {
   double a = p.mode == 1 ? posy : posx, b = p.mode == 1 ? posx : posy;
   double tx = fabs(a) * p.ia, ty = fabs(b) * p.ib;
-  return exp(-(tx * tx) / 2.0 - (ty * ty) / 2.0);
+  return exp_neg(0.5 * fma(tx, tx, ty * ty));
 }
 
 // Field from the prepared constants, the two w values and the Gaussian factor.
@@ -159,24 +155,15 @@ CG_HD void field_finish(const FieldPrep& p, double posx, double posy, cplx w1, c
   field_finish_g(p, posx, posy, w1, w2, g, fx, fy);
 }
 
-// The same with the kick kernels' w(z) (w_quadrant1_wide).
+// The same with the kick kernels' w(z) (w_quadrant1_wide2).
 CG_HD void gaussian_field_kick(const FieldPrep& p, double posx, double posy, double* fx,
                                double* fy) {
   double z1r, z1i, z2r, z2i;
   field_zargs(p, posx, posy, &z1r, &z1i, &z2r, &z2i);
-  cplx w1 = w_quadrant1_wide(z1r, z1i);
-  cplx w2 = w_quadrant1_wide(z2r, z2i);
-  field_finish(p, posx, posy, w1, w2, fx, fy);
-}
-
-template <bool LowLat = false>
-CG_HD void gaussian_field_prep(const FieldPrep& p, double posx, double posy, double* fx,
-                               double* fy) {
-  double z1r, z1i, z2r, z2i;
-  field_zargs(p, posx, posy, &z1r, &z1i, &z2r, &z2i);
-  cplx w1 = LowLat ? w_quadrant1_lowlat(z1r, z1i) : w_quadrant1(z1r, z1i);
-  cplx w2 = LowLat ? w_quadrant1_lowlat(z2r, z2i) : w_quadrant1(z2r, z2i);
-  field_finish(p, posx, posy, w1, w2, fx, fy);
+  const double zr[2] = {z1r, z2r}, zi[2] = {z1i, z2i};
+  cplx w[2];
+  w_quadrant1_wide2(zr, zi, w);
+  field_finish(p, posx, posy, w[0], w[1], fx, fy);
 }
 
 }  // namespace cg

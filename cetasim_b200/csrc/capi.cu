@@ -133,7 +133,7 @@ void free_beam(Handle& h) {
   h.cbm_cap = h.cbm_n = 0;
   IonWalk& w = d.iw;
   dfree(w.births); dfree(w.prep); dfree(w.bunch); dfree(w.spec); dfree(w.bound); dfree(w.part);
-  dfree(w.traj); dfree(w.alive); dfree(w.carry);
+  dfree(w.traj); dfree(w.alive); dfree(w.carry); dfree(w.done);
   w = IonWalk();
   d.c = nullptr; d.surv = nullptr; d.tile_bunch = nullptr; d.chunk_bunch = nullptr;
   d.chunk_loc = nullptr;
@@ -853,15 +853,18 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
     // ion-chain scratch: trajectories = the cloud's capacity + the births of one walk
     IonWalk& w = d.iw;
     const size_t NM = (size_t)h.cfg.ion.macro_ions_per_ip, P = (size_t)h.P;
-    w.tcap = (int64_t)h.ion_cap + (int64_t)M * (int64_t)NM;
-    w.grid = ion_walk_grid(w.tcap, 8);  // the most walk CTAs of any shape
+    // whole 16s: the compaction reads the survivors' flags 16 at a time
+    w.tcap = ((int64_t)h.ion_cap + (int64_t)M * (int64_t)NM + 15) / 16 * 16;
+    w.grid = ion_walk_grid(w.tcap, 16);  // the most walk CTAs of any shape
     if (dalloc(&w.births, P * M * NM * 2) || dalloc(&w.prep, (size_t)M) ||
         dalloc(&w.bunch, 3 * (size_t)M) || dalloc(&w.spec, P * M * 2) || dalloc(&w.bound, 2) ||
         dalloc(&w.part, P * M * (size_t)w.grid * 5) || dalloc(&w.traj, P * 6 * (size_t)w.tcap) ||
-        dalloc(&w.alive, P * (size_t)w.tcap) || dalloc(&w.carry, 4 * P)) {
+        dalloc(&w.alive, P * (size_t)w.tcap) || dalloc(&w.carry, 5 * P) ||
+        dalloc(&w.done, 2 * P)) {
       free_beam(h);
       return fail(&h, CG_ERR_OOM, "ion chain scratch");
     }
+    cudaMemset(w.done, 0, sizeof(unsigned) * 2 * P);
   }
   if (h.cfg.flag_lr_wake) {
     if (dalloc(&d.lr_hist, (size_t)h.cfg.lr_turns * 3 * M) || dalloc(&d.lr_force, 3 * (size_t)M)) {

@@ -90,8 +90,10 @@ struct IonWalk {
   double* part = nullptr;     // P x M x grid x (count, sum x, sum y, sum x^2, sum y^2)
   double* traj = nullptr;     // P x 6 x tcap: x, y, vx, vy after the walk, last kick fx, fy
   uint8_t* alive = nullptr;   // P x tcap
-  double* carry = nullptr;    // P x (centroid x, y carried between steps, last rms x, y)
-  int64_t tcap = 0;           // trajectories per species: cloud capacity + M x NM
+  double* carry = nullptr;    // P x (centroid x, y carried between steps, last rms x, y), then
+                              // P survivor counts of the compaction
+  unsigned* done = nullptr;   // P x 2: finished CTAs of k_ion_records, k_ion_compact (0 between)
+  int64_t tcap = 0;           // trajectories per species: cloud capacity + M x NM, whole 16s
   int grid = 0;               // CTAs of k_ion_walk per species
 };
 
@@ -220,9 +222,9 @@ struct Handle {
   std::vector<double*> phase_bufs; // their device buffers (6 x n each)
   std::vector<double> bbi_table;  // the copy of cfg.bbi.table
   int pipe_groups = 4;
-  // trajectories per walk CTA (8, 16, 32, 64): smaller CTAs spread the
-  // walk's FP64 work over more SMs and find room sooner while the kicks and
-  // maps of earlier segments fill the GPU
+  // trajectories per walk CTA (8, 16, 32, 64; 8 runs as 16, one warp): smaller
+  // CTAs spread the walk's FP64 work over more SMs and find room sooner while
+  // the kicks and maps of earlier segments fill the GPU
   int walk_ions = 64;
   bool pipe_ramp = false;  // last walk segment half as long as the others
   bool walk_reserve = false;  // walk CTAs take their SM's whole shared memory

@@ -37,6 +37,7 @@ void weideman_table_init(WeidemanTable* t) {
     t->a[N - n] = (double)(s / M2);
   }
   t->L = (double)L;
+  for (int i = 0; i < kWeidemanTail; ++i) t->t[i] = (float)t->a[i];
 }
 
 }  // namespace cg

@@ -16,15 +16,15 @@
 // couple them are the cloud moments each bunch sees, which are per-step sums
 // over the ions alive at that step.
 //
-// Three kernels per IP:
+// Four kernels per IP:
 //   k_ion_prep    per bunch: loss bounds, birth positions (Philox, attempts in
 //                 order), field constants, coefficients;
-//   k_ion_walk    each CTA walks 16 to 64 trajectories (four lanes per ion: w(z1)
-//                 and w(z2) each split into halves of the series) through all bunches
-//                 without a barrier per bunch, and writes per-step partial
+//   k_ion_walk    each CTA walks 16 to 128 trajectories (two lanes per ion, one
+//                 for w(z1) and one for w(z2), or one lane for both) through all
+//                 bunches without a barrier per bunch, and writes per-step partial
 //                 sums (count, sum x, y, x^2, y^2) every kWin bunches;
-//   k_ion_records per step: sums in CTA order -> cloud centroid and rms ->
-//                 the record the electron kick reads;
+//   k_ion_records one warp per step: sums in a fixed order -> cloud centroid and
+//                 rms -> the record the electron kick reads;
 //   k_ion_compact stable compaction of the survivors into the cloud (birth
 //                 order, as the reference's erase keeps it) and the cloud state.
 // The walk and the records also run as consecutive segments of bunch steps.
@@ -38,14 +38,18 @@ namespace cg {
 
 #define FULL_MASK 0xffffffffu
 
-// The walk's CTA shape: IONS trajectories per block (8, 16, 32 or 64), four
-// lanes per ion; per step the block's ions are summed in groups of 4 (in
-// trajectory order), then the groups in order.
+// The walk's CTA shape: IONS trajectories per block (16, 32 or 64) with two
+// lanes each, or 2 IONS with one lane each (see k_ion_walk).
 constexpr int kWin = 16;                       // steps per shared-memory window
-constexpr int kGroupIons = 4;
+// Trajectories of one species above which one lane walks a whole ion: at two
+// lanes per ion the 592 sub-partitions then hold two warps each, which take
+// 870 cycles a step together, as much as one warp of whole ions (2415 cycles
+// for four); below, the shorter chain of the two lanes wins.
+constexpr int64_t kWalkWide = 148 * 4 * 32;
 constexpr int kPrepThreads = 128;
-constexpr int kFinishThreads = 1024;
-constexpr int kFinishChunk = 2048;             // steps per shared-memory chunk
+constexpr int kRecThreads = 256;
+constexpr int kRecChunk = 2048;                // steps per shared-memory chunk of the carry
+constexpr int kCompactThreads = 1024;
 
 __device__ __forceinline__ void warp_max2(double& a, double& b) {
 #pragma unroll
@@ -145,49 +149,242 @@ __global__ void __launch_bounds__(kPrepThreads) k_ion_prep(ChainParams cp, Chain
   }
 }
 
-// w(z) for a warp in which some lane has |z| >= 30 (an ion far from the
-// bunch), kept out of line: inlined, its continued fraction doubles the
-// walk's code and registers (214 -> 142) and lengthens every step's
-// instruction fetch, although the branch is rarely taken.
-__device__ __noinline__ cplx walk_w_wide(double zr, double zi) {
-  return w_quadrant1_wide_lowlat(zr, zi);
+// One bunch passage as every ion of a window step sees it, in the frame of
+// the bunch's axes (a the larger one): the centroid, the scales of w(z1),
+// w(z2) and of the Gaussian factor, and the ion-side coefficient.
+struct WalkStep {
+  double ma, mb;        // centroid
+  double sa[2], sb[2];  // z1, z2 = (|da| sa, |db| sb)
+  double ga, gb;        // 1/sigma_a, 1/sigma_b
+  double c1;            // coefficient times -sqrt(pi)/sigma
+  double ci;            // coefficient
+  double dt;            // drift time to the next bunch
+  int mode;             // FieldPrep::mode: 1 = a is y
+};
+
+__device__ __forceinline__ WalkStep walk_step_of(const FieldPrep& f, const double* bunch, double ci) {
+  WalkStep s;
+  const bool sw = f.mode == 1;
+  s.ma = sw ? bunch[1] : bunch[0];
+  s.mb = sw ? bunch[0] : bunch[1];
+  s.sa[0] = s.sb[0] = f.isig;
+  s.sa[1] = f.r * f.isig;
+  s.sb[1] = f.isig * f.ir;
+  s.ga = f.ia;
+  s.gb = f.ib;
+  s.c1 = f.coeff * ci;
+  s.ci = ci;
+  s.dt = bunch[2];
+  s.mode = f.mode;
+  return s;
 }
 
-// One CTA block = IONS trajectories: index t < n0 is ion t of the cloud the
-// previous call left, t >= n0 the ion born as number (t - n0) % NM at bunch
-// (t - n0) / NM.  blockIdx.y = species.  The step loop has no block barrier:
-// each ion's position at each step goes to a shared-memory window of kWin
-// steps, and after each window the CTA sums it per step in a fixed order
-// (groups of 4 ions, then the IONS / 4 groups) into the per-step partials.
-// A launch walks the bunch steps [ja, jb): trajectories that started before
-// ja resume from the state the previous segment stored, so the walk can run
-// as consecutive segments (the turn graph kicks the bunches of one segment
-// while the next segment walks).
+// What a window's steps may assume (bits, all steps of the window together).
+enum : int {
+  kWinFlip = 1,  // some bunch has a = y
+  kWinStay = 2,  // some bunch has a = x
+  kWinSlow = 4,  // a round bunch, or an ion within the loss bounds may see |z| >= 30
+};
+// For an ion with |x| <= bx, |y| <= by.
+__device__ __forceinline__ int walk_step_flags(const WalkStep& s, double bx, double by) {
+  if (s.mode == 2) return kWinSlow;
+  const double a = (s.mode == 1 ? by : bx) + fabs(s.ma), b = (s.mode == 1 ? bx : by) + fabs(s.mb);
+  const double ar = a * fmax(s.sa[0], s.sa[1]), bi = b * fmax(s.sb[0], s.sb[1]);
+  return (s.mode == 1 ? kWinFlip : kWinStay) | (fma(ar, ar, bi * bi) < 900.0 ? 0 : kWinSlow);
+}
+
+// An ion in the frame (a, b).
+struct IonState {
+  double a, b, va, vb;
+  double ka, kb;  // the last bunch's velocity kick (ionAccumuFx/Fy)
+  bool alive;
+  __device__ __forceinline__ void flip() {
+    double t = a; a = b; b = t;
+    t = va; va = vb; vb = t;
+    t = ka; ka = kb; kb = t;
+  }
+};
+
+// The constants of one step in registers: PAIR: of this lane's w(z) alone.
+template <bool PAIR>
+struct StepRegs {
+  double ma, mb, sa[2], sb[2], ga, gb, c1, dt;
+};
+template <bool PAIR>
+__device__ __forceinline__ StepRegs<PAIR> step_regs(const WalkStep& s, int sub) {
+  StepRegs<PAIR> r;
+  r.ma = s.ma;
+  r.mb = s.mb;
+  r.sa[0] = s.sa[sub];
+  r.sb[0] = s.sb[sub];
+  if (!PAIR) {
+    r.sa[1] = s.sa[1];
+    r.sb[1] = s.sb[1];
+  }
+  r.ga = s.ga;
+  r.gb = s.gb;
+  r.c1 = s.c1;
+  r.dt = s.dt;
+  return r;
+}
+
+// Velocity kick, drift and loss test (LIP::IonTransferDueToBunch).
+__device__ __forceinline__ void walk_move(double fa, double fb, double dt, bool active, double ba,
+                                          double bb, IonState& q) {
+  if (active) {
+    q.ka = fa;
+    q.kb = fb;
+    q.va += fa;
+    q.vb += fb;
+    q.a += q.va * dt;
+    q.b += q.vb * dt;
+    q.alive = !(fabs(q.a) > ba || fabs(q.b) > bb);
+  }
+}
+
+// The ion side of MPBunch::SSIonBunchInteraction for one ion and one bunch
+// that is not round, all |z| < 30.  PAIR: two lanes per ion, lane `sub`
+// evaluates w(z1) or w(z2) and the halves of the field are added by one
+// shuffle; else one lane evaluates both.  Called by full warps.  The step is
+// one dependent chain from the position to the position; it holds no branch
+// and no vote, so that the Gaussian factor and the scales are worked out
+// beside the series.
+template <bool PAIR>
+__device__ __forceinline__ void walk_step(const StepRegs<PAIR>& st, int sub, bool active, double ba,
+                                          double bb, IonState& q) {
+  const double da = q.a - st.ma, db = q.b - st.mb;
+  const double aa = fabs(da), ab = fabs(db);
+  const double ua = aa * st.ga, ub = ab * st.gb;
+  const double g = exp_neg(0.5 * fma(ua, ua, ub * ub));
+  cplx f;
+  if (PAIR) {
+    f = weideman_scaled(aa * st.sa[0], ab * st.sb[0], sub ? -(st.c1 * g) : st.c1);
+    f.re += __shfl_xor_sync(FULL_MASK, f.re, 1);
+    f.im += __shfl_xor_sync(FULL_MASK, f.im, 1);
+  } else {
+    const double zr[2] = {aa * st.sa[0], aa * st.sa[1]}, zi[2] = {ab * st.sb[0], ab * st.sb[1]};
+    cplx w[2];
+    w_weideman_fast<2>(zr, zi, w);
+    f = {st.c1 * fma(-g, w[1].re, w[0].re), st.c1 * fma(-g, w[1].im, w[0].im)};
+  }
+  double fa = da <= 0 ? -f.im : f.im, fb = db <= 0 ? -f.re : f.re;
+  if (ua + ub < 1.0e-5) fa = fb = 0.0;  // MPBunch.cpp:1128
+  walk_move(fa, fb, st.dt, active, ba, bb, q);
+}
+
+// The same for any bunch and any ion, one lane for both w(z), out of line: a
+// round bunch, or an ion far from the bunch (|z| >= 30).
+__device__ __noinline__ cplx walk_field_any(const WalkStep& st, double da, double db) {
+  double fa, fb;
+  if (st.mode == 2) {
+    gaussian_round_field(da, db, 1.0 / st.ga, &fa, &fb);
+    return {st.ci * fa, st.ci * fb};
+  }
+  const double aa = fabs(da), ab = fabs(db), ua = aa * st.ga, ub = ab * st.gb;
+  const double zr[2] = {aa * st.sa[0], aa * st.sa[1]}, zi[2] = {ab * st.sb[0], ab * st.sb[1]};
+  const double g = exp_neg(0.5 * fma(ua, ua, ub * ub));
+  cplx w[2];
+  w_quadrant1_wide2(zr, zi, w);
+  const cplx f = {st.c1 * fma(-g, w[1].re, w[0].re), st.c1 * fma(-g, w[1].im, w[0].im)};
+  return {da <= 0 ? -f.im : f.im, db <= 0 ? -f.re : f.re};
+}
+
+// The nw steps of a window for one ion born at step `born` of it (or before),
+// its position at each step into the window's rows; flags: what walk_step_flags
+// gives for the window's bunches.  Called by full warps.
+template <bool PAIR, int ROW, int ACT>
+__device__ __forceinline__ void walk_window(const WalkStep* s_st, int flags, int nw, int born,
+                                            int sub, int slot, double (*s_x)[ROW],
+                                            double (*s_y)[ROW], uint8_t (*s_act)[ACT], double bx,
+                                            double by, IonState& q) {
+  if (!__any_sync(FULL_MASK, q.alive && born < nw)) {
+    if (sub == 0)
+      for (int s = 0; s < nw; ++s) s_act[s][slot] = 0;
+    return;
+  }
+  // ions start a call anywhere (a cloud kept from the last one, a birth)
+  const bool inside = __all_sync(FULL_MASK, !q.alive || (fabs(q.a) <= bx && fabs(q.b) <= by));
+  if (inside && (flags == kWinFlip || flags == kWinStay)) {
+    if (flags == kWinFlip) {
+      q.flip();
+      double t = bx; bx = by; by = t;
+      double(*r)[ROW] = s_x; s_x = s_y; s_y = r;
+    }
+    // PAIR, a lone chain: the next step's constants are loaded while this one's
+    // runs (with one lane per ion other warps fill the wait)
+    StepRegs<PAIR> cur = step_regs<PAIR>(s_st[0], sub), nxt;
+#pragma unroll 1
+    for (int s = 0; s < nw; ++s) {
+      if (PAIR) nxt = step_regs<PAIR>(s_st[min(s + 1, nw - 1)], sub);
+      else cur = step_regs<PAIR>(s_st[s], sub);
+      const bool active = q.alive && s >= born;
+      if (sub == 0) {  // the cloud bunch j sees: ions alive after the births of bunch j
+        s_x[s][slot] = q.a;
+        s_y[s][slot] = q.b;
+        s_act[s][slot] = active ? 1 : 0;
+      }
+      walk_step<PAIR>(cur, sub, active, bx, by, q);
+      if (PAIR) cur = nxt;
+    }
+    if (flags == kWinFlip) q.flip();
+    return;
+  }
+#pragma unroll 1
+  for (int s = 0; s < nw; ++s) {
+    const bool active = q.alive && s >= born;
+    if (sub == 0) {
+      s_x[s][slot] = q.a;
+      s_y[s][slot] = q.b;
+      s_act[s][slot] = active ? 1 : 0;
+    }
+    const WalkStep& st = s_st[s];
+    const bool sw = st.mode == 1;
+    const double da = (sw ? q.b : q.a) - st.ma, db = (sw ? q.a : q.b) - st.mb;
+    cplx f = walk_field_any(st, da, db);
+    if (fabs(da) * st.ga + fabs(db) * st.gb < 1.0e-5) f = {0.0, 0.0};  // MPBunch.cpp:1128
+    walk_move(sw ? f.im : f.re, sw ? f.re : f.im, st.dt, active, bx, by, q);
+  }
+}
+
+// One CTA block = IONS trajectories (two lanes each) or, when the clouds hold
+// enough ions to fill the GPU with one lane each (T > kWalkWide), 2 IONS
+// trajectories: index t < n0 is ion t of the cloud the previous call left, t
+// >= n0 the ion born as number (t - n0) % NM at bunch (t - n0) / NM.
+// blockIdx.y = species.  The step loop has no block barrier: each ion's
+// position at each step goes to a shared-memory window of kWin steps, and
+// after each window the CTA sums it per step in a fixed order into the
+// per-step partials.  A launch walks the bunch steps [ja, jb): trajectories
+// that started before ja resume from the state the previous segment stored,
+// so the walk can run as consecutive segments (the turn graph kicks the
+// bunches of one segment while the next segment walks).
+// A train of few ions is bound by the chain of one ion (0.38 us a step alone,
+// of which the FP64 pipe issues 270 cycles), a large cloud by the FP64 pipe:
+// 219 FP64 operations per ion and step with one lane, 2 x 136 with two, 4 x
+// 165 in the form with four lanes per ion that this replaced.  200,000 ions
+// through 1000 bunches: 19.7 -> 3.5 ms per interaction point; the 900-bunch
+// train from empty clouds: 848 -> 521 us (prep to compaction).
 template <int IONS>
-__global__ void __launch_bounds__(4 * IONS, 1) k_ion_walk(ChainParams cp, IonWalk w,
-                                                      const CloudDev* __restrict__ clouds,
-                                                      const CloudState* __restrict__ cst,
-                                                      int ja, int jb) {
-  constexpr int kWalkIons = IONS;
-  constexpr int kWalkThreads = 4 * IONS;
-  constexpr int kGroups = IONS / kGroupIons;   // ion groups summed per step
-  static_assert(kGroups * kWin == kWalkThreads, "the group sums of a window cover the block");
-  __shared__ double s_x[kWin][kWalkIons], s_y[kWin][kWalkIons];
-  __shared__ uint8_t s_act[kWin][kWalkIons];
+__global__ void __launch_bounds__(2 * IONS, 256 / IONS) k_ion_walk(ChainParams cp, IonWalk w,
+                                                                 const CloudDev* __restrict__ clouds,
+                                                                 const CloudState* __restrict__ cst,
+                                                                 int ja, int jb) {
+  constexpr int NT = 2 * IONS;
+  constexpr int kGroups = NT / kWin;  // groups of ions summed per step
+  constexpr int kRow = NT + 8;        // row stride: the rows of one half-warp in distinct banks
+  __shared__ double s_x[kWin][kRow], s_y[kWin][kRow];
+  __shared__ uint8_t s_act[kWin][NT];
   __shared__ double s_grp[kWin][kGroups][5];
-  __shared__ FieldPrep s_fp[kWin];
-  __shared__ double s_bc[kWin][4];  // mean x, mean y, drift time, ion coefficient
-  __shared__ double s_a[kWeidemanN];  // Weideman coefficients (lanes read different ones)
+  __shared__ WalkStep s_st[kWin];
+  __shared__ int s_flags;
   const int p = blockIdx.y, G = gridDim.x, c = blockIdx.x;
   const int M = cp.n_bunches, NM = cp.macro_per_ip;
   const int n0 = cst[p].n;
   const int64_t T = (int64_t)n0 + (int64_t)M * NM;
-  const int nblk = (int)((T + kWalkIons - 1) / kWalkIons);
+  const bool wide = T > kWalkWide;
+  const int per = wide ? NT : IONS;  // trajectories per block
+  const int nblk = (int)((T + per - 1) / per);
   if (c >= nblk) return;
-  const int tid = threadIdx.x, slot = tid >> 2, sub = tid & 3;
-  const bool second = (sub >> 1) != 0, upper = (sub & 1) != 0;
-  for (int i = tid; i < kWeidemanN; i += kWalkThreads) s_a[i] = weideman_table().a[i];
-  const double L = weideman_table().L;
+  const int tid = threadIdx.x, slot = wide ? tid : tid >> 1, sub = wide ? 0 : tid & 1;
   const CloudDev cd = clouds[p];
   const double bx = w.bound[0], by = w.bound[1];
   const double* births = w.births + 2 * (size_t)p * M * NM;
@@ -197,108 +394,59 @@ __global__ void __launch_bounds__(4 * IONS, 1) k_ion_walk(ChainParams cp, IonWal
   uint8_t* alive_out = w.alive + (size_t)p * w.tcap;
   bool first = true;
   for (int blk = c; blk < nblk; blk += G, first = false) {
-    const int64_t t = (int64_t)blk * kWalkIons + slot;
-    const int64_t tb = (int64_t)blk * kWalkIons;
+    const int64_t t = (int64_t)blk * per + slot;
+    const int64_t tb = (int64_t)blk * per;
     const int jfirst = tb < n0 ? 0 : (int)((tb - n0) / NM);
     const int js = max(jfirst, ja);
-    if (first && tid < 5)
-      for (int j = ja; j < min(js, jb); ++j) part[((size_t)j * G + c) * 5 + tid] = 0.0;
-    bool alive = t < T;
+    if (first)
+      for (int e = tid; e < 5 * (min(js, jb) - ja); e += NT)
+        part[((size_t)(ja + e / 5) * G + c) * 5 + e % 5] = 0.0;
+    IonState q = {0, 0, 0, 0, 0, 0, t < T};
     int j0 = 0;
-    double x = 0, y = 0, vx = 0, vy = 0;
-    double kx = 0, ky = 0;  // the last bunch's velocity kick (ionAccumuFx/Fy)
-    if (alive) {
+    if (q.alive) {
       const int start = t < n0 ? 0 : (int)((t - n0) / NM);
       if (t >= n0) j0 = start;
       if (start < ja) {  // walked by an earlier segment
-        x = traj[t];
-        y = traj[w.tcap + t];
-        vx = traj[2 * w.tcap + t];
-        vy = traj[3 * w.tcap + t];
-        alive = alive_out[t] != 0;
+        q.a = traj[t];
+        q.b = traj[w.tcap + t];
+        q.va = traj[2 * w.tcap + t];
+        q.vb = traj[3 * w.tcap + t];
+        q.alive = alive_out[t] != 0;
       } else if (t < n0) {
-        x = cd.x[0][t];
-        y = cd.y[0][t];
-        vx = cd.vx[0][t];
-        vy = cd.vy[0][t];
+        q.a = cd.x[0][t];
+        q.b = cd.y[0][t];
+        q.va = cd.vx[0][t];
+        q.vb = cd.vy[0][t];
       } else {
         const int64_t b = t - n0;
-        x = births[2 * b];
-        y = births[2 * b + 1];
+        q.a = births[2 * b];
+        q.b = births[2 * b + 1];
       }
     }
     for (int jw = js; jw < jb; jw += kWin) {
       const int nw = min(kWin, jb - jw);
       // the window's bunch constants in shared memory (global loads would sit
       // on the latency chain of every step)
+      int flags = 0;
       if (tid < nw) {
         const int j = jw + tid;
-        s_fp[tid] = w.prep[j];
-        s_bc[tid][0] = w.bunch[3 * j];
-        s_bc[tid][1] = w.bunch[3 * j + 1];
-        s_bc[tid][2] = w.bunch[3 * j + 2];
-        s_bc[tid][3] = spec[2 * j + 1];
+        const WalkStep st = walk_step_of(w.prep[j], w.bunch + 3 * j, spec[2 * j + 1]);
+        flags = walk_step_flags(st, bx, by);
+        s_st[tid] = st;
+      }
+      if (tid < 32) {
+        flags = __reduce_or_sync(FULL_MASK, flags);
+        if (tid == 0) s_flags = flags;
       }
       __syncthreads();
-      for (int s = 0; s < nw; ++s) {
-        const int j = jw + s;
-        const bool active = alive && j >= j0;
-        // the cloud bunch j sees: ions alive after the births of bunch j
-        if (sub == 0) {
-          s_x[s][slot] = x;
-          s_y[s][slot] = y;
-          s_act[s][slot] = active ? 1 : 0;
-        }
-        // ion side of MPBunch::SSIonBunchInteraction and the drift/loss of
-        // LIP::IonTransferDueToBunch
-        if (__any_sync(FULL_MASK, active)) {
-          const FieldPrep& fp = s_fp[s];
-          const double mx = s_bc[s][0], my = s_bc[s][1], dt = s_bc[s][2], coeffI = s_bc[s][3];
-          const double dx = x - mx, dy = y - my;
-          double z1r = 0, z1i = 0, z2r = 0, z2i = 0;
-          if (active) field_zargs(fp, dx, dy, &z1r, &z1i, &z2r, &z2i);
-          // lanes 0, 1 of the quad: w(z1); lanes 2, 3: w(z2), which also
-          // evaluate the Gaussian factor alongside the series
-          const double zr = second ? z2r : z1r, zi = second ? z2i : z1i;
-          // every lane evaluates the factor (a per-lane branch would make the
-          // series lanes wait for the exp); lanes 2, 3 keep it
-          const double gall = field_gauss(fp, dx, dy);
-          const double g = (active && second && fp.mode != 2) ? gall : 0.0;
-          cplx wv;
-          if (__all_sync(FULL_MASK, fp.mode == 2 || fma(zr, zr, zi * zi) < 900.0)) {
-            // each w(z) over two lanes: lower and upper halves of the series
-            cplx rden;
-            const cplx ph = weideman_half(zr, zi, L, s_a, upper, &rden);
-            const cplx po = {__shfl_xor_sync(FULL_MASK, ph.re, 1),
-                             __shfl_xor_sync(FULL_MASK, ph.im, 1)};
-            const cplx lo = upper ? po : ph, hi = upper ? ph : po;
-            wv = weideman_from_sum({lo.re + hi.re, lo.im + hi.im}, rden);
-          } else {
-            wv = walk_w_wide(zr, zi);
-          }
-          const cplx wo = {__shfl_xor_sync(FULL_MASK, wv.re, 2),
-                           __shfl_xor_sync(FULL_MASK, wv.im, 2)};
-          const double go = __shfl_xor_sync(FULL_MASK, g, 2);
-          if (active) {
-            double fx, fy;
-            field_finish_g(fp, dx, dy, second ? wo : wv, second ? wv : wo, second ? g : go, &fx,
-                           &fy);
-            kx = coeffI * fx;
-            ky = coeffI * fy;
-            vx += kx;
-            vy += ky;
-            x += vx * dt;
-            y += vy * dt;
-            alive = !(fabs(x) > bx || fabs(y) > by);
-          }
-        }
-      }
+      if (wide) walk_window<false>(s_st, s_flags, nw, j0 - jw, 0, slot, s_x, s_y, s_act, bx, by, q);
+      else walk_window<true>(s_st, s_flags, nw, j0 - jw, sub, slot, s_x, s_y, s_act, bx, by, q);
       __syncthreads();
-      {  // per step and group of 8 ions: (count, sum x, sum y, sum x^2, sum y^2)
+      {  // per step and group of ions: (count, sum x, sum y, sum x^2, sum y^2)
         const int s = tid / kGroups, g = tid % kGroups;
         if (s < nw) {
           double a[5] = {0, 0, 0, 0, 0};
-          for (int i = g * kGroupIons; i < (g + 1) * kGroupIons; ++i) {
+          for (int i = g; i < per; i += kGroups) {
             if (!s_act[s][i]) continue;
             const double xi = s_x[s][i], yi = s_y[s][i];
             a[0] += 1.0;
@@ -308,69 +456,72 @@ __global__ void __launch_bounds__(4 * IONS, 1) k_ion_walk(ChainParams cp, IonWal
             a[4] += yi * yi;
           }
 #pragma unroll
-          for (int q = 0; q < 5; ++q) s_grp[s][g][q] = a[q];
+          for (int e = 0; e < 5; ++e) s_grp[s][g][e] = a[e];
         }
       }
       __syncthreads();
-      for (int e = tid; e < 5 * nw; e += kWalkThreads) {
-        const int s = e / 5, q = e % 5;
+      for (int e = tid; e < 5 * nw; e += NT) {
+        const int s = e / 5;
         double a = 0.0;
 #pragma unroll
-        for (int g = 0; g < kGroups; ++g) a += s_grp[s][g][q];
-        double* dst = part + ((size_t)(jw + s) * G + c) * 5 + q;
+        for (int g = 0; g < kGroups; ++g) a += s_grp[s][g][e % 5];
+        double* dst = part + ((size_t)(jw + s) * G + c) * 5 + e % 5;
         if (first) *dst = a;
         else *dst += a;
       }
     }
     if (t < T && sub == 0) {
-      traj[t] = x;
-      traj[w.tcap + t] = y;
-      traj[2 * w.tcap + t] = vx;
-      traj[3 * w.tcap + t] = vy;
-      traj[4 * w.tcap + t] = kx;
-      traj[5 * w.tcap + t] = ky;
-      alive_out[t] = alive ? 1 : 0;
+      traj[t] = q.a;
+      traj[w.tcap + t] = q.b;
+      traj[2 * w.tcap + t] = q.va;
+      traj[3 * w.tcap + t] = q.vb;
+      traj[4 * w.tcap + t] = q.ka;
+      traj[5 * w.tcap + t] = q.kb;
+      alive_out[t] = q.alive ? 1 : 0;
     }
     __syncthreads();  // shared windows reused by the next block of this CTA
   }
 }
 
-// Records of the bunch steps [ja, jb), one CTA per species: per step the
-// partial sums in CTA order -> cloud centroid and rms -> the record the
-// electron kick reads.  The one-ion quirk keeps the previous centroid, so the
-// centroid is carried from step to step and, across launches, in w.carry
-// (initialised from the cloud state at ja = 0); at jb = M the last rms is
-// kept there too, for the cloud state.
-__global__ void __launch_bounds__(kFinishThreads) k_ion_records(ChainParams cp, IonWalk w,
-                                                              const CloudState* __restrict__ cst,
-                                                              CloudRec* rec, FieldPrep* rec_prep,
-                                                              int* status, int G, int ions,
-                                                              int ja, int jb) {
-  __shared__ double s_ax[kFinishChunk], s_ay[kFinishChunk];
-  __shared__ int s_n[kFinishChunk];
+// Records of the bunch steps [ja, jb), one warp per step and species: the
+// partial sums of the walk's CTAs (each lane every 32nd CTA, then a butterfly:
+// a fixed order) -> cloud centroid and rms -> the record the electron kick
+// reads.  The one-ion quirk keeps the previous centroid, so the last CTA to
+// finish carries the centroid through the steps that hold one ion and, across
+// launches, in w.carry (initialised from the cloud state at ja = 0); at jb = M
+// the last rms is kept there too, for the cloud state.
+// As one CTA for all steps it took 223 us for a segment of 250 steps over 592
+// walk CTAs (23 MB of partials through one SM).
+__global__ void __launch_bounds__(kRecThreads) k_ion_records(ChainParams cp, IonWalk w,
+                                                           const CloudState* __restrict__ cst,
+                                                           CloudRec* rec, FieldPrep* rec_prep,
+                                                           int* status, int G, int ions,
+                                                           int ja, int jb) {
+  __shared__ double s_ax[kRecChunk], s_ay[kRecChunk];
+  __shared__ uint8_t s_one[kRecChunk];
   __shared__ double s_carry[2];
-  const int p = blockIdx.x, P = cp.n_species, tid = threadIdx.x;
+  __shared__ bool s_last;
+  const int p = blockIdx.y, P = cp.n_species, tid = threadIdx.x, lane = tid & 31;
   const int M = cp.n_bunches, NM = cp.macro_per_ip;
   const CloudState st0 = cst[p];
   const int64_t T = (int64_t)st0.n + (int64_t)M * NM;
-  const int nblk = (int)((T + ions - 1) / ions);
+  const int per = T > kWalkWide ? 2 * ions : ions;
+  const int nblk = (int)((T + per - 1) / per);
   const int nwork = nblk < G ? nblk : G;
-  const double* part = w.part + (size_t)p * M * G * 5;
   const double* spec = w.spec + 2 * (size_t)p * M;
   double* carry = w.carry + 4 * (size_t)p;
-  if (tid == 0) {
-    s_carry[0] = ja == 0 ? st0.aver_x : carry[0];
-    s_carry[1] = ja == 0 ? st0.aver_y : carry[1];
-  }
-  for (int j0 = ja; j0 < jb; j0 += kFinishChunk) {
-    const int nj = min(kFinishChunk, jb - j0);
-    __syncthreads();
-    for (int jj = tid; jj < nj; jj += kFinishThreads) {
-      const int j = j0 + jj;
-      double s[5] = {0, 0, 0, 0, 0};
-      for (int cc = 0; cc < nwork; ++cc)
+  const int j = ja + (int)blockIdx.x * (kRecThreads / 32) + (tid >> 5);
+  if (j < jb) {
+    const double* part = w.part + ((size_t)p * M + j) * G * 5;
+    double s[5] = {0, 0, 0, 0, 0};
+    for (int cc = lane; cc < nwork; cc += 32)
 #pragma unroll
-        for (int q = 0; q < 5; ++q) s[q] += part[((size_t)j * G + cc) * 5 + q];
+      for (int q = 0; q < 5; ++q) s[q] += part[5 * cc + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 5; ++q) s[q] += __shfl_xor_sync(FULL_MASK, s[q], o);
+    if (lane == 0) {
       const int n = (int)s[0];
       double ax = 0, ay = 0, rx, ry;
       if (n == 1) {  // one ion: rms = |x| and the centroid stays (LIP.cpp:1125-1129)
@@ -384,15 +535,14 @@ __global__ void __launch_bounds__(kFinishThreads) k_ion_records(ChainParams cp, 
         ry = sqrt(fmax(s[4] * inv_n - ay * ay, 0.0));
       }
       if (n > cp.max_ions) atomicOr(status, kStatusIonOverflow);  // LIP.cpp:1043-1048
-      s_n[jj] = n;
-      s_ax[jj] = ax;
-      s_ay[jj] = ay;
       CloudRec r;
       r.coeff = 2.0 * (spec[2 * j] * n) * kElecClassicRadius / cp.r_gamma;
       r.rms_x = rx;
       r.rms_y = ry;
+      r.aver_x = ax;
+      r.aver_y = ay;
       r.count = n;
-      rec[(size_t)j * P + p] = r;  // centroid filled below
+      rec[(size_t)j * P + p] = r;
       // the field constants of this Gaussian, once for all the kicks that read it
       rec_prep[(size_t)j * P + p] = field_prep(rx, ry);
       if (j == M - 1) {
@@ -400,11 +550,40 @@ __global__ void __launch_bounds__(kFinishThreads) k_ion_records(ChainParams cp, 
         carry[3] = ry;
       }
     }
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&w.done[2 * p], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) {
+    w.done[2 * p] = 0;
+    s_carry[0] = ja == 0 ? st0.aver_x : carry[0];
+    s_carry[1] = ja == 0 ? st0.aver_y : carry[1];
+  }
+  for (int j0 = ja; j0 < jb; j0 += kRecChunk) {
+    const int nj = min(kRecChunk, jb - j0);
+    bool one = false;
     __syncthreads();
-    if (tid == 0) {  // the stale-centroid carry is sequential
+    for (int jj = tid; jj < nj; jj += kRecThreads) {
+      const CloudRec* r = rec + (size_t)(j0 + jj) * P + p;
+      s_one[jj] = __ldcg(&r->count) == 1.0;
+      s_ax[jj] = __ldcg(&r->aver_x);
+      s_ay[jj] = __ldcg(&r->aver_y);
+      one = one || s_one[jj];
+    }
+    if (!__syncthreads_or(one)) {  // no one-ion step: nothing to carry in
+      if (tid == 0) {
+        s_carry[0] = s_ax[nj - 1];
+        s_carry[1] = s_ay[nj - 1];
+      }
+      continue;
+    }
+    if (tid == 0) {
       double cx = s_carry[0], cy = s_carry[1];
       for (int jj = 0; jj < nj; ++jj) {
-        if (s_n[jj] == 1) {
+        if (s_one[jj]) {
           s_ax[jj] = cx;
           s_ay[jj] = cy;
         } else {
@@ -416,13 +595,13 @@ __global__ void __launch_bounds__(kFinishThreads) k_ion_records(ChainParams cp, 
       s_carry[1] = cy;
     }
     __syncthreads();
-    for (int jj = tid; jj < nj; jj += kFinishThreads) {
+    for (int jj = tid; jj < nj; jj += kRecThreads) {
+      if (!s_one[jj]) continue;
       CloudRec* r = rec + (size_t)(j0 + jj) * P + p;
       r->aver_x = s_ax[jj];
       r->aver_y = s_ay[jj];
     }
   }
-  __syncthreads();
   if (tid == 0) {
     carry[0] = s_carry[0];
     carry[1] = s_carry[1];
@@ -431,32 +610,41 @@ __global__ void __launch_bounds__(kFinishThreads) k_ion_records(ChainParams cp, 
 
 // After the last walk segment and the last records: the surviving ions in
 // trajectory order (birth order, as the reference's erase keeps it) into
-// cloud buffer 0, and the cloud state.  One CTA per species.
-__global__ void __launch_bounds__(kFinishThreads) k_ion_compact(ChainParams cp, IonWalk w,
+// cloud buffer 0, and the cloud state.  One CTA per kCompactThreads
+// trajectories and species: it counts the survivors before its own by reading
+// their flags (16 at a time) and keeps its own in order; the CTA that finishes
+// last writes the state, when no other reads it any more.
+// As one CTA it took 100 us for 20,000 ions, one round of barriers per 1024.
+__global__ void __launch_bounds__(kCompactThreads) k_ion_compact(ChainParams cp, IonWalk w,
                                                               CloudDev* clouds, CloudState* cst,
                                                               int* status) {
-  __shared__ int s_wsum[kFinishThreads / 32];
-  __shared__ int s_base;
-  const int p = blockIdx.x, tid = threadIdx.x;
+  __shared__ int s_wsum[kCompactThreads / 32];
+  __shared__ int s_before;
+  const int p = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int M = cp.n_bunches, NM = cp.macro_per_ip;
   const CloudState st0 = cst[p];
   const int64_t T = (int64_t)st0.n + (int64_t)M * NM;
-  const double* spec = w.spec + 2 * (size_t)p * M;
-  const double* carry = w.carry + 4 * (size_t)p;
-  CloudDev cd = clouds[p];
-  const double* traj = w.traj + (size_t)p * 6 * w.tcap;
-  const uint8_t* al = w.alive + (size_t)p * w.tcap;
-  if (tid == 0) s_base = 0;
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int64_t t0 = 0; t0 < T; t0 += kFinishThreads) {
+  const int64_t t0 = (int64_t)blockIdx.x * kCompactThreads;
+  const CloudDev cd = clouds[p];
+  if (t0 < T) {
+    const double* traj = w.traj + (size_t)p * 6 * w.tcap;
+    const uint8_t* al = w.alive + (size_t)p * w.tcap;
+    if (tid == 0) s_before = 0;
+    __syncthreads();
+    int before = 0;  // flags are 0 or 1: a word's set bits are its survivors
+    for (int64_t i = tid; i < t0 / 16; i += kCompactThreads) {
+      const uint4 v = reinterpret_cast<const uint4*>(al)[i];
+      before += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
+    before = __reduce_add_sync(FULL_MASK, before);
+    if (lane == 0 && before) atomicAdd(&s_before, before);
     const int64_t t = t0 + tid;
     const bool keep = t < T && al[t];
     const unsigned bal = __ballot_sync(FULL_MASK, keep);
     if (lane == 0) s_wsum[warp] = __popc(bal);
     __syncthreads();
-    int pre = s_base, tot = 0;
-    for (int u = 0; u < kFinishThreads / 32; ++u) {
+    int pre = s_before, tot = s_before;
+    for (int u = 0; u < kCompactThreads / 32; ++u) {
       pre += u < warp ? s_wsum[u] : 0;
       tot += s_wsum[u];
     }
@@ -469,22 +657,27 @@ __global__ void __launch_bounds__(kFinishThreads) k_ion_compact(ChainParams cp, 
       cd.fx[pre] = traj[4 * w.tcap + t];
       cd.fy[pre] = traj[5 * w.tcap + t];
     }
-    __syncthreads();
-    if (tid == 0) s_base += tot;
-    __syncthreads();
+    if (tid == 0 && t0 + kCompactThreads >= T) w.carry[4 * (size_t)cp.n_species + p] = tot;
   }
-  if (tid == 0) {
-    CloudState st;
-    st.n = s_base < cd.cap ? s_base : cd.cap;
-    if (s_base > cd.cap) atomicOr(status, kStatusIonOverflow);
-    st.cur = 0;
-    st.aver_x = carry[0];
-    st.aver_y = carry[1];
-    st.rms_x = carry[2];
-    st.rms_y = carry[3];
-    st.macro_charge = spec[2 * (M - 1)];
-    cst[p] = st;
-  }
+  __syncthreads();
+  if (tid != 0) return;
+  __threadfence();
+  if (atomicAdd(&w.done[2 * p + 1], 1u) != gridDim.x - 1) return;
+  __threadfence();
+  w.done[2 * p + 1] = 0;
+  const double* spec = w.spec + 2 * (size_t)p * M;
+  const double* carry = w.carry + 4 * (size_t)p;
+  const int total = (int)__ldcg(&w.carry[4 * (size_t)cp.n_species + p]);
+  CloudState st;
+  st.n = total < cd.cap ? total : cd.cap;
+  if (total > cd.cap) atomicOr(status, kStatusIonOverflow);
+  st.cur = 0;
+  st.aver_x = carry[0];
+  st.aver_y = carry[1];
+  st.rms_x = carry[2];
+  st.rms_y = carry[3];
+  st.macro_charge = spec[2 * (M - 1)];
+  cst[p] = st;
 }
 
 static ChainSection chain_section(const Handle& h, int k) {
@@ -510,8 +703,8 @@ cudaError_t launch_ion_prep(Handle& h, int k) {
 // driver keeps per CTA, the whole 228 KB of the SM, so that no kick or map
 // CTA is scheduled beside the walk (their warps would take issue slots and
 // FP64 pipe cycles from the walk's latency-bound chain).  Set per device by
-// prepare_ion_walk; index 0..3 = 8, 16, 32, 64 ions per CTA.
-static int g_walk_reserve_dyn[4] = {0, 0, 0, 0};
+// prepare_ion_walk; index 0..2 = 16, 32, 64 ions per CTA.
+static int g_walk_reserve_dyn[3] = {0, 0, 0};
 
 template <int IONS>
 static cudaError_t prepare_walk_shape(int slot) {
@@ -525,39 +718,41 @@ static cudaError_t prepare_walk_shape(int slot) {
 }
 
 cudaError_t prepare_ion_walk() {
-  cudaError_t e = prepare_walk_shape<8>(0);
-  if (e == cudaSuccess) e = prepare_walk_shape<16>(1);
-  if (e == cudaSuccess) e = prepare_walk_shape<32>(2);
-  if (e == cudaSuccess) e = prepare_walk_shape<64>(3);
+  cudaError_t e = prepare_walk_shape<16>(0);
+  if (e == cudaSuccess) e = prepare_walk_shape<32>(1);
+  if (e == cudaSuccess) e = prepare_walk_shape<64>(2);
   return e;
 }
 
 cudaError_t launch_ion_walk(Handle& h, int k, int ja, int jb, cudaStream_t s) {
-  const int ions = h.walk_ions;
+  const int ions = std::max(16, h.walk_ions);  // 8 runs as 16: one warp
   const dim3 grid(ion_walk_grid(h.d.iw.tcap, ions), h.P);
   const CloudDev* cl = h.d.clouds + (size_t)k * h.P;
   const CloudState* cs = h.d.cloud_state + (size_t)k * h.P;
-  const int slot = ions == 8 ? 0 : ions == 16 ? 1 : ions == 32 ? 2 : 3;
+  const int slot = ions == 16 ? 0 : ions == 32 ? 1 : 2;
   const size_t dyn = h.walk_reserve ? (size_t)g_walk_reserve_dyn[slot] : 0;
-  if (ions == 8) k_ion_walk<8><<<grid, 32, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
-  else if (ions == 16) k_ion_walk<16><<<grid, 64, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
-  else if (ions == 32) k_ion_walk<32><<<grid, 128, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
-  else k_ion_walk<64><<<grid, 256, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
+  if (ions == 16) k_ion_walk<16><<<grid, 32, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
+  else if (ions == 32) k_ion_walk<32><<<grid, 64, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
+  else k_ion_walk<64><<<grid, 128, dyn, s>>>(h.chain, h.d.iw, cl, cs, ja, jb);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ion_records(Handle& h, int k, int ja, int jb, cudaStream_t s) {
-  k_ion_records<<<h.P, kFinishThreads, 0, s>>>(h.chain, h.d.iw, h.d.cloud_state + (size_t)k * h.P,
-                                               h.d.rec + (size_t)k * h.M * h.P,
-                                               h.d.rec_prep + (size_t)k * h.M * h.P, h.d.status,
-                                               ion_walk_grid(h.d.iw.tcap, h.walk_ions),
-                                               h.walk_ions, ja, jb);
+  constexpr int kWarps = kRecThreads / 32;
+  const int ions = std::max(16, h.walk_ions);
+  const dim3 grid((jb - ja + kWarps - 1) / kWarps, h.P);
+  if (jb <= ja) return cudaSuccess;
+  k_ion_records<<<grid, kRecThreads, 0, s>>>(h.chain, h.d.iw, h.d.cloud_state + (size_t)k * h.P,
+                                             h.d.rec + (size_t)k * h.M * h.P,
+                                             h.d.rec_prep + (size_t)k * h.M * h.P, h.d.status,
+                                             ion_walk_grid(h.d.iw.tcap, ions), ions, ja, jb);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ion_compact(Handle& h, int k, cudaStream_t s) {
-  k_ion_compact<<<h.P, kFinishThreads, 0, s>>>(h.chain, h.d.iw, h.d.clouds + (size_t)k * h.P,
-                                               h.d.cloud_state + (size_t)k * h.P, h.d.status);
+  const dim3 grid((unsigned)((h.d.iw.tcap + kCompactThreads - 1) / kCompactThreads), h.P);
+  k_ion_compact<<<grid, kCompactThreads, 0, s>>>(h.chain, h.d.iw, h.d.clouds + (size_t)k * h.P,
+                                                 h.d.cloud_state + (size_t)k * h.P, h.d.status);
   return cudaGetLastError();
 }
 
@@ -574,44 +769,19 @@ cudaError_t upload_weideman_table_ion() {
   return e != cudaSuccess ? e : prepare_ion_walk();
 }
 
-// Latency floor of the walk: one quad of lanes advances one ion through a
-// dependent chain of bunch passages with exactly the walk's step arithmetic
-// (the field arguments, w(z1) and w(z2) each split over two lanes, the
-// Gaussian factor beside them, the shuffles, the field and the velocity and
-// position update) and none of its window stores, barriers and sums.  With
-// coefficient 1e-13 the ion oscillates in the core of the Gaussian (period of
-// ~300 passages), where the walk spends its time (Weideman region of w(z)).
+// Latency floor of the walk: one warp advances 16 ions through a dependent
+// chain of bunch passages with exactly the walk's step (walk_step) and none of
+// its window stores, barriers and sums.  With coefficient 1e-13 the ion
+// oscillates in the core of the Gaussian (period of ~300 passages), where the
+// walk spends its time (Weideman region of w(z)).
 __global__ void k_field_chain(double* out, int n) {
-  __shared__ double s_a[kWeidemanN];
-  const int lane = threadIdx.x & 31, sub = lane & 3;
-  for (int i = lane; i < kWeidemanN; i += 32) s_a[i] = weideman_table().a[i];
-  __syncwarp();
-  if (threadIdx.x >= 32) return;
-  const bool second = (sub >> 1) != 0, upper = (sub & 1) != 0;
-  const double L = weideman_table().L;
-  const FieldPrep fp = field_prep(1.4e-5, 6.3e-6);
-  double x = 3.0e-6, y = 2.0e-6, vx = 0.0, vy = 0.0;
-  const double c = 1.0e-13;
-  for (int i = 0; i < n; ++i) {
-    double z1r, z1i, z2r, z2i;
-    field_zargs(fp, x, y, &z1r, &z1i, &z2r, &z2i);
-    const double zr = second ? z2r : z1r, zi = second ? z2i : z1i;
-    const double g = second ? field_gauss(fp, x, y) : 0.0;
-    cplx rden;
-    const cplx ph = weideman_half(zr, zi, L, s_a, upper, &rden);
-    const cplx po = {__shfl_xor_sync(FULL_MASK, ph.re, 1), __shfl_xor_sync(FULL_MASK, ph.im, 1)};
-    const cplx lo = upper ? po : ph, hi = upper ? ph : po;
-    const cplx wv = weideman_from_sum({lo.re + hi.re, lo.im + hi.im}, rden);
-    const cplx wo = {__shfl_xor_sync(FULL_MASK, wv.re, 2), __shfl_xor_sync(FULL_MASK, wv.im, 2)};
-    const double go = __shfl_xor_sync(FULL_MASK, g, 2);
-    double fx, fy;
-    field_finish_g(fp, x, y, second ? wo : wv, second ? wv : wo, second ? g : go, &fx, &fy);
-    vx += c * fx;
-    vy += c * fy;
-    x += vx;
-    y += vy;
-  }
-  if (lane == 0) out[0] = x + y;
+  const double bunch[3] = {0.0, 0.0, 1.0};
+  const int sub = threadIdx.x & 1;
+  const WalkStep st = walk_step_of(field_prep(1.4e-5, 6.3e-6), bunch, 1.0e-13);
+  const StepRegs<true> r = step_regs<true>(st, sub);
+  IonState q = {3.0e-6, 2.0e-6, 0.0, 0.0, 0.0, 0.0, true};
+  for (int i = 0; i < n; ++i) walk_step<true>(r, sub, true, 1.0, 1.0, q);
+  if (threadIdx.x == 0) out[0] = q.a + q.b;
 }
 
 cudaError_t measure_field_chain_latency(double* us_per_step) {

@@ -228,7 +228,7 @@ __global__ void k_sur_data(uint64_t seed, int64_t n, float* __restrict__ xin,
   const double r = (q.v[3] & 1u) ? exp(log(kSurRmin) * (1.0 - ur))
                                  : kSurRmin + (1.0 - kSurRmin) * ur;
   double fx, fy;
-  gaussian_field<false>(kSurRange * a, kSurRange * b * r, 1.0, r, &fx, &fy);
+  gaussian_field(kSurRange * a, kSurRange * b * r, 1.0, r, &fx, &fy);
   xin[3 * i] = (float)a;
   xin[3 * i + 1] = (float)b;
   xin[3 * i + 2] = (float)r;
