@@ -101,7 +101,7 @@ int launch_ok(Handle& h, cudaError_t e, const char* what) {
 
 void free_beam(Handle& h) {
   DeviceBufs& d = h.d;
-  dfree(d.c); dfree(d.surv); dfree(d.tile_bunch); dfree(d.chunk_bunch); dfree(d.chunk_loc);
+  dfree(d.c); dfree(d.surv); dfree(d.tile_bunch); dfree(d.chunk_loc);
   dfree(d.bunch);
   dfree(d.wpartials);
   dfree(d.counters); dfree(d.mom); dfree(d.loss_count); dfree(d.scratch);
@@ -135,7 +135,7 @@ void free_beam(Handle& h) {
   dfree(w.births); dfree(w.prep); dfree(w.bunch); dfree(w.spec); dfree(w.bound); dfree(w.part);
   dfree(w.traj); dfree(w.alive); dfree(w.carry); dfree(w.done);
   w = IonWalk();
-  d.c = nullptr; d.surv = nullptr; d.tile_bunch = nullptr; d.chunk_bunch = nullptr;
+  d.c = nullptr; d.surv = nullptr; d.tile_bunch = nullptr;
   d.chunk_loc = nullptr;
   d.bunch = nullptr; d.wpartials = nullptr;
   d.counters = nullptr; d.mom = nullptr; d.loss_count = nullptr; d.scratch = nullptr;
@@ -189,7 +189,11 @@ SectionDev make_section_dev(const cg_section& s, const cg_ring& r) {
   std::memcpy(d.b1h1, s.map_b1h1, sizeof d.b1h1);
   std::memcpy(d.h1b1, s.map_h1b1, sizeof d.h1b1);
   std::memcpy(d.h2b2, s.map_h2b2, sizeof d.h2b2);
-  d.twiss_form = fits_twiss_form(d.b1h1) && fits_twiss_form(d.h1b1) && fits_twiss_form(d.h2b2);
+  auto fits = [&](unsigned long long form) {
+    return fits_form(d.b1h1, form) && fits_form(d.h1b1, form) && fits_form(d.h2b2, form);
+  };
+  const bool flat = s.eta_x == 0 && s.etap_x == 0 && s.eta_y == 0 && s.etap_y == 0;
+  d.twiss_form = flat && fits(kPlainForm) ? 2 : fits(kTwissForm) ? 1 : 0;
   return d;
 }
 
@@ -198,7 +202,11 @@ RingDev make_ring_dev(const cg_config& c, const cg_section& s0) {
   RingDev d;
   std::memset(&d, 0, sizeof d);
   d.chrom[0] = r.chrom[0]; d.chrom[1] = r.chrom[1];
-  for (int i = 0; i < 5; ++i) { d.adtx[i] = r.adtx[i]; d.adty[i] = r.adty[i]; }
+  for (int i = 0; i < 5; ++i) {
+    d.adtx[i] = r.adtx[i];
+    d.adty[i] = r.adty[i];
+    if (i > 1 && (r.adtx[i] != 0 || r.adty[i] != 0)) d.adt2 = 1;
+  }
   d.circ_ring = r.circ_ring;
   for (int i = 0; i < 3; ++i) d.alphac[i] = r.alphac[i];
   d.energy = r.electron_energy;
@@ -526,17 +534,22 @@ int cg_create(const cg_config* cfg, int device, cg_handle** out) {
     cg_destroy(H);
     return code;
   };
-  if ((e = cudaStreamCreateWithFlags(&h.side, cudaStreamNonBlocking)) != cudaSuccess)
+  // the ion walk, the turn's critical path, runs on the handle's stream: its
+  // few CTAs go before the waiting CTAs of the particle passes beside it, which
+  // fill every SM's registers and hold them for tens of microseconds
+  int low = 0, high = 0;
+  if ((e = cudaDeviceGetStreamPriorityRange(&low, &high)) != cudaSuccess)
     return bail(CG_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = cudaStreamCreateWithFlags(&h.side2, cudaStreamNonBlocking)) != cudaSuccess)
-    return bail(CG_ERR_CUDA, cudaGetErrorString(e));
+  for (cudaStream_t* st : {&h.side, &h.side2})
+    if ((e = cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, low)) != cudaSuccess)
+      return bail(CG_ERR_CUDA, cudaGetErrorString(e));
   h.pipe_ev.assign(kMaxPipeGroups + 1, nullptr);
   h.kick_ev.assign(kMaxPipeGroups + 1, nullptr);
   for (auto* evs : {&h.pipe_ev, &h.kick_ev})
     for (auto& ev : *evs)
       if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
         return bail(CG_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking)) != cudaSuccess)
+  if ((e = cudaStreamCreateWithPriority(&h.stream, cudaStreamNonBlocking, high)) != cudaSuccess)
     return bail(CG_ERR_CUDA, cudaGetErrorString(e));
   if ((e = dalloc(&h.sec_dev, h.K)) != cudaSuccess) return bail(CG_ERR_OOM, "sections");
   cudaMemcpy(h.sec_dev, h.sec_dev_host.data(), sizeof(SectionDev) * h.K, cudaMemcpyHostToDevice);
@@ -768,10 +781,32 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   for (int j = 0; j < M - 1; ++j) h.gap[j] = harm[j + 1] - harm[j];
   h.gap[M - 1] = Hh - harm[M - 1];
   std::vector<BunchDev> bd(M);
-  std::vector<int> tb, cb;
+  std::vector<int> tb;
   std::vector<int4> cl;
   h.tile_off.assign(M + 1, 0);
   int tiles = 0, chunks = 0;
+  // Tiles per chunk, from the whole train (the same on every rank of a
+  // sharded run): long chunks spread the reduction at a chunk's end over more
+  // particles, but the 592 CTAs that run at once (four a SM) want some six
+  // chunks each to even out; and at most 256 chunks a bunch.
+  int64_t all_tiles = 0, big = 0;
+  for (int j = 0; j < M; ++j) {
+    const int64_t nt = (n_macro[j] + kTile - 1) / kTile;
+    all_tiles += nt;
+    big = std::max(big, nt);
+  }
+  const int64_t share = 592 * 6;
+  const int ct = (int)std::max<int64_t>(
+      (big + 255) / 256,
+      std::min<int64_t>(kMaxChunkTiles, std::max<int64_t>(1, (all_tiles + share / 2) / share)));
+  h.max_chunks = (int)((big + ct - 1) / ct);
+  // Walk segments: a segment's records, its pass and their launches cost some
+  // 15 us beside the 25 us that the pass of 3000 tiles takes, so shorter
+  // segments lose more than the overlap gives (80 x 2e4 particles: 2.81 ms a
+  // turn in 2 segments, 3.00 in 1, 3.28 in 4; 1.74e7: 46.5 ms in 8, 47.5 in 4,
+  // 58.7 in 1).
+  if (!h.pipe_given)
+    h.pipe_groups = (int)std::min<int64_t>(8, std::max<int64_t>(1, (all_tiles + 1500) / 3000));
   // bunch sharding: this rank tracks the particles of bunches [j0, j1)
   const ShardLayout lay = shard_layout(n_macro, M, h.sh_world);
   h.sh_j0 = lay.j0[h.sh_rank];
@@ -780,7 +815,7 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   for (int j = 0; j < M; ++j) {
     const bool local = j >= h.sh_j0 && j < h.sh_j1;
     int nt = local ? (n_macro[j] + kTile - 1) / kTile : 0;
-    int nc = (nt + kMomChunkTiles - 1) / kMomChunkTiles;
+    int nc = (nt + ct - 1) / ct;
     bd[j].n = local ? n_macro[j] : 0;
     bd[j].tile_off = tiles;
     bd[j].n_tiles = nt;
@@ -792,10 +827,8 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
     bd[j].q_macro = ne[j] / n_macro[j];
     h.tile_off[j] = tiles;
     for (int t = 0; t < nt; ++t) tb.push_back(j);
-    for (int t = 0; t < nc; ++t) {
-      cb.push_back(j);
-      cl.push_back(make_int4(j, tiles + t * kMomChunkTiles, t, bd[j].n - t * kMomChunkTiles * kTile));
-    }
+    for (int t = 0; t < nc; ++t)
+      cl.push_back(make_int4(j, tiles + t * ct, std::min(ct, nt - t * ct), 0));
     tiles += nt;
     chunks += nc;
   }
@@ -808,9 +841,9 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   h.npad = (int64_t)tiles * kTile;
   DeviceBufs& d = h.d;
   if (dalloc(&d.c, 6 * (size_t)h.npad) || dalloc(&d.surv, (size_t)h.npad) ||
-      dalloc(&d.tile_bunch, tiles) || dalloc(&d.chunk_bunch, chunks) ||
+      dalloc(&d.tile_bunch, tiles) ||
       dalloc(&d.chunk_loc, chunks) || dalloc(&d.bunch, M) ||
-      dalloc(&d.wpartials, 8 * (size_t)chunks) ||
+      dalloc(&d.wpartials, (size_t)kMomWarps * chunks) ||
       dalloc(&d.counters, M + 1) || dalloc(&d.mom, M) || dalloc(&d.loss_count, M + 1)) {
     free_beam(h);
     return fail(&h, CG_ERR_OOM, "beam allocation failed");
@@ -823,7 +856,6 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   cudaMemset(d.c, 0, sizeof(double) * 6 * h.npad);
   cudaMemset(d.surv, kPadding, h.npad);
   cudaMemcpy(d.tile_bunch, tb.data(), sizeof(int) * tiles, cudaMemcpyHostToDevice);
-  cudaMemcpy(d.chunk_bunch, cb.data(), sizeof(int) * chunks, cudaMemcpyHostToDevice);
   cudaMemcpy(d.chunk_loc, cl.data(), sizeof(int4) * chunks, cudaMemcpyHostToDevice);
   if (h.nccl_comm) {
     const int W = h.sh_world, ml = std::max(1, h.sh_maxlocal);
@@ -1366,6 +1398,8 @@ static cudaError_t enqueue_turn(Handle& h) {
     int mom = -1;
     if (k + 1 < h.K) mom = sec_mom ? k + 1 : -1;
     else mom = post ? h.K - 1 : -1;
+    // the z range with the turn's last moments, the ones cg_get_moments returns
+    const bool zr = k == (post ? h.K - 1 : h.K - 2);
     if (c.flag_beam_ion && G > 1 && !c.flag_sc) {
       // the walk in G segments of bunches on the main stream; as soon as a
       // segment is walked, its records and kick on `side` and its map (with
@@ -1384,7 +1418,8 @@ static cudaError_t enqueue_turn(Handle& h) {
         const int ta = h.tile_off[ja], tb = h.tile_off[jb];
         const int ca = h.chunk_off[ja], cb = h.chunk_off[jb];
         if (fused) {
-          if ((e = launch_map_turn(h, k, mom, true, ca, cb, h.side))) return e;
+          if ((e = launch_map_pass(h, k, mom, true, zr, ca, cb, h.side))) return e;
+          TRACE(h.side, CG_TRACE_ION_KICK, k, g);  // both in one launch
           TRACE(h.side, CG_TRACE_MAP_PASS, k, g);
           continue;
         }
@@ -1395,7 +1430,7 @@ static cudaError_t enqueue_turn(Handle& h) {
         if ((e = cudaEventRecord(h.kick_ev[g], h.side))) return e;
         if ((e = cudaStreamWaitEvent(h.side2, h.kick_ev[g], 0))) return e;
         if (k == h.K - 1 && (e = launch_phase_adv(h, ja, jb, h.side2))) return e;
-        if ((e = launch_map_turn(h, k, mom, false, ca, cb, h.side2))) return e;
+        if ((e = launch_map_pass(h, k, mom, false, zr, ca, cb, h.side2))) return e;
         TRACE(h.side2, CG_TRACE_MAP_PASS, k, g);
       }
       if ((e = launch_ion_compact(h, k, h.side))) return e;
@@ -1406,6 +1441,7 @@ static cudaError_t enqueue_turn(Handle& h) {
         if ((e = cudaEventRecord(h.kick_ev[kMaxPipeGroups], h.side2))) return e;
         if ((e = cudaStreamWaitEvent(h.stream, h.kick_ev[kMaxPipeGroups], 0))) return e;
       }
+      if (mom >= 0 && (e = launch_mom_merge(h, mom))) return e;
     } else {
       if (c.flag_beam_ion) {
         if ((e = launch_ion_chain(h, k))) return e;
@@ -1417,7 +1453,8 @@ static cudaError_t enqueue_turn(Handle& h) {
       }
       if (c.flag_sc && (e = launch_space_charge(h, k))) return e;
       if (k == h.K - 1 && (e = launch_phase_adv(h, 0, h.M))) return e;
-      if ((e = launch_map_turn(h, k, mom, fused))) return e;
+      if ((e = launch_map_pass(h, k, mom, fused, zr))) return e;
+      if (fused) TRACE(h.stream, CG_TRACE_ION_KICK, k, -1);
       TRACE(h.stream, CG_TRACE_MAP_PASS, k, -1);
     }
     if (mom >= 0) {
@@ -1715,9 +1752,9 @@ int cg_time_stage(cg_handle* H, int stage, int k, int reps, double* ms) {
       case 7:
         e = h.cfg.flag_beam_ion ? launch_map_pass(h, k, k, true) : cudaErrorInvalidValue;
         break;
-      case 8: e = launch_map_async(h, k, k); break;
+      case 8: e = launch_map_pass(h, k, k); break;
       case 9:
-        e = h.cfg.flag_beam_ion ? launch_map_async(h, k, k, true) : cudaErrorInvalidValue;
+        e = h.cfg.flag_beam_ion ? launch_map_pass(h, k, k, true) : cudaErrorInvalidValue;
         break;
       case 6:
         e = h.d.sur_w ? launch_ion_kick_sur(h, k) : cudaErrorInvalidValue;
@@ -2120,8 +2157,8 @@ int cg_autotune(cg_handle* H, int k, int reps, int* choice, double* ms) {
   double map_ms = 0, fused_ms = 0, amap_ms = 0, afused_ms = 0;
   if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, false); }, &map_ms);
   if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, true); }, &fused_ms);
-  if (e == cudaSuccess) e = time_it([&]() { return launch_map_async(h, k, mom, false); }, &amap_ms);
-  if (e == cudaSuccess) e = time_it([&]() { return launch_map_async(h, k, mom, true); }, &afused_ms);
+  if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, false); }, &amap_ms);
+  if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, true); }, &afused_ms);
   if (ms) {
     ms[nv] = map_ms;
     ms[nv + 1] = fused_ms;
@@ -2235,6 +2272,7 @@ int cg_set_pipeline(cg_handle* H, int groups, int walk_ions, int ramp) {
     h.turn_graph = nullptr;
   }
   h.pipe_groups = groups;
+  h.pipe_given = true;
   h.walk_ions = walk_ions;
   h.pipe_ramp = rp;
   return CG_OK;

@@ -11,12 +11,12 @@ namespace cg {
 
 constexpr int kTile = 256;            // particles per tile == threads per CTA
 
-constexpr int kMomChunkTiles = 4;     // tiles per CTA of the moments kernel
+constexpr int kMaxChunkTiles = 8;     // most tiles per CTA of the map pass and the moments
 constexpr int kMaxPipeGroups = 16;    // segments of the pipelined ion pass
 
 struct BunchDev {
   int n, tile_off, n_tiles, harm, gap;
-  int chunk_off, n_chunks;  // moments chunks of kMomChunkTiles tiles
+  int chunk_off, n_chunks;  // chunks of the map pass and the moments
   double ne, q_macro;
 };
 
@@ -101,10 +101,9 @@ struct DeviceBufs {
   double* c = nullptr;          // 6 x npad SoA
   uint8_t* surv = nullptr;      // npad
   int* tile_bunch = nullptr;    // n_tiles
-  int* chunk_bunch = nullptr;   // n_chunks: bunch of each moments chunk
-  int4* chunk_loc = nullptr;    // n_chunks: (bunch, first tile, chunk of the bunch, valid slots)
+  int4* chunk_loc = nullptr;    // n_chunks: (bunch, first tile, tiles, -)
   BunchDev* bunch = nullptr;    // M
-  MomPartial* wpartials = nullptr; // n_chunks x 8: per-warp moment partials
+  MomPartial* wpartials = nullptr; // n_chunks x kMomWarps: moment partials
   unsigned* counters = nullptr;    // M (+ spare)
   BunchMomDev* mom = nullptr;      // M
   int* loss_count = nullptr;       // M
@@ -207,7 +206,7 @@ struct Handle {
   cudaStream_t stream = nullptr;
   int K = 0, M = 0, P = 1;
   int n_tiles = 0;
-  int n_chunks = 0;
+  int n_chunks = 0, max_chunks = 0;  // of all bunches, of the largest bunch
   int64_t npad = 0;
   std::vector<int> n_macro, harm, gap, tile_off, chunk_off;
   // pipelined turn: the ion walk of an IP in `pipe_groups` segments of bunches;
@@ -221,7 +220,8 @@ struct Handle {
   std::vector<int> phase_bunches;  // bunches whose particles' phase advance is tracked
   std::vector<double*> phase_bufs; // their device buffers (6 x n each)
   std::vector<double> bbi_table;  // the copy of cfg.bbi.table
-  int pipe_groups = 4;
+  int pipe_groups = 1;      // by the train's size at cg_set_beam unless
+  bool pipe_given = false;  // cg_set_pipeline chose it
   // trajectories per walk CTA (8, 16, 32, 64; 8 runs as 16, one warp): smaller
   // CTAs spread the walk's FP64 work over more SMs and find room sooner while
   // the kicks and maps of earlier segments fill the GPU
@@ -245,8 +245,8 @@ struct Handle {
   int ion_cap = 0;
   cudaGraphExec_t turn_graph = nullptr;
   int kick_variant = 0;         // autotuned shape of the kick kernel
-  bool fuse_kick = false;       // autotuned: kick inside the map pass
-  bool map_async = false;       // autotuned: the map pass with the next chunk in flight
+  bool fuse_kick = true;        // the kick inside the map pass (cg_set_kick_variant, cg_autotune)
+  bool map_async = false;       // cg_set_map_async (no effect: the map pass always prefetches)
   int sh_rank = 0, sh_world = 1;  // bunch sharding over ranks (cg_set_shard)
   int sh_j0 = 0, sh_j1 = 0, sh_maxlocal = 0;
   void* nccl_comm = nullptr;

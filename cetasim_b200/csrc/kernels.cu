@@ -150,204 +150,126 @@ __device__ __forceinline__ void store6(double* __restrict__ c, int64_t npad, int
 
 // ---------------------------------------------------------------------------
 // Moments (MPBunch::GetMPBunchRMS, MPBunch.cpp:342-498): a CTA takes a chunk
-// of up to kMomChunkTiles tiles of one bunch, holds its particles in
-// registers and makes a two-pass partial (mean, then centred co-moments) over
-// the alive ones; the last CTA of each bunch merges the bunch's partials in
-// chunk order (Chan et al. pairwise update: deterministic, and as accurate as
-// the reference's two passes over the whole bunch).
+// (consecutive tiles of one bunch) and each thread adds up its particles of
+// the chunk as deviations from its warp's pivot, the mean of the first 32 that
+// hold an alive particle, so that one pass over the particles is as accurate
+// as the reference's two (the pivot lies within a fraction of sigma of the
+// mean).  Each warp stores its sums as a partial (count, means, centred
+// co-moments) and is done; k_mom_merge, one CTA per bunch, merges a bunch's
+// partials in a fixed order: deterministic.  (A merge by the last CTA of each
+// bunch costs every CTA a fence and an atomic: some 5 us at the end of each.)
+// The map pass and k_moments share these functions: the same moments bit for
+// bit.
 
-// v[u][d]: coordinate d of this thread's particle in tile u of the chunk.
-// Two block reductions with fixed trees: (sums, count, z min, z max), whose
-// totals every thread needs for the centred pass, then the centred
-// co-moments, whose totals only thread 0 needs.  Three barriers; the warp
-// stage of the sums uses the transposed butterfly (warp_sum8_t).
-// The reductions of a chunk partial from this thread's sums over its alive
-// particles (s: six coordinates then the count; mn, mx: the z range), with
-// get(u, d) = coordinate d of the thread's particle in tile u, read again for
-// the centred pass (only where alive[u]).
-template <class Get>
-__device__ __forceinline__ void chunk_moment_reduce(double (&s)[7], double mn, double mx,
-                                                    const bool (&alive)[kMomChunkTiles], Get get,
-                                                    double* smem, MomPartial* out) {
-  constexpr int NW = kTile / 32;
-  double* sa = smem;            // 9 x 32: sums (7), min z, max z
-  double* sb = smem + 9 * 32;   // 9 x 32: centred co-moments
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  {
-    const double s8[8] = {s[0], s[1], s[2], s[3], s[4], s[5], s[6], 0.0};
-    const double t = warp_sum8_t(s8);
-    const int idx = warp_sum8_index(lane);
-    if ((lane & 3) == 0 && idx < 7) sa[idx * 32 + warp] = t;
+struct MomSums {
+  double s[6], q[9], zmin, zmax;
+  int n;
+};
+__device__ __forceinline__ void mom_sums_clear(MomSums& m) {
+#pragma unroll
+  for (int d = 0; d < 6; ++d) m.s[d] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m.q[k] = 0.0;
+  m.zmin = INFINITY;
+  m.zmax = -INFINITY;
+  m.n = 0;
+}
+// ZR: the z range too
+template <bool ZR>
+__device__ __forceinline__ void mom_sums_add(MomSums& m, const double (&v)[6], const double* pivot) {
+  double d[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    d[k] = v[k] - pivot[k];
+    m.s[k] += d[k];
+    m.q[k] = fma(d[k], d[k], m.q[k]);
   }
+  m.q[6] = fma(d[0], d[1], m.q[6]);
+  m.q[7] = fma(d[2], d[3], m.q[7]);
+  m.q[8] = fma(d[4], d[5], m.q[8]);
+  if (ZR) {
+    m.zmin = fmin(m.zmin, v[4]);
+    m.zmax = fmax(m.zmax, v[4]);
+  }
+  m.n += 1;
+}
+
+// Threads of a CTA of the map pass and the moments, and its steps per tile.
+constexpr int kPassThreads = 128;
+constexpr int kPassSteps = kTile / kPassThreads;
+static_assert(kMomWarps * 32 == kPassThreads, "one partial per warp");
+
+// Sets the warp's pivot if some lane's particle is alive; the warp calls it
+// per tile until it returns true.
+__device__ __forceinline__ bool mom_pivot(double* pivot, bool alive, const double (&v)[6]) {
+  const unsigned bal = __ballot_sync(FULL_MASK, alive);
+  if (!bal) return false;
+  const int lane = threadIdx.x & 31, idx = warp_sum8_index(lane);
+  double a[8];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) a[d] = alive ? v[d] : 0.0;
+  a[6] = a[7] = 0.0;
+  const double t = warp_sum8_t(a);
+  if ((lane & 3) == 0 && idx < 6) pivot[idx] = t / __popc(bal);
+  __syncwarp();
+  return true;
+}
+
+// The warp's sums as a partial.
+__device__ __forceinline__ void mom_partial(const MomSums& m, bool have, const double* pivot,
+                                            MomPartial* out) {
+  const int lane = threadIdx.x & 31;
+  // lane 4 i gets total i: s 0..5, n, q8, and q 0..7
+  const double a[8] = {m.s[0], m.s[1], m.s[2], m.s[3], m.s[4], m.s[5], (double)m.n, m.q[8]};
+  const double b[8] = {m.q[0], m.q[1], m.q[2], m.q[3], m.q[4], m.q[5], m.q[6], m.q[7]};
+  const double t = warp_sum8_t(a), q = warp_sum8_t(b);
+  double mn = m.zmin, mx = m.zmax;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     mn = fmin(mn, __shfl_xor_sync(FULL_MASK, mn, o));
     mx = fmax(mx, __shfl_xor_sync(FULL_MASK, mx, o));
   }
-  if (lane == 0) {
-    sa[7 * 32 + warp] = mn;
-    sa[8 * 32 + warp] = mx;
+  const double n = __shfl_sync(FULL_MASK, t, 24);
+  const double inv = n > 0 ? 1.0 / n : 0.0;
+  // co-moment k of lane 4 k: its pair of coordinates
+  const int k = lane >> 2;
+  const int i = k < 6 ? k : 2 * (k - 6), j = k < 6 ? k : 2 * (k - 6) + 1;
+  const double si = __shfl_sync(FULL_MASK, t, 4 * i), sj = __shfl_sync(FULL_MASK, t, 4 * j);
+  const double s4 = __shfl_sync(FULL_MASK, t, 16), s5 = __shfl_sync(FULL_MASK, t, 20);
+  if ((lane & 3) == 0) {
+    out->c[k] = q - si * (sj * inv);
+    if (k < 6) out->mean[k] = have ? pivot[k] + t * inv : 0.0;
+    else if (k == 6) out->n = n;
+    else out->c[8] = t - s4 * (s5 * inv);
   }
-  __syncthreads();
-  // every thread combines the NW warp totals in the same order
+  if (lane == 1) out->zmin = mn;
+  if (lane == 2) out->zmax = mx;
+}
+
+// A CTA of NT threads merges n_parts partials in two passes, the mean of all
+// and then the co-moments about it (thread t takes every NT-th in order, then
+// a butterfly per warp and the warps in order); thread 0 gets the total.
+template <int NT, bool GLOBAL = true>
+__device__ __forceinline__ void mom_merge_block(const MomPartial* partials, int n_parts,
+                                                MomPartial* total) {
+  constexpr int NW = NT / 32;
+  __shared__ double s_sum[NW][20];
+  auto get = [](const double* p) { return GLOBAL ? __ldcg(p) : *p; };
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t0 = NW > 1 ? (int)threadIdx.x : lane;
+  // perhaps written by other CTAs of this launch: read through L2
+  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, mn = INFINITY, mx = -INFINITY;
+  for (int t = t0; t < n_parts; t += NT) {
+    const MomPartial* q = partials + t;
+    const double n = get(&q->n);
 #pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    double a = sa[k * 32];
-#pragma unroll
-    for (int w = 1; w < NW; ++w) a += sa[k * 32 + w];
-    s[k] = a;
-  }
-  mn = sa[7 * 32];
-  mx = sa[8 * 32];
-#pragma unroll
-  for (int w = 1; w < NW; ++w) {
-    mn = fmin(mn, sa[7 * 32 + w]);
-    mx = fmax(mx, sa[8 * 32 + w]);
-  }
-  const double n = s[6];
-  double mean[6];
-#pragma unroll
-  for (int d = 0; d < 6; ++d) mean[d] = n > 0 ? s[d] / n : 0.0;
-  double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    double dv[6];
-#pragma unroll
-    for (int d = 0; d < 6; ++d) dv[d] = alive[u] ? get(u, d) - mean[d] : 0.0;
-#pragma unroll
-    for (int d = 0; d < 6; ++d) q[d] = fma(dv[d], dv[d], q[d]);
-    q[6] = fma(dv[0], dv[1], q[6]);
-    q[7] = fma(dv[2], dv[3], q[7]);
-    q[8] = fma(dv[4], dv[5], q[8]);
+    for (int d = 0; d < 6; ++d) s[d] = fma(n, get(&q->mean[d]), s[d]);
+    s[6] += n;
+    mn = fmin(mn, get(&q->zmin));
+    mx = fmax(mx, get(&q->zmax));
   }
   {
-    const double q8[8] = {q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]};
-    const double t = warp_sum8_t(q8);
-    if ((lane & 3) == 0) sb[warp_sum8_index(lane) * 32 + warp] = t;
-    double q9 = q[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) q9 += __shfl_xor_sync(FULL_MASK, q9, o);
-    if (lane == 0) sb[8 * 32 + warp] = q9;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    MomPartial p;
-    p.n = n;
-#pragma unroll
-    for (int d = 0; d < 6; ++d) p.mean[d] = mean[d];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      double a = sb[k * 32];
-#pragma unroll
-      for (int w = 1; w < NW; ++w) a += sb[k * 32 + w];
-      p.c[k] = a;
-    }
-    p.zmin = mn;
-    p.zmax = mx;
-    *out = p;
-  }
-}
-
-// The thread's sums over its alive particles in tile order, as the reductions
-// take them.
-__device__ __forceinline__ void chunk_sums_add(const double (&v)[6], double (&s)[7], double& mn,
-                                               double& mx) {
-#pragma unroll
-  for (int d = 0; d < 6; ++d) s[d] += v[d];
-  s[6] += 1.0;
-  mn = fmin(mn, v[4]);
-  mx = fmax(mx, v[4]);
-}
-
-__device__ void chunk_moment_partial(const double (&v)[kMomChunkTiles][6],
-                                     const bool (&alive)[kMomChunkTiles], double* smem,
-                                     MomPartial* out) {
-  double s[7] = {0, 0, 0, 0, 0, 0, 0};
-  double mn = INFINITY, mx = -INFINITY;
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u)
-    if (alive[u]) chunk_sums_add(v[u], s, mn, mx);
-  chunk_moment_reduce(s, mn, mx, alive, [&](int u, int d) { return v[u][d]; }, smem, out);
-}
-
-__device__ __noinline__ void merge_partials_warp(int b, int part_off, int n_parts,
-                                                 const MomPartial* partials, unsigned* counters,
-                                                 BunchMomDev* mom, double beta_x, double beta_y,
-                                                 const double* z0);
-
-// Called by all threads of every CTA after its partial is stored: the last of
-// the n_parts CTAs of bunch b merges partials [part_off, part_off + n_parts)
-// and finalises.  z0 = z of the bunch's first particle (GetZMinMax seeds the
-// range with it, MPBunch.cpp:1862-1863).
-__device__ __noinline__ void bunch_moment_finish(int b, int part_off, int n_parts, const MomPartial* partials,
-                                    unsigned* counters, BunchMomDev* mom, double beta_x,
-                                    double beta_y, const double* z0) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned prev = atomicAdd(&counters[b], 1u);
-    last = (prev == (unsigned)(n_parts - 1));
-  }
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  __threadfence();
-  merge_partials_warp(b, part_off, n_parts, partials, counters, mom, beta_x, beta_y, z0);
-}
-
-// One full warp: lane l merges partials part_off + l, + l + 32, ... in order,
-// then a fixed shuffle tree (lane i absorbs lane i + o) leaves the bunch total
-// in lane 0, which finalises it and rearms the bunch's counter.
-__device__ __noinline__ void merge_partials_warp(int b, int part_off, int n_parts,
-                                                 const MomPartial* partials, unsigned* counters,
-                                                 BunchMomDev* mom, double beta_x, double beta_y,
-                                                 const double* z0) {
-  constexpr int ND = (int)(sizeof(MomPartial) / sizeof(double));
-  const int lane = threadIdx.x & 31;
-  MomPartial acc;
-  mom_clear(acc);
-  for (int t = lane; t < n_parts; t += 32) {
-    // partials written by other CTAs: read through L2 (no stale L1 lines)
-    const double* src = reinterpret_cast<const double*>(partials + part_off + t);
-    MomPartial q;
-    double* dst = reinterpret_cast<double*>(&q);
-#pragma unroll
-    for (int e = 0; e < ND; ++e) dst[e] = __ldcg(src + e);
-    mom_merge(acc, q);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    MomPartial q;
-    double* dq = reinterpret_cast<double*>(&q);
-    const double* da = reinterpret_cast<const double*>(&acc);
-#pragma unroll
-    for (int e = 0; e < ND; ++e) dq[e] = __shfl_down_sync(FULL_MASK, da[e], o);
-    if (lane < o) mom_merge(acc, q);
-  }
-  if (lane == 0) {
-    BunchMomDev m = mom[b];
-    double tr = m.transmission;
-    mom_finalize(acc, beta_x, beta_y, __ldcg(z0), m);  // may have been mapped by another CTA
-    m.transmission = tr;
-    mom[b] = m;
-    counters[b] = 0;
-  }
-}
-
-// Warp-level moments for the map passes: each warp makes the two-pass partial
-// of its kMomChunkTiles x 32 particles of the chunk with shuffles only (no
-// block barrier), and the last warp of each bunch merges the bunch's warp
-// partials, index 8 x chunk + warp, in index order (deterministic).
-constexpr int kWarpsPerChunk = kTile / 32;
-
-// From this thread's first-pass sums (chunk_sums_add over its alive slots in
-// tile order) and its particles v(u, d): the warp's two-pass partial.
-template <int UNROLL, class A, class V>
-__device__ __forceinline__ void warp_moment_reduce(double (&s)[7], double mn, double mx, A alive,
-                                                   V v, MomPartial* out) {
-  const int lane = threadIdx.x & 31;
-  {  // warp totals to every lane: lanes 4 i hold total i after the transposed butterfly
-    const double s8[8] = {s[0], s[1], s[2], s[3], s[4], s[5], s[6], 0.0};
-    const double t = warp_sum8_t(s8);
+    const double t = warp_sum8_t(s);
 #pragma unroll
     for (int k = 0; k < 7; ++k) s[k] = __shfl_sync(FULL_MASK, t, 4 * k);
   }
@@ -356,104 +278,119 @@ __device__ __forceinline__ void warp_moment_reduce(double (&s)[7], double mn, do
     mn = fmin(mn, __shfl_xor_sync(FULL_MASK, mn, o));
     mx = fmax(mx, __shfl_xor_sync(FULL_MASK, mx, o));
   }
-  const double n = s[6];
-  double mean[6];
+  if (NW > 1) {
+    if (lane == 0) {
 #pragma unroll
-  for (int d = 0; d < 6; ++d) mean[d] = n > 0 ? s[d] / n : 0.0;
-  double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll UNROLL
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    double dv[6];
-    const bool al = alive(u);
+      for (int k = 0; k < 7; ++k) s_sum[warp][k] = s[k];
+      s_sum[warp][7] = mn;
+      s_sum[warp][8] = mx;
+    }
+    __syncthreads();
+    mn = s_sum[0][7];
+    mx = s_sum[0][8];
 #pragma unroll
-    for (int d = 0; d < 6; ++d) dv[d] = al ? v(u, d) - mean[d] : 0.0;
+    for (int k = 0; k < 7; ++k) s[k] = s_sum[0][k];
+    for (int w = 1; w < NW; ++w) {
 #pragma unroll
-    for (int d = 0; d < 6; ++d) q[d] = fma(dv[d], dv[d], q[d]);
-    q[6] = fma(dv[0], dv[1], q[6]);
-    q[7] = fma(dv[2], dv[3], q[7]);
-    q[8] = fma(dv[4], dv[5], q[8]);
+      for (int k = 0; k < 7; ++k) s[k] += s_sum[w][k];
+      mn = fmin(mn, s_sum[w][7]);
+      mx = fmax(mx, s_sum[w][8]);
+    }
   }
-  const double q8[8] = {q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]};
-  const double t = warp_sum8_t(q8);
-  double q9 = q[8];
+  const double inv = s[6] > 0 ? 1.0 / s[6] : 0.0;
+  double c[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int t = t0; t < n_parts; t += NT) {
+    const MomPartial* q = partials + t;
+    const double n = get(&q->n);
+    double d[6];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) q9 += __shfl_xor_sync(FULL_MASK, q9, o);
-  if ((lane & 3) == 0) out->c[warp_sum8_index(lane)] = t;
-  if (lane == 0) {
-    out->n = n;
+    for (int k = 0; k < 6; ++k) d[k] = get(&q->mean[k]) - s[k] * inv;
 #pragma unroll
-    for (int d = 0; d < 6; ++d) out->mean[d] = mean[d];
-    out->c[8] = q9;
-    out->zmin = mn;
-    out->zmax = mx;
+    for (int k = 0; k < 6; ++k) c[k] += fma(n * d[k], d[k], get(&q->c[k]));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) c[6 + k] += fma(n * d[2 * k], d[2 * k + 1], get(&q->c[6 + k]));
   }
-}
-
-__device__ __forceinline__ void warp_moment_partial(const double (&v)[kMomChunkTiles][6],
-                                                    const bool (&alive)[kMomChunkTiles],
-                                                    MomPartial* out) {
-  double s[7] = {0, 0, 0, 0, 0, 0, 0};
-  double mn = INFINITY, mx = -INFINITY;
+  const double c8[8] = {c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7]};
+  const double t = warp_sum8_t(c8);
+  double u = c[8];
 #pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u)
-    if (alive[u]) chunk_sums_add(v[u], s, mn, mx);
-  warp_moment_reduce<kMomChunkTiles>(s, mn, mx, [&](int u) { return alive[u]; },
-                                     [&](int u, int d) { return v[u][d]; }, out);
-}
-
-// After the warp's partial is stored: whether this warp is the last of the
-// bunch's n_parts warps to arrive (it then merges them).
-__device__ __forceinline__ bool warp_moment_arrive(int b, int n_parts, unsigned* counters) {
-  __threadfence();
-  __syncwarp();
-  unsigned prev = 0;
-  if ((threadIdx.x & 31) == 0) prev = atomicAdd(&counters[b], 1u);
-  prev = __shfl_sync(FULL_MASK, prev, 0);
-  return prev == (unsigned)(n_parts - 1);
-}
-
-__device__ __forceinline__ void warp_moment_finish(int b, int part_off, int n_parts,
-                                                   const MomPartial* partials,
-                                                   unsigned* counters, BunchMomDev* mom,
-                                                   double beta_x, double beta_y,
-                                                   const double* z0) {
-  if (!warp_moment_arrive(b, n_parts, counters)) return;
-  __threadfence();
-  merge_partials_warp(b, part_off, n_parts, partials, counters, mom, beta_x, beta_y, z0);
-}
-
-__global__ void __launch_bounds__(kTile, 2) k_moments(const double* __restrict__ c, int64_t npad,
-                                                   const uint8_t* __restrict__ surv,
-                                                   const int* __restrict__ chunk_bunch,
-                                                   const BunchDev* __restrict__ bunch,
-                                                   MomPartial* partials, unsigned* counters,
-                                                   BunchMomDev* mom, double beta_x, double beta_y) {
-  const int b = chunk_bunch[blockIdx.x];
-  const BunchDev B = bunch[b];
-  const int tile0 = B.tile_off + (blockIdx.x - B.chunk_off) * kMomChunkTiles;
-  const int i0 = (tile0 - B.tile_off) * kTile + threadIdx.x;
-  double v[kMomChunkTiles][6];
-  bool alive[kMomChunkTiles];
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    const int64_t g = (int64_t)(tile0 + u) * kTile + threadIdx.x;
-    const bool valid = i0 + u * kTile < B.n;
-    alive[u] = valid && surv[g] == kAlive;
-#pragma unroll
-    for (int d = 0; d < 6; ++d) v[u][d] = valid ? c[d * npad + g] : 0.0;
+  for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(FULL_MASK, u, o);
+  if ((lane & 3) == 0) s_sum[warp][9 + warp_sum8_index(lane)] = t;
+  if (lane == 0) s_sum[warp][17] = u;
+  if (NW > 1) __syncthreads();
+  else __syncwarp();
+  if (threadIdx.x != 0) return;
+  total->n = s[6];
+  for (int k = 0; k < 6; ++k) total->mean[k] = s[k] * inv;
+  for (int k = 0; k < 9; ++k) {
+    double a = s_sum[0][9 + k];
+    for (int w = 1; w < NW; ++w) a += s_sum[w][9 + k];
+    total->c[k] = a;
   }
-  // the same warp partials and merge as the map passes (bitwise the same moments)
+  total->zmin = mn;
+  total->zmax = mx;
+}
+
+// One CTA of NT threads per bunch: its partials merged and finalised.  z0 = z of
+// the bunch's first particle (GetZMinMax seeds the range with it,
+// MPBunch.cpp:1862-1863).
+template <int NT>
+__global__ void __launch_bounds__(NT) k_mom_merge(const double* __restrict__ c, int64_t npad,
+                                                  const BunchDev* __restrict__ bunch,
+                                                  const MomPartial* partials, BunchMomDev* mom,
+                                                  double beta_x, double beta_y) {
+  const int b = blockIdx.x;
+  const BunchDev& B = bunch[b];
+  if (B.n_chunks == 0) return;  // held by another rank
+  MomPartial total;
+  mom_merge_block<NT>(partials + (size_t)B.chunk_off * kMomWarps, B.n_chunks * kMomWarps, &total);
+  if (threadIdx.x != 0) return;
+  BunchMomDev m;
+  mom_finalize(total, beta_x, beta_y, c[4 * npad + (int64_t)B.tile_off * kTile], m);
+  m.transmission = mom[b].transmission;
+  m.pad = 0.0;
+  mom[b] = m;
+}
+
+// A warp per bunch while it has at most eight rounds of partials to read.
+cudaError_t launch_mom_merge(Handle& h, int k, cudaStream_t s) {
+  const SectionDev& sec = h.sec_dev_host[k];
+  auto kern = h.max_chunks * kMomWarps <= 8 * 32 ? k_mom_merge<32> : k_mom_merge<256>;
+  kern<<<h.M, h.max_chunks * kMomWarps <= 8 * 32 ? 32 : 256, 0, s ? s : h.stream>>>(
+      h.d.c, h.npad, h.d.bunch, h.d.wpartials, h.d.mom, sec.beta_x, sec.beta_y);
+  return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(kPassThreads, 6) k_moments(const double* __restrict__ c,
+                                                          int64_t npad,
+                                                          const uint8_t* __restrict__ surv,
+                                                          const int4* __restrict__ chunk_loc,
+                                                          MomPartial* partials) {
+  __shared__ double s_pivot[kMomWarps][6];
+  const int4 l = chunk_loc[blockIdx.x];
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
   const int warp = threadIdx.x >> 5;
-  warp_moment_partial(v, alive, &partials[(size_t)blockIdx.x * kWarpsPerChunk + warp]);
-  warp_moment_finish(b, B.chunk_off * kWarpsPerChunk, B.n_chunks * kWarpsPerChunk, partials,
-                     counters, mom, beta_x, beta_y, c + 4 * npad + (int64_t)B.tile_off * kTile);
+  MomSums m;
+  mom_sums_clear(m);
+  bool have = false;
+#pragma unroll 1
+  for (int u = 0; u < kPassSteps * l.z; ++u, g += kPassThreads) {
+    const bool alive = surv[g] == kAlive;
+    double w[6];
+    load6(c, npad, g, w);
+    if (!have) have = mom_pivot(s_pivot[warp], alive, w);
+    if (alive) mom_sums_add<true>(m, w, s_pivot[warp]);
+  }
+  mom_partial(m, have, s_pivot[warp], &partials[(size_t)blockIdx.x * kMomWarps + warp]);
 }
 
 cudaError_t launch_moments(Handle& h, int k) {
-  const SectionDev& s = h.sec_dev_host[k];
-  k_moments<<<h.n_chunks, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_bunch, h.d.bunch,
-                                                h.d.wpartials, h.d.counters, h.d.mom, s.beta_x,
-                                                s.beta_y);
+  if (h.n_chunks < 1) return cudaSuccess;
+  k_moments<<<h.n_chunks, kPassThreads, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc,
+                                                       h.d.wpartials);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_mom_merge(h, k, h.stream);
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
@@ -490,7 +427,6 @@ template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_ion_kick(double* __restrict__ c, int64_t npad,
                                                       const uint8_t* __restrict__ surv,
                                                       const int* __restrict__ tile_bunch,
-                                                      const BunchDev* __restrict__ bunch,
                                                       const CloudRec* __restrict__ rec,
                                                       const FieldPrep* __restrict__ rec_prep,
                                                       int P, int tile_base) {
@@ -498,84 +434,30 @@ __global__ void __launch_bounds__(NT, MINB) k_ion_kick(double* __restrict__ c, i
   const int tile = tile_base + (int)(blockIdx.x / kSub);
   const int b = tile_bunch[tile];
   const int lane = (blockIdx.x % kSub) * NT + threadIdx.x;
-  const int i = (tile - bunch[b].tile_off) * kTile + lane;
-  const int64_t g = (int64_t)tile * kTile + lane;
-  if (i >= bunch[b].n) return;
+  const int64_t g = (int64_t)tile * kTile + lane;  // padding slots hold kPadding
+  __shared__ KickConst s_kc[CG_MAX_SPECIES];
   // every load of the particle at once (one memory round trip); the field
   // constants of the bunch's records come precomputed with the records
+  rec += (size_t)b * P;
+  rec_prep += (size_t)b * P;
+  if ((int)threadIdx.x < P) s_kc[threadIdx.x] = kick_const(rec[threadIdx.x], rec_prep[threadIdx.x]);
   const uint8_t alive = surv[g];
   const double x = c[0 * npad + g], y = c[2 * npad + g];
   const double px = c[1 * npad + g], py = c[3 * npad + g];
+  __syncthreads();
   if (alive != kAlive) return;
   double dpx, dpy;
-  ion_kick_particle_prep(rec + (size_t)b * P, rec_prep + (size_t)b * P, P, x, y, &dpx, &dpy);
+  ion_kick_particle(s_kc, rec, rec_prep, P, x, y, &dpx, &dpy);
   c[1 * npad + g] = px + dpx;
   c[3 * npad + g] = py + dpy;
 }
 
-// The same kick with IPC items per CTA (an item = the NT particles of one
-// tile that one CTA of k_ion_kick covers): the CTA issues the loads of its
-// next item before it evaluates the field of the current one, so after the
-// first item its warps find their coordinates loaded instead of waiting a
-// memory round trip at the start with nothing else to issue.  The padding
-// slots of a tile hold the survival mark kPadding, so the loads need no
-// bunch lookup first; results are bitwise those of k_ion_kick.
-template <int NT, int MINB, int IPC>
-__global__ void __launch_bounds__(NT, MINB) k_ion_kick_run(double* __restrict__ c, int64_t npad,
-                                                          const uint8_t* __restrict__ surv,
-                                                          const int* __restrict__ tile_bunch,
-                                                          const BunchDev* __restrict__ bunch,
-                                                          const CloudRec* __restrict__ rec,
-                                                          const FieldPrep* __restrict__ rec_prep,
-                                                          int P, int tile_base, int n_items) {
-  constexpr int kSub = kTile / NT;
-  const int it0 = blockIdx.x * IPC, it1 = min(it0 + IPC, n_items);
-  auto index = [&](int it) {
-    return (int64_t)(tile_base + it / kSub) * kTile + (it % kSub) * NT + threadIdx.x;
-  };
-  int64_t g = index(it0);
-  uint8_t alive = surv[g];
-  double x = c[0 * npad + g], y = c[2 * npad + g];
-  double px = c[1 * npad + g], py = c[3 * npad + g];
-  for (int it = it0; it < it1; ++it) {
-    // the next item's loads, in flight while this item's field is evaluated
-    int64_t gn = g;
-    uint8_t an = kPadding;
-    double xn = 0, yn = 0, pxn = 0, pyn = 0;
-    if (it + 1 < it1) {
-      gn = index(it + 1);
-      an = surv[gn];
-      xn = c[0 * npad + gn];
-      yn = c[2 * npad + gn];
-      pxn = c[1 * npad + gn];
-      pyn = c[3 * npad + gn];
-    }
-    if (alive == kAlive) {
-      const int tile = tile_base + it / kSub;
-      const int b = tile_bunch[tile];
-      const int i = (tile - bunch[b].tile_off) * kTile + (it % kSub) * NT + threadIdx.x;
-      if (i < bunch[b].n) {
-        double dpx, dpy;
-        ion_kick_particle_prep(rec + (size_t)b * P, rec_prep + (size_t)b * P, P, x, y, &dpx,
-                               &dpy);
-        c[1 * npad + g] = px + dpx;
-        c[3 * npad + g] = py + dpy;
-      }
-    }
-    g = gn;
-    alive = an;
-    x = xn;
-    y = yn;
-    px = pxn;
-    py = pyn;
-  }
-}
-
-// The kick shapes of autotune choice v: threads per CTA, minimum CTAs per SM
-// (the register budget) and items per CTA (1 = k_ion_kick, one tile or half
-// of one per CTA; more = k_ion_kick_run).
-static const int kKickShapes[][3] = {{256, 3, 1}, {256, 4, 1}, {128, 4, 1}, {128, 6, 1},
-                                     {256, 3, 4}, {128, 6, 4}, {128, 6, 8}, {256, 3, 8}};
+// The kick shapes of autotune choice v: threads per CTA and minimum CTAs per SM
+// (the register budget).  Three kernels; the numbers 1 and 4 to 7 once stood
+// for a 64-register shape, which spills, and for several tiles per CTA, which
+// the occupancy of these makes needless (359 us against 361 for 1.74e7 kicks).
+static const int kKickShapes[][2] = {{256, 3}, {256, 3}, {128, 4}, {128, 6},
+                                     {256, 3}, {128, 6}, {128, 6}, {256, 3}};
 constexpr int kKickVariants = 8;
 
 cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a, int tile_b,
@@ -586,38 +468,19 @@ cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a, int til
   if (!s) s = h.stream;
   const int nt = tile_b - tile_a;
   if (nt <= 0) return cudaSuccess;
-  switch (v) {
-    case 1:
-      k_ion_kick<256, 4><<<nt, 256, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                            rec, rp, h.P, tile_a);
-      break;
-    case 2:
-      k_ion_kick<128, 4><<<2 * nt, 128, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                h.d.bunch, rec, rp, h.P, tile_a);
-      break;
-    case 3:
-      k_ion_kick<128, 6><<<2 * nt, 128, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                h.d.bunch, rec, rp, h.P, tile_a);
-      break;
+  const int* shape = kKickShapes[v];
+  switch (shape[0] == 128 ? shape[1] : 0) {
     case 4:
-      k_ion_kick_run<256, 3, 4><<<(nt + 3) / 4, 256, 0, s>>>(
-          h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, rec, rp, h.P, tile_a, nt);
-      break;
-    case 5:
-      k_ion_kick_run<128, 6, 4><<<(2 * nt + 3) / 4, 128, 0, s>>>(
-          h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, rec, rp, h.P, tile_a, 2 * nt);
+      k_ion_kick<128, 4><<<2 * nt, 128, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
+                                                rec, rp, h.P, tile_a);
       break;
     case 6:
-      k_ion_kick_run<128, 6, 8><<<(2 * nt + 7) / 8, 128, 0, s>>>(
-          h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, rec, rp, h.P, tile_a, 2 * nt);
-      break;
-    case 7:
-      k_ion_kick_run<256, 3, 8><<<(nt + 7) / 8, 256, 0, s>>>(
-          h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, rec, rp, h.P, tile_a, nt);
+      k_ion_kick<128, 6><<<2 * nt, 128, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
+                                                rec, rp, h.P, tile_a);
       break;
     default:
-      k_ion_kick<256, 3><<<nt, 256, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                            rec, rp, h.P, tile_a);
+      k_ion_kick<256, 3><<<nt, 256, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, rec, rp,
+                                            h.P, tile_a);
   }
   return cudaGetLastError();
 }
@@ -628,223 +491,91 @@ void kick_variant_shape(int v, int* threads, int* min_ctas) {
   *min_ctas = kKickShapes[v][1];
 }
 
-// The map of section k with the moments the next stage reads (MOM: at the
-// twiss of section `mom_section`, MPBeam.cpp:1061/1069) in one pass over
-// chunks of kMomChunkTiles tiles of one bunch: all loads of a chunk are issued
-// first, the mapped particles stay in registers for the moments, and each
-// particle is read and written once.  Results equal k_map followed by
-// k_moments.
-template <bool MOM, bool KICK>
-__global__ void __launch_bounds__(kTile, 2) k_map_pass(double* __restrict__ c, int64_t npad,
-                                                    const uint8_t* __restrict__ surv,
+// The particles' pass of one interaction point: the electron-side ion kick
+// (KICK), the map of section k and the moments the next stage reads (MOM: at
+// the twiss of section `mom_section`, MPBeam.cpp:1061/1069), each particle
+// read and written once.  A CTA takes one chunk, tile by tile, and issues the
+// next tile's loads before it works on the current one.  Results equal
+// k_ion_kick, k_map and k_moments in turn, bit for bit.
+// Bound by issue: 795 instructions a particle of which 327 on the FP64 pipe (48 %
+// busy) at 16 warps an SM, the accumulators of the moments beside the two
+// series leaving no registers for more.  1.74e7 particles: 623 us (kick 359 and
+// map with moments 403 apart; 471 and 441 before); floors 316 us of FP64 and
+// 260 us of HBM.  Two particles at a time spill (810 us); the next tile's
+// loads in registers or by cp.async gain nothing (660 us); an unrolled loop
+// misses the instruction cache (729 us).
+// MOM: 0 no moments, 1 moments without the z range (which only the turn's last
+// moments, the ones that callers can read, need), 2 all.
+template <int MOM, bool KICK>
+__global__ void __launch_bounds__(kPassThreads, KICK ? 4 : 5) k_map_pass(double* __restrict__ c,
+                                                    int64_t npad, const uint8_t* __restrict__ surv,
                                                     const int4* __restrict__ chunk_loc,
-                                                    const BunchDev* __restrict__ bunch,
                                                     const __grid_constant__ SectionDev sec,
                                                     const __grid_constant__ RingDev r,
-                                                    MomPartial* partials, unsigned* counters,
-                                                    BunchMomDev* mom, double beta_x, double beta_y,
-                                                    const CloudRec* __restrict__ rec, int P,
+                                                    MomPartial* partials,
+                                                    const CloudRec* __restrict__ rec,
+                                                    const FieldPrep* __restrict__ rec_prep, int P,
                                                     int chunk_base) {
-  __shared__ FieldPrep s_prep[CG_MAX_SPECIES];
+  __shared__ double s_pivot[kMomWarps][6];
+  __shared__ KickConst s_kc[KICK ? CG_MAX_SPECIES : 1];
   const int chunk = chunk_base + (int)blockIdx.x;
-  // the chunk's place from one table load (x bunch, y first tile, z chunk of
-  // the bunch, w valid slots), so the coordinate loads wait for one round
-  // trip, not two
+  // the chunk's place from one table load (x bunch, y first tile, z tiles), so
+  // the coordinate loads wait for one round trip; the padding slots of a tile
+  // hold the survival mark kPadding
   const int4 l = chunk_loc[chunk];
-  const int b = l.x, tile0 = l.y;
-  double v[kMomChunkTiles][6];
-  bool alive[kMomChunkTiles];
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    const int64_t g = (int64_t)(tile0 + u) * kTile + threadIdx.x;
-    const bool valid = u * kTile + (int)threadIdx.x < l.w;
-    alive[u] = valid && surv[g] == kAlive;
-#pragma unroll
-    for (int d = 0; d < 6; ++d) v[u][d] = valid ? c[d * npad + g] : 0.0;
-  }
-  const CloudRec* rb = rec + (size_t)b * P;
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
+  rec += (size_t)l.x * P;
+  rec_prep += (size_t)l.x * P;
   if (KICK) {
-    if ((int)threadIdx.x < P)
-      s_prep[threadIdx.x] = field_prep(rb[threadIdx.x].rms_x, rb[threadIdx.x].rms_y);
+    if ((int)threadIdx.x < P) s_kc[threadIdx.x] = kick_const(rec[threadIdx.x], rec_prep[threadIdx.x]);
     __syncthreads();
   }
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    if (!alive[u]) continue;
-    if (KICK) {
-      double dpx, dpy;
-      ion_kick_particle_prep(rb, s_prep, P, v[u][0], v[u][2], &dpx, &dpy);
-      v[u][1] += dpx;
-      v[u][3] += dpy;
-    }
-    section_map_particle(sec, r, v[u]);
-    store6(c, npad, (int64_t)(tile0 + u) * kTile + threadIdx.x, v[u]);
-  }
-  if (MOM) {
-    const BunchDev& B = bunch[b];
-    const int warp = threadIdx.x >> 5;
-    warp_moment_partial(v, alive, &partials[(size_t)chunk * kWarpsPerChunk + warp]);
-    warp_moment_finish(b, B.chunk_off * kWarpsPerChunk, B.n_chunks * kWarpsPerChunk, partials,
-                       counters, mom, beta_x, beta_y, c + 4 * npad + (int64_t)B.tile_off * kTile);
-  }
-}
-
-cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick, int chunk_a,
-                            int chunk_b, cudaStream_t s) {
-  const bool m = mom_section >= 0;
-  const double bx = m ? h.sec_dev_host[mom_section].beta_x : 0.0;
-  const double by = m ? h.sec_dev_host[mom_section].beta_y : 0.0;
-  const CloudRec* rec = kick ? h.d.rec + (size_t)k * h.M * h.P : nullptr;
-  if (chunk_b < 0) chunk_b = h.n_chunks;
-  if (!s) s = h.stream;
-  if (chunk_b <= chunk_a) return cudaSuccess;
-  auto kern = m ? (kick ? k_map_pass<true, true> : k_map_pass<true, false>)
-                : (kick ? k_map_pass<false, true> : k_map_pass<false, false>);
-  kern<<<chunk_b - chunk_a, kTile, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.d.bunch,
-                                           h.sec_dev_host[k], h.ring, h.d.wpartials,
-                                           h.d.counters, h.d.mom, bx, by, rec, h.P, chunk_a);
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// The map pass with the chunk staged in shared memory.  k_map_pass holds the
-// 24 coordinates of its four particles per thread in registers while their
-// loads are in flight, which needs 128 registers and so allows two CTAs per
-// SM: at most two chunks per SM are loading at any time.  Here every thread
-// copies its slots of the chunk into shared memory with cp.async (8 bytes per
-// coordinate, the aligned 4-byte word holding each survival byte), waits for
-// its own copies (a thread reads back only what it copied, so no CTA barrier
-// is needed) and then maps one particle at a time, writing the mapped
-// particle back to its slots for the second pass of the moments.  The
-// registers of one particle instead of four let more CTAs, and so more
-// chunks in flight, share an SM.  The chunk's place (bunch, first tile,
-// tiles, valid slots) comes from a per-chunk table, one load with no
-// dependent lookup.  The arithmetic and the reductions are those of
-// k_map_pass (with the kick, the records' precomputed field constants, as
-// k_ion_kick reads them), so the results are bitwise the same.
-
-struct ChunkStage {
-  double v[kMomChunkTiles][6][kTile];  // [tile of the chunk][coordinate][thread]
-  uint32_t sw[kMomChunkTiles][kTile];  // the 4-byte word holding each slot's survival byte
-};
-constexpr size_t kStageSmem = sizeof(ChunkStage);
-constexpr int kStagedCtasPerSm = 2;
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-template <bool MOM, bool KICK>
-__global__ void __launch_bounds__(kTile, kStagedCtasPerSm)
-    k_map_staged(double* __restrict__ c, int64_t npad, const uint8_t* __restrict__ surv,
-                 const int4* __restrict__ chunk_loc, const BunchDev* __restrict__ bunch,
-                 const __grid_constant__ SectionDev sec, const __grid_constant__ RingDev r,
-                 MomPartial* partials, unsigned* counters, BunchMomDev* mom, double beta_x,
-                 double beta_y, const CloudRec* __restrict__ rec,
-                 const FieldPrep* __restrict__ rec_prep, int P, int chunk_base) {
-  extern __shared__ __align__(128) unsigned char dyn_smem[];
-  ChunkStage& sb = *reinterpret_cast<ChunkStage*>(dyn_smem);
-  const int tid = threadIdx.x;
-  const int chunk = chunk_base + (int)blockIdx.x;
-  const int4 l = chunk_loc[chunk];  // x bunch, y first tile, z chunk of the bunch, w valid slots
-#pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    if (u * kTile < l.w) {  // a tile of this bunch
-      const int64_t g = (int64_t)(l.y + u) * kTile + tid;
-#pragma unroll
-      for (int d = 0; d < 6; ++d) cp_async8(&sb.v[u][d][tid], c + d * npad + g);
-      cp_async4(&sb.sw[u][tid], surv + (g & ~(int64_t)3));  // surv rows are 256-byte aligned
-    }
-  }
-  cp_async_wait_all();
-  const int byte = 8 * (tid & 3);
-  uint32_t alive = 0;
-  double s[7] = {0, 0, 0, 0, 0, 0, 0};
-  double mn = INFINITY, mx = -INFINITY;
+  const int warp = threadIdx.x >> 5;
+  MomSums m;
+  if (MOM) mom_sums_clear(m);
+  bool have = false;
 #pragma unroll 1
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    const bool valid = u * kTile + tid < l.w;
-    if (!(valid && ((sb.sw[u][tid] >> byte) & 0xFFu) == kAlive)) continue;
-    alive |= 1u << u;
-    double v[6];
-#pragma unroll
-    for (int d = 0; d < 6; ++d) v[d] = sb.v[u][d][tid];
-    if (KICK) {
-      double dpx, dpy;
-      ion_kick_particle_prep(rec + (size_t)l.x * P, rec_prep + (size_t)l.x * P, P, v[0], v[2],
-                             &dpx, &dpy);
-      v[1] += dpx;
-      v[3] += dpy;
+  for (int u = 0; u < kPassSteps * l.z; ++u, g += kPassThreads) {
+    const bool alive = surv[g] == kAlive;
+    double w[6];
+    load6(c, npad, g, w);
+    if (alive) {
+      if (KICK) {
+        double dpx, dpy;
+        ion_kick_particle(s_kc, rec, rec_prep, P, w[0], w[2], &dpx, &dpy);
+        w[1] += dpx;
+        w[3] += dpy;
+      }
+      section_map_particle(sec, r, w);
+      store6(c, npad, g, w);
     }
-    section_map_particle(sec, r, v);
-    store6(c, npad, (int64_t)(l.y + u) * kTile + tid, v);
     if (MOM) {
-#pragma unroll
-      for (int d = 0; d < 6; ++d) sb.v[u][d][tid] = v[d];
-      chunk_sums_add(v, s, mn, mx);
+      if (!have) have = mom_pivot(s_pivot[warp], alive, w);
+      if (alive) mom_sums_add<MOM == 2>(m, w, s_pivot[warp]);
     }
   }
-  if (MOM) {
-    const int warp = tid >> 5;
-    warp_moment_reduce<1>(s, mn, mx, [&](int u) { return ((alive >> u) & 1u) != 0; },
-                          [&](int u, int d) { return sb.v[u][d][tid]; },
-                          &partials[(size_t)chunk * kWarpsPerChunk + warp]);
-    const BunchDev& B = bunch[l.x];
-    warp_moment_finish(l.x, B.chunk_off * kWarpsPerChunk, B.n_chunks * kWarpsPerChunk, partials,
-                       counters, mom, beta_x, beta_y, c + 4 * npad + (int64_t)B.tile_off * kTile);
-  }
+  if (MOM) mom_partial(m, have, s_pivot[warp], &partials[(size_t)chunk * kMomWarps + warp]);
 }
 
-// Per device, once: the dynamic shared memory the staged map pass asks for
-// (above the 48 KB default) and a shared-memory carveout that holds
-// kStagedCtasPerSm of its CTAs.
-cudaError_t prepare_map_async() {
-  const void* kerns[] = {(const void*)k_map_staged<true, false>,
-                         (const void*)k_map_staged<true, true>,
-                         (const void*)k_map_staged<false, false>,
-                         (const void*)k_map_staged<false, true>};
-  const int carve = (int)std::min<size_t>(
-      100, (kStagedCtasPerSm * (kStageSmem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
-  for (const void* f : kerns) {
-    cudaError_t e =
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_map_turn(Handle& h, int k, int mom_section, bool kick, int chunk_a,
-                            int chunk_b, cudaStream_t s) {
-  return h.map_async ? launch_map_async(h, k, mom_section, kick, chunk_a, chunk_b, s)
-                     : launch_map_pass(h, k, mom_section, kick, chunk_a, chunk_b, s);
-}
-
-cudaError_t launch_map_async(Handle& h, int k, int mom_section, bool kick, int chunk_a,
-                             int chunk_b, cudaStream_t s) {
-  const bool m = mom_section >= 0;
-  const double bx = m ? h.sec_dev_host[mom_section].beta_x : 0.0;
-  const double by = m ? h.sec_dev_host[mom_section].beta_y : 0.0;
+cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick, bool z_range,
+                            int chunk_a, int chunk_b, cudaStream_t s) {
+  const int m = mom_section < 0 ? 0 : z_range ? 2 : 1;
   const CloudRec* rec = kick ? h.d.rec + (size_t)k * h.M * h.P : nullptr;
   const FieldPrep* rp = kick ? h.d.rec_prep + (size_t)k * h.M * h.P : nullptr;
-  if (chunk_b < 0) chunk_b = h.n_chunks;
+  const bool all = chunk_b < 0;
+  if (all) chunk_b = h.n_chunks;
   if (!s) s = h.stream;
-  if (chunk_b <= chunk_a) return cudaSuccess;
-  auto kern = m ? (kick ? k_map_staged<true, true> : k_map_staged<true, false>)
-                : (kick ? k_map_staged<false, true> : k_map_staged<false, false>);
-  kern<<<chunk_b - chunk_a, kTile, kStageSmem, s>>>(
-      h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.d.bunch, h.sec_dev_host[k], h.ring,
-      h.d.wpartials, h.d.counters, h.d.mom, bx, by, rec, rp, h.P, chunk_a);
-  return cudaGetLastError();
+  if (chunk_b > chunk_a) {
+    auto kern = m == 2   ? (kick ? k_map_pass<2, true> : k_map_pass<2, false>)
+                : m == 1 ? (kick ? k_map_pass<1, true> : k_map_pass<1, false>)
+                         : (kick ? k_map_pass<0, true> : k_map_pass<0, false>);
+    kern<<<chunk_b - chunk_a, kPassThreads, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc,
+                                                    h.sec_dev_host[k], h.ring, h.d.wpartials, rec,
+                                                    rp, h.P, chunk_a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return m && all ? launch_mom_merge(h, mom_section, s) : cudaSuccess;
 }
 
 cudaError_t launch_ion_kick(Handle& h, int k) { return launch_ion_kick_variant(h, k, h.kick_variant); }
@@ -1421,7 +1152,6 @@ cudaError_t measure_fp64_peak(double* flops) {
 
 cudaError_t upload_weideman_table() {
   cudaError_t e = cudaMemcpyToSymbol(c_weideman, &h_weideman, sizeof(WeidemanTable));
-  if (e == cudaSuccess) e = prepare_map_async();
   if (e == cudaSuccess) e = upload_weideman_table_ion();
   if (e == cudaSuccess) e = upload_weideman_table_sc();
   return e != cudaSuccess ? e : upload_weideman_table_sur();
@@ -1433,28 +1163,26 @@ cudaError_t upload_weideman_table() {
 // (another code's tracking loop, a PyTorch program whose caching allocator owns
 // the device memory) cannot afford a cudaMalloc/cudaFree pair per call: both
 // synchronise the device and stall the caller's other streams.  The per-tile
-// partials, the finished moments and the completion counter therefore live in
-// one file-scope device array of fixed size.
+// partials and the completion counter therefore live in one file-scope device
+// array of fixed size.
 //
-// Layout of the array (doubles): one partial per CTA, i.e. per chunk of
-// kMomChunkTiles tiles (kNoAllocMaxChunks of them), then one BunchMomDev slot
-// (32 doubles), then the completion counter (32 doubles).
+// Layout of the array (doubles): one partial per CTA (kNoAllocMaxParts), then
+// the completion counter (32 doubles).
 // Only the counter must read zero when a call starts: it is zero at module
 // load, zeroed again when the address is first resolved on a device, and the
-// last CTA of every call puts it back to zero.  The partials and the moments
-// slot are written before they are read in every call.  Two calls that overlap
+// last CTA of every call puts it back to zero.  The partials are written before
+// they are read in every call.  Two calls that overlap
 // on one device (different streams, or different host threads without
 // ordering) share this array and race.
-constexpr int kNoAllocMaxChunks = kNoAllocMaxTiles / kMomChunkTiles;
+constexpr int kNoAllocThreads = 256;
+constexpr int kNoAllocMaxParts = 148 * 3;  // CTAs
 constexpr int kNoAllocPartialDoubles = (int)(sizeof(MomPartial) / sizeof(double));
-constexpr size_t kNoAllocMomOff = (size_t)kNoAllocMaxChunks * kNoAllocPartialDoubles;
-constexpr size_t kNoAllocCounterOff = kNoAllocMomOff + 32;
+constexpr size_t kNoAllocCounterOff =
+    ((size_t)kNoAllocMaxParts * kNoAllocPartialDoubles + 31) / 32 * 32;
 constexpr size_t kNoAllocDoubles = kNoAllocCounterOff + 32;
 static_assert(sizeof(MomPartial) % sizeof(double) == 0, "partial is a whole number of doubles");
-static_assert(sizeof(BunchMomDev) <= 32 * sizeof(double), "moments slot holds a BunchMomDev");
-static_assert(kNoAllocMaxTiles % kMomChunkTiles == 0 &&
-                  (long long)kNoAllocMaxChunks * kMomChunkTiles * kTile >= CG_NOALLOC_MAX_PARTICLES,
-              "one partial per chunk covers the largest accepted call");
+static_assert((long long)kNoAllocMaxTiles * kTile >= CG_NOALLOC_MAX_PARTICLES,
+              "the largest accepted call");
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
 cudaError_t noalloc_scratch_address(double** ptr) {
@@ -1463,34 +1191,65 @@ cudaError_t noalloc_scratch_address(double** ptr) {
   return cudaMemset(*ptr + kNoAllocCounterOff, 0, 32 * sizeof(double));
 }
 
-__global__ void __launch_bounds__(kTile, 2) k_moments_noalloc(const double* __restrict__ c,
+__global__ void __launch_bounds__(kNoAllocThreads, 3) k_moments_noalloc(const double* __restrict__ c,
                                                            int64_t stride,
                                                            const uint8_t* __restrict__ surv, int n,
-                                                           double beta_x, double beta_y,
-                                                           double* scratch) {
-  __shared__ double smem[18 * 32];
+                                                           int steps, double beta_x, double beta_y,
+                                                           double* scratch, cg_bunch_moments* out) {
+  __shared__ double s_pivot[kNoAllocThreads / 32][6];
+  __shared__ MomPartial s_part[kNoAllocThreads / 32];
+  __shared__ bool s_last;
   MomPartial* partials = reinterpret_cast<MomPartial*>(scratch);
-  BunchMomDev* mom = reinterpret_cast<BunchMomDev*>(scratch + kNoAllocMomOff);
   unsigned* counter = reinterpret_cast<unsigned*>(scratch + kNoAllocCounterOff);
-  double v[kMomChunkTiles][6];
-  bool alive[kMomChunkTiles];
+  const int warp = threadIdx.x >> 5;
+  double* pivot = s_pivot[warp];
+  MomSums m;
+  mom_sums_clear(m);
+  bool have = false;
+  int i = blockIdx.x * steps * kNoAllocThreads + threadIdx.x;
+  // the next step's loads in flight while this one's are added up
+  auto load = [&](int at, double (&v)[6]) {
+    const bool valid = at < n;
+    const bool alive = valid && surv[at] == kAlive;
 #pragma unroll
-  for (int u = 0; u < kMomChunkTiles; ++u) {
-    const int i = (blockIdx.x * kMomChunkTiles + u) * kTile + threadIdx.x;
-    const bool valid = i < n;
-    alive[u] = valid && surv[i] == kAlive;
+    for (int d = 0; d < 6; ++d) v[d] = valid ? c[d * stride + at] : 0.0;
+    return alive;
+  };
+  double v[6];
+  bool next = load(i, v);
+#pragma unroll 1
+  for (int u = 0; u < steps; ++u) {
+    const bool alive = next;
+    double w[6];
 #pragma unroll
-    for (int d = 0; d < 6; ++d) v[u][d] = valid ? c[d * stride + i] : 0.0;
+    for (int d = 0; d < 6; ++d) w[d] = v[d];
+    if (u + 1 < steps) {
+      i += kNoAllocThreads;
+      next = load(i, v);
+    }
+    if (!have) have = mom_pivot(pivot, alive, w);
+    if (alive) mom_sums_add<true>(m, w, pivot);
   }
-  chunk_moment_partial(v, alive, smem, &partials[blockIdx.x]);
-  bunch_moment_finish(0, 0, (int)gridDim.x, partials, counter, mom, beta_x, beta_y, c + 4 * stride);
-}
-
-// Converts the finished moments into the public record (one thread; the
-// transmission of a record made this way is n_alive / n).
-__global__ void k_moments_noalloc_out(const double* __restrict__ scratch, int n,
-                                      cg_bunch_moments* out) {
-  const BunchMomDev s = *reinterpret_cast<const BunchMomDev*>(scratch + kNoAllocMomOff);
+  mom_partial(m, have, pivot, &s_part[warp]);
+  __syncthreads();
+  MomPartial total;
+  if (warp == 0) {
+    mom_merge_block<32, false>(s_part, kNoAllocThreads / 32, &total);
+    if (threadIdx.x == 0) partials[blockIdx.x] = total;
+  }
+  // the last CTA merges
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  mom_merge_block<kNoAllocThreads>(partials, (int)gridDim.x, &total);
+  if (threadIdx.x != 0) return;
+  *counter = 0;
+  BunchMomDev s;
+  mom_finalize(total, beta_x, beta_y, c[4 * stride], s);
+  // the public record (its transmission is n_alive / n)
   cg_bunch_moments o;
   o.n_alive = (int)s.n_alive;
   o.n_macro = n;
@@ -1511,15 +1270,16 @@ __global__ void k_moments_noalloc_out(const double* __restrict__ scratch, int n,
   *out = o;
 }
 
+// Steps per CTA: enough that at most kNoAllocMaxParts CTAs cover the call, so
+// that every CTA of the largest runs at once.
 cudaError_t launch_moments_noalloc(const double* c, int64_t stride, const uint8_t* surv, int n,
                                    double beta_x, double beta_y, double* scratch,
                                    cg_bunch_moments* out, cudaStream_t s) {
-  const int chunks = (n + kTile * kMomChunkTiles - 1) / (kTile * kMomChunkTiles);
-  if (n < 1 || chunks > kNoAllocMaxChunks) return cudaErrorInvalidValue;
-  k_moments_noalloc<<<chunks, kTile, 0, s>>>(c, stride, surv, n, beta_x, beta_y, scratch);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_moments_noalloc_out<<<1, 1, 0, s>>>(scratch, n, out);
+  if (n < 1 || n > kNoAllocMaxTiles * kTile) return cudaErrorInvalidValue;
+  const int all = (n + kNoAllocThreads - 1) / kNoAllocThreads;
+  const int steps = (all + kNoAllocMaxParts - 1) / kNoAllocMaxParts;
+  k_moments_noalloc<<<(all + steps - 1) / steps, kNoAllocThreads, 0, s>>>(
+      c, stride, surv, n, steps, beta_x, beta_y, scratch, out);
   return cudaGetLastError();
 }
 

@@ -54,20 +54,16 @@ cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a = 0, int
 int kick_variants();
 void kick_variant_shape(int v, int* threads, int* min_ctas);
 // (ion kick of IP k if `kick`) + map of section k + moments at section
-// `mom_section` (if >= 0), over the moments chunks [chunk_a, chunk_b)
-// (chunk_b < 0: all) on stream s (null: h.stream)
-cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick = false, int chunk_a = 0,
-                            int chunk_b = -1, cudaStream_t s = nullptr);
-// The same pass with the next chunk in flight: a persistent grid (two CTAs
-// per SM) in which every thread stages its slots of the CTA's next chunk in
-// shared memory by cp.async while it maps and reduces the current one.
-cudaError_t launch_map_async(Handle& h, int k, int mom_section, bool kick = false,
-                             int chunk_a = 0, int chunk_b = -1, cudaStream_t s = nullptr);
-// the map pass of the turn: the asynchronous form when h.map_async is set
-cudaError_t launch_map_turn(Handle& h, int k, int mom_section, bool kick = false,
-                            int chunk_a = 0, int chunk_b = -1, cudaStream_t s = nullptr);
-// per device, once: the dynamic shared memory of the asynchronous map pass
-cudaError_t prepare_map_async();
+// `mom_section` (if >= 0; their z range if `z_range`), over the chunks
+// [chunk_a, chunk_b) (chunk_b < 0: all, and the moments merged; over parts the
+// caller merges them) on stream s (null: h.stream)
+cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick = false,
+                            bool z_range = true, int chunk_a = 0, int chunk_b = -1,
+                            cudaStream_t s = nullptr);
+// the bunches' moments from the passes' partials, at the twiss of section k
+cudaError_t launch_mom_merge(Handle& h, int k, cudaStream_t s = nullptr);
+// warps per CTA of the passes: moment partials per chunk
+constexpr int kMomWarps = 4;
 enum LongFlags : unsigned {
   kLongRF = 1,
   kLongDrift = 2,

@@ -21,13 +21,15 @@ struct SectionDev {
   double aperture_x, aperture_y;
   double b1h1[36], h1b1[36], h2b2[36];
   // 1 when all three matrices have the uncoupled Twiss/dispersion form (no
-  // non-zero entry outside kTwissForm): the maps then skip the zero terms
+  // non-zero entry outside kTwissForm), 2 when there is no dispersion either
+  // (kPlainForm): the maps then skip the zero terms
   int twiss_form;
 };
 
 struct RingDev {
   double chrom[2];
   double adtx[5], adty[5];
+  int adt2;                          // some second-order amplitude-dependent term is not zero
   double circ_ring, alphac[3];
   double energy, r_beta2, u0_term;   // u0 / E / beta^2 (Bunch.cpp:490)
   double rf_theta_coeff[4];          // 2 pi h_c f_RF / (c beta), Bunch.cpp:468
@@ -64,9 +66,12 @@ constexpr unsigned long long kTwissForm =
     (1ull << 20) | (1ull << 21) | (1ull << 23) |                    // row 3: 2, 3, 5
     (1ull << 24) | (1ull << 25) | (1ull << 26) | (1ull << 27) | (1ull << 28) |  // row 4
     (1ull << 35);                                                   // row 5: 5
-inline bool fits_twiss_form(const double* A) {
+// the same without dispersion: x, x', y, y', z, dp each on its own plane
+constexpr unsigned long long kPlainForm = (1ull << 0) | (1ull << 6) | (1ull << 7) | (1ull << 14) |
+                                          (1ull << 20) | (1ull << 21) | (1ull << 28) | (1ull << 35);
+inline bool fits_form(const double* A, unsigned long long form) {
   for (int e = 0; e < 36; ++e)
-    if (!((kTwissForm >> e) & 1ull) && A[e] != 0.0) return false;
+    if (!((form >> e) & 1ull) && A[e] != 0.0) return false;
   return true;
 }
 
@@ -81,29 +86,53 @@ CG_HD void matvec6_twiss(const double* A, const double v[6], double out[6]) {
   out[5] = A[35] * v[5];
 }
 
+// matvec6 for a matrix without dispersion terms: 8 operations.
+CG_HD void matvec6_plain(const double* A, const double v[6], double out[6]) {
+  out[0] = A[0] * v[0];
+  out[1] = fma(A[7], v[1], A[6] * v[0]);
+  out[2] = A[14] * v[2];
+  out[3] = fma(A[21], v[3], A[20] * v[2]);
+  out[4] = A[28] * v[4];
+  out[5] = A[35] * v[5];
+}
+
 CG_HD void matvec6_section(const SectionDev& s, const double* A, const double v[6], double out[6]) {
-  if (s.twiss_form) matvec6_twiss(A, v, out);
+  if (s.twiss_form == 2) matvec6_plain(A, v, out);
+  else if (s.twiss_form) matvec6_twiss(A, v, out);
   else matvec6(A, v, out);
 }
 
 // sin and cos of phi0 + d from those of phi0 and a Taylor series of d
-// (|d| <= 1/16: the first omitted terms are below 1e-20 relative); larger d
-// takes sincos of the sum.  The chromatic and amplitude tune shifts of a
-// section are ~1e-3 rad, so the series is the path taken: it costs a dozen
-// FMAs instead of two argument reductions.
+// (the first omitted terms are below 1e-20 relative: five terms each to |d| <=
+// 1/16, three to 1/256); larger d takes sincos of the sum, out of line.  The
+// chromatic and amplitude tune shifts of a section are ~1e-3 rad, so the short
+// series is the path taken: it costs eight FMAs instead of two argument
+// reductions.
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__
+#else
+inline
+#endif
+static void sincos_far(double phi, double* sn, double* cs) { sincos(phi, sn, cs); }
+
 CG_HD void sincos_shifted(double phi0, double c0, double s0, double d, double* sn, double* cs) {
-  if (fabs(d) <= 0.0625) {
+  const double ad = fabs(d);
+  if (ad <= 0.0625) {
     const double d2 = d * d;
-    const double sd =
-        d * fma(d2, fma(d2, fma(d2, fma(d2, fma(d2, -1.0 / 39916800.0, 1.0 / 362880.0),
-                                            -1.0 / 5040.0), 1.0 / 120.0), -1.0 / 6.0), 1.0);
-    const double cd =
-        fma(d2, fma(d2, fma(d2, fma(d2, fma(d2, -1.0 / 3628800.0, 1.0 / 40320.0), -1.0 / 720.0),
-                            1.0 / 24.0), -0.5), 1.0);
+    double sd, cd;
+    if (ad <= 0.00390625) {
+      sd = d * fma(d2, fma(d2, fma(d2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), 1.0);
+      cd = fma(d2, fma(d2, fma(d2, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
+    } else {
+      sd = d * fma(d2, fma(d2, fma(d2, fma(d2, fma(d2, -1.0 / 39916800.0, 1.0 / 362880.0),
+                                           -1.0 / 5040.0), 1.0 / 120.0), -1.0 / 6.0), 1.0);
+      cd = fma(d2, fma(d2, fma(d2, fma(d2, fma(d2, -1.0 / 3628800.0, 1.0 / 40320.0),
+                                       -1.0 / 720.0), 1.0 / 24.0), -0.5), 1.0);
+    }
     *sn = fma(s0, cd, c0 * sd);
     *cs = fma(c0, cd, -(s0 * sd));
   } else {
-    sincos(phi0 + d, sn, cs);
+    sincos_far(phi0 + d, sn, cs);
   }
 }
 
@@ -120,19 +149,24 @@ CG_HD void sincos_shifted(double phi0, double c0, double s0, double d, double* s
 CG_HD void section_map_rotated(const SectionDev& s, const RingDev& r, const double v[6],
                                double v2[6]) {
   const double dp = v[5];
-  double x = v[0] - s.eta_x * dp;
-  double px = v[1] - s.etap_x * dp;
-  double y = v[2] - s.eta_y * dp;
-  double py = v[3] - s.etap_y * dp;
+  double x = v[0], px = v[1], y = v[2], py = v[3];
+  if (s.twiss_form != 2) {
+    x -= s.eta_x * dp;
+    px -= s.etap_x * dp;
+    y -= s.eta_y * dp;
+    py -= s.etap_y * dp;
+  }
   double ux = fma(s.alpha_x, x, s.beta_x * px);
   double uy = fma(s.alpha_y, y, s.beta_y * py);
   double ampX = fma(x, x, ux * ux) * s.inv_beta_x;
   double ampY = fma(y, y, uy * uy) * s.inv_beta_y;
-  double ax2 = ampX * ampX, ay2 = ampY * ampY, axy = ampX * ampY;
-  double dnux = r.chrom[0] * dp + r.adtx[0] * ampX + r.adtx[1] * ampY + r.adtx[2] * ax2 / 2 +
-                r.adtx[3] * ay2 / 2 + r.adtx[4] * axy;
-  double dnuy = r.chrom[1] * dp + r.adty[0] * ampX + r.adty[1] * ampY + r.adty[2] * ax2 / 2 +
-                r.adty[3] * ay2 / 2 + r.adty[4] * axy;
+  double dnux = r.chrom[0] * dp + r.adtx[0] * ampX + r.adtx[1] * ampY;
+  double dnuy = r.chrom[1] * dp + r.adty[0] * ampX + r.adty[1] * ampY;
+  if (r.adt2) {
+    double ax2 = ampX * ampX, ay2 = ampY * ampY, axy = ampX * ampY;
+    dnux = dnux + r.adtx[2] * ax2 / 2 + r.adtx[3] * ay2 / 2 + r.adtx[4] * axy;
+    dnuy = dnuy + r.adty[2] * ax2 / 2 + r.adty[3] * ay2 / 2 + r.adty[4] * axy;
+  }
   dnux *= s.weigh_x;
   dnuy *= s.weigh_y;
   // the reference's rounded phase phi = phaseAdv + 2 pi dnu; phi - phaseAdv is
@@ -260,9 +294,9 @@ CG_HD int mark_lost_particle(const RingDev& r, double ax, double ay, double x, d
 }
 
 // ---------------------------------------------------------------------------
-// Moments: per-tile partials merged with Chan, Golub & LeVeque's pairwise
-// update, in a fixed order, so the result is deterministic and two-pass
-// accurate (the reference makes two passes, MPBunch.cpp:355-455).
+// Moments: partials of groups of particles, merged in a fixed order, so the
+// result is deterministic and two-pass accurate (the reference makes two
+// passes, MPBunch.cpp:355-455).
 
 struct MomPartial {
   double n;
@@ -270,35 +304,6 @@ struct MomPartial {
   double c[9];        // centred co-moments: xx pxpx yy pypy zz pzpz xpx ypy zpz
   double zmin, zmax;  // alive only
 };
-
-CG_HD void mom_clear(MomPartial& p) {
-  p.n = 0;
-  for (int d = 0; d < 6; ++d) p.mean[d] = 0;
-  for (int d = 0; d < 9; ++d) p.c[d] = 0;
-  p.zmin = INFINITY;
-  p.zmax = -INFINITY;
-}
-
-// a <- a (+) b
-CG_HD void mom_merge(MomPartial& a, const MomPartial& b) {
-  if (b.n == 0) return;
-  if (a.n == 0) {
-    a = b;
-    return;
-  }
-  double n = a.n + b.n;
-  double f = b.n / n;
-  double w = a.n * b.n / n;
-  double d[6];
-  for (int k = 0; k < 6; ++k) d[k] = b.mean[k] - a.mean[k];
-  const int ia[9] = {0, 1, 2, 3, 4, 5, 0, 2, 4};
-  const int ib[9] = {0, 1, 2, 3, 4, 5, 1, 3, 5};
-  for (int k = 0; k < 9; ++k) a.c[k] = a.c[k] + b.c[k] + d[ia[k]] * d[ib[k]] * w;
-  for (int k = 0; k < 6; ++k) a.mean[k] = fma(d[k], f, a.mean[k]);
-  a.n = n;
-  a.zmin = fmin(a.zmin, b.zmin);
-  a.zmax = fmax(a.zmax, b.zmax);
-}
 
 // Bunch-level outputs of MPBunch::GetMPBunchRMS (MPBunch.cpp:390-497) from
 // the merged partial.  beta_x/beta_y are the twiss betas of the section k
@@ -350,32 +355,77 @@ struct CloudRec {
   double coeff, rms_x, rms_y, aver_x, aver_y, count;
 };
 
-// Electron-side kick of one particle from all species (MPBunch.cpp:1166-1206).
-CG_HD void ion_kick_particle(const CloudRec* rec, int n_species, double x, double y, double* dpx,
-                             double* dpy) {
-  double fx = 0, fy = 0;
-  for (int p = 0; p < n_species; ++p) {
-    double ex, ey;
-    gaussian_field(x - rec[p].aver_x, y - rec[p].aver_y, rec[p].rms_x, rec[p].rms_y, &ex, &ey);
-    fx = fma(rec[p].coeff, ex, fx);
-    fy = fma(rec[p].coeff, ey, fy);
-  }
-  *dpx = fx;
-  *dpy = fy;
+#if defined(__CUDACC__)
+// One cloud record as the kick kernels read it, in the frame of the cloud's
+// axes (a the larger one): centroid, the scales of w(z1) and w(z2) (z1 = (|da|,
+// |db|) s0, z2 = (|da| sa1, |db| sb1)), of the Gaussian factor, and the whole
+// coefficient.
+struct KickConst {
+  double ma, mb, s0, sa1, sb1, ga, gb, ck;
+  int mode;  // FieldPrep::mode
+};
+CG_D KickConst kick_const(const CloudRec& r, const FieldPrep& f) {
+  KickConst k;
+  const bool sw = f.mode == 1;
+  k.ma = sw ? r.aver_y : r.aver_x;
+  k.mb = sw ? r.aver_x : r.aver_y;
+  k.s0 = f.isig;
+  k.sa1 = f.r * f.isig;
+  k.sb1 = f.isig * f.ir;
+  k.ga = f.ia;
+  k.gb = f.ib;
+  k.ck = r.coeff * f.coeff;
+  k.mode = f.mode;
+  return k;
+}
+// |z1|, |z2| possibly beyond 30, a round cloud, or no number: out of line, so
+// that the common path stays short (the kick's loop has to fit the
+// instruction cache).
+static __device__ __noinline__ void ion_kick_any(const CloudRec* rec, const FieldPrep* prep,
+                                                 double x, double y, double* fx, double* fy) {
+  double ex, ey;
+  gaussian_field_kick(*prep, x - rec->aver_x, y - rec->aver_y, &ex, &ey);
+  *fx = rec->coeff * ex;
+  *fy = rec->coeff * ey;
+}
+CG_D double flip_sign(double v, double s) {  // v times the sign of s
+  return __hiloint2double(__double2hiint(v) ^ (__double2hiint(s) & 0x80000000), __double2loint(v));
 }
 
-// The same with the per-record field constants prepared by the ion chain.
-CG_HD void ion_kick_particle_prep(const CloudRec* rec, const FieldPrep* prep, int n_species,
-                                  double x, double y, double* dpx, double* dpy) {
+// Electron-side kick of one particle from all species (MPBunch.cpp:1166-1206)
+// with the records' constants prepared.
+CG_D void ion_kick_particle(const KickConst* kc, const CloudRec* rec, const FieldPrep* prep,
+                            int n_species, double x, double y, double* dpx, double* dpy) {
   double fx = 0, fy = 0;
   for (int p = 0; p < n_species; ++p) {
-    double ex, ey;
-    gaussian_field_kick(prep[p], x - rec[p].aver_x, y - rec[p].aver_y, &ex, &ey);
-    fx = fma(rec[p].coeff, ex, fx);
-    fy = fma(rec[p].coeff, ey, fy);
+    const KickConst& k = kc[p];
+    const bool sw = k.mode == 1;
+    const double da = (sw ? y : x) - k.ma, db = (sw ? x : y) - k.mb;
+    const double aa = fabs(da), ab = fabs(db);
+    const double zr[2] = {aa * k.s0, aa * k.sa1}, zi[2] = {ab * k.s0, ab * k.sb1};
+    // z1 has the larger real part, z2 the larger imaginary one: both below 21
+    // keeps |z| below 30 (compared by the upper words)
+    constexpr int kHi21 = 0x40350000;
+    if (k.mode != 2 && __double2hiint(zr[0]) < kHi21 && __double2hiint(zi[1]) < kHi21) {
+      const double ua = aa * k.ga, ub = ab * k.gb;
+      const double g = exp_neg(0.5 * fma(ua, ua, ub * ub));
+      cplx w[2];
+      w_weideman_fast<2>(zr, zi, w);
+      double fa = flip_sign(k.ck * fma(-g, w[1].im, w[0].im), da);
+      double fb = flip_sign(k.ck * fma(-g, w[1].re, w[0].re), db);
+      if (ua + ub < 1.0e-5) fa = fb = 0.0;  // MPBunch.cpp:1179
+      fx += sw ? fb : fa;
+      fy += sw ? fa : fb;
+    } else {
+      double ex, ey;
+      ion_kick_any(rec + p, prep + p, x, y, &ex, &ey);
+      fx += ex;
+      fy += ey;
+    }
   }
   *dpx = fx;
   *dpy = fy;
 }
+#endif
 
 }  // namespace cg

@@ -737,8 +737,8 @@ int cg_surrogate_audit_stats(cg_handle* h, int* count, double* last, double* wor
  * the call returns without waiting.
  *
  * It never allocates: the partials live in a fixed static device array,
- * one per CTA of 1024 particles (CG_NOALLOC_MAX_PARTICLES / 1024 of them,
- * about 148 KB per device, held by every device that loads the library), and
+ * one per CTA (at most 444 of them, about 64 KB per device, held by every
+ * device that loads the library), and
  * n > CG_NOALLOC_MAX_PARTICLES is rejected with CG_ERR_INVALID.  The first
  * call on each device resolves that array's address and zeroes its
  * completion counter with a synchronous memset, so make it before any stream
