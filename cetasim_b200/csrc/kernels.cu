@@ -200,17 +200,26 @@ constexpr int kPassSteps = kTile / kPassThreads;
 static_assert(kMomWarps * 32 == kPassThreads, "one partial per warp");
 
 // Sets the warp's pivot if some lane's particle is alive; the warp calls it
-// per tile until it returns true.
+// per tile until it returns true.  The pivot is the mean of the warp's alive
+// particles, or the first one where that is the same to rounding: a coordinate
+// that is equal in all of them has deviations of exactly zero.
 __device__ __forceinline__ bool mom_pivot(double* pivot, bool alive, const double (&v)[6]) {
   const unsigned bal = __ballot_sync(FULL_MASK, alive);
   if (!bal) return false;
   const int lane = threadIdx.x & 31, idx = warp_sum8_index(lane);
   double a[8];
+  if (lane == __ffs(bal) - 1)
+#pragma unroll
+    for (int d = 0; d < 6; ++d) pivot[d] = v[d];
 #pragma unroll
   for (int d = 0; d < 6; ++d) a[d] = alive ? v[d] : 0.0;
   a[6] = a[7] = 0.0;
   const double t = warp_sum8_t(a);
-  if ((lane & 3) == 0 && idx < 6) pivot[idx] = t / __popc(bal);
+  __syncwarp();
+  if ((lane & 3) == 0 && idx < 6) {
+    const double mean = t / __popc(bal);
+    if (fabs(mean - pivot[idx]) > 1e-14 * fabs(mean)) pivot[idx] = mean;
+  }
   __syncwarp();
   return true;
 }
@@ -257,13 +266,17 @@ __device__ __forceinline__ void mom_merge_block(const MomPartial* partials, int 
   auto get = [](const double* p) { return GLOBAL ? __ldcg(p) : *p; };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = NW > 1 ? (int)threadIdx.x : lane;
-  // perhaps written by other CTAs of this launch: read through L2
-  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, mn = INFINITY, mx = -INFINITY;
+  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, mn = INFINITY, mx = -INFINITY, m0[6];
+  // means about that of the first of them with particles: a mean that is the
+  // same in all stays that value exactly
+  const int first = __ffs(__ballot_sync(FULL_MASK, lane < n_parts && get(&partials[lane].n) > 0));
+#pragma unroll
+  for (int d = 0; d < 6; ++d) m0[d] = first ? get(&partials[first - 1].mean[d]) : 0.0;
   for (int t = t0; t < n_parts; t += NT) {
     const MomPartial* q = partials + t;
     const double n = get(&q->n);
 #pragma unroll
-    for (int d = 0; d < 6; ++d) s[d] = fma(n, get(&q->mean[d]), s[d]);
+    for (int d = 0; d < 6; ++d) s[d] = fma(n, n > 0 ? get(&q->mean[d]) - m0[d] : 0.0, s[d]);
     s[6] += n;
     mn = fmin(mn, get(&q->zmin));
     mx = fmax(mx, get(&q->zmax));
@@ -304,7 +317,7 @@ __device__ __forceinline__ void mom_merge_block(const MomPartial* partials, int 
     const double n = get(&q->n);
     double d[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) d[k] = get(&q->mean[k]) - s[k] * inv;
+    for (int k = 0; k < 6; ++k) d[k] = (get(&q->mean[k]) - m0[k]) - s[k] * inv;
 #pragma unroll
     for (int k = 0; k < 6; ++k) c[k] += fma(n * d[k], d[k], get(&q->c[k]));
 #pragma unroll
@@ -321,7 +334,7 @@ __device__ __forceinline__ void mom_merge_block(const MomPartial* partials, int 
   else __syncwarp();
   if (threadIdx.x != 0) return;
   total->n = s[6];
-  for (int k = 0; k < 6; ++k) total->mean[k] = s[k] * inv;
+  for (int k = 0; k < 6; ++k) total->mean[k] = m0[k] + s[k] * inv;
   for (int k = 0; k < 9; ++k) {
     double a = s_sum[0][9 + k];
     for (int w = 1; w < NW; ++w) a += s_sum[w][9 + k];

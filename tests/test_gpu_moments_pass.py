@@ -79,3 +79,21 @@ def test_moments(n, lost, off):
     a = bytes(g.moments())
     g.MPBeamRMSCal(0)
     assert a == bytes(g.moments())
+
+
+@pytest.mark.parametrize("n,lost", [(45, 0), (300, 7), (5000, 1100), (70001, 257)])
+def test_equal_coordinates_have_zero_size(n, lost):
+    """A coordinate that is the same in every alive particle: its mean is that
+    value and its size zero exactly (a zero size is an error further on)."""
+    wl = small("plain_single", n / 1e5)
+    wl.n_macro[0] = n
+    c = particles(wl, seed=n)[0]
+    s = np.zeros(n, dtype=np.uint8)
+    s[:lost] = 1
+    c[4, lost:], c[5, lost:] = 1.1e-3, 0.7e-4
+    g = MPBeam(wl)
+    g.upload(0, c, s)
+    g.MPBeamRMSCal(0)
+    m = g.moments()[0]
+    assert (m.bunch_length, m.energy_spread) == (0.0, 0.0)
+    assert (m.mean[4], m.mean[5]) == (1.1e-3, 0.7e-4)
