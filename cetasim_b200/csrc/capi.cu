@@ -127,9 +127,10 @@ void free_beam(Handle& h) {
   dfree(d.phase_slot); dfree(d.phase_ptr);
   d.phase_slot = nullptr; d.phase_ptr = nullptr;
   dfree(d.sc_geom); dfree(d.sc_cnt); dfree(d.sc_acc); dfree(d.sc_field);
-  dfree(d.sc_slice_of); dfree(d.sc_list); dfree(d.sc_start); dfree(d.sc_cursor);
+  dfree(d.sc_slices); dfree(d.sc_xy); dfree(d.sc_start); dfree(d.sc_cursor); dfree(d.sc_range);
   d.sc_geom = nullptr; d.sc_cnt = nullptr; d.sc_acc = nullptr; d.sc_field = nullptr;
-  d.sc_slice_of = nullptr; d.sc_list = nullptr; d.sc_start = nullptr; d.sc_cursor = nullptr;
+  d.sc_slices = nullptr; d.sc_xy = nullptr; d.sc_start = nullptr; d.sc_cursor = nullptr;
+  d.sc_range = nullptr;
   h.cbm_cap = h.cbm_n = 0;
   IonWalk& w = d.iw;
   dfree(w.births); dfree(w.prep); dfree(w.bunch); dfree(w.spec); dfree(w.bound); dfree(w.part);
@@ -677,7 +678,6 @@ int cg_create(const cg_config* cfg, int device, cg_handle** out) {
     p.nx = h.cfg.sc_mesh[0];
     p.ny = h.cfg.sc_mesh[1];
     p.nz = h.cfg.sc_mesh[2];
-    p.acc_per_slice = p.flag == 2 ? p.nx * p.ny : 4;
     // PIC2D::UpdateTransverseMomentum (PIC2D.cpp): the reference momentum
     const double gamma0 = h.cfg.ring.electron_energy / 0.51099906e6;
     const double beta0 = std::sqrt(1 - 1 / std::pow(gamma0, 2));
@@ -970,16 +970,16 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
       return fail(&h, CG_ERR_UNSUPPORTED, "space charge with bunch sharding is not supported");
     }
     const size_t slices = (size_t)M * p.nz;
-    if (dalloc(&d.sc_geom, (size_t)M * 11) || dalloc(&d.sc_cnt, slices) ||
-        (p.flag != 2 && dalloc(&d.sc_acc, slices * p.acc_per_slice)) ||
+    if (dalloc(&d.sc_geom, (size_t)M * kScGeom) || dalloc(&d.sc_cnt, slices) ||
+        dalloc(&d.sc_range, (size_t)M * 4) ||
+        (p.flag != 2 && (dalloc(&d.sc_acc, slices * 4) || dalloc(&d.sc_slices, slices * sc_slice_bytes()))) ||
         (p.flag == 2 && (dalloc(&d.sc_field, slices * 2 * p.nx * p.ny) ||
-                         dalloc(&d.sc_slice_of, (size_t)h.npad) || dalloc(&d.sc_list, (size_t)h.npad) ||
+                         dalloc(&d.sc_xy, 2 * (size_t)h.npad) ||
                          dalloc(&d.sc_start, slices) || dalloc(&d.sc_cursor, slices)))) {
       free_beam(h);
       return fail(&h, CG_ERR_OOM, "space-charge buffers");
     }
-    cudaMemset(d.sc_geom, 0, sizeof(double) * M * 11);
-    if (d.sc_acc) cudaMemset(d.sc_acc, 0, sizeof(unsigned long long) * slices * p.acc_per_slice);
+    cudaMemset(d.sc_geom, 0, sizeof(double) * M * kScGeom);
   }
   if (h.cfg.bbi.flag) {
     const size_t wc = h.bbi.wcap;

@@ -11,6 +11,7 @@ namespace cg {
 
 constexpr int kTile = 256;            // particles per tile == threads per CTA
 
+constexpr int kScGeom = 16;           // doubles per bunch of the space-charge geometry
 constexpr int kMaxChunkTiles = 8;     // most tiles per CTA of the map pass and the moments
 constexpr int kMaxPipeGroups = 16;    // segments of the pipelined ion pass
 
@@ -39,7 +40,6 @@ struct BbiParams {
 struct ScParams {
   int flag = 0;                // 1 Bassetti-Erskine slices, 2 2.5-D PIC, 3 linear
   int nx = 0, ny = 0, nz = 0;  // mesh nodes (PIC) and slices
-  int acc_per_slice = 0;       // accumulators per slice: nx ny (PIC) or 4
   double range = 10.0;         // mesh half-width in rms sizes (PIC3D.h:62, PIC3D.cpp:152)
   double p0 = 0;               // beta0 gamma0 of the reference particle (PIC2D.cpp)
 };
@@ -164,13 +164,14 @@ struct DeviceBufs {
   double* bbi_pot = nullptr;       // M x 6 x wcap: profile and potentials of the last kick
   int2* bbi_win = nullptr;         // M: first bin and bin count of bbi_pot
   // space charge
-  double* sc_geom = nullptr;       // M x 11: slices, mesh, fixed-point scales
+  double* sc_geom = nullptr;       // M x kScGeom: slices, mesh, fixed-point scales
+  unsigned long long* sc_range = nullptr;  // M x 4: z range, largest |x|, |y| (ordered bits)
   int* sc_cnt = nullptr;           // M x nz particles per slice
-  unsigned long long* sc_acc = nullptr;  // M x nz x acc_per_slice fixed-point sums
-  double* sc_field = nullptr;      // M x nz x 2 x nx x ny mesh field (PIC)
-  int* sc_slice_of = nullptr;      // npad: each particle's slice (PIC)
-  int* sc_list = nullptr;          // npad: particle indices grouped by bunch and slice (PIC)
-  int* sc_start = nullptr;         // M x nz: first list entry of each slice (PIC)
+  unsigned long long* sc_acc = nullptr;  // M x nz x 4 fixed-point sums (slice models)
+  double* sc_field = nullptr;      // M x nz x nx x ny x 2 mesh field (PIC)
+  unsigned char* sc_slices = nullptr;  // M x nz slice constants (slice models)
+  double* sc_xy = nullptr;         // npad x (x, y) grouped by bunch and slice (PIC)
+  int* sc_start = nullptr;         // M x nz: first entry of each slice (PIC)
   int* sc_cursor = nullptr;        // M x nz: fill cursors (PIC)
   double* sc_sin = nullptr;        // nx x nx + ny x ny: 2 sin(pi (i + 1)(k + 1) / (n + 1))
   // phase advance of the tracked bunches: slot per bunch (-1 untracked),

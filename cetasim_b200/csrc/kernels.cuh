@@ -25,6 +25,7 @@ cudaError_t launch_phase_adv(Handle& h, int ja, int jb, cudaStream_t s = nullptr
 // space charge (sc.cu)
 cudaError_t launch_space_charge(Handle& h, int k);
 size_t sc_solve_smem(const ScParams& p);
+size_t sc_slice_bytes();  // of one slice's constants (slice models)
 cudaError_t prepare_sc(const ScParams& p);
 
 // broadband impedance (bbi.cu)

@@ -16,20 +16,33 @@
 //   flag 3: the linear field of a uniform beam of those sizes (:764-831).
 // Every flag ends in the same momentum update (PIC2D.cpp, MPBunch.cpp:740-760).
 //
-//  k_sc_geom     one CTA per bunch: the survivors' z range (GetZMinMax,
-//                seeded with particle 0), the slice width, the mesh
-//                (PIC2D::Set2DMesh(rms, centroid), PIC2D.cpp), the largest
-//                |x|, |y| for the fixed-point scales.
-//  k_sc_deposit  per tile: slice counts; PIC: each particle's slice;
-//                analytic: per-slice sums of x and y in 64-bit fixed point
+//  k_sc_range    per chunk: the survivors' z range (GetZMinMax, seeded with
+//                particle 0) and the largest |x|, |y| (ordered bit patterns
+//                under atomics).
+//  k_sc_geom     per bunch: the slice width, the mesh (PIC2D::Set2DMesh(rms,
+//                centroid), PIC2D.cpp), the fixed-point scales.
+//  k_sc_count    per chunk: particles per slice in shared memory, then added to
+//                the bunch's; slice models: also the sums of x, y, x^2, y^2
+//                about the bunch centroid in 64-bit fixed point
 //                (order-independent sums under atomics).
-//  k_sc_offsets, k_sc_scatter (PIC): the particles grouped by slice.
-//  k_sc_second   per tile (analytic): per-slice sums of (x - <x>)^2, (y - <y>)^2.
+//  k_sc_slices   slice models: per slice the centroid, the sizes and the
+//                field's constants.
+//  k_sc_offsets, k_sc_scatter (PIC): the particles' x, y grouped by slice.
 //  k_sc_solve    one CTA per (bunch, slice) (PIC): the slice's cloud-in-cell
 //                charge in shared memory (fixed point), the DST-I Poisson
-//                solve as two matrix products each way, then the field on
-//                the mesh.
+//                solve as two matrix products each way on the FP64 tensor
+//                instructions, then the field on the mesh.
 //  k_sc_kick     per tile: the field at each particle and the kick.
+// Bound by: the passes over the particles by HBM and by shared-memory atomics,
+// the solve by its products and its barriers (one slice is a few hundred tile
+// products), the field models by the FP64 pipe.  A section of 80 bunches of
+// 20,000, us: PIC 32 x 32 x 33 468 -> 232 (solve 95, kick 41, scatter 25, range
+// and count 13 each, merge 12, geom 5, offsets 4, with the map pass's 46 in the
+// sum); Bassetti-Erskine slices 373 -> 143.  Before, the transforms were plain
+// FP64 dot products, the deposit went through 64-bit shared atomics
+// (compare-and-swap loops) from the whole bunch's particles, and the kick
+// evaluated w(z) through the general path.
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include "be_field.cuh"
@@ -43,68 +56,118 @@ constexpr double kEpsilon0 = 8.854187817E-12;  // Global.h:26
 constexpr double kElectronMassKg = 9.10938215E-31;
 
 // per-bunch geometry, sc_geom[b * kScGeom + ...]
-enum { kGZmin = 0, kGDz, kGMx0, kGMy0, kGHx, kGHy, kGDv, kGExp0, kGExp1, kGExp2, kGExp3, kScGeom };
+enum {
+  kGZmin = 0, kGDz, kGIDz, kGMx0, kGMy0, kGHx, kGHy, kGIHx, kGIHy, kGIDv,
+  kGExp0, kGExp1, kGExp2, kGExp3, kGPx, kGPy
+};
+static_assert(kGPy + 1 == kScGeom, "geometry record");
 
 __device__ __forceinline__ int sc_fix_exp(double amax, double n) {
   if (!(amax > 0) || isinf(amax)) return 0;
   const int nb = 32 - __clz((int)n);
   return 60 - ilogb(amax) - nb;
 }
-
-__device__ __forceinline__ double sc_block_reduce(double v, double* red, bool is_max) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double u = __shfl_xor_sync(SC_FULL, v, o);
-    v = is_max ? fmax(v, u) : fmin(v, u);
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = red[0];
-  for (int q = 1; q < kScThreads / 32; ++q) t = is_max ? fmax(t, red[q]) : fmin(t, red[q]);
-  return t;
+__device__ __forceinline__ double sc_fix(unsigned long long v, int e) {
+  return scalbn((double)(long long)v, -e);
 }
 
-__global__ void __launch_bounds__(kScThreads) k_sc_geom(const double* __restrict__ c, int64_t npad,
-                                                        const uint8_t* __restrict__ surv,
-                                                        const BunchDev* __restrict__ bunch,
-                                                        const BunchMomDev* __restrict__ mom,
-                                                        ScParams p, double* geom, int* status) {
-  __shared__ double red[kScThreads / 32];
-  const int b = blockIdx.x;
-  const BunchDev& Bd = bunch[b];
-  if (Bd.n < 1) return;
-  const int64_t g0 = (int64_t)Bd.tile_off * kTile;
-  const double z0 = c[4 * npad + g0];
-  double zmn = z0, zmx = z0, ax = 0, ay = 0;
-  for (int i = threadIdx.x; i < Bd.n; i += kScThreads) {
-    const int64_t g = g0 + i;
-    if (surv[g] == kAlive) {
-      const double z = c[4 * npad + g];
+// Doubles as integers in the same order (for atomicMin / atomicMax).
+__device__ __forceinline__ unsigned long long sc_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return (unsigned long long)b ^ (b < 0 ? ~0ull : 1ull << 63);
+}
+__device__ __forceinline__ double sc_unkey(unsigned long long k) {
+  return __longlong_as_double((long long)(k ^ (k >> 63 ? 1ull << 63 : ~0ull)));
+}
+
+// range[4 b ..]: keys of the survivors' lowest and highest z (particle 0 not
+// yet in them), bit patterns of the largest |x|, |y|.
+__global__ void k_sc_clear(unsigned long long* range, int* cnt, unsigned long long* acc, int M,
+                           int nz, int per) {
+  const int n = M * nz;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    cnt[i] = 0;
+    for (int q = 0; q < per; ++q) acc[(size_t)i * per + q] = 0ull;
+  }
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < M; b += gridDim.x * blockDim.x) {
+    range[4 * b] = sc_key(INFINITY);
+    range[4 * b + 1] = sc_key(-INFINITY);
+    range[4 * b + 2] = range[4 * b + 3] = 0ull;
+  }
+}
+
+template <bool XY>
+__global__ void __launch_bounds__(kScThreads) k_sc_range(const double* __restrict__ c, int64_t npad,
+                                                         const uint8_t* __restrict__ surv,
+                                                         const int4* __restrict__ chunk_loc,
+                                                         unsigned long long* range) {
+  __shared__ double red[4][kScThreads / 32];
+  const int4 l = chunk_loc[blockIdx.x];
+  double zmn = INFINITY, zmx = -INFINITY, ax = 0, ay = 0;
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
+  for (int u = 0; u < l.z; ++u, g += kTile) {
+    const uint8_t s = surv[g];
+    if (s == kPadding) break;  // the tail of the bunch's last tile
+    const double z = c[4 * npad + g];
+    if (s == kAlive) {
       zmn = fmin(zmn, z);
       zmx = fmax(zmx, z);
     }
-    ax = fmax(ax, fabs(c[g]));
-    ay = fmax(ay, fabs(c[2 * npad + g]));
+    if (XY) {
+      ax = fmax(ax, fabs(c[g]));
+      ay = fmax(ay, fabs(c[2 * npad + g]));
+    }
   }
-  zmn = sc_block_reduce(zmn, red, false);
-  zmx = sc_block_reduce(zmx, red, true);
-  ax = sc_block_reduce(ax, red, true);
-  ay = sc_block_reduce(ay, red, true);
-  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    zmn = fmin(zmn, __shfl_xor_sync(SC_FULL, zmn, o));
+    zmx = fmax(zmx, __shfl_xor_sync(SC_FULL, zmx, o));
+    if (XY) {
+      ax = fmax(ax, __shfl_xor_sync(SC_FULL, ax, o));
+      ay = fmax(ay, __shfl_xor_sync(SC_FULL, ay, o));
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = zmn;
+    red[1][threadIdx.x >> 5] = zmx;
+    red[2][threadIdx.x >> 5] = ax;
+    red[3][threadIdx.x >> 5] = ay;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 4) return;
+  double v = red[threadIdx.x][0];
+  for (int w = 1; w < kScThreads / 32; ++w)
+    v = threadIdx.x == 0 ? fmin(v, red[0][w]) : fmax(v, red[threadIdx.x][w]);
+  unsigned long long* r = range + 4 * (size_t)l.x + threadIdx.x;
+  if (threadIdx.x == 0) atomicMin(r, sc_key(v));
+  else if (threadIdx.x == 1) atomicMax(r, sc_key(v));
+  else if (XY) atomicMax(r, (unsigned long long)__double_as_longlong(v));
+}
+
+__global__ void k_sc_geom(const double* __restrict__ c, int64_t npad,
+                          const BunchDev* __restrict__ bunch, const BunchMomDev* __restrict__ mom,
+                          ScParams p, const unsigned long long* __restrict__ range, double* geom,
+                          int* status, int M) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= M) return;
+  const BunchDev& Bd = bunch[b];
+  if (Bd.n < 1) return;
+  const double z0 = c[4 * npad + (int64_t)Bd.tile_off * kTile];
+  const double zmn = fmin(z0, sc_unkey(range[4 * b])), zmx = fmax(z0, sc_unkey(range[4 * b + 1]));
   double* G = geom + (size_t)b * kScGeom;
   // GetZMinMax (MPBunch.cpp:1883-1884) and SetSlicedBunchInfo (:670)
   const double zMin = zmn - 1.e-6, zMax = zmx + 1.e-6;
   G[kGZmin] = zMin;
   G[kGDz] = (zMax - zMin) / (p.nz - 1);
+  G[kGIDz] = 1.0 / G[kGDz];
   const double charge = Bd.q_macro * kElectronCharge / G[kGDz];  // [C/m], MPBunch.cpp:689
+  const BunchMomDev& m = mom[b];
   if (p.flag == 2) {
     // PIC2D::Set2DMesh(rmsXY, averXY) (PIC2D.cpp) from the moments of this section
-    const BunchMomDev& m = mom[b];
     const double rms[2] = {m.rms_x, m.rms_y}, cen[2] = {m.mean[0], m.mean[2]};
     if (rms[0] == 0 || rms[1] == 0) {
       atomicOr(status, kStatusScMesh);  // MPBunch.cpp:893-897
-      G[kGDv] = 0;
+      G[kGIDv] = 0;
       return;
     }
     double len[2];
@@ -115,142 +178,242 @@ __global__ void __launch_bounds__(kScThreads) k_sc_geom(const double* __restrict
     for (int q = 0; q < 2; ++q) {
       const double w = lmax / (n[q] - 1);
       G[q ? kGHy : kGHx] = w;
+      G[q ? kGIHy : kGIHx] = 1.0 / w;
       G[q ? kGMy0 : kGMx0] = cen[q] - lmax / 2;
       dv *= w;
     }
-    G[kGDv] = dv;
+    G[kGIDv] = 1.0 / dv;
     // a deposit is at most charge / dv (weights <= 1)
     G[kGExp0] = sc_fix_exp(charge / dv, Bd.n);
   } else {
+    // the sums' pivot: the bunch centroid (zero if there is none)
+    const double px = isfinite(m.mean[0]) ? m.mean[0] : 0.0;
+    const double py = isfinite(m.mean[2]) ? m.mean[2] : 0.0;
+    const double ax = __longlong_as_double((long long)range[4 * b + 2]) + fabs(px);
+    const double ay = __longlong_as_double((long long)range[4 * b + 3]) + fabs(py);
+    G[kGPx] = px;
+    G[kGPy] = py;
     G[kGExp0] = sc_fix_exp(ax, Bd.n);
     G[kGExp1] = sc_fix_exp(ay, Bd.n);
-    G[kGExp2] = sc_fix_exp(4 * ax * ax, Bd.n);
-    G[kGExp3] = sc_fix_exp(4 * ay * ay, Bd.n);
+    G[kGExp2] = sc_fix_exp(ax * ax, Bd.n);
+    G[kGExp3] = sc_fix_exp(ay * ay, Bd.n);
   }
 }
 
 // slice of a particle (MPBunch.cpp:679-681)
 __device__ __forceinline__ int sc_slice(double z, const double* G, int nz) {
-  const double t = floor((z - G[kGZmin]) / G[kGDz]);
+  const double t = floor((z - G[kGZmin]) * G[kGIDz]);
   return t < 0 ? 0 : (t > nz - 1 ? nz - 1 : (int)t);
 }
 
-// mesh cell and cloud-in-cell weights (PIC2D::Set2DRho, PIC2D.cpp); false
-// when the particle is outside the mesh
+// mesh cell and cloud-in-cell distances (PIC2D::Set2DRho, PIC2D.cpp: the
+// weights times the cell's area); false when the particle is outside the mesh
 __device__ __forceinline__ bool sc_cell(double x, double y, const double* G, const ScParams& p,
                                         int* ix, int* iy, double w[4]) {
-  const double tx = floor((x - G[kGMx0]) / G[kGHx]);
-  const double ty = floor((y - G[kGMy0]) / G[kGHy]);
+  const double tx = floor((x - G[kGMx0]) * G[kGIHx]);
+  const double ty = floor((y - G[kGMy0]) * G[kGIHy]);
   if (!(tx >= 0 && tx < p.nx - 1 && ty >= 0 && ty < p.ny - 1)) return false;
   *ix = (int)tx;
   *iy = (int)ty;
-  for (int j = 0; j < 4; ++j) {
-    const int dx = (j % 2 == 0) ? 1 : 0, dy = (j % 4 < 2) ? 1 : 0;
-    const double mx = G[kGMx0] + G[kGHx] * (*ix + dx);
-    const double my = G[kGMy0] + G[kGHy] * (*iy + dy);
-    w[j] = fabs(x - mx) * fabs(y - my) / G[kGDv];
-  }
+  const double x1 = fabs(x - (G[kGMx0] + G[kGHx] * (*ix + 1))), x0 = fabs(x - (G[kGMx0] + G[kGHx] * *ix));
+  const double y1 = fabs(y - (G[kGMy0] + G[kGHy] * (*iy + 1))), y0 = fabs(y - (G[kGMy0] + G[kGHy] * *iy));
+  w[0] = x1 * y1;
+  w[1] = x0 * y1;
+  w[2] = x1 * y0;
+  w[3] = x0 * y0;
   return true;
 }
 
-__global__ void __launch_bounds__(kTile) k_sc_deposit(const double* __restrict__ c, int64_t npad,
-                                                      const int* __restrict__ tile_bunch,
-                                                      const BunchDev* __restrict__ bunch,
-                                                      ScParams p, const double* __restrict__ geom,
-                                                      int* cnt, unsigned long long* acc,
-                                                      int* slice_of) {
-  const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  if (i >= Bd.n) return;
-  const double* G = geom + (size_t)b * kScGeom;
-  if (p.flag == 2 && G[kGDv] == 0) return;
-  const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int s = sc_slice(c[4 * npad + g], G, p.nz);
-  const size_t bs = (size_t)b * p.nz + s;
-  atomicAdd(&cnt[bs], 1);
-  if (p.flag == 2) {
-    slice_of[g] = s;  // the slice's CTA deposits its particles (k_sc_solve)
-  } else {
-    const double x = c[g], y = c[2 * npad + g];
-    unsigned long long* A = acc + bs * p.acc_per_slice;
-    atomicAdd(&A[0], (unsigned long long)__double2ll_rn(scalbn(x, (int)G[kGExp0])));
-    atomicAdd(&A[1], (unsigned long long)__double2ll_rn(scalbn(y, (int)G[kGExp1])));
+// A 64-bit sum in shared memory as two words (a 64-bit shared atomic is a
+// compare-and-swap loop, which retries under contention; the carry of a 32-bit
+// add is exact).
+__device__ __forceinline__ void sc_add64(unsigned* lo, unsigned* hi, long long v) {
+  const unsigned vl = (unsigned)v, old = atomicAdd(lo, vl);
+  const unsigned vh = (unsigned)((unsigned long long)v >> 32) + (old + vl < vl ? 1u : 0u);
+  if (vh) atomicAdd(hi, vh);
+}
+
+// Slices up to which a CTA keeps its counts (and the models' sums) in shared
+// memory; beyond, it adds to the bunch's directly.
+constexpr int kScSharedSlices = 1024;
+
+template <bool PIC>
+__global__ void __launch_bounds__(kScThreads) k_sc_count(const double* __restrict__ c, int64_t npad,
+                                                         const uint8_t* __restrict__ surv,
+                                                         const int4* __restrict__ chunk_loc,
+                                                         ScParams p, const double* __restrict__ geom,
+                                                         int* cnt, unsigned long long* acc) {
+  extern __shared__ unsigned s_sum[];  // nz counts; models: then 4 x (lo, hi) x nz
+  const int4 l = chunk_loc[blockIdx.x];
+  const double* G = geom + (size_t)l.x * kScGeom;
+  if (PIC && G[kGIDv] == 0) return;
+  const int nz = p.nz;
+  const bool shared = nz <= kScSharedSlices;
+  if (shared) {
+    for (int i = threadIdx.x; i < nz * (PIC ? 1 : 9); i += kScThreads) s_sum[i] = 0u;
+    __syncthreads();
+  }
+  const size_t b0 = (size_t)l.x * nz;
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
+  for (int u = 0; u < l.z; ++u, g += kTile) {
+    if (surv[g] == kPadding) break;
+    const int s = sc_slice(c[4 * npad + g], G, nz);
+    if (shared) atomicAdd(&s_sum[s], 1u);
+    else atomicAdd(&cnt[b0 + s], 1);
+    if (!PIC) {
+      const double dx = c[g] - G[kGPx], dy = c[2 * npad + g] - G[kGPy];
+      const double v[4] = {dx, dy, dx * dx, dy * dy};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long t = __double2ll_rn(scalbn(v[q], (int)G[kGExp0 + q]));
+        if (shared) sc_add64(&s_sum[(1 + 2 * q) * nz + s], &s_sum[(2 + 2 * q) * nz + s], t);
+        else atomicAdd(&acc[(b0 + s) * 4 + q], (unsigned long long)t);
+      }
+    }
+  }
+  if (!shared) return;
+  __syncthreads();
+  for (int s = threadIdx.x; s < nz; s += kScThreads) {
+    if (!s_sum[s]) continue;
+    atomicAdd(&cnt[b0 + s], (int)s_sum[s]);
+    if (!PIC)
+      for (int q = 0; q < 4; ++q)
+        atomicAdd(&acc[(b0 + s) * 4 + q],
+                  (unsigned long long)s_sum[(2 + 2 * q) * nz + s] << 32 | s_sum[(1 + 2 * q) * nz + s]);
   }
 }
 
-__device__ __forceinline__ double sc_fix(unsigned long long v, int e) {
-  return scalbn((double)(long long)v, -e);
+// Slice models: one slice as the kick reads it.
+struct ScSlice {
+  double cx, cy, rx, ry;  // centroid, sizes
+  double lambda;          // line charge over pi epsilon0
+  KickConst k;            // flag 1: the field's constants, in the frame of the larger axis
+};
+
+__global__ void k_sc_slices(ScParams p, const BunchDev* __restrict__ bunch,
+                            const double* __restrict__ geom, const int* __restrict__ cnt,
+                            const unsigned long long* __restrict__ acc, ScSlice* slices, int M) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= M * p.nz) return;
+  const int b = i / p.nz, n = cnt[i];
+  if (n < 2) return;
+  const double* G = geom + (size_t)b * kScGeom;
+  const unsigned long long* A = acc + 4 * (size_t)i;
+  const double mx = sc_fix(A[0], (int)G[kGExp0]) / n, my = sc_fix(A[1], (int)G[kGExp1]) / n;
+  ScSlice s;
+  s.cx = G[kGPx] + mx;
+  s.cy = G[kGPy] + my;
+  s.rx = sqrt(fmax(sc_fix(A[2], (int)G[kGExp2]) / n - mx * mx, 0.0));
+  s.ry = sqrt(fmax(sc_fix(A[3], (int)G[kGExp3]) / n - my * my, 0.0));
+  s.lambda = n * (bunch[b].q_macro * kElectronCharge / G[kGDz]) / kPi / kEpsilon0;  // n charge: [C/m]
+  CloudRec r;
+  r.coeff = -0.5 * s.lambda;
+  r.rms_x = s.rx;
+  r.rms_y = s.ry;
+  r.aver_x = s.cx;
+  r.aver_y = s.cy;
+  r.count = n;
+  s.k = kick_const(r, field_prep(s.rx, s.ry));
+  slices[i] = s;
 }
 
-// PIC: each bunch's particles grouped by slice (a counting sort: the
-// slices' starts, then every particle's index at its slice's cursor), so
-// that one CTA per slice deposits its own particles in shared memory
+// PIC: each bunch's particles grouped by slice (a counting sort: the slices'
+// starts, then every particle's x, y at its slice's cursor), so that one CTA
+// per slice deposits its own particles in shared memory.  One warp per bunch.
 __global__ void k_sc_offsets(const BunchDev* __restrict__ bunch, int nz, const int* __restrict__ cnt,
-                             int* start, int* cursor, int M) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= M) return;
-  int pos = bunch[b].tile_off * kTile;
-  for (int s = 0; s < nz; ++s) {
-    start[(size_t)b * nz + s] = pos;
-    cursor[(size_t)b * nz + s] = pos;
-    pos += cnt[(size_t)b * nz + s];
+                             int* start, int* cursor) {
+  const int b = blockIdx.x, lane = threadIdx.x;
+  int base = bunch[b].tile_off * kTile;
+  for (int s0 = 0; s0 < nz; s0 += 32) {
+    const int s = s0 + lane, n = s < nz ? cnt[(size_t)b * nz + s] : 0;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(SC_FULL, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (s < nz) start[(size_t)b * nz + s] = cursor[(size_t)b * nz + s] = base + inc - n;
+    base += __shfl_sync(SC_FULL, inc, 31);
   }
 }
 
-__global__ void __launch_bounds__(kTile) k_sc_scatter(const int* __restrict__ tile_bunch,
-                                                      const BunchDev* __restrict__ bunch, int nz,
-                                                      const double* __restrict__ geom,
-                                                      const int* __restrict__ slice_of, int* cursor,
-                                                      int* list) {
-  const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const bool in = i < Bd.n && geom[(size_t)b * kScGeom + kGDv] != 0;
-  const int key = in ? b * nz + slice_of[g] : -1;
-  // one cursor increment per slice and warp
-  const unsigned peers = __match_any_sync(SC_FULL, key);
-  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-  int base = 0;
-  if (in && lane == leader) base = atomicAdd(&cursor[key], __popc(peers));
-  base = __shfl_sync(SC_FULL, base, leader);
-  if (in) list[base + __popc(peers & ((1u << lane) - 1u))] = (int)g;
+__global__ void __launch_bounds__(kScThreads) k_sc_scatter(const double* __restrict__ c, int64_t npad,
+                                                           const uint8_t* __restrict__ surv,
+                                                           const int4* __restrict__ chunk_loc,
+                                                           ScParams p,
+                                                           const double* __restrict__ geom,
+                                                           int* cursor, double2* xy) {
+  extern __shared__ unsigned s_sum[];  // nz counts, then nz first places
+  const int4 l = chunk_loc[blockIdx.x];
+  const double* G = geom + (size_t)l.x * kScGeom;
+  if (G[kGIDv] == 0) return;
+  const int nz = p.nz;
+  const bool shared = nz <= kScSharedSlices;
+  const size_t b0 = (size_t)l.x * nz;
+  const int64_t g0 = (int64_t)l.y * kTile + threadIdx.x;
+  unsigned rank[kMaxChunkTiles];
+  if (shared) {
+    // the chunk's places in each slice with one global atomic per slice
+    for (int i = threadIdx.x; i < nz; i += kScThreads) s_sum[i] = 0u;
+    __syncthreads();
+    for (int u0 = 0; u0 < l.z; u0 += kMaxChunkTiles) {
+      const int nu = min(kMaxChunkTiles, l.z - u0);
+#pragma unroll
+      for (int u = 0; u < kMaxChunkTiles; ++u) {
+        const int64_t g = g0 + (int64_t)(u0 + u) * kTile;
+        if (u < nu && surv[g] != kPadding) rank[u] = atomicAdd(&s_sum[sc_slice(c[4 * npad + g], G, nz)], 1u);
+      }
+      __syncthreads();
+      for (int s = threadIdx.x; s < nz; s += kScThreads) {
+        s_sum[nz + s] = s_sum[s] ? (unsigned)atomicAdd(&cursor[b0 + s], (int)s_sum[s]) : 0u;
+        s_sum[s] = 0u;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kMaxChunkTiles; ++u) {
+        const int64_t g = g0 + (int64_t)(u0 + u) * kTile;
+        if (u < nu && surv[g] != kPadding)
+          xy[s_sum[nz + sc_slice(c[4 * npad + g], G, nz)] + rank[u]] = make_double2(c[g], c[2 * npad + g]);
+      }
+      __syncthreads();
+    }
+  } else {
+    for (int u = 0; u < l.z; ++u) {
+      const int64_t g = g0 + (int64_t)u * kTile;
+      if (surv[g] != kPadding)
+        xy[atomicAdd(&cursor[b0 + sc_slice(c[4 * npad + g], G, nz)], 1)] = make_double2(c[g], c[2 * npad + g]);
+    }
+  }
 }
 
-// analytic models: second pass, (x - <x>)^2 and (y - <y>)^2 per slice
-__global__ void __launch_bounds__(kTile) k_sc_second(const double* __restrict__ c, int64_t npad,
-                                                     const int* __restrict__ tile_bunch,
-                                                     const BunchDev* __restrict__ bunch,
-                                                     ScParams p, const double* __restrict__ geom,
-                                                     const int* __restrict__ cnt,
-                                                     unsigned long long* acc) {
-  const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  if (i >= Bd.n) return;
-  const double* G = geom + (size_t)b * kScGeom;
-  const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int s = sc_slice(c[4 * npad + g], G, p.nz);
-  const size_t bs = (size_t)b * p.nz + s;
-  unsigned long long* A = acc + bs * p.acc_per_slice;
-  const double n = cnt[bs];
-  const double cx = sc_fix(A[0], (int)G[kGExp0]) / n, cy = sc_fix(A[1], (int)G[kGExp1]) / n;
-  const double dx = c[g] - cx, dy = c[2 * npad + g] - cy;
-  atomicAdd(&A[2], (unsigned long long)__double2ll_rn(scalbn(dx * dx, (int)G[kGExp2])));
-  atomicAdd(&A[3], (unsigned long long)__double2ll_rn(scalbn(dy * dy, (int)G[kGExp3])));
+// D = A B on the FP64 tensor instructions (m8n8k4): one 8 x 8 tile of the
+// product of A (rows, K) and B (K, columns), both row by row in shared memory
+// with a row stride of 4 or 12 modulo 16 doubles (no bank conflicts).  Lane l
+// gets the elements (l / 4, 2 (l % 4)) and the next.
+__device__ __forceinline__ void sc_mma_tile(const double* A, int lda, const double* B, int ldb, int K,
+                                            double (&d)[2]) {
+  const int lane = threadIdx.x & 31;
+  const double* a = A + (lane >> 2) * lda + (lane & 3);
+  const double* b = B + (lane & 3) * ldb + (lane >> 2);
+  d[0] = d[1] = 0.0;
+  for (int k = 0; k < K; k += 4) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a[k]), "d"(b[k * ldb]));
+  }
 }
+
+__host__ __device__ inline int sc_pad(int n) { return (n + 7) / 8 * 8; }
 
 // One CTA per (bunch, slice): PIC2D::Set2DPhi and Set2DEField (PIC2D.cpp).
 // The 2-D DST-I (RODFT00, Y_k = 2 sum_j X_j sin(pi (j + 1)(k + 1) / (n + 1))
-// along each axis) as S_x R S_y^T in shared memory; sx, sy hold 2 sin(...).
-__global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const double* __restrict__ c,
-                                                         int64_t npad,
-                                                         const BunchDev* __restrict__ bunch,
+// along each axis) as S_x R S_y^T in shared memory; sx, sy hold 2 sin(...),
+// the mesh padded with zeros to whole 8 x 8 tiles.
+__global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const BunchDev* __restrict__ bunch,
                                                          const double* __restrict__ geom,
                                                          const int* __restrict__ cnt,
                                                          const int* __restrict__ start,
-                                                         const int* __restrict__ list,
+                                                         const double2* __restrict__ xy,
                                                          const double* __restrict__ sxy,
                                                          double* field) {
   extern __shared__ double sm[];
@@ -259,169 +422,172 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const doubl
   const size_t bs = blockIdx.x;
   const double* G = geom + (size_t)b * kScGeom;
   const int n = cnt[bs];
-  if (n < 2 || G[kGDv] == 0) return;  // a skipped slice (MPBunch.cpp:916)
-  double* R = sm;
-  double* T = sm + N;
-  double* Sx = sm + 2 * N;
-  double* Sy = Sx + nx * nx;
-  unsigned long long* S = reinterpret_cast<unsigned long long*>(Sy + ny * ny);
+  if (n < 2 || G[kGIDv] == 0) return;  // a skipped slice (MPBunch.cpp:916)
+  const int px = sc_pad(nx), py = sc_pad(ny), lx = px + 4, ly = py + 4;
+  double* R = sm;                // px x ly
+  double* T = R + px * ly;       // px x ly
+  double* Sx = T + px * ly;      // px x lx
+  double* Sy = Sx + px * lx;     // py x ly
+  unsigned* lo = reinterpret_cast<unsigned*>(T);  // the fixed-point charge, in T's place
+  unsigned* hi = lo + N;
   const int e = (int)G[kGExp0];
-  for (int t = threadIdx.x; t < N; t += kScThreads) S[t] = 0ull;
+  for (int t = threadIdx.x; t < 2 * N; t += kScThreads) lo[t] = 0u;
+  for (int t = threadIdx.x; t < px * lx; t += kScThreads) {
+    const int i = t / lx, k = t % lx;
+    Sx[t] = i < nx && k < nx ? sxy[i * nx + k] : 0.0;
+  }
+  for (int t = threadIdx.x; t < py * ly; t += kScThreads) {
+    const int i = t / ly, k = t % ly;
+    Sy[t] = i < ny && k < ny ? sxy[nx * nx + i * ny + k] : 0.0;
+  }
   __syncthreads();
   // PIC2D::Set2DRho (PIC2D.cpp): cloud-in-cell charge [C/m^3] of the slice's
   // particles, in 64-bit fixed point (order-independent)
   const double charge = bunch[b].q_macro * kElectronCharge / G[kGDz];
-  const int* L = list + start[bs];
+  const double unit = scalbn(charge * G[kGIDv] * G[kGIDv], e);
+  const double2* L = xy + start[bs];
   for (int t = threadIdx.x; t < n; t += kScThreads) {
-    const int64_t g = L[t];
+    const double2 v = L[t];
     int ix, iy;
     double w[4];
-    if (!sc_cell(c[g], c[2 * npad + g], G, p, &ix, &iy, w)) continue;
+    if (!sc_cell(v.x, v.y, G, p, &ix, &iy, w)) continue;
     const int node[4] = {ix * ny + iy, (ix + 1) * ny + iy, ix * ny + iy + 1, (ix + 1) * ny + iy + 1};
-    for (int j = 0; j < 4; ++j) {
-      const double v = w[j] * charge / G[kGDv];
-      atomicAdd(&S[node[j]], (unsigned long long)__double2ll_rn(scalbn(v, e)));
-    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sc_add64(&lo[node[j]], &hi[node[j]], __double2ll_rn(w[j] * unit));
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < N; t += kScThreads) R[t] = sc_fix(S[t], e);
-  for (int t = threadIdx.x; t < nx * nx; t += kScThreads) Sx[t] = sxy[t];
-  for (int t = threadIdx.x; t < ny * ny; t += kScThreads) Sy[t] = sxy[nx * nx + t];
+  for (int t = threadIdx.x; t < px * ly; t += kScThreads) {
+    const int i = t / ly, j = t % ly;
+    R[t] = i < nx && j < ny
+               ? sc_fix((unsigned long long)hi[i * ny + j] << 32 | lo[i * ny + j], e)
+               : 0.0;
+  }
   __syncthreads();
   const double hx = G[kGHx], hy = G[kGHy];
   const double* __restrict__ eig = sxy + nx * nx + ny * ny;
-  // A thread keeps four rows k0..k0+3 of one column: the column's element
-  // is loaded once for the four sums (rows past the mesh are clamped for the
-  // loads and not stored); every sum runs in the index order of a plain
-  // product, so the results do not depend on the grouping.
-  const int groups = ny * ((nx + 3) / 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tx = px / 8, ty = py / 8, tiles = tx * ty;
   for (int pass = 0; pass < 2; ++pass) {
-    // T = Sx R (along x)
-    for (int q = threadIdx.x; q < groups; q += kScThreads) {
-      const int j = q % ny, k0 = (q / ny) * 4;
-      const int k1 = min(k0 + 1, nx - 1), k2 = min(k0 + 2, nx - 1), k3 = min(k0 + 3, nx - 1);
-      double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-      for (int i = 0; i < nx; ++i) {
-        const double r = R[i * ny + j];
-        s0 = fma(Sx[k0 * nx + i], r, s0);
-        s1 = fma(Sx[k1 * nx + i], r, s1);
-        s2 = fma(Sx[k2 * nx + i], r, s2);
-        s3 = fma(Sx[k3 * nx + i], r, s3);
-      }
-      T[k0 * ny + j] = s0;
-      if (k0 + 1 < nx) T[k1 * ny + j] = s1;
-      if (k0 + 2 < nx) T[k2 * ny + j] = s2;
-      if (k0 + 3 < nx) T[k3 * ny + j] = s3;
+    for (int q = warp; q < tiles; q += kScThreads / 32) {  // T = Sx R (along x)
+      const int i = q / ty * 8, j = q % ty * 8;
+      double d[2];
+      sc_mma_tile(Sx + i * lx, lx, R + j, ly, px, d);
+      double* o = T + (i + (lane >> 2)) * ly + j + 2 * (lane & 3);
+      o[0] = d[0];
+      o[1] = d[1];
     }
     __syncthreads();
-    // R = T Sy^T (along y); the DST-I matrix is symmetric, Sy[j][l] =
-    // Sy[l][j], so it is read along the lanes' l (distinct banks)
-    for (int q = threadIdx.x; q < groups; q += kScThreads) {
-      const int l = q % ny, k0 = (q / ny) * 4;
-      const int kk[4] = {k0, min(k0 + 1, nx - 1), min(k0 + 2, nx - 1), min(k0 + 3, nx - 1)};
-      double sum[4] = {0, 0, 0, 0};
-      for (int j = 0; j < ny; ++j) {
-        const double y = Sy[j * ny + l];
+    for (int q = warp; q < tiles; q += kScThreads / 32) {  // R = T Sy^T (along y; Sy is symmetric)
+      const int i = q / ty * 8, j = q % ty * 8;
+      double d[2];
+      sc_mma_tile(T + i * ly, ly, Sy + j, ly, py, d);
+      const int k = i + (lane >> 2);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sum[u] = fma(T[kk[u] * ny + j], y, sum[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (k0 + u >= nx) break;
-        const int k = kk[u], t = k * ny + l;
-        if (pass == 0) {
-          // the Laplacian's eigenvalue (PIC2D.cpp Set2DPhi): out / K / Epsilon,
-          // with the sines of pi / 2 (k + 1) / (n + 1) from the table
-          const double ax = 2 * eig[k] / hx, ay = 2 * eig[nx + l] / hy;
-          const double K = ax * ax + ay * ay;
-          R[t] = sum[u] / K / kEpsilon0;
-        } else {
-          R[t] = sum[u] / (4.0 * (nx + 1) * (ny + 1));  // phi [V]
+      for (int u = 0; u < 2; ++u) {
+        const int m = j + 2 * (lane & 3) + u;
+        double v = 0.0;
+        if (k < nx && m < ny) {
+          if (pass == 0) {
+            // the Laplacian's eigenvalue (PIC2D.cpp Set2DPhi): out / K / Epsilon,
+            // with the sines of pi / 2 (k + 1) / (n + 1) from the table
+            const double ax = 2 * eig[k] / hx, ay = 2 * eig[nx + m] / hy;
+            v = d[u] / (ax * ax + ay * ay) / kEpsilon0;
+          } else {
+            v = d[u] / (4.0 * (nx + 1) * (ny + 1));  // phi [V]
+          }
         }
+        R[k * ly + m] = v;
       }
     }
     __syncthreads();
   }
   // Set2DEField: central differences, zero potential beyond the mesh
   double* F = field + bs * 2 * N;
+  const double fx = -0.5 / hx, fy = -0.5 / hy;
   for (int t = threadIdx.x; t < N; t += kScThreads) {
     const int i = t / ny, j = t % ny;
-    const double x1 = i == 0 ? 0 : R[(i - 1) * ny + j], x2 = i == nx - 1 ? 0 : R[(i + 1) * ny + j];
-    const double y1 = j == 0 ? 0 : R[i * ny + j - 1], y2 = j == ny - 1 ? 0 : R[i * ny + j + 1];
-    F[t] = -(x2 - x1) / (2 * hx);
-    F[N + t] = -(y2 - y1) / (2 * hy);
+    const double x1 = i == 0 ? 0 : R[(i - 1) * ly + j], x2 = i == nx - 1 ? 0 : R[(i + 1) * ly + j];
+    const double y1 = j == 0 ? 0 : R[i * ly + j - 1], y2 = j == ny - 1 ? 0 : R[i * ly + j + 1];
+    reinterpret_cast<double2*>(F)[t] = make_double2((x2 - x1) * fx, (y2 - y1) * fy);
   }
 }
 
+// A point beyond the series' range or a round slice, out of line.
+__device__ __noinline__ void sc_field_any(const ScSlice& s, double posx, double posy, double* fx,
+                                          double* fy) {
+  if ((s.rx - s.ry) / s.ry > 1.e-4) bassetti_erskine(posx, posy, s.rx, s.ry, fx, fy);
+  else if ((s.rx - s.ry) / s.ry < -1.e-4) bassetti_erskine(posy, posx, s.ry, s.rx, fy, fx);
+  else gaussian_round_field(posx, posy, s.rx, fx, fy);
+}
+
 // The kick (PIC2D::SetPartSCField / UpdateTransverseMomentum, PIC2D.cpp;
-// MPBunch.cpp:713-760 and 781-829), in the reference's operation order; its
-// total momentum is formed from (delta, y, px) as there.
+// MPBunch.cpp:713-760 and 781-829); its total momentum p is formed from
+// (delta, y, px) as there, and E / gamma^2 e ds / (beta c) / (m p c) is
+// evaluated as E e ds / (m c^2) / (gamma p^2).
+template <int FLAG>
 __global__ void __launch_bounds__(kTile) k_sc_kick(double* __restrict__ c, int64_t npad,
-                                                   const int* __restrict__ tile_bunch,
-                                                   const BunchDev* __restrict__ bunch, ScParams p,
+                                                   const uint8_t* __restrict__ surv,
+                                                   const int* __restrict__ tile_bunch, ScParams p,
                                                    const double* __restrict__ geom,
                                                    const int* __restrict__ cnt,
-                                                   const unsigned long long* __restrict__ acc,
+                                                   const ScSlice* __restrict__ slices,
                                                    const double* __restrict__ field, double ds) {
   const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  if (i >= Bd.n) return;
-  const double* G = geom + (size_t)b * kScGeom;
-  if (p.flag == 2 && G[kGDv] == 0) return;
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int s = sc_slice(c[4 * npad + g], G, p.nz);
+  if (surv[g] == kPadding) return;
+  const double* G = geom + (size_t)b * kScGeom;
+  if (FLAG == 2 && G[kGIDv] == 0) return;
+  const double z = c[4 * npad + g], x = c[g], y = c[2 * npad + g];
+  const double px0 = c[npad + g], py0 = c[3 * npad + g], dp = c[5 * npad + g];
+  const int s = sc_slice(z, G, p.nz);
   const size_t bs = (size_t)b * p.nz + s;
-  const int n = cnt[bs];
-  if (n < 2) return;  // MPBunch.cpp:916
-  const double x = c[g], y = c[2 * npad + g];
+  if (cnt[bs] < 2) return;  // MPBunch.cpp:916
   double ex = 0, ey = 0;
-  if (p.flag == 2) {
+  if (FLAG == 2) {
     int ix, iy;
     double w[4];
     if (sc_cell(x, y, G, p, &ix, &iy, w)) {
-      const int N = p.nx * p.ny;
-      const double* F = field + bs * 2 * N;
-      const int n0 = ix * p.ny + iy, n1 = (ix + 1) * p.ny + iy, n2 = ix * p.ny + iy + 1,
-                n3 = (ix + 1) * p.ny + iy + 1;
-      ex = F[n0] * w[0] + F[n1] * w[1] + F[n2] * w[2] + F[n3] * w[3];
-      ey = F[N + n0] * w[0] + F[N + n1] * w[1] + F[N + n2] * w[2] + F[N + n3] * w[3];
+      const double2* F = reinterpret_cast<const double2*>(field) + bs * p.nx * p.ny;
+      const int n0 = ix * p.ny + iy;
+      const double2 f0 = F[n0], f1 = F[n0 + p.ny], f2 = F[n0 + 1], f3 = F[n0 + p.ny + 1];
+      ex = (f0.x * w[0] + f1.x * w[1] + f2.x * w[2] + f3.x * w[3]) * G[kGIDv];
+      ey = (f0.y * w[0] + f1.y * w[1] + f2.y * w[2] + f3.y * w[3]) * G[kGIDv];
+    }
+  } else if (FLAG == 1) {
+    const ScSlice& S = slices[bs];
+    const KickConst& k = S.k;
+    const bool sw = k.mode == 1;
+    const double da = (sw ? y : x) - k.ma, db = (sw ? x : y) - k.mb;
+    const double aa = fabs(da), ab = fabs(db);
+    const double zr[2] = {aa * k.s0, aa * k.sa1}, zi[2] = {ab * k.s0, ab * k.sb1};
+    constexpr int kHi21 = 0x40350000;  // |z| < 30 in both series (see ion_kick_particle)
+    if (k.mode != 2 && __double2hiint(zr[0]) < kHi21 && __double2hiint(zi[1]) < kHi21) {
+      const double ua = aa * k.ga, ub = ab * k.gb;
+      const double gs = exp_neg(0.5 * fma(ua, ua, ub * ub));
+      cplx w[2];
+      w_weideman_fast<2>(zr, zi, w);
+      const double fa = flip_sign(k.ck * fma(-gs, w[1].im, w[0].im), da);
+      const double fb = flip_sign(k.ck * fma(-gs, w[1].re, w[0].re), db);
+      ex = sw ? fb : fa;
+      ey = sw ? fa : fb;
+    } else {
+      double fx, fy;
+      sc_field_any(S, x - S.cx, y - S.cy, &fx, &fy);
+      ex = -0.5 * S.lambda * fx;
+      ey = -0.5 * S.lambda * fy;
     }
   } else {
-    const unsigned long long* A = acc + bs * p.acc_per_slice;
-    const double cx = sc_fix(A[0], (int)G[kGExp0]) / n, cy = sc_fix(A[1], (int)G[kGExp1]) / n;
-    const double rx = sqrt(sc_fix(A[2], (int)G[kGExp2]) / n);
-    const double ry = sqrt(sc_fix(A[3], (int)G[kGExp3]) / n);
-    const double lambda = n * (Bd.q_macro * kElectronCharge / G[kGDz]);  // [C/m]
-    const double posx = x - cx, posy = y - cy;
-    double fx, fy;
-    if (p.flag == 1) {
-      if ((rx - ry) / ry > 1.e-4)
-        bassetti_erskine(posx, posy, rx, ry, &fx, &fy);
-      else if ((rx - ry) / ry < -1.e-4)
-        bassetti_erskine(posy, posx, ry, rx, &fy, &fx);
-      else
-        gaussian_round_field(posx, posy, rx, &fx, &fy);
-      ex = -lambda / kPi / 2.0 / kEpsilon0 * fx;
-      ey = -lambda / kPi / 2.0 / kEpsilon0 * fy;
-    } else {
-      fx = posx / (rx * (rx + ry));
-      fy = posy / (ry * (rx + ry));
-      ex = lambda / kPi / kEpsilon0 * fx;
-      ey = lambda / kPi / kEpsilon0 * fy;
-    }
+    const ScSlice& S = slices[bs];
+    const double q = S.lambda / (S.rx + S.ry);
+    ex = q * ((x - S.cx) / S.rx);
+    ey = q * ((y - S.cy) / S.ry);
   }
-  const double px0 = c[npad + g];
-  const double pz = (1 + c[5 * npad + g]) * p.p0;
+  const double pz = (1 + dp) * p.p0;
   const double tpx = pz * y, tpy = pz * px0;
-  const double pp = sqrt(pz * pz + tpx * tpx + tpy * tpy);
-  const double gamma = sqrt(1 + pp * pp);
-  const double beta = pp / gamma;
-  const double g2 = gamma * gamma;
-  const double dpx = ex / g2 * kElectronCharge * ds / (beta * kCLight) / (kElectronMassKg * pp * kCLight);
-  const double dpy = ey / g2 * kElectronCharge * ds / (beta * kCLight) / (kElectronMassKg * pp * kCLight);
-  c[npad + g] = px0 + dpx;
-  c[3 * npad + g] += dpy;
+  const double p2 = pz * pz + tpx * tpx + tpy * tpy;
+  const double f = kElectronCharge * ds / (kElectronMassKg * kCLight * kCLight) / (sqrt(1 + p2) * p2);
+  c[npad + g] = px0 + ex * f;
+  c[3 * npad + g] = py0 + ey * f;
 }
 
 // this translation unit's copy of the w(z) table (faddeeva.cuh keeps one
@@ -431,8 +597,11 @@ cudaError_t upload_weideman_table_sc() {
 }
 
 size_t sc_solve_smem(const ScParams& p) {
-  return sizeof(double) * ((size_t)3 * p.nx * p.ny + p.nx * p.nx + p.ny * p.ny);
+  const size_t px = sc_pad(p.nx), py = sc_pad(p.ny);
+  return sizeof(double) * (2 * px * (py + 4) + px * (px + 4) + py * (py + 4));
 }
+
+size_t sc_slice_bytes() { return sizeof(ScSlice); }
 
 cudaError_t prepare_sc(const ScParams& p) {
   if (p.flag != 2) return cudaSuccess;
@@ -442,33 +611,35 @@ cudaError_t prepare_sc(const ScParams& p) {
 
 cudaError_t launch_space_charge(Handle& h, int k) {
   const ScParams& p = h.sc;
-  cudaError_t e = cudaMemsetAsync(h.d.sc_cnt, 0, sizeof(int) * (size_t)h.M * p.nz, h.stream);
-  if (e != cudaSuccess) return e;
-  if (p.flag != 2) {
-    e = cudaMemsetAsync(h.d.sc_acc, 0,
-                        sizeof(unsigned long long) * (size_t)h.M * p.nz * p.acc_per_slice, h.stream);
-    if (e != cudaSuccess) return e;
-  }
-  k_sc_geom<<<h.M, kScThreads, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.bunch, h.d.mom, p,
-                                             h.d.sc_geom, h.d.status);
-  k_sc_deposit<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.tile_bunch, h.d.bunch, p,
-                                                  h.d.sc_geom, h.d.sc_cnt, h.d.sc_acc,
-                                                  h.d.sc_slice_of);
-  if (p.flag == 2) {
-    k_sc_offsets<<<(h.M + 127) / 128, 128, 0, h.stream>>>(h.d.bunch, p.nz, h.d.sc_cnt,
-                                                         h.d.sc_start, h.d.sc_cursor, h.M);
-    k_sc_scatter<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.tile_bunch, h.d.bunch, p.nz, h.d.sc_geom,
-                                                    h.d.sc_slice_of, h.d.sc_cursor, h.d.sc_list);
-    k_sc_solve<<<h.M * p.nz, kScThreads, sc_solve_smem(p), h.stream>>>(
-        p, h.d.c, h.npad, h.d.bunch, h.d.sc_geom, h.d.sc_cnt, h.d.sc_start, h.d.sc_list, h.d.sc_sin,
-        h.d.sc_field);
+  const DeviceBufs& d = h.d;
+  const cudaStream_t st = h.stream;
+  const bool pic = p.flag == 2;
+  const int slices = h.M * p.nz;
+  const size_t shared = p.nz <= kScSharedSlices ? sizeof(unsigned) * p.nz : 0;
+  if (h.n_chunks < 1) return cudaSuccess;
+  ScSlice* sl = reinterpret_cast<ScSlice*>(d.sc_slices);
+  double2* xy = reinterpret_cast<double2*>(d.sc_xy);
+  k_sc_clear<<<std::min(148, (slices + 255) / 256), 256, 0, st>>>(d.sc_range, d.sc_cnt, d.sc_acc, h.M,
+                                                                p.nz, pic ? 0 : 4);
+  (pic ? k_sc_range<false> : k_sc_range<true>)<<<h.n_chunks, kScThreads, 0, st>>>(
+      d.c, h.npad, d.surv, d.chunk_loc, d.sc_range);
+  k_sc_geom<<<(h.M + 31) / 32, 32, 0, st>>>(d.c, h.npad, d.bunch, d.mom, p, d.sc_range, d.sc_geom,
+                                            d.status, h.M);
+  (pic ? k_sc_count<true> : k_sc_count<false>)<<<h.n_chunks, kScThreads, shared * (pic ? 1 : 9), st>>>(
+      d.c, h.npad, d.surv, d.chunk_loc, p, d.sc_geom, d.sc_cnt, d.sc_acc);
+  if (pic) {
+    k_sc_offsets<<<h.M, 32, 0, st>>>(d.bunch, p.nz, d.sc_cnt, d.sc_start, d.sc_cursor);
+    k_sc_scatter<<<h.n_chunks, kScThreads, 2 * shared, st>>>(d.c, h.npad, d.surv, d.chunk_loc, p,
+                                                             d.sc_geom, d.sc_cursor, xy);
+    k_sc_solve<<<slices, kScThreads, sc_solve_smem(p), st>>>(p, d.bunch, d.sc_geom, d.sc_cnt,
+                                                             d.sc_start, xy, d.sc_sin, d.sc_field);
   } else {
-    k_sc_second<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.tile_bunch, h.d.bunch, p,
-                                                   h.d.sc_geom, h.d.sc_cnt, h.d.sc_acc);
+    k_sc_slices<<<(slices + 127) / 128, 128, 0, st>>>(p, d.bunch, d.sc_geom, d.sc_cnt, d.sc_acc, sl,
+                                                      h.M);
   }
-  k_sc_kick<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.tile_bunch, h.d.bunch, p,
-                                               h.d.sc_geom, h.d.sc_cnt, h.d.sc_acc, h.d.sc_field,
-                                               h.sections[k].length);
+  auto kick = pic ? k_sc_kick<2> : p.flag == 1 ? k_sc_kick<1> : k_sc_kick<3>;
+  kick<<<h.n_tiles, kTile, 0, st>>>(d.c, h.npad, d.surv, d.tile_bunch, p, d.sc_geom, d.sc_cnt, sl,
+                                    d.sc_field, h.sections[k].length);
   return cudaGetLastError();
 }
 
