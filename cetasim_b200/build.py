@@ -17,7 +17,7 @@ LIB = os.path.join(HERE, "libcetagpu.so")
 
 SOURCES = ["capi.cu", "kernels.cu", "kernels_sr.cu", "kernels_ion.cu", "surrogate.cu", "shard.cu",
            "cbm.cu", "beam_loading.cu", "bbi.cu", "sc.cu", "faddeeva_table.cpp", "input_settings.cpp", "rw_wake.cpp"]
-HEADERS = ["cg_common.cuh", "faddeeva.cuh", "be_field.cuh", "track_math.cuh", "cg_internal.h",
+HEADERS = ["cg_common.cuh", "faddeeva.cuh", "be_field.cuh", "track_math.cuh", "normals.cuh", "cg_internal.h",
            "kernels.cuh", "umma.cuh", "surrogate.cuh", "rw_wake.h"]
 
 NVCC_FLAGS = [

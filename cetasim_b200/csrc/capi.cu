@@ -210,8 +210,7 @@ RingDev make_ring_dev(const cg_config& c, const cg_section& s0) {
   }
   d.circ_ring = r.circ_ring;
   for (int i = 0; i < 3; ++i) d.alphac[i] = r.alphac[i];
-  d.energy = r.electron_energy;
-  d.r_beta2 = std::pow(r.r_beta, 2);
+  d.inv_e_beta2 = 1.0 / r.electron_energy / std::pow(r.r_beta, 2);
   d.u0_term = r.u0 / r.electron_energy / std::pow(r.r_beta, 2);
   double fRF = r.f0 * r.harmonics;
   d.n_cav = r.n_cav;
@@ -1329,6 +1328,7 @@ int cg_fir(cg_handle* H, int turn) {
 int cg_mark_lost(cg_handle* H, double* trans) {
   STAGE_PROLOGUE
   int st = launch_ok(h, launch_mark_lost(h, false, true), "mark lost");
+  if (!st) st = launch_ok(h, launch_turn_end(h, false), "transmission");
   int s2 = check_status(h);
   if (!st) st = s2;
   if (trans) {
@@ -1471,6 +1471,10 @@ static cudaError_t enqueue_turn(Handle& h) {
   // the LR kick joins the longitudinal kernel unless the broadband impedance
   // kicks in between (MPBeam.cpp:1084-1085)
   if (c.flag_lr_wake && !c.bbi.flag) fl |= kLongLR;
+  // and the loss check, unless a stage in between takes the survivors of the
+  // turn before
+  const bool mark = !c.bbi.flag && !c.flag_sr_wake && !c.flag_fir;
+  if (mark) fl |= kLongMark;
   if ((e = launch_long(h, fl))) return e;
   TRACE(h.stream, CG_TRACE_LONG, -1, -1);
   if (c.bbi.flag) {
@@ -1487,8 +1491,8 @@ static cudaError_t enqueue_turn(Handle& h) {
     if ((e = launch_fir_compute(h))) return e;
     TRACE(h.stream, CG_TRACE_FIR, -1, -1);
   }
-  if ((e = launch_mark_lost(h, c.flag_fir != 0, true))) return e;
-  if ((e = launch_turn_advance(h))) return e;
+  if (!mark && (e = launch_mark_lost(h, c.flag_fir != 0, true))) return e;
+  if ((e = launch_turn_end(h, true))) return e;
   TRACE(h.stream, CG_TRACE_MARK_LOST, -1, -1);
   return cudaSuccess;
 }

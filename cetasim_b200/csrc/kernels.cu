@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "kernels.cuh"
+#include "normals.cuh"
 
 namespace cg {
 
@@ -597,59 +598,99 @@ cudaError_t launch_ion_kick(Handle& h, int k) { return launch_ion_kick_variant(h
 // Turn tail: RF kick, drift, energy loss (all particles), synchrotron
 // radiation (alive), long-range wake kick (all particles).
 
-__global__ void __launch_bounds__(kTile) k_long(double* __restrict__ c, int64_t npad,
-                                                const uint8_t* __restrict__ surv,
-                                                const int* __restrict__ tile_bunch,
-                                                const BunchDev* __restrict__ bunch,
-                                                const __grid_constant__ SectionDev sec0,
-                                                const __grid_constant__ RingDev r,
-                                                unsigned flags, uint64_t seed,
-                                                const int* __restrict__ d_turn,
-                                                const double* __restrict__ lr_force,
-                                                const double* __restrict__ rf_zr,
-                                                const double* __restrict__ rf_kick,
-                                                const double* __restrict__ rf_fbk, int M,
-                                                double* rf_info) {
+//
+// Bound by instruction issue: the quantum excitation's three pairs of normals
+// are half of the work.  With the library's log, square root and sincospi (and
+// two divisions per cavity) a particle took 1016 instructions; the branch-free
+// forms of normals.cuh take 725.  1.6e6 particles with one cavity:
+// 73 -> 54 us.
+//
+// If nothing after it in the turn depends on the survival marks before the
+// loss check (kLongMark), the check is made here on the final position; the
+// bunches' counts end up in the transmission (k_turn_end).
+
+// Bunch::MarkLostParticle (Bunch.cpp:172-200) for the warp's particles, their
+// number of loss conditions added to the bunch's.  A position clearly inside
+// the aperture by the reciprocals takes no division; the others take the
+// reference's.
+struct Aperture {
+  double ax, ay, iax, iay;
+};
+__device__ __forceinline__ void mark_lost_warp(const RingDev& r, const Aperture& ap, bool valid,
+                                               double x, double y, double z, uint8_t* surv,
+                                               int* loss_count) {
+  const double tx = x * ap.iax, ty = y * ap.iay;
+  int count = 0;
+  if (valid && !(fma(tx, tx, ty * ty) < 0.999 && fabs(z) <= r.z_loss)) {
+    uint8_t s = *surv;
+    count = mark_lost_particle(r, ap.ax, ap.ay, x, y, z, &s);
+    if (count) *surv = s;
+  }
+  if (__any_sync(FULL_MASK, count)) {
+    count = __reduce_add_sync(FULL_MASK, count);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss_count, count);
+  }
+}
+
+// LOADING: some cavity has beam loading; MARK: kLongMark
+template <bool LOADING, bool MARK>
+__global__ void __launch_bounds__(kTile, 3) k_long(double* __restrict__ c, int64_t npad,
+                                                  uint8_t* __restrict__ surv,
+                                                  const int* __restrict__ tile_bunch,
+                                                  const BunchDev* __restrict__ bunch,
+                                                  const __grid_constant__ SectionDev sec0,
+                                                  const __grid_constant__ RingDev r,
+                                                  unsigned flags, uint64_t seed,
+                                                  const int* __restrict__ d_turn,
+                                                  const double* __restrict__ lr_force,
+                                                  const double* __restrict__ rf_zr,
+                                                  const double* __restrict__ rf_kick,
+                                                  const double* __restrict__ rf_fbk, int M,
+                                                  double* rf_info,
+                                                  const __grid_constant__ Aperture ap,
+                                                  int* loss_count) {
   TileIdx t = tile_index(tile_bunch, bunch);
-  if (!t.valid) return;
-  double v[6];
-  load6(c, npad, t.g, v);
-  if ((flags & kLongRF) && t.i == bunch[t.b].n - 1) {
-    // the ideal cavities' BunchRFModeInfo: the voltage the bunch's last
-    // particle sees (Bunch.cpp:466-478; cavity = generator, no induced or
-    // self-loss voltage)
-    for (int q = 0; q < r.n_cav; ++q) {
-      if (r.bl_any && r.bl_index[q] >= 0) continue;
-      double sn, co;
-      sincos(v[4] * r.rf_theta_coeff[q], &sn, &co);
-      const double re = fma(r.vreq_re[q], co, r.vreq_im[q] * sn);
-      const double im = fma(r.vreq_im[q], co, -r.vreq_re[q] * sn);
-      double* o = rf_info + ((size_t)t.b * CG_MAX_CAVITIES + q) * 8;
-      o[0] = re; o[1] = im; o[2] = re; o[3] = im;
-      o[4] = 0.0; o[5] = 0.0; o[6] = 0.0; o[7] = 0.0;
+  double v[6] = {0, 0, 0, 0, 0, 0};
+  if (t.valid) {
+    load6(c, npad, t.g, v);
+    const bool alive = (LOADING || (flags & kLongSynrad)) && surv[t.g] == kAlive;
+    if (flags & kLongRF) {
+      if (t.i == bunch[t.b].n - 1) {
+        // the ideal cavities' BunchRFModeInfo: the voltage the bunch's last
+        // particle sees (Bunch.cpp:466-478; cavity = generator, no induced or
+        // self-loss voltage)
+        for (int q = 0; q < r.n_cav; ++q) {
+          if (LOADING && r.bl_index[q] >= 0) continue;
+          double sn, co;
+          sincos_far(v[4] * r.rf_theta_coeff[q], &sn, &co);
+          const double re = fma(r.vreq_re[q], co, r.vreq_im[q] * sn);
+          const double im = fma(r.vreq_im[q], co, -r.vreq_re[q] * sn);
+          double* o = rf_info + ((size_t)t.b * CG_MAX_CAVITIES + q) * 8;
+          o[0] = re; o[1] = im; o[2] = re; o[3] = im;
+          o[4] = 0.0; o[5] = 0.0; o[6] = 0.0; o[7] = 0.0;
+        }
+      }
+      if (LOADING) v[5] = rf_kick_dp_loading(r, v[4], v[5], alive, t.b, M, rf_zr, rf_kick, rf_fbk);
+      else v[5] = rf_kick_dp(r, v[4], v[5]);
     }
+    if (flags & kLongDrift) v[4] = drift_z(r, v[4], v[5]);
+    if (flags & kLongLoss) v[5] -= r.u0_term;
+    if ((flags & kLongSynrad) && alive) {
+      double g[6] = {0, 0, 0, 0, 0, 0};
+      const bool excite = bunch[t.b].n != 1;
+      if (excite && (r.qe_coeff[0] != 0 || r.qe_coeff[1] != 0 || r.qe_coeff[2] != 0))
+        synrad_normals(seed, (uint32_t)t.i, (uint32_t)t.b, (uint32_t)(*d_turn), g);
+      synrad_particle(sec0, r, v, g, excite);
+    }
+    if (flags & kLongLR) {
+      const double* f = lr_force + 3 * t.b;
+      v[1] += f[0];
+      v[3] += f[1];
+      v[5] += f[2];
+    }
+    store6(c, npad, t.g, v);
   }
-  if (flags & kLongRF) {
-    if (r.bl_any)
-      v[5] = rf_kick_dp_loading(r, v[4], v[5], surv[t.g] == kAlive, t.b, M, rf_zr, rf_kick,
-                                rf_fbk);
-    else
-      v[5] = rf_kick_dp(r, v[4], v[5]);
-  }
-  if (flags & kLongDrift) v[4] = drift_z(r, v[4], v[5]);
-  if (flags & kLongLoss) v[5] -= r.u0_term;
-  if ((flags & kLongSynrad) && surv[t.g] == kAlive) {
-    double g[6];
-    synrad_normals(seed, (uint32_t)t.i, (uint32_t)t.b, (uint32_t)(*d_turn), g);
-    synrad_particle(sec0, r, v, g, bunch[t.b].n != 1);
-  }
-  if (flags & kLongLR) {
-    const double* f = lr_force + 3 * t.b;
-    v[1] += f[0];
-    v[3] += f[1];
-    v[5] += f[2];
-  }
-  store6(c, npad, t.g, v);
+  if (MARK) mark_lost_warp(r, ap, t.valid, v[0], v[2], v[4], surv + t.g, loss_count + t.b);
 }
 
 // The accumulated phase advance of the tracked bunches' particles
@@ -725,16 +766,24 @@ cudaError_t launch_phase_adv(Handle& h, int ja, int jb, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+static Aperture aperture(const Handle& h) {
+  const cg_section& s = h.sections[0];
+  return {s.aperture_x, s.aperture_y, 1.0 / s.aperture_x, 1.0 / s.aperture_y};
+}
+
 cudaError_t launch_long(Handle& h, unsigned flags) {
   if ((flags & kLongRF) && h.ring.bl_any) {
     // the cavities' recurrence over the train first: the kicks of each bin
     cudaError_t e = launch_rf_beam_loading(h);
     if (e != cudaSuccess) return e;
   }
-  k_long<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                            h.sec_dev_host[0], h.ring, flags, h.cfg.seed, h.d.turn,
-                                            h.d.lr_force, h.d.rf_zr, h.d.rf_kick, h.d.rf_fbk, h.M,
-                                            h.d.rf_info);
+  const bool mark = flags & kLongMark;
+  auto kern = h.ring.bl_any ? (mark ? k_long<true, true> : k_long<true, false>)
+                            : (mark ? k_long<false, true> : k_long<false, false>);
+  kern<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
+                                          h.sec_dev_host[0], h.ring, flags, h.cfg.seed, h.d.turn,
+                                          h.d.lr_force, h.d.rf_zr, h.d.rf_kick, h.d.rf_fbk, h.M,
+                                          h.d.rf_info, aperture(h), h.d.loss_count);
   return cudaGetLastError();
 }
 
@@ -893,21 +942,19 @@ cudaError_t launch_fir_compute(Handle& h) {
 }
 
 // ---------------------------------------------------------------------------
-// FIR kick (all particles) + Bunch::MarkLostParticle (Bunch.cpp:172-200).
+// FIR kick (all particles) + Bunch::MarkLostParticle (Bunch.cpp:172-200): a
+// pass over x, y, z, bound by HBM latency (1.6e6 particles 23 -> 16 us; it used
+// to sum each tile over the CTA, fence, and divide twice per particle).
 
 __global__ void __launch_bounds__(kTile) k_mark_lost(double* __restrict__ c, int64_t npad,
                                                      uint8_t* __restrict__ surv,
                                                      const int* __restrict__ tile_bunch,
-                                                     const BunchDev* __restrict__ bunch, RingDev r,
-                                                     double ax, double ay, int mode,
+                                                     const BunchDev* __restrict__ bunch,
+                                                     const __grid_constant__ RingDev r,
+                                                     const __grid_constant__ Aperture ap, int mode,
                                                      const double* __restrict__ fir_kick,
-                                                     double inv_beta2, int* loss_count,
-                                                     unsigned* counters, BunchMomDev* mom,
-                                                     int* status, bool mark) {
-  __shared__ double smem[32];
-  __shared__ bool last;
+                                                     double inv_beta2, int* loss_count, bool mark) {
   TileIdx t = tile_index(tile_bunch, bunch);
-  double cnt[1] = {0.0};
   if (t.valid && mode > 0) {
     const double* k = fir_kick + 3 * t.b;
     c[1 * npad + t.g] += k[0];
@@ -916,47 +963,41 @@ __global__ void __launch_bounds__(kTile) k_mark_lost(double* __restrict__ c, int
     else c[5 * npad + t.g] += k[2];
   }
   if (!mark) return;
+  double x = 0, y = 0, z = 0;
   if (t.valid) {
-    double x = c[t.g], y = c[2 * npad + t.g], z = c[4 * npad + t.g];
-    uint8_t s = surv[t.g];
-    cnt[0] = (double)mark_lost_particle(r, ax, ay, x, y, z, &s);
-    surv[t.g] = s;
+    x = c[t.g];
+    y = c[2 * npad + t.g];
+    z = c[4 * npad + t.g];
   }
-  block_sum<1, kTile>(cnt, smem);
-  const BunchDev& B = bunch[t.b];
-  if (threadIdx.x == 0) atomicAdd(&loss_count[t.b], (int)cnt[0]);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned prev = atomicAdd(&counters[t.b], 1u);
-    last = (prev == (unsigned)(B.n_tiles - 1));
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    int count = atomicAdd(&loss_count[t.b], 0);
-    double tr = (B.n - count) / (double)B.n;
-    mom[t.b].transmission = tr;
-    if (tr < 0.5) atomicOr(status, kStatusTransmission);
-    loss_count[t.b] = 0;
-    counters[t.b] = 0;
-  }
+  mark_lost_warp(r, ap, t.valid, x, y, z, surv + t.g, loss_count + t.b);
 }
 
 cudaError_t launch_mark_lost(Handle& h, bool fir_kick, bool mark) {
   int mode = 0;
   if (fir_kick) mode = (h.cfg.fir.mode == 0) ? 2 : 1;
   double inv_beta2 = 1.0 / (h.cfg.ring.r_beta * h.cfg.ring.r_beta);
-  k_mark_lost<<<h.n_tiles, kTile, 0, h.stream>>>(
-      h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, h.ring, h.sections[0].aperture_x,
-      h.sections[0].aperture_y, mode, h.d.fir_kick, inv_beta2, h.d.loss_count, h.d.counters,
-      h.d.mom, h.d.status, mark);
+  k_mark_lost<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
+                                                 h.d.bunch, h.ring, aperture(h), mode,
+                                                 h.d.fir_kick, inv_beta2, h.d.loss_count, mark);
   return cudaGetLastError();
 }
 
-__global__ void k_turn_advance(int* turn) { *turn += 1; }
-cudaError_t launch_turn_advance(Handle& h) {
-  k_turn_advance<<<1, 1, 0, h.stream>>>(h.d.turn);
+// After the loss check: the bunches' transmission, and the turn's end.
+__global__ void k_turn_end(const BunchDev* __restrict__ bunch, int M, int* loss_count,
+                           BunchMomDev* mom, int* status, int* turn, int advance) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b == 0) *turn += advance;
+  if (b >= M || bunch[b].n_tiles == 0) return;  // no particles here: another rank's
+  const int n = bunch[b].n;
+  const double tr = (n - loss_count[b]) / (double)n;
+  loss_count[b] = 0;
+  mom[b].transmission = tr;
+  if (tr < 0.5) atomicOr(status, kStatusTransmission);
+}
+
+cudaError_t launch_turn_end(Handle& h, bool advance) {
+  k_turn_end<<<(h.M + 127) / 128, 128, 0, h.stream>>>(h.d.bunch, h.M, h.d.loss_count, h.d.mom,
+                                                      h.d.status, h.d.turn, advance ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -71,6 +71,7 @@ enum LongFlags : unsigned {
   kLongLoss = 4,
   kLongSynrad = 8,
   kLongLR = 16,
+  kLongMark = 32,  // the loss check too
 };
 cudaError_t launch_long(Handle& h, unsigned flags);
 // cavities with beam loading: z ranges and bins of the RF step, then the
@@ -84,8 +85,9 @@ cudaError_t launch_lr_compute(Handle& h);
 cudaError_t launch_lr_kick(Handle& h);
 cudaError_t launch_fir_compute(Handle& h);
 cudaError_t launch_mark_lost(Handle& h, bool fir_kick, bool mark);
+// after the loss check: the transmissions; the turn counter if `advance`
+cudaError_t launch_turn_end(Handle& h, bool advance);
 cudaError_t launch_sr_wake(Handle& h);
-cudaError_t launch_turn_advance(Handle& h);
 cudaError_t launch_gaussian(Handle& h, double emit_x, double emit_y, double sigma_z,
                             double sigma_dp, uint64_t seed);
 cudaError_t launch_faddeeva(const double* zr, const double* zi, double* wr, double* wi, int64_t n,

@@ -31,7 +31,7 @@ struct RingDev {
   double adtx[5], adty[5];
   int adt2;                          // some second-order amplitude-dependent term is not zero
   double circ_ring, alphac[3];
-  double energy, r_beta2, u0_term;   // u0 / E / beta^2 (Bunch.cpp:490)
+  double inv_e_beta2, u0_term;       // 1 / (E beta^2), u0 / E / beta^2 (Bunch.cpp:490)
   double rf_theta_coeff[4];          // 2 pi h_c f_RF / (c beta), Bunch.cpp:468
   double vreq_re[4], vreq_im[4];
   int n_cav;
@@ -192,52 +192,6 @@ CG_HD void section_map_particle(const SectionDev& s, const RingDev& r, double v[
   matvec6_section(s, s.h2b2, v2, v);
 }
 
-// Bunch::BunchMomentumUpdateDueToRFCA (Bunch.cpp:466-472), every particle.
-// The RF step with cavities that load (MPBeam.cpp:2621-2704): per cavity in
-// order, the ideal cavity's kick or, for an alive particle, the two
-// increments of its bin from the recurrence's table (kick[((b M + j) nb +
-// bin) 2 ..]); then the direct-feedback kicks of the bunch, to every
-// particle.
-CG_HD double rf_kick_dp_loading(const RingDev& r, double z, double dp, bool alive, int j, int M,
-                                const double* zr, const double* kick, const double* fbk) {
-  int bin = -1;
-  if (alive) {
-    const double zmin = zr[2 * j], zmax = zr[2 * j + 1];
-    const double dz = (zmax - zmin) / r.rf_bins;
-    bin = (int)floor((zmax - z) / dz);
-    bin = bin < 0 ? 0 : (bin >= r.rf_bins ? r.rf_bins - 1 : bin);
-  }
-  for (int c = 0; c < r.n_cav; ++c) {
-    const int b = r.bl_index[c];
-    if (b < 0) {
-      double th = z * r.rf_theta_coeff[c];
-      double s, co;
-      sincos(th, &s, &co);
-      double re = fma(r.vreq_re[c], co, r.vreq_im[c] * s);
-      dp += re / r.energy / r.r_beta2;
-    } else if (bin >= 0) {
-      const double* k = kick + (((size_t)b * M + j) * r.rf_bins + bin) * 2;
-      dp += k[0];
-      dp += k[1];
-    }
-  }
-  for (int c = 0; c < r.n_cav; ++c)
-    if (r.bl_index[c] >= 0 && r.bl_fb[c]) dp += fbk[(size_t)r.bl_index[c] * M + j];
-  return dp;
-}
-
-CG_HD double rf_kick_dp(const RingDev& r, double z, double dp) {
-  for (int c = 0; c < r.n_cav; ++c) {
-    double th = z * r.rf_theta_coeff[c];
-    double s, co;
-    sincos(th, &s, &co);
-    // Re(V e^{-i th}) = Vr cos th + Vi sin th
-    double re = fma(r.vreq_re[c], co, r.vreq_im[c] * s);
-    dp += re / r.energy / r.r_beta2;
-  }
-  return dp;
-}
-
 // Bunch::BunchLongPosTransferOneTurn (Bunch.cpp:499-500).
 CG_HD double drift_z(const RingDev& r, double z, double dp) {
   double poly = fma(r.alphac[2], dp * dp * dp, fma(r.alphac[1], dp * dp, r.alphac[0] * dp));
@@ -263,16 +217,6 @@ CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
     X[5] = fma(r.qe_coeff[2], g[5], X[5]);
   }
   matvec6_section(s0, s0.h1b1, X, v);
-}
-
-// Six synrad normals of particle i of bunch j at turn `turn`.
-CG_HD void synrad_normals(uint64_t seed, uint32_t i, uint32_t j, uint32_t turn, double g[6]) {
-  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32) ^ kStreamSynrad;
-#pragma unroll
-  for (uint32_t q = 0; q < 3; ++q) {
-    u32x4 c = {{i, j, turn, q}};
-    normal2(philox4x32_10(c, k0, k1), &g[2 * q], &g[2 * q + 1]);
-  }
 }
 
 // Bunch::MarkLostParticle per particle (Bunch.cpp:179-191): returns the
