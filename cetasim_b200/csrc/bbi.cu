@@ -20,376 +20,387 @@
 // the two FFTs of length 2n - 1 and needs no FFT library.  The sums are the
 // same up to rounding.
 //
-//  k_bbi_range  per tile: the bin of every particle, per-bunch lowest and
-//               highest bin and the largest |x|, |y| (atomics).
-//  k_bbi_hist   per tile: per-bin counts and sums of x and y in 64-bit fixed
+//  k_bbi_range  per-bunch lowest and highest bin and the largest |x|, |y|
+//               (atomics); in the turn the longitudinal pass before it does
+//               this with the positions that it writes (bbi_span_cta).
+//  k_bbi_hist   per chunk: per-bin counts and sums of x and y in 64-bit fixed
 //               point (the scale from the bunch's largest |x|, |y|), so the
-//               result does not depend on the order of the atomics.
+//               result does not depend on the order of the atomics; in shared
+//               memory, then added to the bunch's.
 //  k_bbi_conv   one CTA per bunch: profiles, the Gaussian filter and its
 //               renormalisation, the potentials of the bins that hold
-//               particles; resets the per-bunch accumulators.
-//  k_bbi_kick   per tile: the kicks, plane by plane in the reference's order.
+//               particles, and each bin's kick; resets the accumulators.
+//  k_bbi_kick   per tile: the kicks, plane by plane in the reference's order,
+//               and the turn's loss check if no stage comes between.
+//
+// Bound by: the passes by HBM (38 MB to count, 115 MB to kick 1.6e6 particles)
+// and its latency, the convolution by its chains of FMAs and barriers.  80
+// bunches of 20,000, five planes, us: range 25 -> in the longitudinal pass,
+// hist 53 -> 21 (global 64-bit atomics), conv 28 -> 15 (256 threads, a
+// filter with bounds checks per tap, one chain of 600 FMAs per bin and plane),
+// kick 40 and the loss check 16 -> 24 together (up to fourteen divisions a particle).
+#include <algorithm>
 #include <climits>
 #include <cuda_runtime.h>
 
-#include "kernels.cuh"
+#include "turn_tail.cuh"
 
 namespace cg {
 
 #define BBI_FULL 0xffffffffu
 constexpr int kBbiThreads = 256;
-
-// The bin of a particle, or -1 when the reference would index outside its
-// profile.  Frequency domain (z - zMin + dz / 2) / dz (MPBunch.cpp:2170),
-// time domain (z - zMin) / dz (MPBunch.cpp:2052), truncated as int() does
-// (so -1 < t < 0 is bin 0).
-__device__ __forceinline__ int bbi_bin(const BbiParams& p, double z) {
-  const double t = p.td ? (z - p.zmin) / p.dz : ((z - p.zmin) + p.dz / 2) / p.dz;
-  return (t > -1.0 && t < (double)p.nbins) ? (int)t : -1;
-}
+constexpr int kBbiConvThreads = 1024;
+// Bins up to which a CTA counts in shared memory (20 bytes each); beyond, it
+// adds to the bunch's bins directly.
+constexpr int kBbiSharedBins = 1024;
 
 // Power-of-two scale of the fixed-point sums: |v| 2^s < 2^(61 - nb) for
 // |v| <= amax and n < 2^nb values, so a sum of n of them stays below 2^61.
-__device__ __forceinline__ int bbi_fix_exp(unsigned long long amax_bits, int n) {
-  const double a = __longlong_as_double((long long)amax_bits);
+__device__ __forceinline__ int bbi_fix_exp(unsigned amax_hi, int n) {
+  const double a = __hiloint2double((int)amax_hi, 0);
   if (!(a > 0) || isinf(a)) return 0;
   const int nb = 32 - __clz(n);
   return 60 - ilogb(a) - nb;
 }
 
-__device__ __forceinline__ double bbi_warp_max(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(BBI_FULL, v, o));
-  return v;
-}
-
 __global__ void __launch_bounds__(kTile) k_bbi_range(const double* __restrict__ c, int64_t npad,
                                                      const uint8_t* __restrict__ surv,
                                                      const int* __restrict__ tile_bunch,
-                                                     const BunchDev* __restrict__ bunch, BbiParams p,
-                                                     int* lo, int* hi, unsigned long long* amax,
-                                                     int* status) {
-  __shared__ int s_lo[kTile / 32], s_hi[kTile / 32];
-  __shared__ double s_ax[kTile / 32], s_ay[kTile / 32];
+                                                     const BunchDev* __restrict__ bunch,
+                                                     const __grid_constant__ BbiParams p,
+                                                     BbiSpan* span, int* status) {
   const int b = tile_bunch[blockIdx.x];
   const BunchDev& Bd = bunch[b];
-  if (Bd.q_macro == 0) return;  // MPBeam.cpp:1335
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  int mn = INT_MAX, mx = -1;
-  double ax = 0, ay = 0;
-  if (i < Bd.n) {
-    const int idx = bbi_bin(p, c[4 * npad + g]);
-    if (idx < 0) {
-      atomicOr(status, kStatusBbiRange);
-    } else {
-      mn = mx = idx;
-      // frequency domain: every particle enters the dipole profiles
-      // (MPBunch.cpp:2265-2270); time domain: the survivors' means (:2061-2070)
-      if (!p.td || surv[g] == kAlive) {
-        ax = fabs(c[g]);
-        ay = fabs(c[2 * npad + g]);
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = min(mn, __shfl_xor_sync(BBI_FULL, mn, o));
-    mx = max(mx, __shfl_xor_sync(BBI_FULL, mx, o));
-  }
-  ax = bbi_warp_max(ax);
-  ay = bbi_warp_max(ay);
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    s_lo[w] = mn;
-    s_hi[w] = mx;
-    s_ax[w] = ax;
-    s_ay[w] = ay;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < kTile / 32; ++q) {
-      mn = min(mn, s_lo[q]);
-      mx = max(mx, s_hi[q]);
-      ax = fmax(ax, s_ax[q]);
-      ay = fmax(ay, s_ay[q]);
-    }
-    if (mx >= 0) {
-      atomicMin(&lo[b], mn);
-      atomicMax(&hi[b], mx);
-      // non-negative doubles order as their bit patterns
-      atomicMax(&amax[2 * b], (unsigned long long)__double_as_longlong(ax));
-      atomicMax(&amax[2 * b + 1], (unsigned long long)__double_as_longlong(ay));
-    }
-  }
+  const bool valid = (blockIdx.x - Bd.tile_off) * kTile + (int)threadIdx.x < Bd.n;
+  bbi_span_cta(p, span + b, status, valid && Bd.q_macro != 0, valid && surv[g] == kAlive,
+               valid ? c[g] : 0.0, valid ? c[2 * npad + g] : 0.0, valid ? c[4 * npad + g] : 0.0);
 }
 
-__global__ void __launch_bounds__(kTile) k_bbi_hist(const double* __restrict__ c, int64_t npad,
-                                                    const uint8_t* __restrict__ surv,
-                                                    const int* __restrict__ tile_bunch,
-                                                    const BunchDev* __restrict__ bunch, BbiParams p,
-                                                    const int* __restrict__ lo,
-                                                    const int* __restrict__ hi,
-                                                    const unsigned long long* __restrict__ amax,
-                                                    int* cnt, unsigned long long* sxy, int* status) {
-  const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
+__global__ void __launch_bounds__(kBbiThreads) k_bbi_hist(const double* __restrict__ c, int64_t npad,
+                                                          const uint8_t* __restrict__ surv,
+                                                          const int4* __restrict__ chunk_loc,
+                                                          const BunchDev* __restrict__ bunch,
+                                                          const __grid_constant__ BbiParams p,
+                                                          const BbiSpan* __restrict__ span,
+                                                          int* status, int* cnt,
+                                                          unsigned long long* sxy) {
+  extern __shared__ unsigned s_bin[];  // W counts, then x (lo, hi), y (lo, hi)
+  const int4 l = chunk_loc[blockIdx.x];
+  const BunchDev& Bd = bunch[l.x];
   if (Bd.q_macro == 0) return;
-  const int l = lo[b], W = hi[b] - l + 1;
+  const int b = l.x;
+  const BbiSpan S = span[b];
+  const int first = S.lo(), W = S.bins();
   if (W < 1) return;
   if (W > CG_BBI_MAX_BINS) {
     if (threadIdx.x == 0) atomicOr(status, kStatusBbiWide);
     return;
   }
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  if (i >= Bd.n) return;
-  const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int idx = bbi_bin(p, c[4 * npad + g]);
-  if (idx < 0) return;
-  const int j = idx - l;
+  const bool shared = W <= kBbiSharedBins;
+  if (shared) {
+    for (int t = threadIdx.x; t < 5 * W; t += kBbiThreads) s_bin[t] = 0u;
+    __syncthreads();
+  }
+  const Pow2 fx = pow2_split(bbi_fix_exp(S.ax, Bd.n));
+  const Pow2 fy = pow2_split(bbi_fix_exp(S.ay, Bd.n));
   const size_t base = (size_t)b * p.wcap;
-  atomicAdd(&cnt[base + j], 1);
-  if (!p.td || surv[g] == kAlive) {
-    const int ex = bbi_fix_exp(amax[2 * b], Bd.n), ey = bbi_fix_exp(amax[2 * b + 1], Bd.n);
-    const long long qx = __double2ll_rn(scalbn(c[g], ex));
-    const long long qy = __double2ll_rn(scalbn(c[2 * npad + g], ey));
-    atomicAdd(&sxy[2 * base + j], (unsigned long long)qx);  // two's complement sums
-    atomicAdd(&sxy[2 * base + p.wcap + j], (unsigned long long)qy);
-  }
-}
-
-// Block-wide sum over kBbiThreads threads, fixed order (deterministic).
-__device__ double bbi_block_sum(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(BBI_FULL, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0;
-  for (int q = 0; q < kBbiThreads / 32; ++q) t += red[q];
-  return t;
-}
-
-// GetSmoothedBunchProfileGassionFilter (MPBunch.cpp:2349-2414): the K = 51
-// Gaussian filter with end-value padding over the bins [s0, s1), then the
-// filtered profile scaled so that its sum over [s0, s1) equals the raw one.
-// raw / out hold the bins [a, a + n); bins outside [s0, s1) pass unchanged.
-// Every other bin of the profile is zero and stays zero.
-__device__ void bbi_smooth(const BbiParams& p, const double* raw, double* out, int a, int n,
-                           double* red) {
-  double s_raw = 0, s_out = 0;
-  for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-    const int i = a + t;
-    double y = raw[t];
-    if (i >= p.s0 && i < p.s1) {
-      y = 0;
-      for (int k = -kBbiHalf; k <= kBbiHalf; ++k) {
-        int jj = i + k;
-        jj = jj < p.s0 ? p.s0 : (jj >= p.s1 ? p.s1 - 1 : jj);  // end-value padding
-        const double v = (jj >= a && jj < a + n) ? raw[jj - a] : 0.0;
-        y = fma(p.g[k + kBbiHalf], v, y);
-      }
-      s_raw += raw[t];
-      s_out += y;
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
+  int i = (l.y - Bd.tile_off) * kTile + threadIdx.x;
+  for (int u = 0; u < l.z && i < Bd.n; ++u, g += kTile, i += kTile) {
+    const double x = c[g], y = c[2 * npad + g];
+    const int idx = bbi_bin(p, c[4 * npad + g]);
+    const bool sums = !p.td || surv[g] == kAlive;
+    if (idx < 0) continue;
+    const int t = idx - first;
+    if (shared) atomicAdd(&s_bin[t], 1u);
+    else atomicAdd(&cnt[base + t], 1);
+    if (!sums) continue;
+    const long long qx = __double2ll_rn(pow2_scale(x, fx)), qy = __double2ll_rn(pow2_scale(y, fy));
+    if (shared) {
+      add64_split(&s_bin[W + t], &s_bin[2 * W + t], qx);
+      add64_split(&s_bin[3 * W + t], &s_bin[4 * W + t], qy);
+    } else {
+      atomicAdd(&sxy[2 * base + t], (unsigned long long)qx);  // two's complement sums
+      atomicAdd(&sxy[2 * base + p.wcap + t], (unsigned long long)qy);
     }
-    out[t] = y;
   }
-  const double sum0 = bbi_block_sum(s_raw, red);
-  const double sum1 = bbi_block_sum(s_out, red);
-  const double f = sum0 / sum1;  // MPBunch.cpp:2404-2407 (0 / 0 when empty, as there)
+  if (!shared) return;
   __syncthreads();
-  for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-    const int i = a + t;
-    if (i >= p.s0 && i < p.s1) out[t] *= f;
+  for (int t = threadIdx.x; t < W; t += kBbiThreads) {
+    if (!s_bin[t]) continue;
+    atomicAdd(&cnt[base + t], (int)s_bin[t]);
+    atomicAdd(&sxy[2 * base + t], (unsigned long long)s_bin[2 * W + t] << 32 | s_bin[W + t]);
+    atomicAdd(&sxy[2 * base + p.wcap + t],
+              (unsigned long long)s_bin[4 * W + t] << 32 | s_bin[3 * W + t]);
   }
-  __syncthreads();
 }
+
+// The kick of a bin: what its particles add, in the order of the reference's
+// operations up to the particle's own factor.
+struct alignas(16) BbiKick {
+  double z, dx, dy, qx, qy, pad;
+};
 
 // One CTA per bunch.  pot[(b * 6 + q) * wcap + t] for the bins a + t:
 // q = 0 the smoothed charge profile; q = 1..5 the potentials of the planes
 // Z, Dx, Dy, Qx, Qy at the bins that hold particles (frequency domain: the
 // wakePotenFromBBI arrays, MPBunch.cpp:2193-2341; time domain: temp[0..4],
-// MPBunch.cpp:2100-2111), 0 at the other bins.
-__global__ void __launch_bounds__(kBbiThreads) k_bbi_conv(const BunchDev* __restrict__ bunch,
-                                                          BbiParams p,
-                                                          const double* __restrict__ w, int* lo,
-                                                          int* hi, unsigned long long* amax,
-                                                          int* cnt, unsigned long long* sxy,
-                                                          double* pot, int2* win) {
+// MPBunch.cpp:2100-2111), 0 at the other bins; kick[b * wcap + t] the kicks.
+//
+// Three profiles side by side (the charge, the dipoles x and y; time domain:
+// the charge and the mean x and y, which are not smoothed), the tasks
+// (profile, bin) and (plane, bin) over the threads; a sum over bins runs in
+// four chains.  Smoothing is GetSmoothedBunchProfileGassionFilter
+// (MPBunch.cpp:2349-2414): the K = 51 Gaussian filter with end-value padding
+// over the bins [s0, s1), then the filtered profile scaled so that its sum
+// over [s0, s1) equals the raw one; bins outside pass unchanged, every other
+// bin of the profile is zero and stays zero.  The raw profiles keep kBbiHalf
+// zeros on both sides, so that a tap away from s0 and s1 needs no check.
+__global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
+    const BunchDev* __restrict__ bunch, const __grid_constant__ BbiParams p,
+    const double* __restrict__ w, BbiSpan* span, int* cnt,
+    unsigned long long* sxy, double* pot, BbiKick* kick, int2* win) {
   extern __shared__ double sm[];
-  __shared__ double red[kBbiThreads / 32];
+  __shared__ double red[kBbiConvThreads / 32][6];
+  __shared__ double scale[3];
   const int b = blockIdx.x;
   const BunchDev& Bd = bunch[b];
-  const int l = lo[b], h = hi[b];
-  const int W = h - l + 1;
+  const BbiSpan S = span[b];
+  const int W = S.bins(), l = S.lo(), h = l + W - 1;
   if (Bd.q_macro == 0 || W < 1 || W > CG_BBI_MAX_BINS) {
     if (threadIdx.x == 0) {
       win[b] = make_int2(0, 0);
-      lo[b] = INT_MAX;
-      hi[b] = -1;
-      amax[2 * b] = amax[2 * b + 1] = 0ull;
+      span[b] = BbiSpan{0u, 0u, 0u, 0u};
     }
     return;
   }
   const int a = max(l - kBbiHalf, 0);
   const int e = min(h + kBbiHalf, p.nbins - 1);
   const int n = e - a + 1;
-  double* s_raw = sm;
-  double* s_p0 = sm + p.wcap;
-  double* s_p1 = sm + 2 * p.wcap;
-  double* s_p2 = sm + 3 * p.wcap;
+  const int nr = n + 2 * kBbiHalf;    // raw bins a - kBbiHalf ..
+  double* s_raw = sm;                 // 3 x nr
+  double* s_p = sm + 3 * (size_t)nr;  // 3 x n
   const size_t base = (size_t)b * p.wcap;
-  const int ex = bbi_fix_exp(amax[2 * b], Bd.n), ey = bbi_fix_exp(amax[2 * b + 1], Bd.n);
+  const int ex = bbi_fix_exp(S.ax, Bd.n), ey = bbi_fix_exp(S.ay, Bd.n);
   // the charge per bin: frequency domain a line charge [C/s]
   // (macroEleCharge e / dz c, MPBunch.cpp:2172), time domain [C] (:2054)
   const double unit = p.td ? Bd.q_macro * kElectronCharge
                            : Bd.q_macro * kElectronCharge / p.dz * kCLight;
-  for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-    const int j = a + t - l;
-    s_raw[t] = (j >= 0 && j < W) ? cnt[base + j] * unit : 0.0;
+  const int smooth = p.td ? 1 : 3;  // profiles that are smoothed
+  for (int t = threadIdx.x; t < nr; t += kBbiConvThreads) {
+    const int j = a - kBbiHalf + t - l;
+    double r0 = 0, r1 = 0, r2 = 0;
+    if (j >= 0 && j < W) {
+      const int n0 = cnt[base + j];
+      r0 = n0 * unit;
+      const double sx = scalbn((double)(long long)sxy[2 * base + j], -ex);
+      const double sy = scalbn((double)(long long)sxy[2 * base + p.wcap + j], -ey);
+      if (!p.td) {  // the dipole profiles (MPBunch.cpp:2261-2273, 2304-2316)
+        r1 = unit * sx;
+        r2 = unit * sy;
+      } else if (n0 > 0) {
+        // mean x, y of the survivors over all the bin's particles (MPBunch.cpp:2061-2082)
+        r1 = sx / n0;
+        r2 = sy / n0;
+      }
+      // leave the accumulators zero for the next call
+      cnt[base + j] = 0;
+      sxy[2 * base + j] = 0ull;
+      sxy[2 * base + p.wcap + j] = 0ull;
+    }
+    s_raw[t] = r0;
+    s_raw[nr + t] = r1;
+    s_raw[2 * nr + t] = r2;
   }
   __syncthreads();
-  bbi_smooth(p, s_raw, s_p0, a, n, red);
-  if (!p.td) {
-    // the dipole profiles (MPBunch.cpp:2261-2273, 2304-2316)
-    for (int q = 0; q < 2; ++q) {
-      if (!p.sim[1 + q]) continue;
-      const int ee = q ? ey : ex;
-      for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-        const int j = a + t - l;
-        s_raw[t] = (j >= 0 && j < W)
-                       ? unit * scalbn((double)(long long)sxy[2 * base + q * p.wcap + j], -ee)
-                       : 0.0;
+  double sum[6] = {0, 0, 0, 0, 0, 0};  // raw and filtered sums of the profiles
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double* raw = s_raw + q * nr + kBbiHalf;
+    // the profiles one after the other over the threads
+    for (int t = ((int)threadIdx.x + kBbiConvThreads - q * n % kBbiConvThreads) % kBbiConvThreads;
+         t < n; t += kBbiConvThreads) {
+      const int i = a + t;
+      double y = raw[t];
+      if (q < smooth && i >= p.s0 && i < p.s1) {
+        if (i - kBbiHalf >= p.s0 && i + kBbiHalf < p.s1) {
+          double y0 = p.g[0] * raw[t - kBbiHalf], y1 = 0, y2 = 0;
+#pragma unroll
+          for (int k = 1; k <= 2 * kBbiHalf; k += 2) {
+            y1 = fma(p.g[k], raw[t + k - kBbiHalf], y1);
+            y2 = fma(p.g[k + 1], raw[t + k + 1 - kBbiHalf], y2);
+          }
+          y = y0 + (y1 + y2);
+        } else {
+          y = 0;
+          for (int k = -kBbiHalf; k <= kBbiHalf; ++k) {
+            int jj = i + k;
+            jj = jj < p.s0 ? p.s0 : (jj >= p.s1 ? p.s1 - 1 : jj);  // end-value padding
+            y = fma(p.g[k + kBbiHalf], jj >= a && jj <= e ? raw[jj - a] : 0.0, y);
+          }
+        }
+        sum[2 * q] += raw[t];
+        sum[2 * q + 1] += y;
       }
-      __syncthreads();
-      bbi_smooth(p, s_raw, q ? s_p2 : s_p1, a, n, red);
+      s_p[q * n + t] = y;
     }
-  } else {
-    // mean x, y of the survivors over all the bin's particles (MPBunch.cpp:2061-2082)
-    for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-      const int j = a + t - l;
-      double mx = 0, my = 0;
-      if (j >= 0 && j < W && cnt[base + j] > 0) {
-        const double c0 = cnt[base + j];
-        mx = scalbn((double)(long long)sxy[2 * base + j], -ex) / c0;
-        my = scalbn((double)(long long)sxy[2 * base + p.wcap + j], -ey) / c0;
-      }
-      s_p1[t] = mx;
-      s_p2[t] = my;
+  }
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_xor_sync(BBI_FULL, sum[q], o);
+  }
+  if ((threadIdx.x & 31) == 0)
+    for (int q = 0; q < 6; ++q) red[threadIdx.x >> 5][q] = sum[q];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      double v = red[threadIdx.x][q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(BBI_FULL, v, o);
+      sum[q] = v;
     }
-    __syncthreads();
+    // MPBunch.cpp:2404-2407 (0 / 0 when empty, as there)
+    if (threadIdx.x < 3) {
+      const double s0 = threadIdx.x == 0 ? sum[0] : threadIdx.x == 1 ? sum[2] : sum[4];
+      const double s1 = threadIdx.x == 0 ? sum[1] : threadIdx.x == 1 ? sum[3] : sum[5];
+      scale[threadIdx.x] = s0 / s1;
+    }
   }
-  // leave the accumulators zero for the next call
-  for (int j = threadIdx.x; j < W; j += kBbiThreads) {
-    cnt[base + j] = 0;
-    sxy[2 * base + j] = 0ull;
-    sxy[2 * base + p.wcap + j] = 0ull;
+  __syncthreads();
+  for (int t = threadIdx.x; t < smooth * n; t += kBbiConvThreads) {
+    const int q = t >= 2 * n ? 2 : t >= n ? 1 : 0, i = a + t - q * n;
+    if (i >= p.s0 && i < p.s1) s_p[t] *= scale[q];
   }
+  __syncthreads();
   double* out = pot + (size_t)b * 6 * p.wcap;
-  for (int t = threadIdx.x; t < n; t += kBbiThreads) {
-    out[t] = s_p0[t];
-    const int i = a + t;
-    double v[5] = {0, 0, 0, 0, 0};
-    if (i >= l && i <= h) {
+  for (int t = threadIdx.x; t < n; t += kBbiConvThreads) out[t] = s_p[t];
+  const int N = p.nbins;
+  for (int task = threadIdx.x; task < 5 * n; task += kBbiConvThreads) {
+    const int q = task / n, t = task - q * n, i = a + t;
+    double v = 0;
+    if (i >= l && i <= h && p.sim[q]) {
+      const double* wq = w + (size_t)q * p.nw;
+      double s[4] = {0, 0, 0, 0};
       if (!p.td) {
         // V_q(i) = sum_j P(j) w_q((i - j) mod N): the c2r of the profile's
         // spectrum times Z_q, over N (MPBunch.cpp:2193-2198 and after)
-        const int N = p.nbins;
-        for (int q = 0; q < 5; ++q) {
-          if (!p.sim[q]) continue;
-          const double* P = q == 1 ? s_p1 : (q == 2 ? s_p2 : s_p0);
-          const double* wq = w + (size_t)q * p.nw;
-          double s = 0;
-          for (int u = 0; u < n; ++u) {
-            int m = i - (a + u);
-            if (m < 0) m += N;
-            s = fma(P[u], __ldg(wq + m), s);
+        const double* P = s_p + (q == 1 ? n : q == 2 ? 2 * n : 0);
+        int u = 0;
+        for (; u + 4 <= n; u += 4)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int m = t - u - k;
+            s[k] = fma(P[u + k], __ldg(wq + (m < 0 ? m + N : m)), s[k]);
           }
-          v[q] = q == 0 ? -s : s;  // wakePotenZ = -temp / nBins (MPBunch.cpp:2198)
-        }
+        for (; u < n; ++u) s[0] = fma(P[u], __ldg(wq + (t - u < 0 ? t - u + N : t - u)), s[0]);
+        v = (s[0] + s[1]) + (s[2] + s[3]);
+        if (q == 0) v = -v;  // wakePotenZ = -temp / nBins (MPBunch.cpp:2198)
       } else {
         // the bins ahead, j = i .. (MPBunch.cpp:2102-2111), wake sample j - i
-        double t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0;
-        const int stop = min(e, i + p.nw - 1);
-        for (int j = i; j <= stop; ++j) {
-          const int u = j - i;
-          const double rho = s_p0[j - a];
-          if (p.sim[0]) t0 -= w[u] * rho;
-          if (p.sim[1]) t1 -= w[p.nw + u] * rho * s_p1[j - a];
-          if (p.sim[2]) t2 -= w[2 * p.nw + u] * rho * s_p2[j - a];
-          if (p.sim[3]) t3 -= w[3 * p.nw + u] * rho;
-          if (p.sim[4]) t4 -= w[4 * p.nw + u] * rho;
+        const double* P = s_p + t;
+        const double* D = q == 1 ? s_p + n + t : q == 2 ? s_p + 2 * n + t : nullptr;
+        const int m = min(e, i + p.nw - 1) - i + 1;
+        int u = 0;
+        for (; u + 4 <= m; u += 4)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const double f = __ldg(wq + u + k) * P[u + k];
+            s[k] = D ? fma(-f, D[u + k], s[k]) : s[k] - f;
+          }
+        for (; u < m; ++u) {
+          const double f = __ldg(wq + u) * P[u];
+          s[0] = D ? fma(-f, D[u], s[0]) : s[0] - f;
         }
-        v[0] = t0; v[1] = t1; v[2] = t2; v[3] = t3; v[4] = t4;
+        v = (s[0] + s[1]) + (s[2] + s[3]);
       }
     }
-#pragma unroll
-    for (int q = 0; q < 5; ++q) out[(size_t)(1 + q) * p.wcap + t] = v[q];
+    out[(size_t)(1 + q) * p.wcap + t] = v;
+    const double f = v / p.energy / p.beta2;
+    reinterpret_cast<double*>(kick + base + t)[q] =
+        q == 0 ? f : f / (q & 1 ? p.beta_x : p.beta_y);
   }
   if (threadIdx.x == 0) {
     win[b] = make_int2(a, n);
-    lo[b] = INT_MAX;
-    hi[b] = -1;
-    amax[2 * b] = amax[2 * b + 1] = 0ull;
+    span[b] = BbiSpan{0u, 0u, 0u, 0u};
   }
 }
 
 // The kicks (frequency domain MPBunch.cpp:2201-2342, time domain
-// MPBunch.cpp:2113-2121), each written in the reference's operation order.
+// MPBunch.cpp:2113-2121), the planes in the reference's order.
+template <bool MARK>
 __global__ void __launch_bounds__(kTile) k_bbi_kick(double* __restrict__ c, int64_t npad,
+                                                    uint8_t* __restrict__ surv,
                                                     const int* __restrict__ tile_bunch,
                                                     const BunchDev* __restrict__ bunch,
-                                                    BbiParams p, const int2* __restrict__ win,
-                                                    const double* __restrict__ pot) {
+                                                    const __grid_constant__ BbiParams p,
+                                                    const int2* __restrict__ win,
+                                                    const BbiKick* __restrict__ kick,
+                                                    const __grid_constant__ Aperture ap,
+                                                    int* loss_count) {
   const int b = tile_bunch[blockIdx.x];
   const BunchDev& Bd = bunch[b];
-  const int2 wn = win[b];
-  if (Bd.q_macro == 0 || wn.y == 0) return;
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  if (i >= Bd.n) return;
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int idx = bbi_bin(p, c[4 * npad + g]);
-  if (idx < 0) return;
-  const double* v = pot + (size_t)b * 6 * p.wcap + (idx - wn.x);
-  const double E = p.energy, b2 = p.beta2, bx = p.beta_x, by = p.beta_y;
-  const double x = c[g], y = c[2 * npad + g];
-  double px = c[npad + g], py = c[3 * npad + g], dp = c[5 * npad + g];
-  if (!p.td) {
-    if (p.sim[0]) dp += v[1 * p.wcap] / E / b2;
-    if (p.sim[3]) px += v[4 * p.wcap] / E / b2 * x / bx;
-    if (p.sim[4]) py += v[5 * p.wcap] / E / b2 * y / by;
-    if (p.sim[1]) px += v[2 * p.wcap] / E / b2 / bx;
-    if (p.sim[2]) py += v[3 * p.wcap] / E / b2 / by;
-  } else {
-    if (p.sim[0]) dp += v[1 * p.wcap] / E / b2;
-    if (p.sim[1]) px += v[2 * p.wcap] / E / b2 / bx;
-    if (p.sim[2]) py += v[3 * p.wcap] / E / b2 / by;
-    if (p.sim[3]) px += v[4 * p.wcap] / E / b2 / bx * x;
-    if (p.sim[4]) py += v[5 * p.wcap] / E / b2 / by * y;
+  const bool valid = (blockIdx.x - Bd.tile_off) * kTile + (int)threadIdx.x < Bd.n;
+  double x = 0, y = 0, z = 0;
+  if (valid) {
+    x = c[g];
+    y = c[2 * npad + g];
+    z = c[4 * npad + g];
   }
-  c[npad + g] = px;
-  c[3 * npad + g] = py;
-  c[5 * npad + g] = dp;
+  const int2 wn = win[b];
+  const int idx = valid && Bd.q_macro != 0 && wn.y != 0 ? bbi_bin(p, z) : -1;
+  if (idx >= 0) {
+    double px = c[npad + g], py = c[3 * npad + g], dp = c[5 * npad + g];
+    const double2* K = reinterpret_cast<const double2*>(kick + (size_t)b * p.wcap + (idx - wn.x));
+    const double2 k0 = K[0], k1 = K[1];
+    const double qy = K[2].x;
+    if (p.sim[0]) dp += k0.x;
+    if (!p.td) {
+      if (p.sim[3]) px = fma(k1.y, x, px);
+      if (p.sim[4]) py = fma(qy, y, py);
+      if (p.sim[1]) px += k0.y;
+      if (p.sim[2]) py += k1.x;
+    } else {
+      if (p.sim[1]) px += k0.y;
+      if (p.sim[2]) py += k1.x;
+      if (p.sim[3]) px = fma(k1.y, x, px);
+      if (p.sim[4]) py = fma(qy, y, py);
+    }
+    c[npad + g] = px;
+    c[3 * npad + g] = py;
+    c[5 * npad + g] = dp;
+  }
+  if (MARK) mark_lost_warp(ap, valid, x, y, z, surv + g, loss_count + b);
 }
 
-cudaError_t launch_bbi(Handle& h) {
+size_t bbi_span_bytes() { return sizeof(BbiSpan); }
+
+cudaError_t launch_bbi(Handle& h, bool have_range, bool mark) {
   const BbiParams& p = h.bbi;
-  k_bbi_range<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                 h.d.bunch, p, h.d.bbi_lo, h.d.bbi_hi,
-                                                 h.d.bbi_amax, h.d.status);
-  k_bbi_hist<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                h.d.bunch, p, h.d.bbi_lo, h.d.bbi_hi,
-                                                h.d.bbi_amax, h.d.bbi_cnt, h.d.bbi_sxy,
-                                                h.d.status);
-  k_bbi_conv<<<h.M, kBbiThreads, bbi_conv_smem(p), h.stream>>>(
-      h.d.bunch, p, h.d.bbi_w, h.d.bbi_lo, h.d.bbi_hi, h.d.bbi_amax, h.d.bbi_cnt, h.d.bbi_sxy,
-      h.d.bbi_pot, h.d.bbi_win);
-  k_bbi_kick<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.tile_bunch, h.d.bunch, p,
-                                                h.d.bbi_win, h.d.bbi_pot);
+  BbiSpan* span = reinterpret_cast<BbiSpan*>(h.d.bbi_span);
+  BbiKick* kick = reinterpret_cast<BbiKick*>(h.d.bbi_kick);
+  if (!have_range)
+    k_bbi_range<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
+                                                   h.d.bunch, p, span, h.d.status);
+  k_bbi_hist<<<h.n_chunks, kBbiThreads, 5 * sizeof(unsigned) * std::min(p.wcap, kBbiSharedBins),
+               h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.d.bunch, p, span, h.d.status,
+                           h.d.bbi_cnt, h.d.bbi_sxy);
+  k_bbi_conv<<<h.M, kBbiConvThreads, bbi_conv_smem(p), h.stream>>>(
+      h.d.bunch, p, h.d.bbi_w, span, h.d.bbi_cnt, h.d.bbi_sxy, h.d.bbi_pot, kick, h.d.bbi_win);
+  (mark ? k_bbi_kick<true> : k_bbi_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(
+      h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, p, h.d.bbi_win, kick, aperture(h),
+      h.d.loss_count);
   return cudaGetLastError();
 }
 
-size_t bbi_conv_smem(const BbiParams& p) { return (size_t)4 * p.wcap * sizeof(double); }
+size_t bbi_kick_bytes() { return sizeof(BbiKick); }
+
+size_t bbi_conv_smem(const BbiParams& p) {
+  return (size_t)(6 * p.wcap + 6 * kBbiHalf) * sizeof(double);
+}
 
 cudaError_t prepare_bbi(const BbiParams& p) {
   return cudaFuncSetAttribute(k_bbi_conv, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -117,10 +117,11 @@ void free_beam(Handle& h) {
   dfree(d.rf_info); dfree(d.rf_work);
   d.res_state = nullptr; d.rf_zr = nullptr; d.rf_counts = nullptr; d.rf_kick = nullptr;
   d.rf_fbk = nullptr; d.rf_info = nullptr; d.rf_work = nullptr;
-  dfree(d.bbi_lo); dfree(d.bbi_hi); dfree(d.bbi_amax); dfree(d.bbi_cnt); dfree(d.bbi_sxy);
-  dfree(d.bbi_pot); dfree(d.bbi_win);
-  d.bbi_lo = nullptr; d.bbi_hi = nullptr; d.bbi_amax = nullptr; d.bbi_cnt = nullptr;
-  d.bbi_sxy = nullptr; d.bbi_pot = nullptr; d.bbi_win = nullptr;
+  dfree(d.bbi_span); dfree(d.bbi_cnt); dfree(d.bbi_sxy);
+  dfree(d.bbi_pot); dfree(d.bbi_kick); dfree(d.bbi_win);
+  d.bbi_span = nullptr; d.bbi_cnt = nullptr;
+  d.bbi_sxy = nullptr; d.bbi_pot = nullptr; d.bbi_kick = nullptr;
+  d.bbi_win = nullptr;
   for (double* b : h.phase_bufs) dfree(b);
   h.phase_bufs.clear();
   h.phase_bunches.clear();
@@ -425,6 +426,7 @@ static std::string bbi_plan(const cg_config& cfg, BbiParams& p, std::vector<doub
     p.s1 = p.nbins;
   }
   p.wcap = std::min(CG_BBI_MAX_BINS, p.nbins) + 2 * kBbiHalf;
+  p.inv_dz = 1.0 / p.dz;
   p.energy = r.electron_energy;
   p.beta2 = std::pow(r.r_beta, 2);
   p.beta_x = cfg.sections[0].beta_x;
@@ -982,16 +984,15 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   }
   if (h.cfg.bbi.flag) {
     const size_t wc = h.bbi.wcap;
-    if (dalloc(&d.bbi_lo, (size_t)M) || dalloc(&d.bbi_hi, (size_t)M) ||
-        dalloc(&d.bbi_amax, 2 * (size_t)M) || dalloc(&d.bbi_cnt, (size_t)M * wc) ||
+    if (dalloc(reinterpret_cast<char**>(&d.bbi_span), bbi_span_bytes() * M) ||
+        dalloc(&d.bbi_cnt, (size_t)M * wc) ||
         dalloc(&d.bbi_sxy, 2 * (size_t)M * wc) || dalloc(&d.bbi_pot, 6 * (size_t)M * wc) ||
-        dalloc(&d.bbi_win, (size_t)M)) {
+        dalloc(&d.bbi_win, (size_t)M) ||
+        dalloc(reinterpret_cast<char**>(&d.bbi_kick), bbi_kick_bytes() * M * wc)) {
       free_beam(h);
       return fail(&h, CG_ERR_OOM, "broadband-impedance buffers");
     }
-    cudaMemset(d.bbi_lo, 0x7f, sizeof(int) * M);  // above every bin
-    cudaMemset(d.bbi_hi, 0xff, sizeof(int) * M);  // -1
-    cudaMemset(d.bbi_amax, 0, sizeof(unsigned long long) * 2 * M);
+    cudaMemset(d.bbi_span, 0, bbi_span_bytes() * M);
     cudaMemset(d.bbi_cnt, 0, sizeof(int) * M * wc);
     cudaMemset(d.bbi_sxy, 0, sizeof(unsigned long long) * 2 * M * wc);
     cudaMemset(d.bbi_pot, 0, sizeof(double) * 6 * M * wc);
@@ -1229,7 +1230,7 @@ int cg_space_charge(cg_handle* H, int k) {
 int cg_bbi_kick(cg_handle* H) {
   STAGE_PROLOGUE
   if (!h.cfg.bbi.flag) return fail(&h, CG_ERR_NOT_READY, "runBBIFlag is off");
-  int st = launch_ok(h, launch_bbi(h), "bbi");
+  int st = launch_ok(h, launch_bbi(h, false, false), "bbi");
   return st ? st : check_status(h);
 }
 int cg_bbi_profile(cg_handle* H, int j, int* lo, int* n, double* out, int cap) {
@@ -1473,13 +1474,14 @@ static cudaError_t enqueue_turn(Handle& h) {
   if (c.flag_lr_wake && !c.bbi.flag) fl |= kLongLR;
   // and the loss check, unless a stage in between takes the survivors of the
   // turn before
-  const bool mark = !c.bbi.flag && !c.flag_sr_wake && !c.flag_fir;
-  if (mark) fl |= kLongMark;
+  const bool mark = !c.flag_sr_wake && !c.flag_fir;
+  if (c.bbi.flag) fl |= kLongBbi;
+  else if (mark) fl |= kLongMark;
   if ((e = launch_long(h, fl))) return e;
   TRACE(h.stream, CG_TRACE_LONG, -1, -1);
   if (c.bbi.flag) {
-    if ((e = launch_bbi(h))) return e;
-    if (c.flag_lr_wake && (e = launch_lr_kick(h))) return e;
+    if ((e = launch_bbi(h, true, mark && !c.flag_lr_wake))) return e;
+    if (c.flag_lr_wake && (e = launch_long(h, kLongLR | (mark ? kLongMark : 0u)))) return e;
   }
   if (c.flag_sr_wake) {
     if ((e = launch_sr_wake(h))) return e;

@@ -31,6 +31,7 @@ struct BbiParams {
   int s0 = 0, s1 = 0;          // the filter runs over the bins [s0, s1)
   int wcap = 0;                // bins kept per bunch: min(CG_BBI_MAX_BINS, nbins) + 2 kBbiHalf
   double zmin = 0, dz = 0;     // left edge of bin 0 (frequency domain: its centre), width
+  double inv_dz = 0;
   double energy = 0, beta2 = 0;  // electronBeamEnergy, pow(rBeta, 2)
   double beta_x = 0, beta_y = 0; // twissBetaX[0], twissBetaY[0]
   double g[2 * kBbiHalf + 1];  // normalised Gaussian filter kernel
@@ -156,12 +157,11 @@ struct DeviceBufs {
   double* rf_info = nullptr;       // M x CG_MAX_CAVITIES x 8: BunchRFModeInfo
   // broadband impedance
   double* bbi_w = nullptr;         // 5 x nw wake samples (planes Z, Dx, Dy, Qx, Qy)
-  int* bbi_lo = nullptr;           // M: lowest bin holding a particle (INT_MAX between calls)
-  int* bbi_hi = nullptr;           // M: highest (-1 between calls)
-  unsigned long long* bbi_amax = nullptr;  // M x 2: largest |x|, |y| (bit patterns)
+  void* bbi_span = nullptr;        // M: bin range and largest |x|, |y| (empty between calls)
   int* bbi_cnt = nullptr;          // M x wcap per-bin counts (zero between calls)
   unsigned long long* bbi_sxy = nullptr;  // M x 2 x wcap fixed-point sums of x, y
   double* bbi_pot = nullptr;       // M x 6 x wcap: profile and potentials of the last kick
+  void* bbi_kick = nullptr;        // M x wcap: the bins' kicks
   int2* bbi_win = nullptr;         // M: first bin and bin count of bbi_pot
   // space charge
   double* sc_geom = nullptr;       // M x kScGeom: slices, mesh, fixed-point scales

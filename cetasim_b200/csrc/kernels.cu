@@ -11,6 +11,7 @@
 #include <algorithm>
 #include "kernels.cuh"
 #include "normals.cuh"
+#include "turn_tail.cuh"
 
 namespace cg {
 
@@ -607,34 +608,12 @@ cudaError_t launch_ion_kick(Handle& h, int k) { return launch_ion_kick_variant(h
 //
 // If nothing after it in the turn depends on the survival marks before the
 // loss check (kLongMark), the check is made here on the final position; the
-// bunches' counts end up in the transmission (k_turn_end).
+// bunches' counts end up in the transmission (k_turn_end).  If the broadband
+// impedance comes next (kLongBbi), its bunches' bin ranges are collected.
 
-// Bunch::MarkLostParticle (Bunch.cpp:172-200) for the warp's particles, their
-// number of loss conditions added to the bunch's.  A position clearly inside
-// the aperture by the reciprocals takes no division; the others take the
-// reference's.
-struct Aperture {
-  double ax, ay, iax, iay;
-};
-__device__ __forceinline__ void mark_lost_warp(const RingDev& r, const Aperture& ap, bool valid,
-                                               double x, double y, double z, uint8_t* surv,
-                                               int* loss_count) {
-  const double tx = x * ap.iax, ty = y * ap.iay;
-  int count = 0;
-  if (valid && !(fma(tx, tx, ty * ty) < 0.999 && fabs(z) <= r.z_loss)) {
-    uint8_t s = *surv;
-    count = mark_lost_particle(r, ap.ax, ap.ay, x, y, z, &s);
-    if (count) *surv = s;
-  }
-  if (__any_sync(FULL_MASK, count)) {
-    count = __reduce_add_sync(FULL_MASK, count);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss_count, count);
-  }
-}
-
-// LOADING: some cavity has beam loading; MARK: kLongMark
-template <bool LOADING, bool MARK>
-__global__ void __launch_bounds__(kTile, 3) k_long(double* __restrict__ c, int64_t npad,
+// LOADING: some cavity has beam loading; TAIL: kLongMark or kLongBbi
+template <bool LOADING, unsigned TAIL>
+__global__ void __launch_bounds__(kTile, 4) k_long(double* __restrict__ c, int64_t npad,
                                                   uint8_t* __restrict__ surv,
                                                   const int* __restrict__ tile_bunch,
                                                   const BunchDev* __restrict__ bunch,
@@ -648,12 +627,15 @@ __global__ void __launch_bounds__(kTile, 3) k_long(double* __restrict__ c, int64
                                                   const double* __restrict__ rf_fbk, int M,
                                                   double* rf_info,
                                                   const __grid_constant__ Aperture ap,
-                                                  int* loss_count) {
+                                                  int* loss_count,
+                                                  const __grid_constant__ BbiParams bbi,
+                                                  BbiSpan* span, int* status) {
   TileIdx t = tile_index(tile_bunch, bunch);
   double v[6] = {0, 0, 0, 0, 0, 0};
+  bool alive = false;
   if (t.valid) {
     load6(c, npad, t.g, v);
-    const bool alive = (LOADING || (flags & kLongSynrad)) && surv[t.g] == kAlive;
+    alive = (LOADING || TAIL == kLongBbi || (flags & kLongSynrad)) && surv[t.g] == kAlive;
     if (flags & kLongRF) {
       if (t.i == bunch[t.b].n - 1) {
         // the ideal cavities' BunchRFModeInfo: the voltage the bunch's last
@@ -690,7 +672,11 @@ __global__ void __launch_bounds__(kTile, 3) k_long(double* __restrict__ c, int64
     }
     store6(c, npad, t.g, v);
   }
-  if (MARK) mark_lost_warp(r, ap, t.valid, v[0], v[2], v[4], surv + t.g, loss_count + t.b);
+  if (TAIL == kLongMark)
+    mark_lost_warp(ap, t.valid, v[0], v[2], v[4], surv + t.g, loss_count + t.b);
+  if (TAIL == kLongBbi)
+    bbi_span_cta(bbi, span + t.b, status, t.valid && bunch[t.b].q_macro != 0, alive, v[0], v[2],
+                 v[4]);
 }
 
 // The accumulated phase advance of the tracked bunches' particles
@@ -766,9 +752,9 @@ cudaError_t launch_phase_adv(Handle& h, int ja, int jb, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-static Aperture aperture(const Handle& h) {
+Aperture aperture(const Handle& h) {
   const cg_section& s = h.sections[0];
-  return {s.aperture_x, s.aperture_y, 1.0 / s.aperture_x, 1.0 / s.aperture_y};
+  return {s.aperture_x, s.aperture_y, 1.0 / s.aperture_x, 1.0 / s.aperture_y, h.ring.z_loss};
 }
 
 cudaError_t launch_long(Handle& h, unsigned flags) {
@@ -777,13 +763,16 @@ cudaError_t launch_long(Handle& h, unsigned flags) {
     cudaError_t e = launch_rf_beam_loading(h);
     if (e != cudaSuccess) return e;
   }
-  const bool mark = flags & kLongMark;
-  auto kern = h.ring.bl_any ? (mark ? k_long<true, true> : k_long<true, false>)
-                            : (mark ? k_long<false, true> : k_long<false, false>);
+  auto pick = [&](auto none, auto mark, auto bbi) {
+    return flags & kLongMark ? mark : flags & kLongBbi ? bbi : none;
+  };
+  auto kern = h.ring.bl_any ? pick(k_long<true, 0>, k_long<true, kLongMark>, k_long<true, kLongBbi>)
+                            : pick(k_long<false, 0>, k_long<false, kLongMark>, k_long<false, kLongBbi>);
   kern<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
                                           h.sec_dev_host[0], h.ring, flags, h.cfg.seed, h.d.turn,
                                           h.d.lr_force, h.d.rf_zr, h.d.rf_kick, h.d.rf_fbk, h.M,
-                                          h.d.rf_info, aperture(h), h.d.loss_count);
+                                          h.d.rf_info, aperture(h), h.d.loss_count, h.bbi,
+                                          reinterpret_cast<BbiSpan*>(h.d.bbi_span), h.d.status);
   return cudaGetLastError();
 }
 
@@ -950,7 +939,6 @@ __global__ void __launch_bounds__(kTile) k_mark_lost(double* __restrict__ c, int
                                                      uint8_t* __restrict__ surv,
                                                      const int* __restrict__ tile_bunch,
                                                      const BunchDev* __restrict__ bunch,
-                                                     const __grid_constant__ RingDev r,
                                                      const __grid_constant__ Aperture ap, int mode,
                                                      const double* __restrict__ fir_kick,
                                                      double inv_beta2, int* loss_count, bool mark) {
@@ -969,7 +957,7 @@ __global__ void __launch_bounds__(kTile) k_mark_lost(double* __restrict__ c, int
     y = c[2 * npad + t.g];
     z = c[4 * npad + t.g];
   }
-  mark_lost_warp(r, ap, t.valid, x, y, z, surv + t.g, loss_count + t.b);
+  mark_lost_warp(ap, t.valid, x, y, z, surv + t.g, loss_count + t.b);
 }
 
 cudaError_t launch_mark_lost(Handle& h, bool fir_kick, bool mark) {
@@ -977,7 +965,7 @@ cudaError_t launch_mark_lost(Handle& h, bool fir_kick, bool mark) {
   if (fir_kick) mode = (h.cfg.fir.mode == 0) ? 2 : 1;
   double inv_beta2 = 1.0 / (h.cfg.ring.r_beta * h.cfg.ring.r_beta);
   k_mark_lost<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                 h.d.bunch, h.ring, aperture(h), mode,
+                                                 h.d.bunch, aperture(h), mode,
                                                  h.d.fir_kick, inv_beta2, h.d.loss_count, mark);
   return cudaGetLastError();
 }

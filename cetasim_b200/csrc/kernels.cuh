@@ -29,7 +29,11 @@ size_t sc_slice_bytes();  // of one slice's constants (slice models)
 cudaError_t prepare_sc(const ScParams& p);
 
 // broadband impedance (bbi.cu)
-cudaError_t launch_bbi(Handle& h);
+// the bunches' ranges already collected by the longitudinal pass; the loss
+// check with the kick
+cudaError_t launch_bbi(Handle& h, bool have_range, bool mark);
+size_t bbi_kick_bytes();  // of one bin's kicks
+size_t bbi_span_bytes();  // of one bunch's span
 size_t bbi_conv_smem(const BbiParams& p);
 cudaError_t prepare_bbi(const BbiParams& p);
 // w (5 x (2n - 1)) from the impedances X (5 x n, device) on stream st
@@ -72,6 +76,7 @@ enum LongFlags : unsigned {
   kLongSynrad = 8,
   kLongLR = 16,
   kLongMark = 32,  // the loss check too
+  kLongBbi = 64,   // the broadband impedance's ranges too (not with kLongMark)
 };
 cudaError_t launch_long(Handle& h, unsigned flags);
 // cavities with beam loading: z ranges and bins of the RF step, then the

@@ -47,6 +47,7 @@
 
 #include "be_field.cuh"
 #include "kernels.cuh"
+#include "turn_tail.cuh"
 
 namespace cg {
 
@@ -224,15 +225,6 @@ __device__ __forceinline__ bool sc_cell(double x, double y, const double* G, con
   return true;
 }
 
-// A 64-bit sum in shared memory as two words (a 64-bit shared atomic is a
-// compare-and-swap loop, which retries under contention; the carry of a 32-bit
-// add is exact).
-__device__ __forceinline__ void sc_add64(unsigned* lo, unsigned* hi, long long v) {
-  const unsigned vl = (unsigned)v, old = atomicAdd(lo, vl);
-  const unsigned vh = (unsigned)((unsigned long long)v >> 32) + (old + vl < vl ? 1u : 0u);
-  if (vh) atomicAdd(hi, vh);
-}
-
 // Slices up to which a CTA keeps its counts (and the models' sums) in shared
 // memory; beyond, it adds to the bunch's directly.
 constexpr int kScSharedSlices = 1024;
@@ -254,6 +246,9 @@ __global__ void __launch_bounds__(kScThreads) k_sc_count(const double* __restric
     __syncthreads();
   }
   const size_t b0 = (size_t)l.x * nz;
+  Pow2 f[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) f[q] = PIC ? Pow2{0, 0} : pow2_split((int)G[kGExp0 + q]);
   int64_t g = (int64_t)l.y * kTile + threadIdx.x;
   for (int u = 0; u < l.z; ++u, g += kTile) {
     if (surv[g] == kPadding) break;
@@ -265,8 +260,8 @@ __global__ void __launch_bounds__(kScThreads) k_sc_count(const double* __restric
       const double v[4] = {dx, dy, dx * dx, dy * dy};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const long long t = __double2ll_rn(scalbn(v[q], (int)G[kGExp0 + q]));
-        if (shared) sc_add64(&s_sum[(1 + 2 * q) * nz + s], &s_sum[(2 + 2 * q) * nz + s], t);
+        const long long t = __double2ll_rn(pow2_scale(v[q], f[q]));
+        if (shared) add64_split(&s_sum[(1 + 2 * q) * nz + s], &s_sum[(2 + 2 * q) * nz + s], t);
         else atomicAdd(&acc[(b0 + s) * 4 + q], (unsigned long long)t);
       }
     }
@@ -453,7 +448,7 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const Bunch
     if (!sc_cell(v.x, v.y, G, p, &ix, &iy, w)) continue;
     const int node[4] = {ix * ny + iy, (ix + 1) * ny + iy, ix * ny + iy + 1, (ix + 1) * ny + iy + 1};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sc_add64(&lo[node[j]], &hi[node[j]], __double2ll_rn(w[j] * unit));
+    for (int j = 0; j < 4; ++j) add64_split(&lo[node[j]], &hi[node[j]], __double2ll_rn(w[j] * unit));
   }
   __syncthreads();
   for (int t = threadIdx.x; t < px * ly; t += kScThreads) {

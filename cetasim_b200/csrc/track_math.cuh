@@ -222,10 +222,10 @@ CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
 // Bunch::MarkLostParticle per particle (Bunch.cpp:179-191): returns the
 // number of loss conditions met (0, 1 or 2; the reference counts both) and
 // updates the survival code.
-CG_HD int mark_lost_particle(const RingDev& r, double ax, double ay, double x, double y, double z,
+CG_HD int mark_lost_particle(double z_loss, double ax, double ay, double x, double y, double z,
                              uint8_t* surv) {
   int count = 0;
-  if (fabs(z) > r.z_loss) {
+  if (fabs(z) > z_loss) {
     *surv = 2;
     count++;
   }
