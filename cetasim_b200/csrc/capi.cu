@@ -106,6 +106,7 @@ void free_beam(Handle& h) {
   dfree(d.wpartials);
   dfree(d.counters); dfree(d.mom); dfree(d.loss_count); dfree(d.scratch);
   dfree(d.rec); dfree(d.rec_prep); dfree(d.lr_hist); dfree(d.lr_force); dfree(d.fir_hist); dfree(d.fir_kick);
+  dfree(d.sr_span); d.sr_span = nullptr;
   dfree(d.sr_geom); dfree(d.sr_counts); dfree(d.sr_sumx); dfree(d.sr_sumy); dfree(d.sr_lag);
   dfree(d.sr_pot); dfree(d.sr_potxy);
   d.sr_potxy = nullptr;
@@ -954,7 +955,8 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   }
   if (h.cfg.flag_sr_wake) {
     int B = h.cfg.sr_bins;
-    if (dalloc(&d.sr_geom, 2 * (size_t)M) || dalloc(&d.sr_counts, (size_t)M * B) ||
+    if (dalloc(reinterpret_cast<char**>(&d.sr_span), sr_span_bytes() * M) ||
+        dalloc(&d.sr_geom, 2 * (size_t)M) || dalloc(&d.sr_counts, (size_t)M * B) ||
         dalloc(&d.sr_sumx, (size_t)M * B) || dalloc(&d.sr_sumy, (size_t)M * B) ||
         dalloc(&d.sr_lag, (size_t)M * 3 * (2 * B - 1)) || dalloc(&d.sr_pot, (size_t)M * B) ||
         (h.sr_xy && dalloc(&d.sr_potxy, (size_t)M * 2 * B))) {
@@ -962,6 +964,7 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
       return fail(&h, CG_ERR_OOM, "SR buffers");
     }
     cudaMemset(d.sr_pot, 0, sizeof(double) * M * B);
+    cudaMemset(d.sr_span, 0, sr_span_bytes() * M);
     if (d.sr_potxy) cudaMemset(d.sr_potxy, 0, sizeof(double) * M * 2 * B);
   }
   if (h.cfg.flag_sc) {
@@ -1261,7 +1264,7 @@ int cg_sr_wake(cg_handle* H, int turn) {
   STAGE_PROLOGUE
   (void)turn;
   if (!h.cfg.flag_sr_wake) return fail(&h, CG_ERR_NOT_READY, "runShortRangeWake is off");
-  int st = launch_ok(h, launch_sr_wake(h), "sr");
+  int st = launch_ok(h, launch_sr_wake(h, false, false), "sr");
   return st ? st : check_status(h);
 }
 int cg_set_sr_potentials(cg_handle* H, int on) {
@@ -1472,19 +1475,20 @@ static cudaError_t enqueue_turn(Handle& h) {
   // the LR kick joins the longitudinal kernel unless the broadband impedance
   // kicks in between (MPBeam.cpp:1084-1085)
   if (c.flag_lr_wake && !c.bbi.flag) fl |= kLongLR;
-  // and the loss check, unless a stage in between takes the survivors of the
-  // turn before
+  // the loss check with the last of the kicks, unless the feedback takes the
+  // survivors of the turn before
   const bool mark = !c.flag_sr_wake && !c.flag_fir;
-  if (c.bbi.flag) fl |= kLongBbi;
-  else if (mark) fl |= kLongMark;
+  // or the ranges of the kick after it
+  const unsigned tail = c.flag_sr_wake ? kLongSr : mark ? kLongMark : 0u;
+  fl |= c.bbi.flag ? kLongBbi : tail;
   if ((e = launch_long(h, fl))) return e;
   TRACE(h.stream, CG_TRACE_LONG, -1, -1);
   if (c.bbi.flag) {
     if ((e = launch_bbi(h, true, mark && !c.flag_lr_wake))) return e;
-    if (c.flag_lr_wake && (e = launch_long(h, kLongLR | (mark ? kLongMark : 0u)))) return e;
+    if (c.flag_lr_wake && (e = launch_long(h, kLongLR | tail))) return e;
   }
   if (c.flag_sr_wake) {
-    if ((e = launch_sr_wake(h))) return e;
+    if ((e = launch_sr_wake(h, !c.bbi.flag || c.flag_lr_wake, !c.flag_fir))) return e;
     TRACE(h.stream, CG_TRACE_SR_WAKE, -1, -1);
   }
   if (c.flag_fir) {
@@ -1493,7 +1497,7 @@ static cudaError_t enqueue_turn(Handle& h) {
     if ((e = launch_fir_compute(h))) return e;
     TRACE(h.stream, CG_TRACE_FIR, -1, -1);
   }
-  if (!mark && (e = launch_mark_lost(h, c.flag_fir != 0, true))) return e;
+  if (c.flag_fir && (e = launch_mark_lost(h, true, true))) return e;
   if ((e = launch_turn_end(h, true))) return e;
   TRACE(h.stream, CG_TRACE_MARK_LOST, -1, -1);
   return cudaSuccess;

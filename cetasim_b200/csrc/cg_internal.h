@@ -136,6 +136,7 @@ struct DeviceBufs {
   double* fir_kick = nullptr;      // M x 3
   double* fir_coeff = nullptr;     // 3 x order
   // short-range wake
+  void* sr_span = nullptr;         // M: range of z (empty between calls)
   double* sr_geom = nullptr;       // M x 2 (zlo, dz)
   int* sr_counts = nullptr;        // M x B
   double* sr_sumx = nullptr;       // M x B

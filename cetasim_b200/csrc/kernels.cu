@@ -609,9 +609,10 @@ cudaError_t launch_ion_kick(Handle& h, int k) { return launch_ion_kick_variant(h
 // If nothing after it in the turn depends on the survival marks before the
 // loss check (kLongMark), the check is made here on the final position; the
 // bunches' counts end up in the transmission (k_turn_end).  If the broadband
-// impedance comes next (kLongBbi), its bunches' bin ranges are collected.
+// impedance (kLongBbi) or the short-range wake (kLongSr) comes next, the
+// bunches' ranges that it starts from are collected.
 
-// LOADING: some cavity has beam loading; TAIL: kLongMark or kLongBbi
+// LOADING: some cavity has beam loading; TAIL: kLongMark, kLongBbi or kLongSr
 template <bool LOADING, unsigned TAIL>
 __global__ void __launch_bounds__(kTile, 4) k_long(double* __restrict__ c, int64_t npad,
                                                   uint8_t* __restrict__ surv,
@@ -629,13 +630,13 @@ __global__ void __launch_bounds__(kTile, 4) k_long(double* __restrict__ c, int64
                                                   const __grid_constant__ Aperture ap,
                                                   int* loss_count,
                                                   const __grid_constant__ BbiParams bbi,
-                                                  BbiSpan* span, int* status) {
+                                                  BbiSpan* span, int* status, const SrDev sr) {
   TileIdx t = tile_index(tile_bunch, bunch);
   double v[6] = {0, 0, 0, 0, 0, 0};
   bool alive = false;
   if (t.valid) {
     load6(c, npad, t.g, v);
-    alive = (LOADING || TAIL == kLongBbi || (flags & kLongSynrad)) && surv[t.g] == kAlive;
+    alive = (LOADING || TAIL == kLongBbi || TAIL == kLongSr || (flags & kLongSynrad)) && surv[t.g] == kAlive;
     if (flags & kLongRF) {
       if (t.i == bunch[t.b].n - 1) {
         // the ideal cavities' BunchRFModeInfo: the voltage the bunch's last
@@ -677,6 +678,7 @@ __global__ void __launch_bounds__(kTile, 4) k_long(double* __restrict__ c, int64
   if (TAIL == kLongBbi)
     bbi_span_cta(bbi, span + t.b, status, t.valid && bunch[t.b].q_macro != 0, alive, v[0], v[2],
                  v[4]);
+  if (TAIL == kLongSr) sr_span_cta(sr, t.b, (int)blockIdx.x == bunch[t.b].tile_off, alive, v[4]);
 }
 
 // The accumulated phase advance of the tracked bunches' particles
@@ -763,16 +765,19 @@ cudaError_t launch_long(Handle& h, unsigned flags) {
     cudaError_t e = launch_rf_beam_loading(h);
     if (e != cudaSuccess) return e;
   }
-  auto pick = [&](auto none, auto mark, auto bbi) {
-    return flags & kLongMark ? mark : flags & kLongBbi ? bbi : none;
+  auto pick = [&](auto none, auto mark, auto bbi, auto sr) {
+    return flags & kLongMark ? mark : flags & kLongBbi ? bbi : flags & kLongSr ? sr : none;
   };
-  auto kern = h.ring.bl_any ? pick(k_long<true, 0>, k_long<true, kLongMark>, k_long<true, kLongBbi>)
-                            : pick(k_long<false, 0>, k_long<false, kLongMark>, k_long<false, kLongBbi>);
+  auto kern = h.ring.bl_any ? pick(k_long<true, 0>, k_long<true, kLongMark>, k_long<true, kLongBbi>,
+                                   k_long<true, kLongSr>)
+                            : pick(k_long<false, 0>, k_long<false, kLongMark>,
+                                   k_long<false, kLongBbi>, k_long<false, kLongSr>);
   kern<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
                                           h.sec_dev_host[0], h.ring, flags, h.cfg.seed, h.d.turn,
                                           h.d.lr_force, h.d.rf_zr, h.d.rf_kick, h.d.rf_fbk, h.M,
                                           h.d.rf_info, aperture(h), h.d.loss_count, h.bbi,
-                                          reinterpret_cast<BbiSpan*>(h.d.bbi_span), h.d.status);
+                                          reinterpret_cast<BbiSpan*>(h.d.bbi_span), h.d.status,
+                                          sr_dev(h));
   return cudaGetLastError();
 }
 

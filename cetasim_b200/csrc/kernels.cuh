@@ -76,7 +76,9 @@ enum LongFlags : unsigned {
   kLongSynrad = 8,
   kLongLR = 16,
   kLongMark = 32,  // the loss check too
-  kLongBbi = 64,   // the broadband impedance's ranges too (not with kLongMark)
+  // or the ranges of the broadband impedance or of the short-range wake
+  kLongBbi = 64,
+  kLongSr = 128,
 };
 cudaError_t launch_long(Handle& h, unsigned flags);
 // cavities with beam loading: z ranges and bins of the RF step, then the
@@ -92,7 +94,8 @@ cudaError_t launch_fir_compute(Handle& h);
 cudaError_t launch_mark_lost(Handle& h, bool fir_kick, bool mark);
 // after the loss check: the transmissions; the turn counter if `advance`
 cudaError_t launch_turn_end(Handle& h, bool advance);
-cudaError_t launch_sr_wake(Handle& h);
+cudaError_t launch_sr_wake(Handle& h, bool have_range, bool mark);  // as launch_bbi
+size_t sr_span_bytes();
 cudaError_t launch_gaussian(Handle& h, double emit_x, double emit_y, double sigma_z,
                             double sigma_dp, uint64_t seed);
 cudaError_t launch_faddeeva(const double* zr, const double* zi, double* wr, double* wi, int64_t n,

@@ -1,14 +1,17 @@
 // Short-range wake (MPBunch::BunchTransferDueToSRWake, MPBunch.cpp:1887-2025).
 //
-//  k_sr_geom  per-bunch bin geometry from the alive z range (GetZMinMax,
-//             MPBunch.cpp:1860-1884) and the last rms bunch length:
-//             [zMin - 2 sigma_z, zMax + 2 sigma_z] in B bins.
-//  k_sr_hist  shared-memory histogram with warp-aggregated atomics
-//             (__match_any_sync groups lanes hitting the same bin), integer
-//             counts so the result is exact and order-independent; per-bin
-//             sums of x and y over alive particles for the transverse
-//             potentials.
-//  k_sr_lag   the 1 mm pseudo-Green wake W_z at the 2B-1 distinct lags
+//  k_sr_range per-bunch range of z over the survivors (GetZMinMax,
+//             MPBunch.cpp:1860-1884), and the last call's counts cleared; in
+//             the turn the longitudinal pass before it does this with the
+//             positions that it writes (sr_span_cta).
+//  k_sr_bins  two independent jobs in one launch.  Histogram CTAs: the
+//             bunch's bins [zMin - 2 sigma_z, zMax + 2 sigma_z] (the last rms
+//             bunch length) filled in shared memory with warp-aggregated
+//             atomics (__match_any_sync groups lanes hitting the same bin),
+//             integer counts so the result is exact and order-independent,
+//             and for the transverse potentials the per-bin sums of x and y
+//             over alive particles.  Lag CTAs: below.
+//             The 1 mm pseudo-Green wake W_z at the 2B-1 distinct lags
 //             tau = (i - j) dtBin (WakeFunction.cpp:558-653).  The reference
 //             evaluates it for all B^2 bin pairs; the lag set is identical.
 //             The 1000-term sum per resonator splits over a CTA; the
@@ -16,9 +19,16 @@
 //  k_sr_pot   V_i = (V_i(previous turn) + sum_j W(i - j) n_j) (-e q/E)
 //             (the reference keeps srWakePoten between turns,
 //             MPBunch.cpp:1894-1897, and only the longitudinal plane kicks).
-//  k_sr_kick  dp += V[bin] for alive particles.
+//             A warp per bin, its lanes over j.
+//  k_sr_kick  dp += V[bin] for alive particles, and the turn's loss check if
+//             no stage comes between.
+//
+// Bound by latency for a single bunch (five dependent launches of a few
+// thousand cycles), by HBM for a train.  One bunch of 1e5 particles, 100 bins,
+// us: range 44 (one thread over the tiles) -> in the longitudinal pass, histogram and lags 8 + 5 -> 6.4 together, potentials 7 -> 4.1 (a
+// thread per bin), kick and loss check 5 + 7 -> 5.0 together.
 #include <cuda_runtime.h>
-#include "kernels.cuh"
+#include "turn_tail.cuh"
 
 namespace cg {
 
@@ -38,130 +48,82 @@ __device__ __forceinline__ double warp_sum1(double v) {
   return v;
 }
 
-__global__ void __launch_bounds__(kTile) k_sr_geom(const double* __restrict__ c, int64_t npad,
-                                                   const uint8_t* __restrict__ surv,
-                                                   const int* __restrict__ tile_bunch,
-                                                   const BunchDev* __restrict__ bunch,
-                                                   double* part, unsigned* counters,
-                                                   const BunchMomDev* __restrict__ mom,
-                                                   double* geom, int* counts, double* sumx,
-                                                   double* sumy, int B) {
-  __shared__ double smin[32], smax[32];
-  __shared__ bool last;
+__global__ void __launch_bounds__(kTile) k_sr_range(const double* __restrict__ c, int64_t npad,
+                                                    const uint8_t* __restrict__ surv,
+                                                    const int* __restrict__ tile_bunch,
+                                                    const BunchDev* __restrict__ bunch, SrDev sr) {
   const int b = tile_bunch[blockIdx.x];
   const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  double mn = INFINITY, mx = -INFINITY;
-  if (i < Bd.n && surv[g] == kAlive) {
-    double z = c[4 * npad + g];
-    mn = z;
-    mx = z;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fmin(mn, __shfl_xor_sync(FULL_MASK, mn, o));
-    mx = fmax(mx, __shfl_xor_sync(FULL_MASK, mx, o));
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    smin[warp] = mn;
-    smax[warp] = mx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < kTile / 32; ++w) {
-      mn = fmin(mn, smin[w]);
-      mx = fmax(mx, smax[w]);
-    }
-    part[2 * blockIdx.x] = mn;
-    part[2 * blockIdx.x + 1] = mx;
-    __threadfence();
-    unsigned prev = atomicAdd(&counters[b], 1u);
-    last = (prev == (unsigned)(Bd.n_tiles - 1));
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (threadIdx.x == 0) {
-    // GetZMinMax seeds both extremes with particle 0 (alive or not)
-    double z0 = c[4 * npad + (int64_t)Bd.tile_off * kTile];
-    double zmin = z0, zmax = z0;
-    for (int t = 0; t < Bd.n_tiles; ++t) {
-      zmin = fmin(zmin, __ldcg(part + 2 * (Bd.tile_off + t)));
-      zmax = fmax(zmax, __ldcg(part + 2 * (Bd.tile_off + t) + 1));
-    }
-    zmin = zmin - 1.e-6;
-    zmax = zmax + 1.e-6;
-    double sl = mom[b].bunch_length;
-    double lo = zmin - 2 * sl;
-    double hi = zmax + 2 * sl;
-    geom[2 * b] = lo;
-    geom[2 * b + 1] = (hi - lo) / B;
-    counters[b] = 0;
-  }
-  for (int q = threadIdx.x; q < B; q += kTile) {
-    counts[(size_t)b * B + q] = 0;
-    sumx[(size_t)b * B + q] = 0.0;
-    sumy[(size_t)b * B + q] = 0.0;
-  }
+  const bool valid = (blockIdx.x - Bd.tile_off) * kTile + (int)threadIdx.x < Bd.n;
+  sr_span_cta(sr, b, (int)blockIdx.x == Bd.tile_off, valid && surv[g] == kAlive,
+              valid ? c[4 * npad + g] : 0.0);
 }
 
-__device__ __forceinline__ int sr_bin(double z, double lo, double dz, int B) {
-  int idx = (int)((z - lo) / dz);  // truncation toward zero, as int() in the reference
-  return (idx >= 0 && idx < B) ? idx : -1;
+// A bunch's bins (GetZMinMax seeds both extremes with particle 0, alive or not).
+struct SrGeom {
+  double lo, dz;
+};
+__device__ __forceinline__ SrGeom sr_geometry(const SrSpan& s, double z0, double bunch_length, int B) {
+  double zmin = z0, zmax = z0;
+  if (s.top) {
+    zmin = fmin(zmin, -sr_unkey(s.bottom));
+    zmax = fmax(zmax, sr_unkey(s.top));
+  }
+  zmin = zmin - 1.e-6;
+  zmax = zmax + 1.e-6;
+  const double lo = zmin - 2 * bunch_length, hi = zmax + 2 * bunch_length;
+  return {lo, (hi - lo) / B};
 }
 
-__global__ void __launch_bounds__(kTile) k_sr_hist(const double* __restrict__ c, int64_t npad,
-                                                   const uint8_t* __restrict__ surv,
-                                                   const int* __restrict__ tile_bunch,
-                                                   const BunchDev* __restrict__ bunch,
-                                                   const double* __restrict__ geom, int* counts,
-                                                   double* sumx, double* sumy, int B) {
-  extern __shared__ unsigned char sm_raw[];
+// truncation toward zero, as int() in the reference; the product with 1 / dz
+// decides unless a whole number lies within 2^-50 of it (bbi_bin)
+__device__ __forceinline__ int sr_bin(double z, double lo, double dz, double inv, int B) {
+  double t = (z - lo) * inv;
+  const double whole = (t + 0x1.8p52) - 0x1.8p52;
+  if (!(fabs(t - whole) > 0x1p-50 * fabs(t))) t = (z - lo) / dz;
+  return (t > -1.0 && t < (double)B) ? (int)t : -1;
+}
+
+// One chunk of particles into its bunch's bins.  XY: the sums of x and y too.
+template <bool XY>
+__device__ __forceinline__ void sr_hist_chunk(const double* __restrict__ c, int64_t npad,
+                                              const uint8_t* __restrict__ surv, const int4& l, int n,
+                                              int tile_off, const SrGeom& G, int* counts,
+                                              double* sumx, double* sumy, int B,
+                                              unsigned char* sm_raw) {
   int* s_cnt = reinterpret_cast<int*>(sm_raw);
   double* s_x = reinterpret_cast<double*>(sm_raw + ((B * sizeof(int) + 15) & ~(size_t)15));
   double* s_y = s_x + B;
   for (int q = threadIdx.x; q < B; q += kTile) {
     s_cnt[q] = 0;
-    s_x[q] = 0.0;
-    s_y[q] = 0.0;
+    if (XY) s_x[q] = s_y[q] = 0.0;
   }
   __syncthreads();
-  const int b = tile_bunch[blockIdx.x];
-  const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
-  const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const double lo = geom[2 * b], dz = geom[2 * b + 1];
-  int idx = -1;
-  bool alive = false;
-  double x = 0, y = 0;
-  if (i < Bd.n) {
-    idx = sr_bin(c[4 * npad + g], lo, dz, B);
-    alive = surv[g] == kAlive;
-    x = c[g];
-    y = c[2 * npad + g];
-  }
-  // warp-aggregated count: one shared atomic per distinct bin in the warp
-  unsigned peers = __match_any_sync(FULL_MASK, idx);
-  int leader = __ffs(peers) - 1;
-  if (idx >= 0 && (threadIdx.x & 31) == leader) atomicAdd(&s_cnt[idx], __popc(peers));
-  if (idx >= 0 && alive) {
-    atomicAdd(&s_x[idx], x);
-    atomicAdd(&s_y[idx], y);
+  const double inv = 1.0 / G.dz;
+  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
+  int i = (l.y - tile_off) * kTile + threadIdx.x;
+  for (int u = 0; u < l.z; ++u, g += kTile, i += kTile) {
+    const int idx = i < n ? sr_bin(c[4 * npad + g], G.lo, G.dz, inv, B) : -1;
+    // warp-aggregated count: one shared atomic per distinct bin in the warp
+    const unsigned peers = __match_any_sync(FULL_MASK, idx);
+    if (idx >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&s_cnt[idx], __popc(peers));
+    if (XY && idx >= 0 && surv[g] == kAlive) {
+      atomicAdd(&s_x[idx], c[g]);
+      atomicAdd(&s_y[idx], c[2 * npad + g]);
+    }
   }
   __syncthreads();
   for (int q = threadIdx.x; q < B; q += kTile) {
-    int n = s_cnt[q];
-    if (n) {
-      atomicAdd(&counts[(size_t)b * B + q], n);
-      atomicAdd(&sumx[(size_t)b * B + q], s_x[q]);
-      atomicAdd(&sumy[(size_t)b * B + q], s_y[q]);
+    if (!s_cnt[q]) continue;
+    atomicAdd(&counts[q], s_cnt[q]);
+    if (XY) {
+      atomicAdd(&sumx[q], s_x[q]);
+      atomicAdd(&sumy[q], s_y[q]);
     }
   }
 }
 
-// One CTA per (bunch, lag): W_z(tau) summed over resonators.
 // e^{-x} I_nu(x) for nu = 1/4, 5/4, 3/4, 7/4 (in that order), over the 256
 // threads of the CTA: the power series sum_k (x/2)^{2k+nu} / (k! Gamma(k+nu+1)),
 // each term formed in logarithms (so e^{-x} and the peak near k = x/2 stay in
@@ -208,16 +170,14 @@ __device__ double rw_pseudo_fz(double u, double (*sw4)[8]) {
   return c1 * (c2 * (m025 - p075) + (-p025 + m075));
 }
 
-__global__ void __launch_bounds__(256) k_sr_lag(const double* __restrict__ geom,
-                                                const SrResonator* __restrict__ res,
-                                                const double* __restrict__ green, int n_res,
-                                                int B, double sigmat, double rw_coeff,
-                                                double* lag, const double* __restrict__ green_t) {
+// One CTA per (bunch, lag): W_z(tau) summed over resonators, lag bin m = i - j.
+__device__ __forceinline__ void sr_lag_cta(int b, int m, double dz, const SrResonator* __restrict__ res,
+                                           const double* __restrict__ green, int n_res, int B,
+                                           double sigmat, double rw_coeff, double* lag,
+                                           const double* __restrict__ green_t) {
   __shared__ double sw[8];
   __shared__ double sw4[4][8];
-  const int b = blockIdx.y;
-  const int m = (int)blockIdx.x - (B - 1);  // i - j
-  const double dtBin = geom[2 * b + 1] / kCLight;
+  const double dtBin = dz / kCLight;
   const double tau = m * dtBin;
   const double u = tau / sigmat;
   double total = 0.0;
@@ -246,7 +206,7 @@ __global__ void __launch_bounds__(256) k_sr_lag(const double* __restrict__ geom,
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) lag[(size_t)b * 3 * (2 * B - 1) + blockIdx.x] = total;
+  if (threadIdx.x == 0) lag[(size_t)b * 3 * (2 * B - 1) + m + B - 1] = total;
   if (!green_t) return;
   // the transverse pseudo-Green wakes of the resonators (GetBBRPusdoWakeFun,
   // WakeFunction.cpp:596-629), for the potentials MPBunch.cpp:1981-1985
@@ -274,71 +234,132 @@ __global__ void __launch_bounds__(256) k_sr_lag(const double* __restrict__ geom,
       }
       __syncthreads();
     }
-    if (threadIdx.x == 0) lag[((size_t)b * 3 + 1 + q) * (2 * B - 1) + blockIdx.x] = tq;
+    if (threadIdx.x == 0) lag[((size_t)b * 3 + 1 + q) * (2 * B - 1) + m + B - 1] = tq;
   }
 }
 
-__global__ void k_sr_pot(const BunchDev* __restrict__ bunch, const int* __restrict__ counts,
-                         const double* __restrict__ lag, double* pot, int B, double energy,
-                         const double* __restrict__ sumx, double* potxy) {
-  const int b = blockIdx.x;
-  const int* cnt = counts + (size_t)b * B;
-  const double* lg = lag + (size_t)b * 3 * (2 * B - 1);
+// CTAs [0, n_chunks): a chunk each; then one per (bunch, lag).
+template <bool XY>
+__global__ void __launch_bounds__(kTile) k_sr_bins(const double* __restrict__ c, int64_t npad,
+                                                   const uint8_t* __restrict__ surv,
+                                                   const int4* __restrict__ chunk_loc, int n_chunks,
+                                                   const BunchDev* __restrict__ bunch,
+                                                   const BunchMomDev* __restrict__ mom, SrDev sr,
+                                                   double* geom,
+                                                   const SrResonator* __restrict__ res,
+                                                   const double* __restrict__ green, int n_res,
+                                                   double sigmat, double rw_coeff, double* lag,
+                                                   const double* __restrict__ green_t) {
+  extern __shared__ unsigned char sm_raw[];
+  const int B = sr.B, lags = 2 * B - 1;
+  const bool hist = (int)blockIdx.x < n_chunks;
+  const int q = (int)blockIdx.x - n_chunks;
+  const int4 l = hist ? chunk_loc[blockIdx.x] : make_int4(q / lags, 0, 0, 0);
+  const int b = l.x, tile_off = bunch[b].tile_off;
+  if (bunch[b].n_tiles == 0) return;  // held by another rank
+  const SrGeom G = sr_geometry(sr.span[b], c[4 * npad + (int64_t)tile_off * kTile],
+                               mom[b].bunch_length, B);
+  if (hist) {
+    sr_hist_chunk<XY>(c, npad, surv, l, bunch[b].n, tile_off, G, sr.counts + (size_t)b * B,
+                      sr.sumx + (size_t)b * B, sr.sumy + (size_t)b * B, B, sm_raw);
+    return;
+  }
+  const int m = q % lags;
+  if (m == 0 && threadIdx.x == 0) {
+    geom[2 * b] = G.lo;
+    geom[2 * b + 1] = G.dz;
+  }
+  sr_lag_cta(b, m - (B - 1), G.dz, res, green, n_res, B, sigmat, rw_coeff, lag, XY ? green_t : nullptr);
+}
+
+__global__ void __launch_bounds__(kTile) k_sr_pot(const BunchDev* __restrict__ bunch, SrDev sr,
+                                                  const double* __restrict__ lag, double* pot,
+                                                  double energy, double* potxy) {
+  const int b = blockIdx.y, B = sr.B;
+  if (bunch[b].n_tiles == 0) return;  // held by another rank
+  const int i = blockIdx.x * (kTile / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sr.span[b] = SrSpan{0, 0};  // for the next call
+  if (i >= B) return;
+  const int* cnt = sr.counts + (size_t)b * B;
+  const double* lg = lag + (size_t)b * 3 * (2 * B - 1) + i + B - 1;
   const double scale = (-1) * kElectronCharge * bunch[b].q_macro / energy;
-  for (int i = threadIdx.x; i < B; i += blockDim.x) {
-    double v = pot[(size_t)b * B + i];
-    for (int j = 0; j < B; ++j) v += lg[i - j + B - 1] * cnt[j];
-    pot[(size_t)b * B + i] = v * scale;
+  double v = 0, vx = 0, vy = 0;
+  for (int j = lane; j < B; j += 32) {
+    const int n = cnt[j];
+    v += lg[-j] * n;
     if (!potxy) continue;
     // the transverse potentials, both from the horizontal centroids
     // (averXAlongBunch in both lines, MPBunch.cpp:1981-1985)
-    double vx = potxy[(size_t)b * 2 * B + i], vy = potxy[((size_t)b * 2 + 1) * B + i];
-    for (int j = 0; j < B; ++j) {
-      const double ax = cnt[j] ? sumx[(size_t)b * B + j] / cnt[j] : 0.0;
-      vx += lg[(2 * B - 1) + i - j + B - 1] * cnt[j] * ax;
-      vy += lg[2 * (2 * B - 1) + i - j + B - 1] * cnt[j] * ax;
-    }
-    potxy[(size_t)b * 2 * B + i] = vx * scale;
-    potxy[((size_t)b * 2 + 1) * B + i] = vy * scale;
+    const double ax = n ? sr.sumx[(size_t)b * B + j] / n : 0.0;
+    vx += lg[(2 * B - 1) - j] * n * ax;
+    vy += lg[2 * (2 * B - 1) - j] * n * ax;
+  }
+  v = warp_sum1(v);
+  if (lane == 0) pot[(size_t)b * B + i] = (pot[(size_t)b * B + i] + v) * scale;
+  if (!potxy) return;
+  vx = warp_sum1(vx);
+  vy = warp_sum1(vy);
+  if (lane == 0) {
+    double *px = potxy + (size_t)b * 2 * B + i, *py = px + B;
+    *px = (*px + vx) * scale;
+    *py = (*py + vy) * scale;
   }
 }
 
+template <bool MARK>
 __global__ void __launch_bounds__(kTile) k_sr_kick(double* __restrict__ c, int64_t npad,
-                                                   const uint8_t* __restrict__ surv,
+                                                   uint8_t* __restrict__ surv,
                                                    const int* __restrict__ tile_bunch,
                                                    const BunchDev* __restrict__ bunch,
                                                    const double* __restrict__ geom,
-                                                   const double* __restrict__ pot, int B) {
+                                                   const double* __restrict__ pot, int B,
+                                                   const __grid_constant__ Aperture ap,
+                                                   int* loss_count) {
   const int b = tile_bunch[blockIdx.x];
   const BunchDev& Bd = bunch[b];
-  const int i = (blockIdx.x - Bd.tile_off) * kTile + threadIdx.x;
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  if (i >= Bd.n || surv[g] != kAlive) return;
-  int idx = sr_bin(c[4 * npad + g], geom[2 * b], geom[2 * b + 1], B);
-  if (idx < 0) return;
-  c[5 * npad + g] += pot[(size_t)b * B + idx];
+  const bool valid = (blockIdx.x - Bd.tile_off) * kTile + (int)threadIdx.x < Bd.n;
+  double x = 0, y = 0, z = 0;
+  if (valid) {
+    z = c[4 * npad + g];
+    if (MARK) {
+      x = c[g];
+      y = c[2 * npad + g];
+    }
+    if (surv[g] == kAlive) {
+      const double lo = geom[2 * b], dz = geom[2 * b + 1];
+      const int idx = sr_bin(z, lo, dz, 1.0 / dz, B);
+      if (idx >= 0) c[5 * npad + g] += pot[(size_t)b * B + idx];
+    }
+  }
+  if (MARK) mark_lost_warp(ap, valid, x, y, z, surv + g, loss_count + b);
 }
 
-cudaError_t launch_sr_wake(Handle& h) {
-  const int B = h.cfg.sr_bins;
-  k_sr_geom<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                               h.d.scratch, h.d.counters, h.d.mom, h.d.sr_geom,
-                                               h.d.sr_counts, h.d.sr_sumx, h.d.sr_sumy, B);
-  size_t sm = ((B * sizeof(int) + 15) & ~(size_t)15) + 2 * B * sizeof(double);
-  k_sr_hist<<<h.n_tiles, kTile, sm, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
-                                                h.d.bunch, h.d.sr_geom, h.d.sr_counts,
-                                                h.d.sr_sumx, h.d.sr_sumy, B);
-  dim3 lg(2 * B - 1, h.M);
+size_t sr_span_bytes() { return sizeof(SrSpan); }
+
+SrDev sr_dev(const Handle& h) {
+  return {reinterpret_cast<SrSpan*>(h.d.sr_span), h.d.sr_counts, h.d.sr_sumx, h.d.sr_sumy,
+          h.cfg.sr_bins};
+}
+
+cudaError_t launch_sr_wake(Handle& h, bool have_range, bool mark) {
+  const SrDev sr = sr_dev(h);
+  const int B = sr.B;
+  if (!have_range)
+    k_sr_range<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
+                                                  h.d.bunch, sr);
   const double sigmat = 1.e-3 / kCLight;
   const bool xy = h.sr_xy && h.d.sr_potxy;
-  k_sr_lag<<<lg, 256, 0, h.stream>>>(h.d.sr_geom, reinterpret_cast<const SrResonator*>(h.d.sr_green),
-                                     h.d.sr_green + 3 * CG_MAX_RESONATORS, h.cfg.sr_bbr.n, B,
-                                     sigmat, h.sr_rw_coeff, h.d.sr_lag, xy ? h.d.sr_green_t : nullptr);
-  k_sr_pot<<<h.M, 128, 0, h.stream>>>(h.d.bunch, h.d.sr_counts, h.d.sr_lag, h.d.sr_pot, B,
-                                      h.cfg.ring.electron_energy, h.d.sr_sumx,
-                                      xy ? h.d.sr_potxy : nullptr);
-  k_sr_kick<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                               h.d.sr_geom, h.d.sr_pot, B);
+  const size_t sm = ((B * sizeof(int) + 15) & ~(size_t)15) + (xy ? 2 * B * sizeof(double) : 0);
+  (xy ? k_sr_bins<true> : k_sr_bins<false>)<<<h.n_chunks + h.M * (2 * B - 1), kTile, sm, h.stream>>>(
+      h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.n_chunks, h.d.bunch, h.d.mom, sr, h.d.sr_geom,
+      reinterpret_cast<const SrResonator*>(h.d.sr_green), h.d.sr_green + 3 * CG_MAX_RESONATORS,
+      h.cfg.sr_bbr.n, sigmat, h.sr_rw_coeff, h.d.sr_lag, h.d.sr_green_t);
+  k_sr_pot<<<dim3((B + kTile / 32 - 1) / (kTile / 32), h.M), kTile, 0, h.stream>>>(
+      h.d.bunch, sr, h.d.sr_lag, h.d.sr_pot, h.cfg.ring.electron_energy, xy ? h.d.sr_potxy : nullptr);
+  (mark ? k_sr_kick<true> : k_sr_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(
+      h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, h.d.sr_geom, h.d.sr_pot, B, aperture(h),
+      h.d.loss_count);
   return cudaGetLastError();
 }
 

@@ -60,6 +60,53 @@ __device__ __forceinline__ void bbi_span_cta(const BbiParams& p, BbiSpan* span, 
   if (threadIdx.x < 4 && s_max[threadIdx.x]) atomicMax(&span->top + threadIdx.x, s_max[threadIdx.x]);
 }
 
+// The same for the short-range wake: the survivors' range of z, as maxima of
+// ordered keys (of z and of -z).
+struct alignas(128) SrSpan {
+  unsigned long long top, bottom;
+};
+struct SrDev {
+  SrSpan* span;
+  int* counts;         // M x B particles per bin
+  double *sumx, *sumy; // M x B
+  int B;
+};
+// doubles as unsigned integers of the same order, none of them zero
+__device__ __forceinline__ unsigned long long sr_key(double z) {
+  const long long b = __double_as_longlong(z);
+  return b < 0 ? ~(unsigned long long)b : (unsigned long long)b | 1ull << 63;
+}
+__device__ __forceinline__ double sr_unkey(unsigned long long k) {
+  return __longlong_as_double((long long)(k >> 63 ? k & ~(1ull << 63) : ~k));
+}
+// A CTA's particles into their bunch's span; every thread of the CTA calls it.
+// The CTA of the bunch's first tile clears the counts of the call before.
+__device__ __forceinline__ void sr_span_cta(const SrDev& sr, int b, bool first, bool alive, double z) {
+  __shared__ unsigned long long s_key[2];
+  if (threadIdx.x < 2) s_key[threadIdx.x] = 0ull;
+  if (first)
+    for (int q = threadIdx.x; q < sr.B; q += blockDim.x) {
+      sr.counts[(size_t)b * sr.B + q] = 0;
+      sr.sumx[(size_t)b * sr.B + q] = sr.sumy[(size_t)b * sr.B + q] = 0.0;
+    }
+  __syncthreads();
+  // the extremes without NaN, as fmin and fmax leave it out
+  double mx = alive ? z : NAN, mn = mx;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+  }
+  if ((threadIdx.x & 31) == 0 && mx == mx) {
+    atomicMax(&s_key[0], sr_key(mx));
+    atomicMax(&s_key[1], sr_key(-mn));
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && s_key[threadIdx.x]) atomicMax(&sr.span[b].top + threadIdx.x, s_key[threadIdx.x]);
+}
+
+SrDev sr_dev(const Handle& h);
+
 // Bunch::MarkLostParticle (Bunch.cpp:172-200) for the warp's particles, their
 // number of loss conditions added to the bunch's.  A position clearly inside
 // the aperture by the reciprocals takes no division; the others take the
