@@ -26,15 +26,19 @@ namespace cg {
 constexpr int kSurRows = 128;              // samples per tile = threads per CTA
 constexpr uint32_t kSurTmemCols = 64;
 constexpr uint32_t kSurWaitLimit = 1u << 26;  // mbarrier polls before giving up
-constexpr int kZs = 65;                    // padded row stride of FP32 tiles
+// Training: four threads per sample, a quarter of each layer's 64 units per
+// thread; warp w works on the samples 32 (w % 4) .. (the TMEM lanes that it may
+// read) and the units 16 (w / 4) ..
+constexpr int kSurTrainThreads = 4 * kSurRows;
+constexpr int kQ = kSurH / 4;              // units of a training thread
+constexpr int kHs = 68;                    // row stride of FP32 tiles (16-byte rows, no conflicts)
 
 // dynamic shared memory (offsets from a 1024-byte aligned base)
 constexpr uint32_t kSmA_hi = 0, kSmA_lo = 16384, kSmW2 = 32768, kSmW3 = 40960;
 constexpr uint32_t kSmW2t = 49152, kSmW3t = 57344;
 constexpr uint32_t kSmFwdBytes = 49152 + 1024;   // + alignment slack
-constexpr uint32_t kSmZ = 65536;                 // training: z1, z2, z3, dz (FP32, 128 x kZs)
-constexpr uint32_t kSmZBytes = kSurRows * kZs * 4;
-constexpr uint32_t kSmTrainBytes = kSmZ + 4 * kSmZBytes + 1024;
+constexpr uint32_t kSmH = 65536;                 // training: h1, h2, h3, dz (FP32, 128 x kHs)
+constexpr uint32_t kSmTrainBytes = kSmH + 4 * kSurRows * kHs * 4 + 1024;
 
 struct SurSmall {
   float w1[kSurH * 3], b1[kSurH], b2[kSurH], b3[kSurH], w4[2 * kSurH], b4[2];
@@ -45,10 +49,6 @@ __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__floa
 // below the BF16 weight rounding of the model); for z < -87 the exponential
 // overflows and the quotient is -0, the limit.
 __device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = 1.0f / (1.0f + __expf(-z));
-  return s * fmaf(z, 1.0f - s, 1.0f);
-}
 
 __device__ __forceinline__ uint8_t* sur_base(unsigned char* dyn) {
   return reinterpret_cast<uint8_t*>(((uintptr_t)dyn + 1023) & ~(uintptr_t)1023);
@@ -78,10 +78,12 @@ __device__ void sur_load(const float* __restrict__ w, uint8_t* base, SurSmall& s
   if (threadIdx.x < 2) sm.b4[threadIdx.x] = w[kSurB4 + threadIdx.x];
 }
 
-// Row `r` of the A tile from 64 FP32 values: hi = bf16(v), lo = bf16(v - hi).
-__device__ __forceinline__ void put_row(uint8_t* base, int r, const float (&h)[kSurH]) {
+// N values of row `r` of the A tile from unit `c0` on, from FP32: hi = bf16(v),
+// lo = bf16(v - hi).
+template <int N>
+__device__ __forceinline__ void put_row(uint8_t* base, int r, const float (&h)[N], int c0 = 0) {
 #pragma unroll
-  for (int c8 = 0; c8 < 8; ++c8) {
+  for (int c8 = 0; c8 < N / 8; ++c8) {
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -92,24 +94,15 @@ __device__ __forceinline__ void put_row(uint8_t* base, int r, const float (&h)[k
       hi[q] = *reinterpret_cast<const uint32_t*>(&b);
       lo[q] = *reinterpret_cast<const uint32_t*>(&l);
     }
-    const uint32_t off = umma::sw128_offset((uint32_t)r, (uint32_t)(c8 * 8));
+    const uint32_t off = umma::sw128_offset((uint32_t)r, (uint32_t)(c0 + c8 * 8));
     *reinterpret_cast<uint4*>(base + kSmA_hi + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(base + kSmA_lo + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
 }
 
-// Element (r, i) of the A tile as hi + lo.
-__device__ __forceinline__ float get_a(const uint8_t* base, int r, int i) {
-  const uint32_t off = umma::sw128_offset((uint32_t)r, (uint32_t)i);
-  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + kSmA_hi + off)) +
-         __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + kSmA_lo + off));
-}
-
-// d[row][0..63] = A_tile[row] . B^T with B the tile at `b_off`; every thread
-// of the CTA calls this after writing its row of A.  False if the
-// tensor-core completion did not arrive within the poll limit.
-__device__ bool sur_gemm(uint8_t* base, uint32_t b_off, uint32_t tmem, uint32_t bar,
-                         uint32_t& phase, float (&d)[kSurH]) {
+// Issues D = A_tile . B^T with B the tile at `b_off`; every thread of the CTA
+// calls this after writing its part of A.
+__device__ __forceinline__ void sur_mma(uint8_t* base, uint32_t b_off, uint32_t tmem, uint32_t bar) {
   umma::fence_async_smem();
   umma::fence_before_sync();
   __syncthreads();
@@ -127,9 +120,21 @@ __device__ bool sur_gemm(uint8_t* base, uint32_t b_off, uint32_t tmem, uint32_t 
                      umma::desc_sw128(sa + b_off + 32 * k), id, 1u);
     umma::commit(bar);
   }
+}
+// Waits for it; false if the tensor-core completion did not arrive within the
+// poll limit.
+__device__ __forceinline__ bool sur_mma_wait(uint32_t bar, uint32_t& phase) {
   const bool ok = umma::mbar_wait(bar, phase, kSurWaitLimit);
   phase ^= 1u;
   umma::fence_after_sync();
+  return ok;
+}
+
+// d[row][0..63] = A_tile[row] . B^T (a thread per row).
+__device__ bool sur_gemm(uint8_t* base, uint32_t b_off, uint32_t tmem, uint32_t bar,
+                         uint32_t& phase, float (&d)[kSurH]) {
+  sur_mma(base, b_off, tmem, bar);
+  const bool ok = sur_mma_wait(bar, phase);
   const uint32_t lane = (uint32_t)(threadIdx.x & ~31) << 16;
   float v[32];
   umma::tmem_ld32(tmem + lane, v);
@@ -153,17 +158,14 @@ __device__ __forceinline__ void sur_norm(float a, float b, float r, float (&x)[3
 __device__ __forceinline__ float sur_a(const float (&x)[3]) { return 0.5f * (x[0] + 1.0f); }
 __device__ __forceinline__ float sur_b(const float (&x)[3]) { return 0.5f * (x[1] + 1.0f); }
 
-// Forward pass of this thread's row; z1/z2/z3 (row stride kZs) are saved
-// when non-null.
+// Forward pass of this thread's row.
 __device__ bool sur_forward(uint8_t* base, const SurSmall& sm, uint32_t tmem, uint32_t bar,
-                            uint32_t& phase, const float (&x)[3], float (&out)[2], float* z1s,
-                            float* z2s, float* z3s) {
+                            uint32_t& phase, const float (&x)[3], float (&out)[2]) {
   const int r = threadIdx.x;
   float h[kSurH], d[kSurH];
 #pragma unroll
   for (int j = 0; j < kSurH; ++j) {
     float z = fmaf(sm.w1[3 * j + 2], x[2], fmaf(sm.w1[3 * j + 1], x[1], fmaf(sm.w1[3 * j], x[0], sm.b1[j])));
-    if (z1s) z1s[r * kZs + j] = z;
     h[j] = silu(z);
   }
   put_row(base, r, h);
@@ -171,7 +173,6 @@ __device__ bool sur_forward(uint8_t* base, const SurSmall& sm, uint32_t tmem, ui
 #pragma unroll
   for (int j = 0; j < kSurH; ++j) {
     const float z = d[j] + sm.b2[j];
-    if (z2s) z2s[r * kZs + j] = z;
     h[j] = silu(z);
   }
   put_row(base, r, h);
@@ -180,7 +181,6 @@ __device__ bool sur_forward(uint8_t* base, const SurSmall& sm, uint32_t tmem, ui
 #pragma unroll
   for (int j = 0; j < kSurH; ++j) {
     const float z = d[j] + sm.b3[j];
-    if (z3s) z3s[r * kZs + j] = z;
     const float hj = silu(z);
     o0 = fmaf(sm.w4[j], hj, o0);
     o1 = fmaf(sm.w4[kSurH + j], hj, o1);
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kSurRows) k_sur_eval(const float* __restrict__
     float x[3], o[2];
     if (i < n) sur_norm(xin[3 * i], xin[3 * i + 1], xin[3 * i + 2], x);
     else x[0] = x[1] = x[2] = 0.0f;
-    ok = sur_forward(base, sm, tmem, bar, phase, x, o, nullptr, nullptr, nullptr) && ok;
+    ok = sur_forward(base, sm, tmem, bar, phase, x, o) && ok;
     if (i < n) {
       out[2 * i] = o[0];
       out[2 * i + 1] = o[1];
@@ -276,35 +276,129 @@ __global__ void __launch_bounds__(kSurRows) k_sur_eval(const float* __restrict__
 // sum of e^2).  m = mean e^2 of the previous step (*e2_prev = its sum, held
 // fixed in the derivative); w = 0 is the plain squared error.
 
-__global__ void __launch_bounds__(kSurRows) k_sur_train_tile(const float* __restrict__ w,
-                                                             const float* __restrict__ xin,
-                                                             const float* __restrict__ tin,
-                                                             int64_t n, int64_t row0, uint64_t mul,
-                                                             uint64_t add, float inv_batch,
-                                                             float l4w, const float* e2_prev,
-                                                             float* __restrict__ part,
-                                                             int* status) {
+//
+// Bound by latency: a batch is few tiles (2048 samples: 16 CTAs), each a chain
+// of four layer products and their activations.  Four threads share a sample
+// so that an SM's schedulers have four warps each to choose from, activations
+// and their derivatives are formed once (derivatives stay in registers for the
+// way back), the weight gradients are 4 x 4 register tiles over the FP32
+// activations in shared memory, and they run while the tensor cores form the
+// next layer's dh.  With a thread per sample, which formed 128 x 32 products
+// from two BF16 loads or a SiLU each, a tile took 184 us; now 30.
+
+// silu(z) and its derivative from one exponential
+__device__ __forceinline__ void silu_both(float z, float* h, float* ds) {
+  const float d = 1.0f + __expf(-z);
+  const float s = 1.0f / d;
+  *h = __fdividef(z, d);
+  *ds = s * fmaf(z, 1.0f - s, 1.0f);
+}
+
+__device__ __forceinline__ void put_quarter(float* t, int r, int c0, const float (&v)[kQ]) {
+#pragma unroll
+  for (int k = 0; k < kQ; k += 4)
+    *reinterpret_cast<float4*>(t + r * kHs + c0 + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+}
+
+// g[o][i] = sum over the tile's rows of dz[row][o] h[row][i]: threads 0 .. 255
+// the first 64 rows, the others the rest, which they leave in h's place.
+__device__ __forceinline__ void sur_outer(const float* dz, const float* h, float (&acc)[4][4]) {
+  const int t = threadIdx.x & 255, i0 = (t & 15) * 4, o0 = (t >> 4) * 4;
+  const int q0 = (threadIdx.x >> 8) * (kSurRows / 2);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0f;
+#pragma unroll 4
+  for (int q = q0; q < q0 + kSurRows / 2; ++q) {
+    const float4 d4 = *reinterpret_cast<const float4*>(dz + q * kHs + o0);
+    const float4 h4 = *reinterpret_cast<const float4*>(h + q * kHs + i0);
+    const float d[4] = {d4.x, d4.y, d4.z, d4.w}, v[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(d[a], v[b], acc[a][b]);
+  }
+}
+__device__ __forceinline__ void sur_outer_leave(float* h, const float (&acc)[4][4]) {
+  if (threadIdx.x < 256) return;
+  const int t = threadIdx.x & 255, i0 = (t & 15) * 4, o0 = (t >> 4) * 4;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+    *reinterpret_cast<float4*>(h + (o0 + a) * kHs + i0) =
+        make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+}
+__device__ __forceinline__ void sur_outer_store(const float* h, const float (&acc)[4][4], float* g) {
+  if (threadIdx.x >= 256) return;
+  const int t = threadIdx.x, i0 = (t & 15) * 4, o0 = (t >> 4) * 4;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      g[(o0 + a) * kSurH + i0 + b] = acc[a][b] + h[(o0 + a) * kHs + i0 + b];
+}
+
+__global__ void __launch_bounds__(kSurTrainThreads, 1)
+    k_sur_train_tile(const float* __restrict__ w, const float* __restrict__ xin,
+                     const float* __restrict__ tin, int64_t n, int64_t row0, uint64_t mul,
+                     uint64_t add, float inv_batch, float l4w, const float* e2_prev,
+                     float* __restrict__ part, int* status) {
   extern __shared__ unsigned char dyn[];
   __shared__ SurSmall sm;
   __shared__ uint32_t s_tmem;
   __shared__ uint64_t s_bar;
-  __shared__ float s_x[kSurRows][3], s_dout[kSurRows][2], s_loss[kSurRows / 32];
+  __shared__ float s_x[kSurRows][3], s_dout[kSurRows][2], s_o[4][kSurRows][2];
+  __shared__ float s_row[4][3];        // per warp of rows: e^2, dout
+  __shared__ float s_col[8][4][kSurH];  // column sums over 16 rows each
   uint8_t* base = sur_base(dyn);
-  float* z1s = reinterpret_cast<float*>(base + kSmZ);
-  float* z2s = z1s + kSurRows * kZs;
-  float* z3s = z2s + kSurRows * kZs;
-  float* dzs = z3s + kSurRows * kZs;
+  float* H1 = reinterpret_cast<float*>(base + kSmH);
+  float* H2 = H1 + kSurRows * kHs;
+  float* H3 = H2 + kSurRows * kHs;
+  float* DZ = H3 + kSurRows * kHs;
   sur_load(w, base, sm, true);
   sur_begin(&s_tmem, &s_bar);
   const uint32_t tmem = s_tmem, bar = umma::smem_addr(&s_bar);
   uint32_t phase = 0;
-  const int r = threadIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = (warp & 3) * 32 + lane, cq = warp >> 2, c0 = cq * kQ;
+  const uint32_t dcol = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)c0;
   const int64_t j = row0 + (int64_t)blockIdx.x * kSurRows + r;
   const int64_t s = (int64_t)((mul * (uint64_t)j + add) % (uint64_t)n);
-  float x[3], out[2];
+  float x[3], h[kQ], d[kQ], ds1[kQ], ds2[kQ], ds3[kQ];
   sur_norm(xin[3 * s], xin[3 * s + 1], xin[3 * s + 2], x);
-  bool ok = sur_forward(base, sm, tmem, bar, phase, x, out, z1s, z2s, z3s);
-  const float e0 = out[0] - tin[2 * s], e1 = out[1] - tin[2 * s + 1];
+  const float t0 = tin[2 * s], t1 = tin[2 * s + 1];
+#pragma unroll
+  for (int k = 0; k < kQ; ++k) {
+    const int c = c0 + k;
+    silu_both(fmaf(sm.w1[3 * c + 2], x[2], fmaf(sm.w1[3 * c + 1], x[1], fmaf(sm.w1[3 * c], x[0], sm.b1[c]))),
+              &h[k], &ds1[k]);
+  }
+  put_quarter(H1, r, c0, h);
+  put_row(base, r, h, c0);
+  sur_mma(base, kSmW2, tmem, bar);
+  bool ok = sur_mma_wait(bar, phase);
+  umma::tmem_ld16(dcol, d);
+#pragma unroll
+  for (int k = 0; k < kQ; ++k) silu_both(d[k] + sm.b2[c0 + k], &h[k], &ds2[k]);
+  put_quarter(H2, r, c0, h);
+  put_row(base, r, h, c0);
+  sur_mma(base, kSmW3, tmem, bar);
+  ok = sur_mma_wait(bar, phase) && ok;
+  umma::tmem_ld16(dcol, d);
+  float o0 = 0.0f, o1 = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kQ; ++k) {
+    silu_both(d[k] + sm.b3[c0 + k], &h[k], &ds3[k]);
+    o0 = fmaf(sm.w4[c0 + k], h[k], o0);
+    o1 = fmaf(sm.w4[kSurH + c0 + k], h[k], o1);
+  }
+  put_quarter(H3, r, c0, h);
+  s_o[cq][r][0] = o0;
+  s_o[cq][r][1] = o1;
+  __syncthreads();
+  o0 = sm.b4[0] + ((s_o[0][r][0] + s_o[1][r][0]) + (s_o[2][r][0] + s_o[3][r][0]));
+  o1 = sm.b4[1] + ((s_o[0][r][1] + s_o[1][r][1]) + (s_o[2][r][1] + s_o[3][r][1]));
+  const float e0 = sur_a(x) * o0 - t0, e1 = sur_b(x) * o1 - t1;
   // dL/de = (e / B) ((1 - w) + 2 w e^2 / m)
   float g0 = 1.0f, g1 = 1.0f;
   if (l4w > 0.0f && e2_prev) {
@@ -316,114 +410,110 @@ __global__ void __launch_bounds__(kSurRows) k_sur_train_tile(const float* __rest
   }
   // dL/d(layer-4 output): through the odd-output factors a, b
   const float d0 = e0 * inv_batch * g0 * sur_a(x), d1 = e1 * inv_batch * g1 * sur_b(x);
-  s_x[r][0] = x[0];
-  s_x[r][1] = x[1];
-  s_x[r][2] = x[2];
-  s_dout[r][0] = d0;
-  s_dout[r][1] = d1;
-  {
-    float l = fmaf(e0, e0, e1 * e1);
+  if (cq == 0) {
+    s_x[r][0] = x[0];
+    s_x[r][1] = x[1];
+    s_x[r][2] = x[2];
+    s_dout[r][0] = d0;
+    s_dout[r][1] = d1;
+    float v[3] = {fmaf(e0, e0, e1 * e1), d0, d1};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((r & 31) == 0) s_loss[r >> 5] = l;
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      if (lane == 0) s_row[warp][q] = v[q];
+    }
   }
   // dz3 = (W4^T dout) * silu'(z3)
-  float dz[kSurH];
 #pragma unroll
-  for (int i = 0; i < kSurH; ++i) {
-    const float dh = fmaf(sm.w4[i], d0, sm.w4[kSurH + i] * d1);
-    dz[i] = dh * dsilu(z3s[r * kZs + i]);
-    dzs[r * kZs + i] = dz[i];
-  }
-  __syncthreads();
+  for (int k = 0; k < kQ; ++k) h[k] = fmaf(sm.w4[c0 + k], d0, sm.w4[kSurH + c0 + k] * d1) * ds3[k];
+  put_quarter(DZ, r, c0, h);
+  put_row(base, r, h, c0);
+  sur_mma(base, kSmW3t, tmem, bar);  // dh2 = dz3 W3, during the sums of layers 3 and 4
   float* g = part + (size_t)blockIdx.x * (kSurParams + 1);
-  // layer 4: dW4[o][i] = sum_r dout[r][o] silu(z3[r][i]); db4
+  const int col = threadIdx.x & 63, grp = threadIdx.x >> 6;
+  float acc[4][4];
   {
-    const int o = r >> 6, i = r & 63;
-    float acc = 0.0f;
-    for (int q = 0; q < kSurRows; ++q) acc = fmaf(s_dout[q][o], silu(z3s[q * kZs + i]), acc);
-    g[kSurW4 + o * kSurH + i] = acc;
-    if (r < 2) {
-      float b = 0.0f;
-      for (int q = 0; q < kSurRows; ++q) b += s_dout[q][r];
-      g[kSurB4 + r] = b;
+    // layer 4: dW4[o][i] = sum_r dout[r][o] h3[r][i]; db3
+    float b = 0.0f, w0 = 0.0f, w1 = 0.0f;
+#pragma unroll
+    for (int q = grp * 16; q < grp * 16 + 16; ++q) {
+      const float hv = H3[q * kHs + col];
+      b += DZ[q * kHs + col];
+      w0 = fmaf(s_dout[q][0], hv, w0);
+      w1 = fmaf(s_dout[q][1], hv, w1);
     }
+    s_col[grp][0][col] = b;
+    s_col[grp][1][col] = w0;
+    s_col[grp][2][col] = w1;
+    // layer 3: dW3[o][i] = sum_r dz3[r][o] h2[r][i]
+    sur_outer(DZ, H2, acc);
+    __syncthreads();
+    sur_outer_leave(H2, acc);
+    if (threadIdx.x < 3 * kSurH) {
+      float v = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v += s_col[q][threadIdx.x >> 6][col];
+      g[(grp == 0 ? kSurB3 : kSurW4 + (grp - 1) * kSurH) + col] = v;
+    }
+    if (threadIdx.x < 3) {
+      const float v = (s_row[0][threadIdx.x] + s_row[1][threadIdx.x]) +
+                      (s_row[2][threadIdx.x] + s_row[3][threadIdx.x]);
+      g[threadIdx.x == 0 ? kSurParams : kSurB4 + threadIdx.x - 1] = v;
+    }
+    __syncthreads();
+    sur_outer_store(H2, acc, g + kSurW3);
   }
-  // layer 3: dW3[o][i] = sum_r dz3[r][o] h2[r][i] (h2 = the A tile, hi + lo); db3
+  ok = sur_mma_wait(bar, phase) && ok;
+  umma::tmem_ld16(dcol, d);
+#pragma unroll
+  for (int k = 0; k < kQ; ++k) h[k] = d[k] * ds2[k];  // dz2
+  put_quarter(DZ, r, c0, h);
+  put_row(base, r, h, c0);
+  sur_mma(base, kSmW2t, tmem, bar);  // dh1 = dz2 W2, during the sums of layer 2
   {
-    const int o = r >> 1, i0 = (r & 1) * 32;
-    float acc[32];
+    float b = 0.0f;
 #pragma unroll
-    for (int t = 0; t < 32; ++t) acc[t] = 0.0f;
-    for (int q = 0; q < kSurRows; ++q) {
-      const float dv = dzs[q * kZs + o];
+    for (int q = grp * 16; q < grp * 16 + 16; ++q) b += DZ[q * kHs + col];
+    s_col[grp][0][col] = b;
+    sur_outer(DZ, H1, acc);
+    __syncthreads();
+    sur_outer_leave(H1, acc);
+    if (threadIdx.x < kSurH) {
+      float v = 0.0f;
 #pragma unroll
-      for (int t = 0; t < 32; ++t) acc[t] = fmaf(dv, get_a(base, q, i0 + t), acc[t]);
+      for (int q = 0; q < 8; ++q) v += s_col[q][0][col];
+      g[kSurB2 + col] = v;
     }
-#pragma unroll
-    for (int t = 0; t < 32; ++t) g[kSurW3 + o * kSurH + i0 + t] = acc[t];
-    if (r < kSurH) {
-      float b = 0.0f;
-      for (int q = 0; q < kSurRows; ++q) b += dzs[q * kZs + r];
-      g[kSurB3 + r] = b;
-    }
+    __syncthreads();
+    sur_outer_store(H1, acc, g + kSurW2);
   }
-  __syncthreads();
-  // dh2 = dz3 W3 -> dz2
-  put_row(base, r, dz);
-  float d[kSurH];
-  ok = sur_gemm(base, kSmW3t, tmem, bar, phase, d) && ok;
+  ok = sur_mma_wait(bar, phase) && ok;
+  umma::tmem_ld16(dcol, d);
 #pragma unroll
-  for (int i = 0; i < kSurH; ++i) {
-    dz[i] = d[i] * dsilu(z2s[r * kZs + i]);
-    dzs[r * kZs + i] = dz[i];
-  }
+  for (int k = 0; k < kQ; ++k) h[k] = d[k] * ds1[k];  // dz1
+  put_quarter(DZ, r, c0, h);
   __syncthreads();
-  // layer 2: dW2[o][i] = sum_r dz2[r][o] silu(z1[r][i]); db2
   {
-    const int o = r >> 1, i0 = (r & 1) * 32;
-    float acc[32];
+    // layer 1: dW1[o][k] = sum_r dz1[r][o] x[r][k]; db1
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int t = 0; t < 32; ++t) acc[t] = 0.0f;
-    for (int q = 0; q < kSurRows; ++q) {
-      const float dv = dzs[q * kZs + o];
-#pragma unroll
-      for (int t = 0; t < 32; ++t) acc[t] = fmaf(dv, silu(z1s[q * kZs + i0 + t]), acc[t]);
+    for (int q = grp * 16; q < grp * 16 + 16; ++q) {
+      const float dv = DZ[q * kHs + col];
+      a[0] = fmaf(dv, s_x[q][0], a[0]);
+      a[1] = fmaf(dv, s_x[q][1], a[1]);
+      a[2] = fmaf(dv, s_x[q][2], a[2]);
+      a[3] += dv;
     }
 #pragma unroll
-    for (int t = 0; t < 32; ++t) g[kSurW2 + o * kSurH + i0 + t] = acc[t];
-    if (r < kSurH) {
-      float b = 0.0f;
-      for (int q = 0; q < kSurRows; ++q) b += dzs[q * kZs + r];
-      g[kSurB2 + r] = b;
-    }
-  }
-  __syncthreads();
-  // dh1 = dz2 W2 -> dz1
-  put_row(base, r, dz);
-  ok = sur_gemm(base, kSmW2t, tmem, bar, phase, d) && ok;
+    for (int k = 0; k < 4; ++k) s_col[grp][k][col] = a[k];
+    __syncthreads();
+    if (threadIdx.x < 4 * kSurH) {
+      float v = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kSurH; ++i) dzs[r * kZs + i] = d[i] * dsilu(z1s[r * kZs + i]);
-  __syncthreads();
-  // layer 1: dW1[o][k] = sum_r dz1[r][o] x[r][k]; db1
-  if (r < kSurH) {
-    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, b = 0.0f;
-    for (int q = 0; q < kSurRows; ++q) {
-      const float dv = dzs[q * kZs + r];
-      a0 = fmaf(dv, s_x[q][0], a0);
-      a1 = fmaf(dv, s_x[q][1], a1);
-      a2 = fmaf(dv, s_x[q][2], a2);
-      b += dv;
+      for (int q = 0; q < 8; ++q) v += s_col[q][grp][col];
+      g[grp == 3 ? kSurB1 + col : kSurW1 + 3 * col + grp] = v;
     }
-    g[kSurW1 + 3 * r] = a0;
-    g[kSurW1 + 3 * r + 1] = a1;
-    g[kSurW1 + 3 * r + 2] = a2;
-    g[kSurB1 + r] = b;
-  }
-  if (r == 0) {
-    float l = 0.0f;
-    for (int u = 0; u < kSurRows / 32; ++u) l += s_loss[u];
-    g[kSurParams] = l;
   }
   if (!ok) atomicOr(status, kStatusSurrogateWait);
   sur_end(tmem);
@@ -438,6 +528,7 @@ __global__ void k_sur_adam(float* __restrict__ w, float* __restrict__ m, float* 
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p > kSurParams) return;
   float gsum = 0.0f;
+#pragma unroll 16
   for (int c = 0; c < ncta; ++c) gsum += part[(size_t)c * (kSurParams + 1) + p];
   if (p == kSurParams) {
     if (loss) *loss += (double)gsum;
@@ -525,7 +616,7 @@ __global__ void __launch_bounds__(kSurRows, 3) k_ion_kick_sur(double* __restrict
       bool dom, sw;
       double u, v, sl;
       sur_frame(rc, x, y, xin, &dom, &sw, &u, &v, &sl);
-      ok = sur_forward(base, sm, tmem, bar, phase, xin, o, nullptr, nullptr, nullptr) && ok;
+      ok = sur_forward(base, sm, tmem, bar, phase, xin, o) && ok;
       double fx, fy;
       if (dom) {
         sur_field(o, sw, u, v, sl, &fx, &fy);
@@ -579,7 +670,7 @@ __global__ void __launch_bounds__(kSurRows, 2) k_sur_audit(const double* __restr
       bool dom, sw;
       double u, v, sl;
       sur_frame(rc, x, y, xin, &dom, &sw, &u, &v, &sl);
-      ok = sur_forward(base, sm, tmem, bar, phase, xin, o, nullptr, nullptr, nullptr) && ok;
+      ok = sur_forward(base, sm, tmem, bar, phase, xin, o) && ok;
       if (alive && dom) {
         double fx, fy, ex, ey;
         sur_field(o, sw, u, v, sl, &fx, &fy);
@@ -638,7 +729,7 @@ cudaError_t launch_sur_step(const float* w, const float* xin, const float* tin, 
                             double* loss, float* grad_out, int* status, cudaStream_t s,
                             float l4w, float* e2_sum) {
   const int ncta = batch / kSurRows;
-  k_sur_train_tile<<<ncta, kSurRows, kSmTrainBytes, s>>>(w, xin, tin, n, row0, mul, add,
+  k_sur_train_tile<<<ncta, kSurTrainThreads, kSmTrainBytes, s>>>(w, xin, tin, n, row0, mul, add,
                                                          1.0f / (float)batch, l4w, e2_sum, part,
                                                          status);
   cudaError_t e = cudaGetLastError();
