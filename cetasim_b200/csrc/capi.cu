@@ -4,8 +4,10 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -38,9 +40,44 @@ int cuda_fail(Handle* h, cudaError_t e, const char* where) {
     if (_e != cudaSuccess) return cuda_fail(h, _e, #call); \
   } while (0)
 
+// Memory of the calls that own none (the surrogate's): one pool per device that
+// keeps up to 16 MB between calls.  An allocation of the library that finds no
+// memory takes it back first.
+constexpr size_t kCallPoolKeep = 16u << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[64] = {};
+
+cudaMemPool_t call_pool(int dev) {
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps p = {};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.location.type = cudaMemLocationTypeDevice;
+    p.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &p) != cudaSuccess) return nullptr;
+    uint64_t keep = kCallPoolKeep;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pool[dev] = pool;
+  }
+  return g_pool[dev];
+}
+
 template <class T>
 cudaError_t dalloc(T** p, size_t count) {
-  return cudaMalloc((void**)p, count * sizeof(T) > 0 ? count * sizeof(T) : 16);
+  const size_t bytes = count * sizeof(T) > 0 ? count * sizeof(T) : 16;
+  cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  int dev = 0;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (cudaGetDevice(&dev) == cudaSuccess && dev < 64) pool = g_pool[dev];
+  }
+  if (!pool || cudaMemPoolTrimTo(pool, 0) != cudaSuccess) return e;
+  cudaGetLastError();
+  return cudaMalloc((void**)p, bytes);
 }
 
 void dfree(void* p) {
@@ -63,10 +100,9 @@ int ensure_weideman(int device) {
 
 // Reads the device status word and maps it to a cg_status.
 int check_status(Handle& h) {
-  cudaError_t e = cudaStreamSynchronize(h.stream);
-  if (e != cudaSuccess) return cuda_fail(&h, e, "cudaStreamSynchronize");
   int st = 0;
-  e = cudaMemcpy(&st, h.d.status, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemcpyAsync(&st, h.d.status, sizeof(int), cudaMemcpyDeviceToHost, h.stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h.stream);
   if (e != cudaSuccess) return cuda_fail(&h, e, "status read");
   if (st == 0) return CG_OK;
   cudaMemsetAsync(h.d.status, 0, sizeof(int), h.stream);
@@ -1109,8 +1145,9 @@ int cg_beam_rms(cg_handle* H, int k) {
 int cg_get_moments(cg_handle* H, cg_bunch_moments* out) {
   STAGE_PROLOGUE
   std::vector<BunchMomDev> m(h.M);
+  CG_CUDA(&h, cudaMemcpyAsync(m.data(), h.d.mom, sizeof(BunchMomDev) * h.M, cudaMemcpyDeviceToHost,
+                              h.stream));
   CG_CUDA(&h, cudaStreamSynchronize(h.stream));
-  CG_CUDA(&h, cudaMemcpy(m.data(), h.d.mom, sizeof(BunchMomDev) * h.M, cudaMemcpyDeviceToHost));
   for (int j = 0; j < h.M; ++j) {
     cg_bunch_moments& o = out[j];
     const BunchMomDev& s = m[j];
@@ -1530,8 +1567,8 @@ int cg_run_turns(cg_handle* H, int turn0, int n_turns) {
       h.sur_audit_worst = std::max(h.sur_audit_worst, h.sur_audit_last);
       h.sur_audits++;
     }
-    // status is polled every 64 turns (and at the end) to keep the GPU fed
-    if (((n + 1) & 63) == 0 || n + 1 == n_turns) {
+    // status is polled every 64 turns (and after the last) to keep the GPU fed
+    if (((n + 1) & 63) == 0 && n + 1 < n_turns) {
       if ((st = check_status(h))) return st;
     }
   }
@@ -2613,16 +2650,21 @@ int cg_autotune_pipeline(cg_handle* H, int turn0, int reps, int* shape, double* 
 
 namespace {
 
-// Device buffers of one surrogate call, freed on every exit path.
+// Device buffers of one surrogate call (from the calls' pool, in the order of
+// the default stream that its kernels run on), freed on every exit path.
 struct DevBufs {
   std::vector<void*> p;
   ~DevBufs() {
-    for (void* q : p) dfree(q);
+    for (void* q : p) cudaFreeAsync(q, 0);
   }
   template <class T>
   T* get(size_t count) {
     void* q = nullptr;
-    if (cudaMalloc(&q, std::max<size_t>(count * sizeof(T), 16)) != cudaSuccess) return nullptr;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaMemPool_t pool = call_pool(dev);
+    if (!pool || cudaMallocFromPoolAsync(&q, std::max<size_t>(count * sizeof(T), 16), pool, 0) != cudaSuccess)
+      return nullptr;
     p.push_back(q);
     return static_cast<T*>(q);
   }
@@ -2640,14 +2682,18 @@ int sur_device_ready() {
   return CG_OK;
 }
 
+int sur_status_code(int st) {
+  if (st & kStatusSurrogateWait)
+    return fail(nullptr, CG_ERR_TIMEOUT, "a tensor-core completion wait gave up");
+  return st ? fail(nullptr, CG_ERR_CUDA, "unexpected device status") : CG_OK;
+}
+
 int sur_status(int* d_status) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "surrogate kernels");
   int st = 0;
   cudaMemcpy(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost);
-  if (st & kStatusSurrogateWait)
-    return fail(nullptr, CG_ERR_TIMEOUT, "a tensor-core completion wait gave up");
-  return st ? fail(nullptr, CG_ERR_CUDA, "unexpected device status") : CG_OK;
+  return sur_status_code(st);
 }
 
 // splitmix64 (Steele, Lea and Flood 2014): the host's seeded stream for the
@@ -2714,25 +2760,27 @@ int cg_surrogate_grad(const float* weights, const float* inputs, const float* ta
   float* x = b.get<float>(3 * (size_t)n);
   float* t = b.get<float>(2 * (size_t)n);
   float* part = b.get<float>((size_t)ncta * (CG_SUR_PARAMS + 1));
-  float* g = b.get<float>(CG_SUR_PARAMS);
-  double* l = b.get<double>(1);
-  int* s = b.get<int>(1);
-  if (!w || !x || !t || !part || !g || !l || !s) return fail(nullptr, CG_ERR_OOM, "surrogate grad");
-  cudaMemcpy(w, weights, CG_SUR_PARAMS * sizeof(float), cudaMemcpyHostToDevice);
-  cudaMemcpy(x, inputs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
-  cudaMemcpy(t, targets, 2 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
-  cudaMemset(l, 0, sizeof(double));
-  cudaMemset(s, 0, sizeof(int));
+  // the results in one block and one copy: the loss, the status, the gradient
+  struct Out {
+    double loss;
+    int status, pad;
+    float g[CG_SUR_PARAMS];
+  };
+  Out* o = b.get<Out>(1);
+  if (!w || !x || !t || !part || !o) return fail(nullptr, CG_ERR_OOM, "surrogate grad");
+  cudaMemcpyAsync(w, weights, CG_SUR_PARAMS * sizeof(float), cudaMemcpyHostToDevice, 0);
+  cudaMemcpyAsync(x, inputs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, 0);
+  cudaMemcpyAsync(t, targets, 2 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, 0);
+  cudaMemsetAsync(o, 0, offsetof(Out, g), 0);
   cudaError_t e = launch_sur_step(w, x, t, n, 0, n, 1, 0, part, nullptr, nullptr, nullptr, 0.0f,
-                                  1.0f, 1.0f, l, g, s, 0);
+                                  1.0f, 1.0f, &o->loss, o->g, &o->status, 0);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "surrogate grad launch");
-  if ((st = sur_status(s))) return st;
-  cudaMemcpy(grads, g, CG_SUR_PARAMS * sizeof(float), cudaMemcpyDeviceToHost);
-  if (loss) {
-    double lh = 0;
-    cudaMemcpy(&lh, l, sizeof(double), cudaMemcpyDeviceToHost);
-    *loss = lh / (2.0 * n);
-  }
+  std::unique_ptr<Out> r(new Out);
+  if ((e = cudaMemcpy(r.get(), o, sizeof(Out), cudaMemcpyDeviceToHost)) != cudaSuccess)
+    return cuda_fail(nullptr, e, "surrogate kernels");
+  if ((st = sur_status_code(r->status))) return st;
+  std::memcpy(grads, r->g, sizeof r->g);
+  if (loss) *loss = r->loss / (2.0 * n);
   return CG_OK;
 }
 
