@@ -163,11 +163,14 @@ __device__ __forceinline__ void store6(double* __restrict__ c, int64_t npad, int
 // The map pass and k_moments share these functions: the same moments bit for
 // bit.
 
-struct MomSums {
+template <class Count>
+struct MomSumsOf {
   double s[6], q[9], zmin, zmax;
-  int n;
+  Count n;
 };
-__device__ __forceinline__ void mom_sums_clear(MomSums& m) {
+using MomSums = MomSumsOf<int>;
+template <class Count>
+__device__ __forceinline__ void mom_sums_clear(MomSumsOf<Count>& m) {
 #pragma unroll
   for (int d = 0; d < 6; ++d) m.s[d] = 0.0;
 #pragma unroll
@@ -227,7 +230,8 @@ __device__ __forceinline__ bool mom_pivot(double* pivot, bool alive, const doubl
 }
 
 // The warp's sums as a partial.
-__device__ __forceinline__ void mom_partial(const MomSums& m, bool have, const double* pivot,
+template <class Count>
+__device__ __forceinline__ void mom_partial(const MomSumsOf<Count>& m, bool have, const double* pivot,
                                             MomPartial* out) {
   const int lane = threadIdx.x & 31;
   // lane 4 i gets total i: s 0..5, n, q8, and q 0..7
@@ -257,93 +261,73 @@ __device__ __forceinline__ void mom_partial(const MomSums& m, bool have, const d
   if (lane == 2) out->zmax = mx;
 }
 
-// A CTA of NT threads merges n_parts partials in two passes, the mean of all
-// and then the co-moments about it (thread t takes every NT-th in order, then
-// a butterfly per warp and the warps in order); thread 0 gets the total.
-template <int NT, bool GLOBAL = true>
-__device__ __forceinline__ void mom_merge_block(const MomPartial* partials, int n_parts,
-                                                MomPartial* total) {
-  constexpr int NW = NT / 32;
-  __shared__ double s_sum[NW][20];
+// A warp merges every stride-th 32 of n_parts partials from `at` on in one pass:
+// sums about the mean of the first non-empty one of its first round with any
+// (means that are the same in all stay that value exactly; the co-moments'
+// correction is as small as that mean is close).  GLOBAL: perhaps written by
+// other CTAs of this launch, read through L2.
+template <bool GLOBAL>
+__device__ __forceinline__ void mom_merge_warp(const MomPartial* partials, int n_parts, int at,
+                                               int stride, double* pivot, MomPartial* out) {
   auto get = [](const double* p) { return GLOBAL ? __ldcg(p) : *p; };
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t0 = NW > 1 ? (int)threadIdx.x : lane;
-  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, mn = INFINITY, mx = -INFINITY, m0[6];
-  // means about that of the first of them with particles: a mean that is the
-  // same in all stays that value exactly
-  const int first = __ffs(__ballot_sync(FULL_MASK, lane < n_parts && get(&partials[lane].n) > 0));
+  const int lane = threadIdx.x & 31;
+  MomSumsOf<double> m;
+  mom_sums_clear(m);
+  bool have = false;
+  for (; at < n_parts; at += stride) {
+    const MomPartial* p = partials + at + lane;
+    const bool valid = at + lane < n_parts;
+    const double n = valid ? get(&p->n) : 0.0;
+    double d[6], c[9];
 #pragma unroll
-  for (int d = 0; d < 6; ++d) m0[d] = first ? get(&partials[first - 1].mean[d]) : 0.0;
-  for (int t = t0; t < n_parts; t += NT) {
-    const MomPartial* q = partials + t;
-    const double n = get(&q->n);
+    for (int k = 0; k < 6; ++k) d[k] = valid ? get(&p->mean[k]) : 0.0;
 #pragma unroll
-    for (int d = 0; d < 6; ++d) s[d] = fma(n, n > 0 ? get(&q->mean[d]) - m0[d] : 0.0, s[d]);
-    s[6] += n;
-    mn = fmin(mn, get(&q->zmin));
-    mx = fmax(mx, get(&q->zmax));
-  }
-  {
-    const double t = warp_sum8_t(s);
+    for (int k = 0; k < 9; ++k) c[k] = valid ? get(&p->c[k]) : 0.0;
+    const double zmin = valid ? get(&p->zmin) : INFINITY, zmax = valid ? get(&p->zmax) : -INFINITY;
+    if (!have) {
+      const unsigned bal = __ballot_sync(FULL_MASK, n > 0);
+      if (lane == __ffs(bal) - 1)
 #pragma unroll
-    for (int k = 0; k < 7; ++k) s[k] = __shfl_sync(FULL_MASK, t, 4 * k);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fmin(mn, __shfl_xor_sync(FULL_MASK, mn, o));
-    mx = fmax(mx, __shfl_xor_sync(FULL_MASK, mx, o));
-  }
-  if (NW > 1) {
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < 7; ++k) s_sum[warp][k] = s[k];
-      s_sum[warp][7] = mn;
-      s_sum[warp][8] = mx;
+        for (int k = 0; k < 6; ++k) pivot[k] = d[k];
+      __syncwarp();
+      have = bal != 0;
     }
-    __syncthreads();
-    mn = s_sum[0][7];
-    mx = s_sum[0][8];
+    m.zmin = fmin(m.zmin, zmin);
+    m.zmax = fmax(m.zmax, zmax);
+    if (!(n > 0)) continue;
 #pragma unroll
-    for (int k = 0; k < 7; ++k) s[k] = s_sum[0][k];
-    for (int w = 1; w < NW; ++w) {
-#pragma unroll
-      for (int k = 0; k < 7; ++k) s[k] += s_sum[w][k];
-      mn = fmin(mn, s_sum[w][7]);
-      mx = fmax(mx, s_sum[w][8]);
+    for (int k = 0; k < 6; ++k) {
+      d[k] -= pivot[k];
+      m.s[k] = fma(n, d[k], m.s[k]);
+      m.q[k] += fma(n * d[k], d[k], c[k]);
     }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m.q[6 + k] += fma(n * d[2 * k], d[2 * k + 1], c[6 + k]);
+    m.n += n;
   }
-  const double inv = s[6] > 0 ? 1.0 / s[6] : 0.0;
-  double c[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int t = t0; t < n_parts; t += NT) {
-    const MomPartial* q = partials + t;
-    const double n = get(&q->n);
-    double d[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) d[k] = (get(&q->mean[k]) - m0[k]) - s[k] * inv;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) c[k] += fma(n * d[k], d[k], get(&q->c[k]));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) c[6 + k] += fma(n * d[2 * k], d[2 * k + 1], get(&q->c[6 + k]));
+  mom_partial(m, have, pivot, out);
+}
+
+// A CTA of NT threads merges n_parts partials: the warps their shares, then one
+// warp the warps' results.  Every thread of the CTA calls it; warp 0 may read
+// the result.
+template <int NT, bool GLOBAL = true>
+__device__ __forceinline__ const MomPartial* mom_merge_block(const MomPartial* partials, int n_parts) {
+  constexpr int NW = NT / 32;
+  __shared__ MomPartial s_part[NW + 1];
+  __shared__ double s_pivot[NW][6];
+  const int warp = NW > 1 ? (int)threadIdx.x >> 5 : 0;
+  mom_merge_warp<GLOBAL>(partials, n_parts, warp * 32, NT, s_pivot[warp], &s_part[warp]);
+  if (NW == 1) {
+    __syncwarp();
+    return s_part;
   }
-  const double c8[8] = {c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7]};
-  const double t = warp_sum8_t(c8);
-  double u = c[8];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(FULL_MASK, u, o);
-  if ((lane & 3) == 0) s_sum[warp][9 + warp_sum8_index(lane)] = t;
-  if (lane == 0) s_sum[warp][17] = u;
-  if (NW > 1) __syncthreads();
-  else __syncwarp();
-  if (threadIdx.x != 0) return;
-  total->n = s[6];
-  for (int k = 0; k < 6; ++k) total->mean[k] = m0[k] + s[k] * inv;
-  for (int k = 0; k < 9; ++k) {
-    double a = s_sum[0][9 + k];
-    for (int w = 1; w < NW; ++w) a += s_sum[w][9 + k];
-    total->c[k] = a;
+  __syncthreads();
+  if (warp == 0) {
+    mom_merge_warp<false>(s_part, NW, 0, 32, s_pivot[0], &s_part[NW]);
+    __syncwarp();
   }
-  total->zmin = mn;
-  total->zmax = mx;
+  return s_part + NW;
 }
 
 // One CTA of NT threads per bunch: its partials merged and finalised.  z0 = z of
@@ -357,11 +341,11 @@ __global__ void __launch_bounds__(NT) k_mom_merge(const double* __restrict__ c, 
   const int b = blockIdx.x;
   const BunchDev& B = bunch[b];
   if (B.n_chunks == 0) return;  // held by another rank
-  MomPartial total;
-  mom_merge_block<NT>(partials + (size_t)B.chunk_off * kMomWarps, B.n_chunks * kMomWarps, &total);
+  const MomPartial* total =
+      mom_merge_block<NT>(partials + (size_t)B.chunk_off * kMomWarps, B.n_chunks * kMomWarps);
   if (threadIdx.x != 0) return;
   BunchMomDev m;
-  mom_finalize(total, beta_x, beta_y, c[4 * npad + (int64_t)B.tile_off * kTile], m);
+  mom_finalize(*total, beta_x, beta_y, c[4 * npad + (int64_t)B.tile_off * kTile], m);
   m.transmission = mom[b].transmission;
   m.pad = 0.0;
   mom[b] = m;
@@ -1279,11 +1263,8 @@ __global__ void __launch_bounds__(kNoAllocThreads, 3) k_moments_noalloc(const do
   }
   mom_partial(m, have, pivot, &s_part[warp]);
   __syncthreads();
-  MomPartial total;
-  if (warp == 0) {
-    mom_merge_block<32, false>(s_part, kNoAllocThreads / 32, &total);
-    if (threadIdx.x == 0) partials[blockIdx.x] = total;
-  }
+  if (warp == 0)
+    mom_merge_warp<false>(s_part, kNoAllocThreads / 32, 0, 32, pivot, &partials[blockIdx.x]);
   // the last CTA merges
   __threadfence();
   __syncthreads();
@@ -1291,11 +1272,11 @@ __global__ void __launch_bounds__(kNoAllocThreads, 3) k_moments_noalloc(const do
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  mom_merge_block<kNoAllocThreads>(partials, (int)gridDim.x, &total);
+  const MomPartial* total = mom_merge_block<kNoAllocThreads>(partials, (int)gridDim.x);
   if (threadIdx.x != 0) return;
   *counter = 0;
   BunchMomDev s;
-  mom_finalize(total, beta_x, beta_y, c[4 * stride], s);
+  mom_finalize(*total, beta_x, beta_y, c[4 * stride], s);
   // the public record (its transmission is n_alive / n)
   cg_bunch_moments o;
   o.n_alive = (int)s.n_alive;
