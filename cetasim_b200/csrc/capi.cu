@@ -575,13 +575,17 @@ int cg_create(const cg_config* cfg, int device, cg_handle** out) {
   };
   // the ion walk, the turn's critical path, runs on the handle's stream: its
   // few CTAs go before the waiting CTAs of the particle passes beside it, which
-  // fill every SM's registers and hold them for tens of microseconds
+  // fill every SM's registers and hold them for tens of microseconds; so do
+  // the segments' records (side2)
   int low = 0, high = 0;
   if ((e = cudaDeviceGetStreamPriorityRange(&low, &high)) != cudaSuccess)
     return bail(CG_ERR_CUDA, cudaGetErrorString(e));
-  for (cudaStream_t* st : {&h.side, &h.side2})
-    if ((e = cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, low)) != cudaSuccess)
+  for (cudaStream_t* st : {&h.side, &h.side2, &h.side3})
+    if ((e = cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, st == &h.side2 ? high : low)) !=
+        cudaSuccess)
       return bail(CG_ERR_CUDA, cudaGetErrorString(e));
+  if ((e = cudaEventCreateWithFlags(&h.side3_ev, cudaEventDisableTiming)) != cudaSuccess)
+    return bail(CG_ERR_CUDA, cudaGetErrorString(e));
   h.pipe_ev.assign(kMaxPipeGroups + 1, nullptr);
   h.kick_ev.assign(kMaxPipeGroups + 1, nullptr);
   for (auto* evs : {&h.pipe_ev, &h.kick_ev})
@@ -786,6 +790,8 @@ int cg_destroy(cg_handle* H) {
   if (h.stream) cudaStreamDestroy(h.stream);
   if (h.side) cudaStreamDestroy(h.side);
   if (h.side2) cudaStreamDestroy(h.side2);
+  if (h.side3) cudaStreamDestroy(h.side3);
+  if (h.side3_ev) cudaEventDestroy(h.side3_ev);
   for (auto* evs : {&h.pipe_ev, &h.kick_ev, &h.trace_ev})
     for (auto ev : *evs)
       if (ev) cudaEventDestroy(ev);
@@ -1403,7 +1409,7 @@ static cudaError_t trace_mark(Handle& h, cudaStream_t s, int kind, int ip, int s
   }
   TraceMark m;
   m.kind = kind;
-  m.stream = s == h.side ? 1 : s == h.side2 ? 2 : 0;
+  m.stream = s == h.side ? 1 : s == h.side2 ? 2 : s == h.side3 ? 3 : 0;
   m.ip = ip;
   m.seg = seg;
   h.trace->push_back(m);
@@ -1442,10 +1448,14 @@ static cudaError_t enqueue_turn(Handle& h) {
     // the z range with the turn's last moments, the ones cg_get_moments returns
     const bool zr = k == (post ? h.K - 1 : h.K - 2);
     if (c.flag_beam_ion && G > 1 && !c.flag_sc) {
-      // the walk in G segments of bunches on the main stream; as soon as a
-      // segment is walked, its records and kick on `side` and its map (with
-      // the next IP's moments) on `side2`, so that the walk of segment g + 1,
-      // the kick of g + 1 and the map of g run at the same time
+      // the walk in G segments of bunches on the main stream.  As soon as a
+      // segment is walked: its records on `side2` (a few CTAs, before those of
+      // the passes), then its pass on `side` or, every other segment, `side3`,
+      // so that the pass of g starts in the tail of that of g - 1 and neither
+      // waits for records (the 80-bunch train 2725 -> 2503 us a turn; in one
+      // stream, records between the passes; passes in one stream 2520).
+      // Kick and map apart: records and kick on `side`, the map on `side2`, so
+      // that the walk of g + 1, the kick of g + 1 and the map of g overlap.
       if ((e = launch_ion_prep(h, k))) return e;
       TRACE(h.stream, CG_TRACE_ION_PREP, k, -1);
       for (int g = 0; g < G; ++g) {
@@ -1453,15 +1463,19 @@ static cudaError_t enqueue_turn(Handle& h) {
         if ((e = launch_ion_walk(h, k, ja, jb, h.stream))) return e;
         TRACE(h.stream, CG_TRACE_ION_WALK, k, g);
         if ((e = cudaEventRecord(h.pipe_ev[g], h.stream))) return e;
-        if ((e = cudaStreamWaitEvent(h.side, h.pipe_ev[g], 0))) return e;
-        if ((e = launch_ion_records(h, k, ja, jb, h.side))) return e;
-        TRACE(h.side, CG_TRACE_ION_RECORDS, k, g);
+        const cudaStream_t rs = fused ? h.side2 : h.side;
+        if ((e = cudaStreamWaitEvent(rs, h.pipe_ev[g], 0))) return e;
+        if ((e = launch_ion_records(h, k, ja, jb, rs))) return e;
+        TRACE(rs, CG_TRACE_ION_RECORDS, k, g);
         const int ta = h.tile_off[ja], tb = h.tile_off[jb];
         const int ca = h.chunk_off[ja], cb = h.chunk_off[jb];
         if (fused) {
-          if ((e = launch_map_pass(h, k, mom, true, zr, ca, cb, h.side))) return e;
-          TRACE(h.side, CG_TRACE_ION_KICK, k, g);  // both in one launch
-          TRACE(h.side, CG_TRACE_MAP_PASS, k, g);
+          const cudaStream_t ps = g & 1 ? h.side3 : h.side;
+          if ((e = cudaEventRecord(h.kick_ev[g], rs))) return e;
+          if ((e = cudaStreamWaitEvent(ps, h.kick_ev[g], 0))) return e;
+          if ((e = launch_map_pass(h, k, mom, true, zr, ca, cb, ps))) return e;
+          TRACE(ps, CG_TRACE_ION_KICK, k, g);  // both in one launch
+          TRACE(ps, CG_TRACE_MAP_PASS, k, g);
           continue;
         }
         e = h.d.sur_w ? launch_ion_kick_sur(h, k, ta, tb, h.side)
@@ -1474,13 +1488,16 @@ static cudaError_t enqueue_turn(Handle& h) {
         if ((e = launch_map_pass(h, k, mom, false, zr, ca, cb, h.side2))) return e;
         TRACE(h.side2, CG_TRACE_MAP_PASS, k, g);
       }
-      if ((e = launch_ion_compact(h, k, h.side))) return e;
-      TRACE(h.side, CG_TRACE_ION_COMPACT, k, -1);
+      const cudaStream_t cs = fused ? h.side2 : h.side;
+      if ((e = launch_ion_compact(h, k, cs))) return e;
+      TRACE(cs, CG_TRACE_ION_COMPACT, k, -1);
       if ((e = cudaEventRecord(h.pipe_ev[kMaxPipeGroups], h.side))) return e;
       if ((e = cudaStreamWaitEvent(h.stream, h.pipe_ev[kMaxPipeGroups], 0))) return e;
-      if (!fused) {
-        if ((e = cudaEventRecord(h.kick_ev[kMaxPipeGroups], h.side2))) return e;
-        if ((e = cudaStreamWaitEvent(h.stream, h.kick_ev[kMaxPipeGroups], 0))) return e;
+      if ((e = cudaEventRecord(h.kick_ev[kMaxPipeGroups], h.side2))) return e;
+      if ((e = cudaStreamWaitEvent(h.stream, h.kick_ev[kMaxPipeGroups], 0))) return e;
+      if (fused && G > 1) {
+        if ((e = cudaEventRecord(h.side3_ev, h.side3))) return e;
+        if ((e = cudaStreamWaitEvent(h.stream, h.side3_ev, 0))) return e;
       }
       if (mom >= 0 && (e = launch_mom_merge(h, mom))) return e;
     } else {

@@ -234,9 +234,11 @@ struct Handle {
   std::vector<TraceMark>* trace = nullptr;
   std::vector<cudaEvent_t> trace_ev;
   cudaStream_t side = nullptr;   // records and kicks of the segments
-  cudaStream_t side2 = nullptr;  // maps of the segments (kick g + 1 overlaps map g)
+  cudaStream_t side2 = nullptr;  // the segments' records, or (kick and map apart) their maps
+  cudaStream_t side3 = nullptr;  // every other segment's pass
+  cudaEvent_t side3_ev = nullptr;    // its join
   std::vector<cudaEvent_t> pipe_ev;  // kMaxPipeGroups + 1: walked segments, then the join
-  std::vector<cudaEvent_t> kick_ev;  // kMaxPipeGroups + 1: kicked segments, then the join
+  std::vector<cudaEvent_t> kick_ev;  // kMaxPipeGroups + 1: recorded or kicked segments, then the join
   std::vector<double> ne;
   DeviceBufs d;
   int lr_np = 0;

@@ -610,7 +610,7 @@ enum {
 
 typedef struct {
   int kind;         /* CG_TRACE_* */
-  int stream;       /* 0 the handle's stream, 1 and 2 the pipelined turn's side streams */
+  int stream;       /* 0 the handle's stream, 1 to 3 the pipelined turn's side streams */
   int ip;           /* interaction point / section, or -1 */
   int segment;      /* walk segment of the pipelined turn, or -1 */
   double t_end_us;  /* completion after the turn's start (CUDA events), microseconds */
