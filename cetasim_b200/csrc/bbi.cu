@@ -23,7 +23,7 @@
 //  k_bbi_range  per-bunch lowest and highest bin and the largest |x|, |y|
 //               (atomics); in the turn the longitudinal pass before it does
 //               this with the positions that it writes (bbi_span_cta).
-//  k_bbi_hist   per chunk: per-bin counts and sums of x and y in 64-bit fixed
+//  k_bbi_hist   per CTA: per-bin counts and sums of x and y in 64-bit fixed
 //               point (the scale from the bunch's largest |x|, |y|), so the
 //               result does not depend on the order of the atomics; in shared
 //               memory, then added to the bunch's.
@@ -36,7 +36,7 @@
 // Bound by: the passes by HBM (38 MB to count, 115 MB to kick 1.6e6 particles)
 // and its latency, the convolution by its chains of FMAs and barriers.  80
 // bunches of 20,000, five planes, us: range 25 -> in the longitudinal pass,
-// hist 53 -> 21 (global 64-bit atomics), conv 28 -> 15 (256 threads, a
+// hist 53 -> 14 (global 64-bit atomics), conv 28 -> 15 (256 threads, a
 // filter with bounds checks per tap, one chain of 600 FMAs per bin and plane),
 // kick 40 and the loss check 16 -> 24 together (up to fourteen divisions a particle).
 #include <algorithm>
@@ -79,17 +79,16 @@ __global__ void __launch_bounds__(kTile) k_bbi_range(const double* __restrict__ 
 
 __global__ void __launch_bounds__(kBbiThreads) k_bbi_hist(const double* __restrict__ c, int64_t npad,
                                                           const uint8_t* __restrict__ surv,
-                                                          const int4* __restrict__ chunk_loc,
                                                           const BunchDev* __restrict__ bunch,
+                                                          int tiles,
                                                           const __grid_constant__ BbiParams p,
                                                           const BbiSpan* __restrict__ span,
                                                           int* status, int* cnt,
                                                           unsigned long long* sxy) {
   extern __shared__ unsigned s_bin[];  // W counts, then x (lo, hi), y (lo, hi)
-  const int4 l = chunk_loc[blockIdx.x];
-  const BunchDev& Bd = bunch[l.x];
-  if (Bd.q_macro == 0) return;
-  const int b = l.x;
+  const int b = blockIdx.x, t0 = blockIdx.y * tiles;
+  const BunchDev& Bd = bunch[b];
+  if (Bd.q_macro == 0 || t0 >= Bd.n_tiles) return;
   const BbiSpan S = span[b];
   const int first = S.lo(), W = S.bins();
   if (W < 1) return;
@@ -105,9 +104,9 @@ __global__ void __launch_bounds__(kBbiThreads) k_bbi_hist(const double* __restri
   const Pow2 fx = pow2_split(bbi_fix_exp(S.ax, Bd.n));
   const Pow2 fy = pow2_split(bbi_fix_exp(S.ay, Bd.n));
   const size_t base = (size_t)b * p.wcap;
-  int64_t g = (int64_t)l.y * kTile + threadIdx.x;
-  int i = (l.y - Bd.tile_off) * kTile + threadIdx.x;
-  for (int u = 0; u < l.z && i < Bd.n; ++u, g += kTile, i += kTile) {
+  int64_t g = (int64_t)(Bd.tile_off + t0) * kTile + threadIdx.x;
+  int i = t0 * kTile + threadIdx.x;
+  for (int u = 0; u < tiles && i < Bd.n; ++u, g += kTile, i += kTile) {
     const double x = c[g], y = c[2 * npad + g];
     const int idx = bbi_bin(p, c[4 * npad + g]);
     const bool sums = !p.td || surv[g] == kAlive;
@@ -385,9 +384,14 @@ cudaError_t launch_bbi(Handle& h, bool have_range, bool mark) {
   if (!have_range)
     k_bbi_range<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
                                                    h.d.bunch, p, span, h.d.status);
-  k_bbi_hist<<<h.n_chunks, kBbiThreads, 5 * sizeof(unsigned) * std::min(p.wcap, kBbiSharedBins),
-               h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.d.bunch, p, span, h.d.status,
-                           h.d.bbi_cnt, h.d.bbi_sxy);
+  // six CTAs per SM: each ends with an atomic per bin and sum, so no more CTAs
+  // than the particles' reads need (two tiles each: 20 us, eight: 13.7)
+  int big = 1;
+  for (int j = 0; j < h.M; ++j) big = std::max(big, h.tile_off[j + 1] - h.tile_off[j]);
+  const int tiles = std::max(1, (h.n_tiles + 148 * 6 - 1) / (148 * 6));
+  k_bbi_hist<<<dim3(h.M, (big + tiles - 1) / tiles), kBbiThreads,
+               5 * sizeof(unsigned) * std::min(p.wcap, kBbiSharedBins), h.stream>>>(
+      h.d.c, h.npad, h.d.surv, h.d.bunch, tiles, p, span, h.d.status, h.d.bbi_cnt, h.d.bbi_sxy);
   k_bbi_conv<<<h.M, kBbiConvThreads, bbi_conv_smem(p), h.stream>>>(
       h.d.bunch, p, h.d.bbi_w, span, h.d.bbi_cnt, h.d.bbi_sxy, h.d.bbi_pot, kick, h.d.bbi_win);
   (mark ? k_bbi_kick<true> : k_bbi_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(

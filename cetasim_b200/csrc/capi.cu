@@ -1437,6 +1437,7 @@ static cudaError_t enqueue_turn(Handle& h) {
     TRACE(h.stream, CG_TRACE_MOMENTS, 0, -1);
   }
   const int G = std::max(1, std::min(h.pipe_groups, h.M));
+  bool long_map = false;  // the last map joins the longitudinal pass
   for (int k = 0; k < h.K; ++k) {
     // the space charge kicks between the ion kick and the map, so neither
     // the kick inside the map pass nor the segmented pipeline
@@ -1511,7 +1512,8 @@ static cudaError_t enqueue_turn(Handle& h) {
       }
       if (c.flag_sc && (e = launch_space_charge(h, k))) return e;
       if (k == h.K - 1 && (e = launch_phase_adv(h, 0, h.M))) return e;
-      if ((e = launch_map_pass(h, k, mom, fused, zr))) return e;
+      long_map = k == h.K - 1 && mom < 0 && !fused && !h.ring.bl_any;
+      if (!long_map && (e = launch_map_pass(h, k, mom, fused, zr))) return e;
       if (fused) TRACE(h.stream, CG_TRACE_ION_KICK, k, -1);
       TRACE(h.stream, CG_TRACE_MAP_PASS, k, -1);
     }
@@ -1535,7 +1537,7 @@ static cudaError_t enqueue_turn(Handle& h) {
   // or the ranges of the kick after it
   const unsigned tail = c.flag_sr_wake ? kLongSr : mark ? kLongMark : 0u;
   fl |= c.bbi.flag ? kLongBbi : tail;
-  if ((e = launch_long(h, fl))) return e;
+  if ((e = launch_long(h, fl, long_map))) return e;
   TRACE(h.stream, CG_TRACE_LONG, -1, -1);
   if (c.bbi.flag) {
     if ((e = launch_bbi(h, true, mark && !c.flag_lr_wake))) return e;

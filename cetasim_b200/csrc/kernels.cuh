@@ -80,7 +80,8 @@ enum LongFlags : unsigned {
   kLongBbi = 64,
   kLongSr = 128,
 };
-cudaError_t launch_long(Handle& h, unsigned flags);
+// map: after the map of the ring's last section (no beam loading)
+cudaError_t launch_long(Handle& h, unsigned flags, bool map = false);
 // cavities with beam loading: z ranges and bins of the RF step, then the
 // cavities' recurrence over the train (beam_loading.cu); k_long applies the
 // kicks
