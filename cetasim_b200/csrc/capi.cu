@@ -580,18 +580,20 @@ int cg_create(const cg_config* cfg, int device, cg_handle** out) {
   int low = 0, high = 0;
   if ((e = cudaDeviceGetStreamPriorityRange(&low, &high)) != cudaSuccess)
     return bail(CG_ERR_CUDA, cudaGetErrorString(e));
-  for (cudaStream_t* st : {&h.side, &h.side2, &h.side3})
-    if ((e = cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, st == &h.side2 ? high : low)) !=
-        cudaSuccess)
-      return bail(CG_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = cudaEventCreateWithFlags(&h.side3_ev, cudaEventDisableTiming)) != cudaSuccess)
-    return bail(CG_ERR_CUDA, cudaGetErrorString(e));
   h.pipe_ev.assign(kMaxPipeGroups + 1, nullptr);
   h.kick_ev.assign(kMaxPipeGroups + 1, nullptr);
-  for (auto* evs : {&h.pipe_ev, &h.kick_ev})
-    for (auto& ev : *evs)
-      if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+  if (cfg->flag_beam_ion) {
+    for (cudaStream_t* st : {&h.side, &h.side2, &h.side3})
+      if ((e = cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, st == &h.side2 ? high : low)) !=
+          cudaSuccess)
         return bail(CG_ERR_CUDA, cudaGetErrorString(e));
+    if ((e = cudaEventCreateWithFlags(&h.side3_ev, cudaEventDisableTiming)) != cudaSuccess)
+      return bail(CG_ERR_CUDA, cudaGetErrorString(e));
+    for (auto* evs : {&h.pipe_ev, &h.kick_ev})
+      for (auto& ev : *evs)
+        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+          return bail(CG_ERR_CUDA, cudaGetErrorString(e));
+  }
   if ((e = cudaStreamCreateWithPriority(&h.stream, cudaStreamNonBlocking, high)) != cudaSuccess)
     return bail(CG_ERR_CUDA, cudaGetErrorString(e));
   if ((e = dalloc(&h.sec_dev, h.K)) != cudaSuccess) return bail(CG_ERR_OOM, "sections");
@@ -727,14 +729,19 @@ int cg_create(const cg_config* cfg, int device, cg_handle** out) {
     if (p.flag == 2) {
       // the DST-I matrices 2 sin(pi (i + 1)(k + 1) / (n + 1)), the argument
       // reduced modulo 2 (n + 1) first
-      std::vector<double> sn((size_t)p.nx * p.nx + (size_t)p.ny * p.ny + p.nx + p.ny);
+      // as the solve keeps them in shared memory, zeros to whole 8 x 8 tiles
+      const int px = sc_pad(p.nx), py = sc_pad(p.ny);
+      std::vector<double> sn((size_t)px * sc_stride(px) + (size_t)py * sc_stride(py) + p.nx + p.ny);
       size_t o = 0;
-      for (int n : {p.nx, p.ny})
+      for (int n : {p.nx, p.ny}) {
+        const int row = sc_stride(sc_pad(n));
         for (int k = 0; k < n; ++k)
           for (int i = 0; i < n; ++i) {
             const long r = (long)(i + 1) * (k + 1) % (2 * (n + 1));
-            sn[o++] = 2 * std::sin(kPi * (double)r / (n + 1));
+            sn[o + (size_t)k * row + i] = 2 * std::sin(kPi * (double)r / (n + 1));
           }
+        o += (size_t)sc_pad(n) * row;
+      }
       // then the sines of the Laplacian's eigenvalues, sin(pi / 2 (k + 1) / (n + 1))
       // as PIC2D::Set2DPhi forms them (PIC2D.cpp:303-307)
       for (int n : {p.nx, p.ny})
@@ -1026,6 +1033,7 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
       return fail(&h, CG_ERR_OOM, "space-charge buffers");
     }
     cudaMemset(d.sc_geom, 0, sizeof(double) * M * kScGeom);
+    cudaMemset(d.sc_range, 0, sizeof(unsigned long long) * M * 4);
   }
   if (h.cfg.bbi.flag) {
     const size_t wc = h.bbi.wcap;
@@ -1270,7 +1278,7 @@ int cg_space_charge(cg_handle* H, int k) {
   STAGE_PROLOGUE
   if (!h.cfg.flag_sc) return fail(&h, CG_ERR_NOT_READY, "runSpaceCharge is off");
   if (k < 0 || k >= h.K) return fail(&h, CG_ERR_INVALID, "section index out of range");
-  int st = launch_ok(h, launch_space_charge(h, k), "space charge");
+  int st = launch_ok(h, launch_space_charge(h, k, false), "space charge");
   return st ? st : check_status(h);
 }
 int cg_bbi_kick(cg_handle* H) {
@@ -1446,8 +1454,9 @@ static cudaError_t enqueue_turn(Handle& h) {
     int mom = -1;
     if (k + 1 < h.K) mom = sec_mom ? k + 1 : -1;
     else mom = post ? h.K - 1 : -1;
-    // the z range with the turn's last moments, the ones cg_get_moments returns
-    const bool zr = k == (post ? h.K - 1 : h.K - 2);
+    // the z range with the turn's last moments, the ones cg_get_moments
+    // returns, and where the space charge's mesh slices it
+    const bool zr = k == (post ? h.K - 1 : h.K - 2) || c.flag_sc == 2;
     if (c.flag_beam_ion && G > 1 && !c.flag_sc) {
       // the walk in G segments of bunches on the main stream.  As soon as a
       // segment is walked: its records on `side2` (a few CTAs, before those of
@@ -1510,7 +1519,7 @@ static cudaError_t enqueue_turn(Handle& h) {
           TRACE(h.stream, CG_TRACE_ION_KICK, k, -1);
         }
       }
-      if (c.flag_sc && (e = launch_space_charge(h, k))) return e;
+      if (c.flag_sc && (e = launch_space_charge(h, k, true))) return e;
       if (k == h.K - 1 && (e = launch_phase_adv(h, 0, h.M))) return e;
       long_map = k == h.K - 1 && mom < 0 && !fused && !h.ring.bl_any;
       if (!long_map && (e = launch_map_pass(h, k, mom, fused, zr))) return e;

@@ -37,6 +37,11 @@ struct BbiParams {
   double g[2 * kBbiHalf + 1];  // normalised Gaussian filter kernel
 };
 
+// The PIC mesh in shared memory: nodes to whole 8 x 8 tiles, and the row stride
+// (4 or 12 modulo 16 doubles: a tile's loads meet no bank twice).
+constexpr int sc_pad(int n) { return (n + 7) / 8 * 8; }
+constexpr int sc_stride(int padded) { return padded + 4; }
+
 // Space charge (cg_config::flag_sc), set up at cg_create.
 struct ScParams {
   int flag = 0;                // 1 Bassetti-Erskine slices, 2 2.5-D PIC, 3 linear
@@ -174,7 +179,7 @@ struct DeviceBufs {
   double* sc_xy = nullptr;         // npad x (x, y) grouped by bunch and slice (PIC)
   int* sc_start = nullptr;         // M x nz: first entry of each slice (PIC)
   int* sc_cursor = nullptr;        // M x nz: fill cursors (PIC)
-  double* sc_sin = nullptr;        // nx x nx + ny x ny: 2 sin(pi (i + 1)(k + 1) / (n + 1))
+  double* sc_sin = nullptr;        // per axis 2 sin(pi (i + 1)(k + 1) / (n + 1)), padded; eigenvalue sines
   // phase advance of the tracked bunches: slot per bunch (-1 untracked),
   // per slot 6 x n (previous angles x, y, z; accumulated x, y, z)
   int* phase_slot = nullptr;

@@ -23,7 +23,8 @@ cudaError_t launch_phase_init(Handle& h);
 cudaError_t launch_phase_adv(Handle& h, int ja, int jb, cudaStream_t s = nullptr);
 
 // space charge (sc.cu)
-cudaError_t launch_space_charge(Handle& h, int k);
+// have_range: the moments are those of section k, with the z range
+cudaError_t launch_space_charge(Handle& h, int k, bool have_range);
 size_t sc_solve_smem(const ScParams& p);
 size_t sc_slice_bytes();  // of one slice's constants (slice models)
 cudaError_t prepare_sc(const ScParams& p);

@@ -17,8 +17,9 @@
 // Every flag ends in the same momentum update (PIC2D.cpp, MPBunch.cpp:740-760).
 //
 //  k_sc_range    per chunk: the survivors' z range (GetZMinMax, seeded with
-//                particle 0) and the largest |x|, |y| (ordered bit patterns
-//                under atomics).
+//                particle 0) and, for the slice models, the largest |x|, |y|
+//                (ordered bit patterns under atomics).  In the turn the PIC
+//                takes the range from the moments formed just before.
 //  k_sc_geom     per bunch: the slice width, the mesh (PIC2D::Set2DMesh(rms,
 //                centroid), PIC2D.cpp), the fixed-point scales.
 //  k_sc_count    per chunk: particles per slice in shared memory, then added to
@@ -33,15 +34,18 @@
 //                solve as two matrix products each way on the FP64 tensor
 //                instructions, then the field on the mesh.
 //  k_sc_kick     per tile: the field at each particle and the kick.
-// Bound by: the passes over the particles by HBM and by shared-memory atomics,
-// the solve by its products and its barriers (one slice is a few hundred tile
-// products), the field models by the FP64 pipe.  A section of 80 bunches of
-// 20,000, us: PIC 32 x 32 x 33 468 -> 232 (solve 95, kick 41, scatter 25, range
-// and count 13 each, merge 12, geom 5, offsets 4, with the map pass's 46 in the
-// sum); Bassetti-Erskine slices 373 -> 143.  Before, the transforms were plain
-// FP64 dot products, the deposit went through 64-bit shared atomics
+// Bound by: the passes over the particles by HBM latency and shared-memory
+// atomics, the solve by its deposit (the beam's core is a few cells wide) and
+// the barriers round four small matrix products, the field models by the FP64
+// pipe.  A section of 80 bunches of 20,000, us: PIC 32 x 32 x 33 468 -> 198
+// (solve 80, map 47, kick 38, scatter 24, count 13, moments' merge 9, geom 4,
+// offsets 3); Bassetti-Erskine slices 373 -> 129.  Before, the transforms were
+// plain FP64 dot products, the deposit went through 64-bit shared atomics
 // (compare-and-swap loops) from the whole bunch's particles, and the kick
-// evaluated w(z) through the general path.
+// evaluated w(z) through the general path.  In the solve index arithmetic and
+// divisions had cost as much as the products (95 -> 80 us with padded tables,
+// two tiles a time and one reciprocal per node); four copies of the charge
+// against the deposit's conflicts gained nothing (97).
 #include <algorithm>
 #include <cuda_runtime.h>
 
@@ -72,31 +76,8 @@ __device__ __forceinline__ double sc_fix(unsigned long long v, int e) {
   return scalbn((double)(long long)v, -e);
 }
 
-// Doubles as integers in the same order (for atomicMin / atomicMax).
-__device__ __forceinline__ unsigned long long sc_key(double v) {
-  const long long b = __double_as_longlong(v);
-  return (unsigned long long)b ^ (b < 0 ? ~0ull : 1ull << 63);
-}
-__device__ __forceinline__ double sc_unkey(unsigned long long k) {
-  return __longlong_as_double((long long)(k ^ (k >> 63 ? 1ull << 63 : ~0ull)));
-}
-
-// range[4 b ..]: keys of the survivors' lowest and highest z (particle 0 not
-// yet in them), bit patterns of the largest |x|, |y|.
-__global__ void k_sc_clear(unsigned long long* range, int* cnt, unsigned long long* acc, int M,
-                           int nz, int per) {
-  const int n = M * nz;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    cnt[i] = 0;
-    for (int q = 0; q < per; ++q) acc[(size_t)i * per + q] = 0ull;
-  }
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < M; b += gridDim.x * blockDim.x) {
-    range[4 * b] = sc_key(INFINITY);
-    range[4 * b + 1] = sc_key(-INFINITY);
-    range[4 * b + 2] = range[4 * b + 3] = 0ull;
-  }
-}
-
+// range[4 b ..]: maxima over bunch b, zero between calls: keys (sr_key) of the
+// survivors' -z and z (particle 0 not yet in them), bit patterns of |x|, |y|.
 template <bool XY>
 __global__ void __launch_bounds__(kScThreads) k_sc_range(const double* __restrict__ c, int64_t npad,
                                                          const uint8_t* __restrict__ surv,
@@ -140,29 +121,44 @@ __global__ void __launch_bounds__(kScThreads) k_sc_range(const double* __restric
   for (int w = 1; w < kScThreads / 32; ++w)
     v = threadIdx.x == 0 ? fmin(v, red[0][w]) : fmax(v, red[threadIdx.x][w]);
   unsigned long long* r = range + 4 * (size_t)l.x + threadIdx.x;
-  if (threadIdx.x == 0) atomicMin(r, sc_key(v));
-  else if (threadIdx.x == 1) atomicMax(r, sc_key(v));
-  else if (XY) atomicMax(r, (unsigned long long)__double_as_longlong(v));
+  if (threadIdx.x < 2) {
+    // no survivor leaves the minimum at infinity, the maximum at minus infinity
+    if (threadIdx.x == 0 ? v < INFINITY : v > -INFINITY) atomicMax(r, sr_key(threadIdx.x == 0 ? -v : v));
+  } else if (XY) atomicMax(r, (unsigned long long)__double_as_longlong(v));
 }
 
+// ranges: from `range`; else the moments' (of this section, of the beam as it
+// is now: the same numbers).  Clears the counts and, per slice, `per` sums.
 __global__ void k_sc_geom(const double* __restrict__ c, int64_t npad,
                           const BunchDev* __restrict__ bunch, const BunchMomDev* __restrict__ mom,
-                          ScParams p, const unsigned long long* __restrict__ range, double* geom,
-                          int* status, int M) {
+                          ScParams p, unsigned long long* range, bool ranges, double* geom,
+                          int* status, int M, int* cnt, unsigned long long* acc, int per) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < M * p.nz) {
+    cnt[b] = 0;
+    for (int q = 0; q < per; ++q) acc[(size_t)b * per + q] = 0ull;
+  }
   if (b >= M) return;
   const BunchDev& Bd = bunch[b];
   if (Bd.n < 1) return;
-  const double z0 = c[4 * npad + (int64_t)Bd.tile_off * kTile];
-  const double zmn = fmin(z0, sc_unkey(range[4 * b])), zmx = fmax(z0, sc_unkey(range[4 * b + 1]));
+  const BunchMomDev& m = mom[b];
+  double zMin = m.z_min, zMax = m.z_max, rx = 0, ry = 0;
+  if (ranges) {
+    unsigned long long* r = range + 4 * (size_t)b;
+    const double z0 = c[4 * npad + (int64_t)Bd.tile_off * kTile];
+    // GetZMinMax (MPBunch.cpp:1883-1884)
+    zMin = (r[0] ? fmin(z0, -sr_unkey(r[0])) : z0) - 1.e-6;
+    zMax = (r[1] ? fmax(z0, sr_unkey(r[1])) : z0) + 1.e-6;
+    rx = __longlong_as_double((long long)r[2]);
+    ry = __longlong_as_double((long long)r[3]);
+    r[0] = r[1] = r[2] = r[3] = 0ull;
+  }
   double* G = geom + (size_t)b * kScGeom;
-  // GetZMinMax (MPBunch.cpp:1883-1884) and SetSlicedBunchInfo (:670)
-  const double zMin = zmn - 1.e-6, zMax = zmx + 1.e-6;
+  // SetSlicedBunchInfo (MPBunch.cpp:670)
   G[kGZmin] = zMin;
   G[kGDz] = (zMax - zMin) / (p.nz - 1);
   G[kGIDz] = 1.0 / G[kGDz];
   const double charge = Bd.q_macro * kElectronCharge / G[kGDz];  // [C/m], MPBunch.cpp:689
-  const BunchMomDev& m = mom[b];
   if (p.flag == 2) {
     // PIC2D::Set2DMesh(rmsXY, averXY) (PIC2D.cpp) from the moments of this section
     const double rms[2] = {m.rms_x, m.rms_y}, cen[2] = {m.mean[0], m.mean[2]};
@@ -190,8 +186,7 @@ __global__ void k_sc_geom(const double* __restrict__ c, int64_t npad,
     // the sums' pivot: the bunch centroid (zero if there is none)
     const double px = isfinite(m.mean[0]) ? m.mean[0] : 0.0;
     const double py = isfinite(m.mean[2]) ? m.mean[2] : 0.0;
-    const double ax = __longlong_as_double((long long)range[4 * b + 2]) + fabs(px);
-    const double ay = __longlong_as_double((long long)range[4 * b + 3]) + fabs(py);
+    const double ax = rx + fabs(px), ay = ry + fabs(py);
     G[kGPx] = px;
     G[kGPy] = py;
     G[kGExp0] = sc_fix_exp(ax, Bd.n);
@@ -251,8 +246,10 @@ __global__ void __launch_bounds__(kScThreads) k_sc_count(const double* __restric
   for (int q = 0; q < 4; ++q) f[q] = PIC ? Pow2{0, 0} : pow2_split((int)G[kGExp0 + q]);
   int64_t g = (int64_t)l.y * kTile + threadIdx.x;
   for (int u = 0; u < l.z; ++u, g += kTile) {
-    if (surv[g] == kPadding) break;
-    const int s = sc_slice(c[4 * npad + g], G, nz);
+    const uint8_t sv = surv[g];
+    const double z = c[4 * npad + g];
+    if (sv == kPadding) break;
+    const int s = sc_slice(z, G, nz);
     if (shared) atomicAdd(&s_sum[s], 1u);
     else atomicAdd(&cnt[b0 + s], 1);
     if (!PIC) {
@@ -347,6 +344,7 @@ __global__ void __launch_bounds__(kScThreads) k_sc_scatter(const double* __restr
   const size_t b0 = (size_t)l.x * nz;
   const int64_t g0 = (int64_t)l.y * kTile + threadIdx.x;
   unsigned rank[kMaxChunkTiles];
+  int slot[kMaxChunkTiles];
   if (shared) {
     // the chunk's places in each slice with one global atomic per slice
     for (int i = threadIdx.x; i < nz; i += kScThreads) s_sum[i] = 0u;
@@ -356,7 +354,11 @@ __global__ void __launch_bounds__(kScThreads) k_sc_scatter(const double* __restr
 #pragma unroll
       for (int u = 0; u < kMaxChunkTiles; ++u) {
         const int64_t g = g0 + (int64_t)(u0 + u) * kTile;
-        if (u < nu && surv[g] != kPadding) rank[u] = atomicAdd(&s_sum[sc_slice(c[4 * npad + g], G, nz)], 1u);
+        if (u >= nu) break;
+        const uint8_t sv = surv[g];
+        const double z = c[4 * npad + g];
+        slot[u] = sv != kPadding ? sc_slice(z, G, nz) : -1;
+        if (slot[u] >= 0) rank[u] = atomicAdd(&s_sum[slot[u]], 1u);
       }
       __syncthreads();
       for (int s = threadIdx.x; s < nz; s += kScThreads) {
@@ -367,8 +369,9 @@ __global__ void __launch_bounds__(kScThreads) k_sc_scatter(const double* __restr
 #pragma unroll
       for (int u = 0; u < kMaxChunkTiles; ++u) {
         const int64_t g = g0 + (int64_t)(u0 + u) * kTile;
-        if (u < nu && surv[g] != kPadding)
-          xy[s_sum[nz + sc_slice(c[4 * npad + g], G, nz)] + rank[u]] = make_double2(c[g], c[2 * npad + g]);
+        if (u >= nu) break;
+        const double2 v = make_double2(c[g], c[2 * npad + g]);
+        if (slot[u] >= 0) xy[s_sum[nz + slot[u]] + rank[u]] = v;
       }
       __syncthreads();
     }
@@ -381,24 +384,36 @@ __global__ void __launch_bounds__(kScThreads) k_sc_scatter(const double* __restr
   }
 }
 
-// D = A B on the FP64 tensor instructions (m8n8k4): one 8 x 8 tile of the
-// product of A (rows, K) and B (K, columns), both row by row in shared memory
-// with a row stride of 4 or 12 modulo 16 doubles (no bank conflicts).  Lane l
-// gets the elements (l / 4, 2 (l % 4)) and the next.
-__device__ __forceinline__ void sc_mma_tile(const double* A, int lda, const double* B, int ldb, int K,
-                                            double (&d)[2]) {
+// D = A B on the FP64 tensor instructions (m8n8k4): one or two neighbouring
+// 8 x 8 tiles of a row of the product of A (rows, K) and B (K, columns), both
+// row by row in shared memory with a row stride of 4 or 12 modulo 16 doubles
+// (no bank conflicts).  Lane l gets the elements (l / 4, 2 (l % 4)) and the
+// next.  Two tiles share A's loads, and one waits while the other multiplies.
+__device__ __forceinline__ void sc_mma(double a, double b, double (&d)[2]) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void sc_mma_tiles(const double* A, int lda, const double* B, int ldb, int K,
+                                             bool two, double (&d)[2][2]) {
   const int lane = threadIdx.x & 31;
   const double* a = A + (lane >> 2) * lda + (lane & 3);
   const double* b = B + (lane & 3) * ldb + (lane >> 2);
-  d[0] = d[1] = 0.0;
-  for (int k = 0; k < K; k += 4) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a[k]), "d"(b[k * ldb]));
+  d[0][0] = d[0][1] = d[1][0] = d[1][1] = 0.0;
+  const int step = 4 * ldb;
+  if (two) {
+#pragma unroll 2
+    for (int k = 0; k < K; k += 8, a += 8, b += 2 * step) {  // K: whole tiles
+      const double a0 = a[0], a1 = a[4], b0 = b[0], c0 = b[8], b1 = b[step], c1 = b[step + 8];
+      sc_mma(a0, b0, d[0]);
+      sc_mma(a0, c0, d[1]);
+      sc_mma(a1, b1, d[0]);
+      sc_mma(a1, c1, d[1]);
+    }
+  } else {
+    for (int k = 0; k < K; k += 4, a += 4, b += step) sc_mma(a[0], b[0], d[0]);
   }
 }
-
-__host__ __device__ inline int sc_pad(int n) { return (n + 7) / 8 * 8; }
 
 // One CTA per (bunch, slice): PIC2D::Set2DPhi and Set2DEField (PIC2D.cpp).
 // The 2-D DST-I (RODFT00, Y_k = 2 sum_j X_j sin(pi (j + 1)(k + 1) / (n + 1))
@@ -418,7 +433,7 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const Bunch
   const double* G = geom + (size_t)b * kScGeom;
   const int n = cnt[bs];
   if (n < 2 || G[kGIDv] == 0) return;  // a skipped slice (MPBunch.cpp:916)
-  const int px = sc_pad(nx), py = sc_pad(ny), lx = px + 4, ly = py + 4;
+  const int px = sc_pad(nx), py = sc_pad(ny), lx = sc_stride(px), ly = sc_stride(py);
   double* R = sm;                // px x ly
   double* T = R + px * ly;       // px x ly
   double* Sx = T + px * ly;      // px x lx
@@ -427,14 +442,9 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const Bunch
   unsigned* hi = lo + N;
   const int e = (int)G[kGExp0];
   for (int t = threadIdx.x; t < 2 * N; t += kScThreads) lo[t] = 0u;
-  for (int t = threadIdx.x; t < px * lx; t += kScThreads) {
-    const int i = t / lx, k = t % lx;
-    Sx[t] = i < nx && k < nx ? sxy[i * nx + k] : 0.0;
-  }
-  for (int t = threadIdx.x; t < py * ly; t += kScThreads) {
-    const int i = t / ly, k = t % ly;
-    Sy[t] = i < ny && k < ny ? sxy[nx * nx + i * ny + k] : 0.0;
-  }
+  // Sx and Sy one after the other, here and in the table
+  for (int t = threadIdx.x; t < (px * lx + py * ly) / 2; t += kScThreads)
+    reinterpret_cast<double2*>(Sx)[t] = __ldg(reinterpret_cast<const double2*>(sxy) + t);
   __syncthreads();
   // PIC2D::Set2DRho (PIC2D.cpp): cloud-in-cell charge [C/m^3] of the slice's
   // particles, in 64-bit fixed point (order-independent)
@@ -451,45 +461,47 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const Bunch
     for (int j = 0; j < 4; ++j) add64_split(&lo[node[j]], &hi[node[j]], __double2ll_rn(w[j] * unit));
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < px * ly; t += kScThreads) {
-    const int i = t / ly, j = t % ly;
-    R[t] = i < nx && j < ny
-               ? sc_fix((unsigned long long)hi[i * ny + j] << 32 | lo[i * ny + j], e)
-               : 0.0;
-  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Pow2 back = pow2_split(-e);
+  for (int i = warp; i < px; i += kScThreads / 32)
+    for (int j = lane; j < ly; j += 32)
+      R[i * ly + j] = i < nx && j < ny
+                          ? pow2_scale((double)(long long)((unsigned long long)hi[i * ny + j] << 32 |
+                                                           lo[i * ny + j]), back)
+                          : 0.0;
   __syncthreads();
   const double hx = G[kGHx], hy = G[kGHy];
-  const double* __restrict__ eig = sxy + nx * nx + ny * ny;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tx = px / 8, ty = py / 8, tiles = tx * ty;
+  const double* __restrict__ eig = sxy + px * lx + py * ly;
+  const int tx = px / 8, ty = py / 8, half = (ty + 1) / 2;
+  const double sx2 = 2 / hx, sy2 = 2 / hy, norm = 1.0 / (4.0 * (nx + 1) * (ny + 1));
   for (int pass = 0; pass < 2; ++pass) {
-    for (int q = warp; q < tiles; q += kScThreads / 32) {  // T = Sx R (along x)
-      const int i = q / ty * 8, j = q % ty * 8;
-      double d[2];
-      sc_mma_tile(Sx + i * lx, lx, R + j, ly, px, d);
+    double d[2][2];
+    for (int q = warp; q < tx * half; q += kScThreads / 32) {  // T = Sx R (along x)
+      const int i = q / half * 8, j = q % half * 16;
+      const bool two = j + 8 < py;
+      sc_mma_tiles(Sx + i * lx, lx, R + j, ly, px, two, d);
       double* o = T + (i + (lane >> 2)) * ly + j + 2 * (lane & 3);
-      o[0] = d[0];
-      o[1] = d[1];
+      *reinterpret_cast<double2*>(o) = make_double2(d[0][0], d[0][1]);
+      if (two) *reinterpret_cast<double2*>(o + 8) = make_double2(d[1][0], d[1][1]);
     }
     __syncthreads();
-    for (int q = warp; q < tiles; q += kScThreads / 32) {  // R = T Sy^T (along y; Sy is symmetric)
-      const int i = q / ty * 8, j = q % ty * 8;
-      double d[2];
-      sc_mma_tile(T + i * ly, ly, Sy + j, ly, py, d);
+    for (int q = warp; q < tx * half; q += kScThreads / 32) {  // R = T Sy^T (along y; Sy is symmetric)
+      const int i = q / half * 8, j = q % half * 16;
+      const bool two = j + 8 < py;
+      sc_mma_tiles(T + i * ly, ly, Sy + j, ly, py, two, d);
       const int k = i + (lane >> 2);
+      // the Laplacian's eigenvalue (PIC2D.cpp Set2DPhi): out / K / Epsilon,
+      // with the sines of pi / 2 (k + 1) / (n + 1) from the table
+      const double ax = k < nx ? sx2 * eig[k] : 0.0;
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int m = j + 2 * (lane & 3) + u;
+      for (int u = 0; u < 4; ++u) {
+        if (u >= 2 && !two) break;
+        const int m = j + 8 * (u >> 1) + 2 * (lane & 3) + (u & 1);
         double v = 0.0;
         if (k < nx && m < ny) {
-          if (pass == 0) {
-            // the Laplacian's eigenvalue (PIC2D.cpp Set2DPhi): out / K / Epsilon,
-            // with the sines of pi / 2 (k + 1) / (n + 1) from the table
-            const double ax = 2 * eig[k] / hx, ay = 2 * eig[nx + m] / hy;
-            v = d[u] / (ax * ax + ay * ay) / kEpsilon0;
-          } else {
-            v = d[u] / (4.0 * (nx + 1) * (ny + 1));  // phi [V]
-          }
+          const double ay = pass == 0 ? sy2 * eig[nx + m] : 0.0;
+          v = d[u >> 1][u & 1] *
+              (pass == 0 ? recip_newton(fma(ax, ax, ay * ay)) * (1.0 / kEpsilon0) : norm);  // phi [V]
         }
         R[k * ly + m] = v;
       }
@@ -499,12 +511,12 @@ __global__ void __launch_bounds__(kScThreads) k_sc_solve(ScParams p, const Bunch
   // Set2DEField: central differences, zero potential beyond the mesh
   double* F = field + bs * 2 * N;
   const double fx = -0.5 / hx, fy = -0.5 / hy;
-  for (int t = threadIdx.x; t < N; t += kScThreads) {
-    const int i = t / ny, j = t % ny;
-    const double x1 = i == 0 ? 0 : R[(i - 1) * ly + j], x2 = i == nx - 1 ? 0 : R[(i + 1) * ly + j];
-    const double y1 = j == 0 ? 0 : R[i * ly + j - 1], y2 = j == ny - 1 ? 0 : R[i * ly + j + 1];
-    reinterpret_cast<double2*>(F)[t] = make_double2((x2 - x1) * fx, (y2 - y1) * fy);
-  }
+  for (int i = warp; i < nx; i += kScThreads / 32)
+    for (int j = lane; j < ny; j += 32) {
+      const double x1 = i == 0 ? 0 : R[(i - 1) * ly + j], x2 = i == nx - 1 ? 0 : R[(i + 1) * ly + j];
+      const double y1 = j == 0 ? 0 : R[i * ly + j - 1], y2 = j == ny - 1 ? 0 : R[i * ly + j + 1];
+      reinterpret_cast<double2*>(F)[i * ny + j] = make_double2((x2 - x1) * fx, (y2 - y1) * fy);
+    }
 }
 
 // A point beyond the series' range or a round slice, out of line.
@@ -529,14 +541,18 @@ __global__ void __launch_bounds__(kTile) k_sc_kick(double* __restrict__ c, int64
                                                    const double* __restrict__ field, double ds) {
   const int b = tile_bunch[blockIdx.x];
   const int64_t g = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  if (surv[g] == kPadding) return;
-  const double* G = geom + (size_t)b * kScGeom;
-  if (FLAG == 2 && G[kGIDv] == 0) return;
+  // every load that waits for no other first, but for the model that the FP64
+  // pipe bounds (padding slots hold numbers)
+  const uint8_t sv = surv[g];
+  if (FLAG == 1 && sv == kPadding) return;
   const double z = c[4 * npad + g], x = c[g], y = c[2 * npad + g];
   const double px0 = c[npad + g], py0 = c[3 * npad + g], dp = c[5 * npad + g];
+  const double* G = geom + (size_t)b * kScGeom;
+  if (sv == kPadding || (FLAG == 2 && G[kGIDv] == 0)) return;
   const int s = sc_slice(z, G, p.nz);
   const size_t bs = (size_t)b * p.nz + s;
-  if (cnt[bs] < 2) return;  // MPBunch.cpp:916
+  const int in_slice = cnt[bs];
+  if (FLAG == 1 && in_slice < 2) return;
   double ex = 0, ey = 0;
   if (FLAG == 2) {
     int ix, iy;
@@ -548,7 +564,9 @@ __global__ void __launch_bounds__(kTile) k_sc_kick(double* __restrict__ c, int64
       ex = (f0.x * w[0] + f1.x * w[1] + f2.x * w[2] + f3.x * w[3]) * G[kGIDv];
       ey = (f0.y * w[0] + f1.y * w[1] + f2.y * w[2] + f3.y * w[3]) * G[kGIDv];
     }
-  } else if (FLAG == 1) {
+  }
+  if (in_slice < 2) return;  // MPBunch.cpp:916 (the mesh's loads do not wait for it)
+  if (FLAG == 1) {
     const ScSlice& S = slices[bs];
     const KickConst& k = S.k;
     const bool sw = k.mode == 1;
@@ -571,7 +589,7 @@ __global__ void __launch_bounds__(kTile) k_sc_kick(double* __restrict__ c, int64
       ex = -0.5 * S.lambda * fx;
       ey = -0.5 * S.lambda * fy;
     }
-  } else {
+  } else if (FLAG == 3) {
     const ScSlice& S = slices[bs];
     const double q = S.lambda / (S.rx + S.ry);
     ex = q * ((x - S.cx) / S.rx);
@@ -604,7 +622,7 @@ cudaError_t prepare_sc(const ScParams& p) {
                               (int)sc_solve_smem(p));
 }
 
-cudaError_t launch_space_charge(Handle& h, int k) {
+cudaError_t launch_space_charge(Handle& h, int k, bool have_range) {
   const ScParams& p = h.sc;
   const DeviceBufs& d = h.d;
   const cudaStream_t st = h.stream;
@@ -614,12 +632,13 @@ cudaError_t launch_space_charge(Handle& h, int k) {
   if (h.n_chunks < 1) return cudaSuccess;
   ScSlice* sl = reinterpret_cast<ScSlice*>(d.sc_slices);
   double2* xy = reinterpret_cast<double2*>(d.sc_xy);
-  k_sc_clear<<<std::min(148, (slices + 255) / 256), 256, 0, st>>>(d.sc_range, d.sc_cnt, d.sc_acc, h.M,
-                                                                p.nz, pic ? 0 : 4);
-  (pic ? k_sc_range<false> : k_sc_range<true>)<<<h.n_chunks, kScThreads, 0, st>>>(
-      d.c, h.npad, d.surv, d.chunk_loc, d.sc_range);
-  k_sc_geom<<<(h.M + 31) / 32, 32, 0, st>>>(d.c, h.npad, d.bunch, d.mom, p, d.sc_range, d.sc_geom,
-                                            d.status, h.M);
+  const bool ranges = !(pic && have_range);
+  if (ranges)
+    (pic ? k_sc_range<false> : k_sc_range<true>)<<<h.n_chunks, kScThreads, 0, st>>>(
+        d.c, h.npad, d.surv, d.chunk_loc, d.sc_range);
+  k_sc_geom<<<(slices + 127) / 128, 128, 0, st>>>(d.c, h.npad, d.bunch, d.mom, p, d.sc_range, ranges,
+                                                  d.sc_geom, d.status, h.M, d.sc_cnt, d.sc_acc,
+                                                  pic ? 0 : 4);
   (pic ? k_sc_count<true> : k_sc_count<false>)<<<h.n_chunks, kScThreads, shared * (pic ? 1 : 9), st>>>(
       d.c, h.npad, d.surv, d.chunk_loc, p, d.sc_geom, d.sc_cnt, d.sc_acc);
   if (pic) {
