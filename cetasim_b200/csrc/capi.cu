@@ -836,20 +836,39 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
   std::vector<int4> cl;
   h.tile_off.assign(M + 1, 0);
   int tiles = 0, chunks = 0;
-  // Tiles per chunk, from the whole train (the same on every rank of a
-  // sharded run): long chunks spread the reduction at a chunk's end over more
-  // particles, but the 592 CTAs that run at once (four a SM) want some six
-  // chunks each to even out; and at most 256 chunks a bunch.
-  int64_t all_tiles = 0, big = 0;
+  // Tiles per chunk, from the whole train (the same on every rank of a sharded
+  // run), at most 256 chunks a bunch.  A pass without ions runs 740 CTAs at
+  // once (five per SM): it takes as long as its rounds times a chunk, and the
+  // start and the end of a chunk cost about as much as a tile, so the fewest
+  // rounds x (tiles + 1).  80 x 2e4 particles with space charge slices, 1 / 2 /
+  // 3 / 4 / 5 tiles: 2964 / 2576 / 2412 / 2467 / 2390 us a turn.  With ions
+  // other kernels take part of the SMs and the rounds blur: for each of the 592
+  // CTAs of the pass four chunks of up to three tiles (80 x 2e4, 1 to 5 tiles:
+  // 2706 / 2507 / 2448 / 2512 / 2610 us), six of more (1.74e7: 46.1 ms with 4
+  // tiles, 45.2 with 8; 4.4e6: 34.4 ms with 7, 33.5 with 5).
+  int64_t all_tiles = 0, big = 0, best = 0;
   for (int j = 0; j < M; ++j) {
     const int64_t nt = (n_macro[j] + kTile - 1) / kTile;
     all_tiles += nt;
     big = std::max(big, nt);
   }
-  const int64_t share = 592 * 6;
-  const int ct = (int)std::max<int64_t>(
-      (big + 255) / 256,
-      std::min<int64_t>(kMaxChunkTiles, std::max<int64_t>(1, (all_tiles + share / 2) / share)));
+  int ct = 0;
+  if (h.cfg.flag_beam_ion) {
+    auto share = [&](int64_t n) { return (all_tiles + n / 2) / n; };
+    const int64_t want = std::max(std::min<int64_t>(3, share(592 * 4)), share(592 * 6));
+    ct = (int)std::max<int64_t>((big + 255) / 256,
+                                std::min<int64_t>(kMaxChunkTiles, std::max<int64_t>(1, want)));
+  }
+  for (int c = 1; !h.cfg.flag_beam_ion && (c <= kMaxChunkTiles || ct == 0); ++c) {
+    if (c < (big + 255) / 256) continue;
+    int64_t n = 0;
+    for (int j = 0; j < M; ++j) n += ((n_macro[j] + kTile - 1) / kTile + c - 1) / c;
+    const int64_t cost = (n + 739) / 740 * (c + 1);
+    if (ct == 0 || cost < best) {
+      best = cost;
+      ct = c;
+    }
+  }
   h.max_chunks = (int)((big + ct - 1) / ct);
   // Walk segments: a segment's records, its pass and their launches cost some
   // 15 us beside the 25 us that the pass of 3000 tiles takes, so shorter
