@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kSurTrainThreads, 1)
   __shared__ SurSmall sm;
   __shared__ uint32_t s_tmem;
   __shared__ uint64_t s_bar;
-  __shared__ float s_x[kSurRows][3], s_dout[kSurRows][2], s_o[4][kSurRows][2];
+  __shared__ float s_x[kSurRows][3], s_dout[kSurRows][2];
   __shared__ float s_row[4][3];        // per warp of rows: e^2, dout
   __shared__ float s_col[8][4][kSurH];  // column sums over 16 rows each
   uint8_t* base = sur_base(dyn);
@@ -385,38 +385,41 @@ __global__ void __launch_bounds__(kSurTrainThreads, 1)
   sur_mma(base, kSmW3, tmem, bar);
   ok = sur_mma_wait(bar, phase) && ok;
   umma::tmem_ld16(dcol, d);
-  float o0 = 0.0f, o1 = 0.0f;
 #pragma unroll
-  for (int k = 0; k < kQ; ++k) {
-    silu_both(d[k] + sm.b3[c0 + k], &h[k], &ds3[k]);
-    o0 = fmaf(sm.w4[c0 + k], h[k], o0);
-    o1 = fmaf(sm.w4[kSurH + c0 + k], h[k], o1);
-  }
+  for (int k = 0; k < kQ; ++k) silu_both(d[k] + sm.b3[c0 + k], &h[k], &ds3[k]);
   put_quarter(H3, r, c0, h);
-  s_o[cq][r][0] = o0;
-  s_o[cq][r][1] = o1;
   __syncthreads();
-  o0 = sm.b4[0] + ((s_o[0][r][0] + s_o[1][r][0]) + (s_o[2][r][0] + s_o[3][r][0]));
-  o1 = sm.b4[1] + ((s_o[0][r][1] + s_o[1][r][1]) + (s_o[2][r][1] + s_o[3][r][1]));
-  const float e0 = sur_a(x) * o0 - t0, e1 = sur_b(x) * o1 - t1;
-  // dL/de = (e / B) ((1 - w) + 2 w e^2 / m)
-  float g0 = 1.0f, g1 = 1.0f;
-  if (l4w > 0.0f && e2_prev) {
-    const float m = *e2_prev * inv_batch * 0.5f;
-    if (m > 0.0f) {
-      g0 = fmaf(2.0f * l4w, e0 * e0 / m, 1.0f - l4w);
-      g1 = fmaf(2.0f * l4w, e1 * e1 / m, 1.0f - l4w);
-    }
-  }
-  // dL/d(layer-4 output): through the odd-output factors a, b
-  const float d0 = e0 * inv_batch * g0 * sur_a(x), d1 = e1 * inv_batch * g1 * sur_b(x);
   if (cq == 0) {
+    // layer 4 in sur_forward's order, so that the loss is that of its outputs
+    // bit for bit
+    float o0 = sm.b4[0], o1 = sm.b4[1];
+#pragma unroll
+    for (int k = 0; k < kSurH; k += 4) {
+      const float4 q = *reinterpret_cast<const float4*>(H3 + r * kHs + k);
+      const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        o0 = fmaf(sm.w4[k + u], v[u], o0);
+        o1 = fmaf(sm.w4[kSurH + k + u], v[u], o1);
+      }
+    }
+    const float e0 = sur_a(x) * o0 - t0, e1 = sur_b(x) * o1 - t1;
+    // dL/de = (e / B) ((1 - w) + 2 w e^2 / m)
+    float g0 = 1.0f, g1 = 1.0f;
+    if (l4w > 0.0f && e2_prev) {
+      const float m = *e2_prev * inv_batch * 0.5f;
+      if (m > 0.0f) {
+        g0 = fmaf(2.0f * l4w, e0 * e0 / m, 1.0f - l4w);
+        g1 = fmaf(2.0f * l4w, e1 * e1 / m, 1.0f - l4w);
+      }
+    }
+    // dL/d(layer-4 output): through the odd-output factors a, b
+    s_dout[r][0] = e0 * inv_batch * g0 * sur_a(x);
+    s_dout[r][1] = e1 * inv_batch * g1 * sur_b(x);
     s_x[r][0] = x[0];
     s_x[r][1] = x[1];
     s_x[r][2] = x[2];
-    s_dout[r][0] = d0;
-    s_dout[r][1] = d1;
-    float v[3] = {fmaf(e0, e0, e1 * e1), d0, d1};
+    float v[3] = {fmaf(e0, e0, e1 * e1), s_dout[r][0], s_dout[r][1]};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
 #pragma unroll
@@ -424,6 +427,8 @@ __global__ void __launch_bounds__(kSurTrainThreads, 1)
       if (lane == 0) s_row[warp][q] = v[q];
     }
   }
+  __syncthreads();
+  const float d0 = s_dout[r][0], d1 = s_dout[r][1];
   // dz3 = (W4^T dout) * silu'(z3)
 #pragma unroll
   for (int k = 0; k < kQ; ++k) h[k] = fmaf(sm.w4[c0 + k], d0, sm.w4[kSurH + c0 + k] * d1) * ds3[k];
@@ -457,8 +462,8 @@ __global__ void __launch_bounds__(kSurTrainThreads, 1)
       g[(grp == 0 ? kSurB3 : kSurW4 + (grp - 1) * kSurH) + col] = v;
     }
     if (threadIdx.x < 3) {
-      const float v = (s_row[0][threadIdx.x] + s_row[1][threadIdx.x]) +
-                      (s_row[2][threadIdx.x] + s_row[3][threadIdx.x]);
+      const float v = ((s_row[0][threadIdx.x] + s_row[1][threadIdx.x]) + s_row[2][threadIdx.x]) +
+                      s_row[3][threadIdx.x];
       g[threadIdx.x == 0 ? kSurParams : kSurB4 + threadIdx.x - 1] = v;
     }
     __syncthreads();
