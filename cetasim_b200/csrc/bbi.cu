@@ -29,16 +29,17 @@
 //               memory, then added to the bunch's.
 //  k_bbi_conv   one CTA per bunch: profiles, the Gaussian filter and its
 //               renormalisation, the potentials of the bins that hold
-//               particles, and each bin's kick; resets the accumulators.
+//               particles; resets the accumulators.
 //  k_bbi_kick   per tile: the kicks, plane by plane in the reference's order,
 //               and the turn's loss check if no stage comes between.
 //
 // Bound by: the passes by HBM (38 MB to count, 115 MB to kick 1.6e6 particles)
 // and its latency, the convolution by its chains of FMAs and barriers.  80
 // bunches of 20,000, five planes, us: range 25 -> in the longitudinal pass,
-// hist 53 -> 14 (global 64-bit atomics), conv 28 -> 15 (256 threads, a
+// hist 53 -> 14 (global 64-bit atomics before), conv 28 -> 15 (256 threads, a
 // filter with bounds checks per tap, one chain of 600 FMAs per bin and plane),
-// kick 40 and the loss check 16 -> 24 together (up to fourteen divisions a particle).
+// kick 40 and the loss check 16 -> 24 together (up to fourteen divisions a
+// particle).
 #include <algorithm>
 #include <climits>
 #include <cuda_runtime.h>
@@ -135,17 +136,11 @@ __global__ void __launch_bounds__(kBbiThreads) k_bbi_hist(const double* __restri
   }
 }
 
-// The kick of a bin: what its particles add, in the order of the reference's
-// operations up to the particle's own factor.
-struct alignas(16) BbiKick {
-  double z, dx, dy, qx, qy, pad;
-};
-
 // One CTA per bunch.  pot[(b * 6 + q) * wcap + t] for the bins a + t:
 // q = 0 the smoothed charge profile; q = 1..5 the potentials of the planes
 // Z, Dx, Dy, Qx, Qy at the bins that hold particles (frequency domain: the
 // wakePotenFromBBI arrays, MPBunch.cpp:2193-2341; time domain: temp[0..4],
-// MPBunch.cpp:2100-2111), 0 at the other bins; kick[b * wcap + t] the kicks.
+// MPBunch.cpp:2100-2111), 0 at the other bins.
 //
 // Three profiles side by side (the charge, the dipoles x and y; time domain:
 // the charge and the mean x and y, which are not smoothed), the tasks
@@ -159,7 +154,7 @@ struct alignas(16) BbiKick {
 __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
     const BunchDev* __restrict__ bunch, const __grid_constant__ BbiParams p,
     const double* __restrict__ w, BbiSpan* span, int* cnt,
-    unsigned long long* sxy, double* pot, BbiKick* kick, int2* win) {
+    unsigned long long* sxy, double* pot, int2* win) {
   extern __shared__ double sm[];
   __shared__ double red[kBbiConvThreads / 32][6];
   __shared__ double scale[3];
@@ -317,9 +312,6 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
       }
     }
     out[(size_t)(1 + q) * p.wcap + t] = v;
-    const double f = v / p.energy / p.beta2;
-    reinterpret_cast<double*>(kick + base + t)[q] =
-        q == 0 ? f : f / (q & 1 ? p.beta_x : p.beta_y);
   }
   if (threadIdx.x == 0) {
     win[b] = make_int2(a, n);
@@ -328,7 +320,11 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
 }
 
 // The kicks (frequency domain MPBunch.cpp:2201-2342, time domain
-// MPBunch.cpp:2113-2121), the planes in the reference's order.
+// MPBunch.cpp:2113-2121), the planes in the reference's order: a potential
+// over E beta^2 and, transversely, the beta function.
+struct BbiScale {
+  double z, x, y;
+};
 template <bool MARK>
 __global__ void __launch_bounds__(kTile) k_bbi_kick(double* __restrict__ c, int64_t npad,
                                                     uint8_t* __restrict__ surv,
@@ -336,7 +332,8 @@ __global__ void __launch_bounds__(kTile) k_bbi_kick(double* __restrict__ c, int6
                                                     const BunchDev* __restrict__ bunch,
                                                     const __grid_constant__ BbiParams p,
                                                     const int2* __restrict__ win,
-                                                    const BbiKick* __restrict__ kick,
+                                                    const double* __restrict__ pot,
+                                                    const __grid_constant__ BbiScale f,
                                                     const __grid_constant__ Aperture ap,
                                                     int* loss_count) {
   const int b = tile_bunch[blockIdx.x];
@@ -353,19 +350,19 @@ __global__ void __launch_bounds__(kTile) k_bbi_kick(double* __restrict__ c, int6
   const int idx = valid && Bd.q_macro != 0 && wn.y != 0 ? bbi_bin(p, z) : -1;
   if (idx >= 0) {
     double px = c[npad + g], py = c[3 * npad + g], dp = c[5 * npad + g];
-    const double2* K = reinterpret_cast<const double2*>(kick + (size_t)b * p.wcap + (idx - wn.x));
-    const double2 k0 = K[0], k1 = K[1];
-    const double qy = K[2].x;
-    if (p.sim[0]) dp += k0.x;
+    const double* v = pot + (size_t)b * 6 * p.wcap + (idx - wn.x);
+    const double z0 = f.z * v[p.wcap], dx = f.x * v[2 * p.wcap], dy = f.y * v[3 * p.wcap];
+    const double qx = f.x * v[4 * p.wcap], qy = f.y * v[5 * p.wcap];
+    if (p.sim[0]) dp += z0;
     if (!p.td) {
-      if (p.sim[3]) px = fma(k1.y, x, px);
+      if (p.sim[3]) px = fma(qx, x, px);
       if (p.sim[4]) py = fma(qy, y, py);
-      if (p.sim[1]) px += k0.y;
-      if (p.sim[2]) py += k1.x;
+      if (p.sim[1]) px += dx;
+      if (p.sim[2]) py += dy;
     } else {
-      if (p.sim[1]) px += k0.y;
-      if (p.sim[2]) py += k1.x;
-      if (p.sim[3]) px = fma(k1.y, x, px);
+      if (p.sim[1]) px += dx;
+      if (p.sim[2]) py += dy;
+      if (p.sim[3]) px = fma(qx, x, px);
       if (p.sim[4]) py = fma(qy, y, py);
     }
     c[npad + g] = px;
@@ -380,7 +377,8 @@ size_t bbi_span_bytes() { return sizeof(BbiSpan); }
 cudaError_t launch_bbi(Handle& h, bool have_range, bool mark) {
   const BbiParams& p = h.bbi;
   BbiSpan* span = reinterpret_cast<BbiSpan*>(h.d.bbi_span);
-  BbiKick* kick = reinterpret_cast<BbiKick*>(h.d.bbi_kick);
+  const double fz = 1.0 / p.energy / p.beta2;
+  const BbiScale f = {fz, fz / p.beta_x, fz / p.beta_y};
   if (!have_range)
     k_bbi_range<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch,
                                                    h.d.bunch, p, span, h.d.status);
@@ -393,14 +391,12 @@ cudaError_t launch_bbi(Handle& h, bool have_range, bool mark) {
                5 * sizeof(unsigned) * std::min(p.wcap, kBbiSharedBins), h.stream>>>(
       h.d.c, h.npad, h.d.surv, h.d.bunch, tiles, p, span, h.d.status, h.d.bbi_cnt, h.d.bbi_sxy);
   k_bbi_conv<<<h.M, kBbiConvThreads, bbi_conv_smem(p), h.stream>>>(
-      h.d.bunch, p, h.d.bbi_w, span, h.d.bbi_cnt, h.d.bbi_sxy, h.d.bbi_pot, kick, h.d.bbi_win);
+      h.d.bunch, p, h.d.bbi_w, span, h.d.bbi_cnt, h.d.bbi_sxy, h.d.bbi_pot, h.d.bbi_win);
   (mark ? k_bbi_kick<true> : k_bbi_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(
-      h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, p, h.d.bbi_win, kick, aperture(h),
+      h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, p, h.d.bbi_win, h.d.bbi_pot, f, aperture(h),
       h.d.loss_count);
   return cudaGetLastError();
 }
-
-size_t bbi_kick_bytes() { return sizeof(BbiKick); }
 
 size_t bbi_conv_smem(const BbiParams& p) {
   return (size_t)(6 * p.wcap + 6 * kBbiHalf) * sizeof(double);

@@ -140,7 +140,7 @@ void free_beam(Handle& h) {
   dfree(d.c); dfree(d.surv); dfree(d.tile_bunch); dfree(d.chunk_loc);
   dfree(d.bunch);
   dfree(d.wpartials);
-  dfree(d.counters); dfree(d.mom); dfree(d.loss_count); dfree(d.scratch);
+  dfree(d.mom); dfree(d.loss_count); dfree(d.scratch);
   dfree(d.rec); dfree(d.rec_prep); dfree(d.lr_hist); dfree(d.lr_force); dfree(d.fir_hist); dfree(d.fir_kick);
   dfree(d.sr_span); d.sr_span = nullptr;
   dfree(d.sr_geom); dfree(d.sr_counts); dfree(d.sr_sumx); dfree(d.sr_sumy); dfree(d.sr_lag);
@@ -155,10 +155,9 @@ void free_beam(Handle& h) {
   d.res_state = nullptr; d.rf_zr = nullptr; d.rf_counts = nullptr; d.rf_kick = nullptr;
   d.rf_fbk = nullptr; d.rf_info = nullptr; d.rf_work = nullptr;
   dfree(d.bbi_span); dfree(d.bbi_cnt); dfree(d.bbi_sxy);
-  dfree(d.bbi_pot); dfree(d.bbi_kick); dfree(d.bbi_win);
+  dfree(d.bbi_pot); dfree(d.bbi_win);
   d.bbi_span = nullptr; d.bbi_cnt = nullptr;
-  d.bbi_sxy = nullptr; d.bbi_pot = nullptr; d.bbi_kick = nullptr;
-  d.bbi_win = nullptr;
+  d.bbi_sxy = nullptr; d.bbi_pot = nullptr; d.bbi_win = nullptr;
   for (double* b : h.phase_bufs) dfree(b);
   h.phase_bufs.clear();
   h.phase_bunches.clear();
@@ -177,7 +176,7 @@ void free_beam(Handle& h) {
   d.c = nullptr; d.surv = nullptr; d.tile_bunch = nullptr;
   d.chunk_loc = nullptr;
   d.bunch = nullptr; d.wpartials = nullptr;
-  d.counters = nullptr; d.mom = nullptr; d.loss_count = nullptr; d.scratch = nullptr;
+  d.mom = nullptr; d.loss_count = nullptr; d.scratch = nullptr;
   d.rec = nullptr; d.rec_prep = nullptr; d.lr_hist = nullptr; d.lr_force = nullptr; d.fir_hist = nullptr;
   d.fir_kick = nullptr; d.sr_geom = nullptr; d.sr_counts = nullptr; d.sr_sumx = nullptr;
   d.sr_sumy = nullptr; d.sr_lag = nullptr; d.sr_pot = nullptr;
@@ -914,7 +913,7 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
       dalloc(&d.tile_bunch, tiles) ||
       dalloc(&d.chunk_loc, chunks) || dalloc(&d.bunch, M) ||
       dalloc(&d.wpartials, (size_t)kMomWarps * chunks) ||
-      dalloc(&d.counters, M + 1) || dalloc(&d.mom, M) || dalloc(&d.loss_count, M + 1)) {
+      dalloc(&d.mom, M) || dalloc(&d.loss_count, M + 1)) {
     free_beam(h);
     return fail(&h, CG_ERR_OOM, "beam allocation failed");
   }
@@ -939,7 +938,6 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
     cudaMemset(d.mom_send, 0, sizeof(BunchMomDev) * ml);
   }
   cudaMemcpy(d.bunch, bd.data(), sizeof(BunchDev) * M, cudaMemcpyHostToDevice);
-  cudaMemset(d.counters, 0, sizeof(unsigned) * (M + 1));
   cudaMemset(d.loss_count, 0, sizeof(int) * (M + 1));
   std::vector<BunchMomDev> m0(M);
   std::memset(m0.data(), 0, sizeof(BunchMomDev) * M);
@@ -1059,8 +1057,7 @@ int cg_set_beam(cg_handle* H, int M, const int* n_macro, const int* harm, const 
     if (dalloc(reinterpret_cast<char**>(&d.bbi_span), bbi_span_bytes() * M) ||
         dalloc(&d.bbi_cnt, (size_t)M * wc) ||
         dalloc(&d.bbi_sxy, 2 * (size_t)M * wc) || dalloc(&d.bbi_pot, 6 * (size_t)M * wc) ||
-        dalloc(&d.bbi_win, (size_t)M) ||
-        dalloc(reinterpret_cast<char**>(&d.bbi_kick), bbi_kick_bytes() * M * wc)) {
+        dalloc(&d.bbi_win, (size_t)M)) {
       free_beam(h);
       return fail(&h, CG_ERR_OOM, "broadband-impedance buffers");
     }

@@ -110,7 +110,6 @@ struct DeviceBufs {
   int4* chunk_loc = nullptr;    // n_chunks: (bunch, first tile, tiles, -)
   BunchDev* bunch = nullptr;    // M
   MomPartial* wpartials = nullptr; // n_chunks x kMomWarps: moment partials
-  unsigned* counters = nullptr;    // M (+ spare)
   BunchMomDev* mom = nullptr;      // M
   int* loss_count = nullptr;       // M
   int* status = nullptr;           // device status word(s)
@@ -167,7 +166,6 @@ struct DeviceBufs {
   int* bbi_cnt = nullptr;          // M x wcap per-bin counts (zero between calls)
   unsigned long long* bbi_sxy = nullptr;  // M x 2 x wcap fixed-point sums of x, y
   double* bbi_pot = nullptr;       // M x 6 x wcap: profile and potentials of the last kick
-  void* bbi_kick = nullptr;        // M x wcap: the bins' kicks
   int2* bbi_win = nullptr;         // M: first bin and bin count of bbi_pot
   // space charge
   double* sc_geom = nullptr;       // M x kScGeom: slices, mesh, fixed-point scales
@@ -238,7 +236,7 @@ struct Handle {
   // turn trace (cg_trace_turn): marks and their timing events
   std::vector<TraceMark>* trace = nullptr;
   std::vector<cudaEvent_t> trace_ev;
-  cudaStream_t side = nullptr;   // records and kicks of the segments
+  cudaStream_t side = nullptr;   // passes of the segments, or their records and kicks
   cudaStream_t side2 = nullptr;  // the segments' records, or (kick and map apart) their maps
   cudaStream_t side3 = nullptr;  // every other segment's pass
   cudaEvent_t side3_ev = nullptr;    // its join

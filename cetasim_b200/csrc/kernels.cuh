@@ -33,7 +33,6 @@ cudaError_t prepare_sc(const ScParams& p);
 // the bunches' ranges already collected by the longitudinal pass; the loss
 // check with the kick
 cudaError_t launch_bbi(Handle& h, bool have_range, bool mark);
-size_t bbi_kick_bytes();  // of one bin's kicks
 size_t bbi_span_bytes();  // of one bunch's span
 size_t bbi_conv_smem(const BbiParams& p);
 cudaError_t prepare_bbi(const BbiParams& p);

@@ -25,8 +25,9 @@
 //
 // Bound by latency for a single bunch (five dependent launches of a few
 // thousand cycles), by HBM for a train.  One bunch of 1e5 particles, 100 bins,
-// us: range 44 (one thread over the tiles) -> in the longitudinal pass, histogram and lags 8 + 5 -> 6.4 together, potentials 7 -> 4.1 (a
-// thread per bin), kick and loss check 5 + 7 -> 5.0 together.
+// us: range 44 (one thread over the tiles) -> in the longitudinal pass,
+// histogram and lags 8 + 5 -> 6.4 together, potentials 7 -> 4.1 (a thread per
+// bin before), kick and loss check 5 + 7 -> 5.0 together.
 #include <cuda_runtime.h>
 #include "turn_tail.cuh"
 

@@ -61,8 +61,9 @@ __device__ __forceinline__ void sincos_rf(double th, double* sn, double* cs) {
 // increments of its bin from the recurrence's table (kick[((b M + j) nb +
 // bin) 2 ..]); then the direct-feedback kicks of the bunch, to every
 // particle.
-__device__ __forceinline__ double rf_kick_dp_loading(const RingDev& r, double z, double dp, bool alive, int j, int M,
-                                const double* zr, const double* kick, const double* fbk) {
+__device__ __forceinline__ double rf_kick_dp_loading(const RingDev& r, double z, double dp,
+                                                     bool alive, int j, int M, const double* zr,
+                                                     const double* kick, const double* fbk) {
   int bin = -1;
   if (alive) {
     const double zmin = zr[2 * j], zmax = zr[2 * j + 1];
