@@ -196,10 +196,11 @@ __global__ void k_sc_geom(const double* __restrict__ c, int64_t npad,
   }
 }
 
-// slice of a particle (MPBunch.cpp:679-681)
+// slice of a particle (MPBunch.cpp:679-681); the first for a z that is no
+// number (converted, it would index far outside the slices)
 __device__ __forceinline__ int sc_slice(double z, const double* G, int nz) {
   const double t = floor((z - G[kGZmin]) * G[kGIDz]);
-  return t < 0 ? 0 : (t > nz - 1 ? nz - 1 : (int)t);
+  return !(t > 0) ? 0 : (t > nz - 1 ? nz - 1 : (int)t);
 }
 
 // mesh cell and cloud-in-cell distances (PIC2D::Set2DRho, PIC2D.cpp: the
