@@ -1511,7 +1511,9 @@ static cudaError_t enqueue_turn(Handle& h) {
         if ((e = cudaEventRecord(h.kick_ev[g], h.side))) return e;
         if ((e = cudaStreamWaitEvent(h.side2, h.kick_ev[g], 0))) return e;
         if (k == h.K - 1 && (e = launch_phase_adv(h, ja, jb, h.side2))) return e;
-        if ((e = launch_map_pass(h, k, mom, false, zr, ca, cb, h.side2))) return e;
+        e = mom < 0 ? launch_map(h, k, ta, tb, h.side2)
+                    : launch_map_pass(h, k, mom, false, zr, ca, cb, h.side2);
+        if (e) return e;
         TRACE(h.side2, CG_TRACE_MAP_PASS, k, g);
       }
       const cudaStream_t cs = fused ? h.side2 : h.side;
@@ -1538,7 +1540,10 @@ static cudaError_t enqueue_turn(Handle& h) {
       if (c.flag_sc && (e = launch_space_charge(h, k, true))) return e;
       if (k == h.K - 1 && (e = launch_phase_adv(h, 0, h.M))) return e;
       long_map = k == h.K - 1 && mom < 0 && !fused && !h.ring.bl_any;
-      if (!long_map && (e = launch_map_pass(h, k, mom, fused, zr))) return e;
+      if (!long_map) {
+        e = mom < 0 && !fused ? launch_map(h, k) : launch_map_pass(h, k, mom, fused, zr);
+        if (e) return e;
+      }
       if (fused) TRACE(h.stream, CG_TRACE_ION_KICK, k, -1);
       TRACE(h.stream, CG_TRACE_MAP_PASS, k, -1);
     }

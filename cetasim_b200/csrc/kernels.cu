@@ -394,25 +394,32 @@ cudaError_t launch_moments(Handle& h, int k) {
 }
 
 // ---------------------------------------------------------------------------
-// Section map (Bunch::BunchTransferDueToLatticeTSymplectic).
+// Section map (Bunch::BunchTransferDueToLatticeTSymplectic) of the tiles from
+// tile_base on, a thread per particle: the pass of a section whose moments
+// nothing reads and where no ions kick.  Bound by HBM: every load of a particle
+// at once (the padding slots hold the survival mark kPadding) and as many warps
+// as the registers allow.  8.7e6 particles through a turn of 20 sections: 3.82 ms
+// (5.00 as the moments' pass without the moments, 3.98 with four particles a
+// thread in flight).
 
 __global__ void __launch_bounds__(kTile) k_map(double* __restrict__ c, int64_t npad,
                                                const uint8_t* __restrict__ surv,
-                                               const int* __restrict__ tile_bunch,
-                                               const BunchDev* __restrict__ bunch,
                                                const __grid_constant__ SectionDev sec,
-                                               const __grid_constant__ RingDev r) {
-  TileIdx t = tile_index(tile_bunch, bunch);
-  if (!t.valid || surv[t.g] != kAlive) return;
+                                               const __grid_constant__ RingDev r, int tile_base) {
+  const int64_t g = (int64_t)(tile_base + (int)blockIdx.x) * kTile + threadIdx.x;
+  const uint8_t alive = surv[g];
   double v[6];
-  load6(c, npad, t.g, v);
+  load6(c, npad, g, v);
+  if (alive != kAlive) return;
   section_map_particle(sec, r, v);
-  store6(c, npad, t.g, v);
+  store6(c, npad, g, v);
 }
 
-cudaError_t launch_map(Handle& h, int k) {
-  k_map<<<h.n_tiles, kTile, 0, h.stream>>>(h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch,
-                                           h.sec_dev_host[k], h.ring);
+cudaError_t launch_map(Handle& h, int k, int tile_a, int tile_b, cudaStream_t s) {
+  if (tile_b < 0) tile_b = h.n_tiles;
+  if (tile_b <= tile_a) return cudaSuccess;
+  k_map<<<tile_b - tile_a, kTile, 0, s ? s : h.stream>>>(h.d.c, h.npad, h.d.surv, h.sec_dev_host[k],
+                                                         h.ring, tile_a);
   return cudaGetLastError();
 }
 
@@ -565,9 +572,10 @@ cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick, bool z
   if (all) chunk_b = h.n_chunks;
   if (!s) s = h.stream;
   if (chunk_b > chunk_a) {
+    if (!m && !kick) return cudaErrorInvalidValue;
     auto kern = m == 2   ? (kick ? k_map_pass<2, true> : k_map_pass<2, false>)
                 : m == 1 ? (kick ? k_map_pass<1, true> : k_map_pass<1, false>)
-                         : (kick ? k_map_pass<0, true> : k_map_pass<0, false>);
+                         : k_map_pass<0, true>;
     kern<<<chunk_b - chunk_a, kPassThreads, 0, s>>>(h.d.c, h.npad, h.d.surv, h.d.chunk_loc,
                                                     h.sec_dev_host[k], h.ring, h.d.wpartials, rec,
                                                     rp, h.P, chunk_a);

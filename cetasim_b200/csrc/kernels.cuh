@@ -40,7 +40,9 @@ cudaError_t prepare_bbi(const BbiParams& p);
 cudaError_t bbi_wake_fd(const double2* d_X, int n, double* d_w, cudaStream_t st);
 
 cudaError_t launch_moments(Handle& h, int k);
-cudaError_t launch_map(Handle& h, int k);
+// map of section k over the tiles [tile_a, tile_b) (tile_b < 0: all) on stream s
+// (null: h.stream)
+cudaError_t launch_map(Handle& h, int k, int tile_a = 0, int tile_b = -1, cudaStream_t s = nullptr);
 cudaError_t launch_ion_chain(Handle& h, int k);
 // the chain in pieces (the pipelined turn): prep, walk / records of the bunch
 // steps [ja, jb), compaction
@@ -59,7 +61,8 @@ cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a = 0, int
 int kick_variants();
 void kick_variant_shape(int v, int* threads, int* min_ctas);
 // (ion kick of IP k if `kick`) + map of section k + moments at section
-// `mom_section` (if >= 0; their z range if `z_range`), over the chunks
+// `mom_section` (if >= 0; their z range if `z_range`; with neither kick nor
+// moments the pass is launch_map's), over the chunks
 // [chunk_a, chunk_b) (chunk_b < 0: all, and the moments merged; over parts the
 // caller merges them) on stream s (null: h.stream)
 cudaError_t launch_map_pass(Handle& h, int k, int mom_section, bool kick = false,
