@@ -77,12 +77,9 @@ __device__ __forceinline__ SrGeom sr_geometry(const SrSpan& s, double z0, double
   return {lo, (hi - lo) / B};
 }
 
-// truncation toward zero, as int() in the reference; the product with 1 / dz
-// decides unless a whole number lies within 2^-50 of it (bbi_bin)
+// truncation toward zero, as int() in the reference; inv = 1 / dz
 __device__ __forceinline__ int sr_bin(double z, double lo, double dz, double inv, int B) {
-  double t = (z - lo) * inv;
-  const double whole = (t + 0x1.8p52) - 0x1.8p52;
-  if (!(fabs(t - whole) > 0x1p-50 * fabs(t))) t = (z - lo) / dz;
+  const double t = bin_quotient(z - lo, dz, inv);
   return (t > -1.0 && t < (double)B) ? (int)t : -1;
 }
 

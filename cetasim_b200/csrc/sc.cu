@@ -199,16 +199,17 @@ __global__ void k_sc_geom(const double* __restrict__ c, int64_t npad,
 // slice of a particle (MPBunch.cpp:679-681); the first for a z that is no
 // number (converted, it would index far outside the slices)
 __device__ __forceinline__ int sc_slice(double z, const double* G, int nz) {
-  const double t = floor((z - G[kGZmin]) * G[kGIDz]);
-  return !(t > 0) ? 0 : (t > nz - 1 ? nz - 1 : (int)t);
+  const double s = z - G[kGZmin];
+  const double t = bin_quotient(s, G[kGDz], G[kGIDz]);
+  return !(s > 0) ? 0 : (t < nz - 1 ? (int)t : nz - 1);
 }
 
 // mesh cell and cloud-in-cell distances (PIC2D::Set2DRho, PIC2D.cpp: the
 // weights times the cell's area); false when the particle is outside the mesh
 __device__ __forceinline__ bool sc_cell(double x, double y, const double* G, const ScParams& p,
                                         int* ix, int* iy, double w[4]) {
-  const double tx = floor((x - G[kGMx0]) * G[kGIHx]);
-  const double ty = floor((y - G[kGMy0]) * G[kGIHy]);
+  const double tx = floor(bin_quotient(x - G[kGMx0], G[kGHx], G[kGIHx]));
+  const double ty = floor(bin_quotient(y - G[kGMy0], G[kGHy], G[kGIHy]));
   if (!(tx >= 0 && tx < p.nx - 1 && ty >= 0 && ty < p.ny - 1)) return false;
   *ix = (int)tx;
   *iy = (int)ty;
