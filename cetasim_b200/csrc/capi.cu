@@ -1590,6 +1590,15 @@ static cudaError_t enqueue_turn(Handle& h) {
 }
 #undef TRACE
 
+static int capture_turn(Handle& h, cudaGraph_t* g) {
+  CG_CUDA(&h, cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
+  cudaError_t e = enqueue_turn(h);
+  cudaError_t e2 = cudaStreamEndCapture(h.stream, g);
+  if (e == cudaSuccess) return e2 == cudaSuccess ? CG_OK : cuda_fail(&h, e2, "end capture");
+  if (e2 == cudaSuccess) cudaGraphDestroy(*g);
+  return cuda_fail(&h, e, "turn capture");
+}
+
 int cg_run_turns(cg_handle* H, int turn0, int n_turns) {
   STAGE_PROLOGUE
   if (n_turns < 0) return fail(&h, CG_ERR_INVALID, "n_turns < 0");
@@ -1597,12 +1606,8 @@ int cg_run_turns(cg_handle* H, int turn0, int n_turns) {
   if (st) return st;
   if (!h.turn_graph) {
     cudaGraph_t g;
-    CG_CUDA(&h, cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = enqueue_turn(h);
-    cudaError_t e2 = cudaStreamEndCapture(h.stream, &g);
-    if (e != cudaSuccess) return cuda_fail(&h, e, "turn capture");
-    if (e2 != cudaSuccess) return cuda_fail(&h, e2, "end capture");
-    e = cudaGraphInstantiate(&h.turn_graph, g, 0);
+    if ((st = capture_turn(h, &g))) return st;
+    cudaError_t e = cudaGraphInstantiate(&h.turn_graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(&h, e, "graph instantiate");
   }
@@ -1797,34 +1802,38 @@ void cg_host_free(void* p) {
 
 void* cg_stream(cg_handle* H) { return H ? (void*)H->h.stream : nullptr; }
 
-static int count_turn_launches(Handle& h) {
-  const cg_config& c = h.cfg;
-  int n = h.K;                                   // map + moments passes
-  const int G = std::max(1, std::min(h.pipe_groups, h.M));
-  if (c.flag_beam_ion) {                         // moments at IP 0, then per IP:
-    if (G > 1) n += 1 + h.K * (2 + 3 * G + (G - 1));  // prep, compact, G x (walk, records,
-                                                       // kick), G - 1 more map passes
-    else n += 1 + 5 * h.K;                       // prep, walk, records, compact, kick
-    if (h.fuse_kick && !h.d.sur_w) n -= h.K * G;  // kicks inside the map passes
-  }
-  if (c.flag_lr_wake) n += 2;                    // push + forces
-  n += 1;                                        // longitudinal tail
-  if (c.flag_sr_wake) n += 5;
-  if (c.flag_fir) n += 2;
-  n += 2;                                        // mark lost + turn counter
-  if (h.nccl_comm) {                             // moments scatter after each exchange
-    int ex = 0;
-    for (int k = 0; k < h.K; ++k)
-      if (k + 1 < h.K ? c.flag_beam_ion : (c.flag_lr_wake || c.flag_sr_wake)) ++ex;
-    ex += (c.flag_beam_ion ? 1 : 0) + (c.flag_fir ? 1 : 0);
-    n += ex;
-  }
-  return n;
-}
-
+// The kernel nodes of a captured turn.  A sharded train's moment exchanges are
+// left out of the capture (a collective that the other ranks do not enter must
+// not be enqueued) and their scatter kernels added.
 int cg_turn_launches(cg_handle* H, int* launches) {
   if (!H || !launches) return CG_ERR_INVALID;
-  *launches = count_turn_launches(H->h);
+  Handle& h = H->h;
+  *launches = 0;
+  if (!h.beam_set) return CG_OK;  // no turn yet
+  cudaSetDevice(h.device);
+  void* comm = h.nccl_comm;
+  h.nccl_comm = nullptr;
+  cudaGraph_t g;
+  int st = capture_turn(h, &g);
+  h.nccl_comm = comm;
+  if (st) return st;
+  size_t n = 0;
+  cudaError_t e = cudaGraphGetNodes(g, nullptr, &n);
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (e == cudaSuccess && n) e = cudaGraphGetNodes(g, nodes.data(), &n);
+  int kernels = 0;
+  for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+    cudaGraphNodeType t;
+    e = cudaGraphNodeGetType(nodes[i], &t);
+    kernels += e == cudaSuccess && t == cudaGraphNodeTypeKernel;
+  }
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return cuda_fail(&h, e, "turn graph's nodes");
+  if (comm) {
+    const cg_config& c = h.cfg;
+    kernels += (c.flag_beam_ion ? h.K : 0) + (c.flag_lr_wake || c.flag_sr_wake) + (c.flag_fir != 0);
+  }
+  *launches = kernels;
   return CG_OK;
 }
 
