@@ -68,7 +68,7 @@ DESC = {
 }
 
 
-# the kick kernel's shapes in the order of cg_autotune's timings
+# the kick kernel's shapes in the order of cg_autotune's timings (three kernels)
 KICK_SHAPES = ["256 thr x3/SM", "256 thr x3/SM", "128 thr x4/SM", "128 thr x6/SM",
                "256 thr x3/SM", "128 thr x6/SM", "128 thr x6/SM", "256 thr x3/SM"]
 
@@ -320,10 +320,10 @@ def main():
     ap.add_argument("--no-surrogate", action="store_true",
                     help="skip the surrogate measurement (training + surrogate turns)")
     ap.add_argument("--kick-variant", type=int, default=None, metavar="V",
-                    help="kick shape V (0-3; 4-7: the same inside the map pass) instead of "
+                    help="kick shape V (0-7; 8-15: the kick inside the map pass) instead of "
                          "the kick autotuner")
     ap.add_argument("--map-async", type=int, default=0, choices=[0, 1],
-                    help="with --kick-variant: the map-pass form (1 = next chunk in flight)")
+                    help="accepted without effect (there is one form of the map pass)")
     ap.add_argument("--pipeline", default=None, metavar="G:IONS:RAMP",
                     help="pipeline shape (walk segments, ions per walk CTA, ramp 0/1) instead "
                          "of the whole-turn pipeline autotuner")
@@ -377,7 +377,6 @@ def main():
     ions = bool(wl.cfg.flag_beam_ion)
     if args.kick_variant is not None:
         beam.set_kick_variant(args.kick_variant)
-        beam.set_map_async(args.map_async)
         tune = (args.kick_variant, None)
     elif ions:
         tune = beam.autotune(0, reps=10)
@@ -575,18 +574,12 @@ def main():
             "roofline": top,
             "cpu_baseline": cpu,
             "autotune": {"kick_shapes_ms": None if tune[1] is None else
-                         [round(float(x), 5) for x in tune[1][:-4]],
+                         {k: round(float(x), 5) for k, x in zip(KICK_SHAPES, tune[1][:-4])},
                          "map_pass_ms": None if tune[1] is None else round(float(tune[1][-4]), 5),
                          "map_pass_with_kick_ms": None if tune[1] is None else
                          round(float(tune[1][-3]), 5),
-                         "map_pass_async_ms": None if tune[1] is None else
-                         round(float(tune[1][-2]), 5),
-                         "map_pass_async_with_kick_ms": None if tune[1] is None else
-                         round(float(tune[1][-1]), 5),
-                         "map_async": beam.map_async(),
-                         "chosen_shape": int(tune[0]) % len(KICK_SHAPES),
+                         "chosen_shape": KICK_SHAPES[int(tune[0]) % len(KICK_SHAPES)],
                          "kick_in_map_pass": bool(tune[0] >= len(KICK_SHAPES)),
-                         "shapes": KICK_SHAPES,
                          "pipeline": None if pipe is None else {
                              "segments": pipe[0][0], "walk_ions": pipe[0][1],
                              "ramp": bool(pipe[0][2]),

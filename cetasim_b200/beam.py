@@ -168,9 +168,9 @@ class MPBeam:
 
     # -- autotuning ---------------------------------------------------------------
     def autotune(self, k: int = 0, reps: int = 10):
-        """Times the kick shapes and the map-pass forms on this beam at IP k;
-        returns (choice, ms) as cg_autotune fills them (n kick shapes, then
-        the map pass, with the kick, and both with the next chunk in flight)."""
+        """Times the kick shapes and the map pass without and with the kick on
+        this beam at IP k; returns (choice, ms) as cg_autotune fills them (n
+        kick shapes, the map pass, with the kick, and these two again)."""
         n = C.c_int()
         self._check(self.lib.cg_kick_variants(C.byref(n)))
         ms = np.zeros(n.value + 4)

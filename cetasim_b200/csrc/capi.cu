@@ -1853,12 +1853,8 @@ int cg_time_stage(cg_handle* H, int stage, int k, int reps, double* ms) {
       case 1: e = launch_ion_kick(h, k); break;
       case 2: e = launch_ion_chain(h, k); break;
       case 3: e = launch_moments(h, k); break;
-      case 5: e = launch_map_pass(h, k, k); break;
-      case 7:
-        e = h.cfg.flag_beam_ion ? launch_map_pass(h, k, k, true) : cudaErrorInvalidValue;
-        break;
-      case 8: e = launch_map_pass(h, k, k); break;
-      case 9:
+      case 5: case 8: e = launch_map_pass(h, k, k); break;
+      case 7: case 9:
         e = h.cfg.flag_beam_ion ? launch_map_pass(h, k, k, true) : cudaErrorInvalidValue;
         break;
       case 6:
@@ -2245,30 +2241,23 @@ int cg_autotune(cg_handle* H, int k, int reps, int* choice, double* ms) {
     return r;
   };
   int best = 0;
-  double best_ms = 0;
   const int nv = kick_variants();
+  std::vector<double> per(nv, 0.0);
   for (int v = 0; v < nv && e == cudaSuccess; ++v) {
-    double per = 0;
-    e = time_it([&]() { return launch_ion_kick_variant(h, k, v); }, &per);
-    if (ms) ms[v] = per;
-    if (v == 0 || per < best_ms) {
-      best = v;
-      best_ms = per;
-    }
+    const int same = kick_variant_first(v);  // each kernel once
+    if (same < v) per[v] = per[same];
+    else e = time_it([&]() { return launch_ion_kick_variant(h, k, v); }, &per[v]);
+    if (per[v] < per[best]) best = v;
   }
-  // the separate kick + map pass against the kick inside the map pass, each
-  // pass in its register form and with the next chunk in flight
+  // the separate kick + map pass against the kick inside the map pass
   const int mom = k + 1 < h.K ? k + 1 : k;
-  double map_ms = 0, fused_ms = 0, amap_ms = 0, afused_ms = 0;
+  double map_ms = 0, fused_ms = 0;
   if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, false); }, &map_ms);
   if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, true); }, &fused_ms);
-  if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, false); }, &amap_ms);
-  if (e == cudaSuccess) e = time_it([&]() { return launch_map_pass(h, k, mom, true); }, &afused_ms);
   if (ms) {
-    ms[nv] = map_ms;
-    ms[nv + 1] = fused_ms;
-    ms[nv + 2] = amap_ms;
-    ms[nv + 3] = afused_ms;
+    std::copy(per.begin(), per.end(), ms);
+    ms[nv] = ms[nv + 2] = map_ms;
+    ms[nv + 1] = ms[nv + 3] = fused_ms;
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h.stream);
   cudaEventDestroy(e0);
@@ -2276,18 +2265,9 @@ int cg_autotune(cg_handle* H, int k, int reps, int* choice, double* ms) {
   dfree(keep);
   dfree(keep_mom);
   if (e != cudaSuccess) return cuda_fail(&h, e, "autotune");
-  const double sep = best_ms + std::min(map_ms, amap_ms), fus = std::min(fused_ms, afused_ms);
-  const bool fuse = fus < sep;
-  const bool async = fuse ? afused_ms < fused_ms : amap_ms < map_ms;
-  if (choice) *choice = best + (fuse ? nv : 0);
-  int st = cg_set_kick_variant(H, best);
-  if ((h.fuse_kick != fuse || h.map_async != async) && h.turn_graph) {
-    cudaGraphExecDestroy(h.turn_graph);
-    h.turn_graph = nullptr;
-  }
-  h.fuse_kick = fuse;
-  h.map_async = async;
-  return st;
+  const int v = best + (fused_ms < per[best] + map_ms ? nv : 0);
+  if (choice) *choice = v;
+  return cg_set_kick_variant(H, v);
 }
 
 int cg_resonator_state(cg_handle* H, int c, double* out6) {
@@ -2347,12 +2327,7 @@ int cg_set_walk_reserve(cg_handle* H, int on) {
 
 int cg_set_map_async(cg_handle* H, int on) {
   if (!H) return CG_ERR_INVALID;
-  Handle& h = H->h;
-  if (h.map_async != (on != 0) && h.turn_graph) {
-    cudaGraphExecDestroy(h.turn_graph);
-    h.turn_graph = nullptr;
-  }
-  h.map_async = on != 0;
+  H->h.map_async = on != 0;
   return CG_OK;
 }
 

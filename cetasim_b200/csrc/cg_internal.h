@@ -253,7 +253,7 @@ struct Handle {
   cudaGraphExec_t turn_graph = nullptr;
   int kick_variant = 0;         // autotuned shape of the kick kernel
   bool fuse_kick = true;        // the kick inside the map pass (cg_set_kick_variant, cg_autotune)
-  bool map_async = false;       // cg_set_map_async (no effect: the map pass always prefetches)
+  bool map_async = false;       // cg_set_map_async (kept for cg_map_async; one map pass)
   int sh_rank = 0, sh_world = 1;  // bunch sharding over ranks (cg_set_shard)
   int sh_j0 = 0, sh_j1 = 0, sh_maxlocal = 0;
   void* nccl_comm = nullptr;

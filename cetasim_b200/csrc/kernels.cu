@@ -492,9 +492,10 @@ cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a, int til
 }
 
 int kick_variants() { return kKickVariants; }
-void kick_variant_shape(int v, int* threads, int* min_ctas) {
-  *threads = kKickShapes[v][0];
-  *min_ctas = kKickShapes[v][1];
+int kick_variant_first(int v) {
+  int u = 0;
+  while (kKickShapes[u][0] != kKickShapes[v][0] || kKickShapes[u][1] != kKickShapes[v][1]) ++u;
+  return u;
 }
 
 // The particles' pass of one interaction point: the electron-side ion kick

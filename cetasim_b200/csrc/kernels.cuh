@@ -59,7 +59,7 @@ cudaError_t launch_ion_kick(Handle& h, int k);
 cudaError_t launch_ion_kick_variant(Handle& h, int k, int v, int tile_a = 0, int tile_b = -1,
                                     cudaStream_t s = nullptr);
 int kick_variants();
-void kick_variant_shape(int v, int* threads, int* min_ctas);
+int kick_variant_first(int v);  // the first choice that runs the kernel of choice v
 // (ion kick of IP k if `kick`) + map of section k + moments at section
 // `mom_section` (if >= 0; their z range if `z_range`; with neither kick nor
 // moments the pass is launch_map's), over the chunks

@@ -424,9 +424,7 @@ int cg_turn_launches(cg_handle* h, int* launches);
  * chain (k), 3 moments (k), 4 longitudinal turn tail, 5 the map + moments
  * pass of the turn graph (section k), 6 the surrogate field kick (k, after
  * cg_set_surrogate), 7 the map + moments pass with the ion kick inside, 8 and
- * 9 the passes 5 and 7 with each CTA's next chunk staged in shared memory by
- * cp.async while it works on the current one (persistent grid).  The beam
- * state is advanced by these launches. */
+ * 9 the same as 5 and 7.  The beam state is advanced by these launches. */
 int cg_time_stage(cg_handle* h, int stage, int k, int reps, double* ms);
 /* FP64 FMA throughput of this device measured by a register-resident FMA
  * chain kernel, in FLOP/s (2 per FMA). */
@@ -484,26 +482,24 @@ int cg_gaussian_field(const double* x, const double* y, const double* sx,
 
 /* ---- autotuning (no counterpart in the reference) ---- */
 
-/* Number n of shapes (threads per CTA, register budget, tiles per CTA) of
- * the field-kick kernel.  Choices 0 .. n-1 run the kick as its own kernel with that shape;
- * n .. 2n-1 the same shape for the staged calls and, in the turn graph, the
- * kick inside the map pass (one particle pass for kick, map and moments). */
+/* Number n of choices of the field-kick kernel's shape (threads per CTA and
+ * register budget; some choices run the same kernel).  Choices 0 .. n-1 run the
+ * kick as its own kernel with that shape; n .. 2n-1 the same shape for the
+ * staged calls and, in the turn graph, the kick inside the map pass (one
+ * particle pass for kick, map and moments; the default). */
 int cg_kick_variants(int* n);
 /* Use choice v for h (the turn graph is rebuilt). */
 int cg_set_kick_variant(cg_handle* h, int v);
-/* Times every kick shape on h's own beam at IP k (reps launches each, after
+/* Times every kick kernel on h's own beam at IP k (reps launches each, after
  * a warm-up; the records of the last ion pass at k), then the map pass with
- * and without the kick inside, each in its register form and with the next
- * chunk in flight; restores the beam after every trial and selects the
- * fastest combination: *choice (as cg_set_kick_variant takes it), ms[0 .. n-1]
- * per kick launch, ms[n] the map pass, ms[n+1] the map pass with the kick,
- * ms[n+2] and ms[n+3] the same with the next chunk in flight (ms holds n + 4
- * values); the map-pass form chosen is set as by cg_set_map_async. */
+ * and without the kick inside; restores the beam after every trial and selects
+ * the fastest combination: *choice (as cg_set_kick_variant takes it), ms[0 ..
+ * n-1] per kick launch (choices of one kernel hold one figure), ms[n] the map
+ * pass, ms[n+1] the map pass with the kick, ms[n+2] and ms[n+3] these two
+ * again (ms holds n + 4 values). */
 int cg_autotune(cg_handle* h, int k, int reps, int* choice, double* ms);
-/* The map pass form of the turn graph: 0 one chunk per CTA with its loads in
- * registers, 1 a persistent grid with each CTA's next chunk staged in shared
- * memory by cp.async while it works on the current one (the turn graph is
- * rebuilt).  Results are bitwise the same. */
+/* Accepted without effect (there is one form of the map pass); cg_map_async
+ * returns the value. */
 int cg_set_map_async(cg_handle* h, int on);
 /* 1: every walk CTA asks for its SM's whole shared memory, so that no other
  * CTA (kick, map pass) runs on an SM while a walk CTA does; 0 (default):
@@ -514,11 +510,13 @@ int cg_map_async(cg_handle* h, int* on);
 
 /* Pipelined turn: the ion walk of each IP runs in `groups` segments of
  * bunches, and the kicks and maps of a walked segment run alongside the next
- * segment's walk (1 = one segment, no overlap; default 4; at most 16); ramp
- * != 0 makes the last segment half as long as the others.  Results do not
+ * segment's walk (1 = one segment, no overlap; at most 16; without this call
+ * cg_set_beam takes a segment per 3000 tiles of 256 particles, at most 8);
+ * ramp != 0 makes the last segment half as long as the others.  Results do not
  * depend on `groups` or `ramp`.  walk_ions: trajectories per walk CTA, 8, 16,
- * 32 or 64 (0 keeps the current shape); the shape sets the summation order of
- * the cloud moments, so results agree to rounding across shapes. */
+ * 32 or 64 (0 keeps the current shape; default 64; 8 runs as 16); the shape
+ * sets the summation order of the cloud moments, so results agree to rounding
+ * across shapes. */
 int cg_set_pipeline(cg_handle* h, int groups, int walk_ions, int ramp);
 
 /* Times whole turns (turn0 to warm up the turn graph, then `reps` turns, CUDA
