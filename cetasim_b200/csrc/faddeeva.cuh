@@ -36,13 +36,14 @@
 namespace cg {
 
 constexpr int kWeidemanN = 40;
-// The coefficients of Z^26 .. Z^39 are below 2e-10 of the leading one, so
-// single precision in their part of the series moves the whole by less than
-// 1e-17: w_weideman_fast sums them in the FP32 pipe.
-// Against binary128 on 5e5 points the errors are those of the all-FP64 series
-// (rms 4.0e-16 of |w| for |z| < 1, 1.4e-16 for 12 < |z| < 30); with 17 or more
-// terms they would grow near the real axis.
-constexpr int kWeidemanTail = 14;
+// The coefficients of Z^28 .. Z^39 are below 2e-11 of the leading one, so
+// single precision in their part of the series moves w by at most 1.4e-18 |w| =
+// 2^-59 |w| for |z| < 30 (14 terms: 1.4e-17): w_weideman_fast sums them in the
+// FP32 pipe.  Against binary128 the rms errors are those of the all-FP64 series
+// to 0.1 % in fourteen ranges of z (4.0e-16 of |w| for |z| < 1, 1.3e-16 for
+// 8 < |z| < 30, 2.4e-16 for 5 < x < 8 near the real axis, where 14 terms left
+// 0.7 % more in places).
+constexpr int kWeidemanTail = 12;
 
 struct WeidemanTable {
   double a[kWeidemanN];  // highest power first (Horner order)
@@ -190,7 +191,8 @@ CG_HD cplx w_quadrant1(double x, double y) {
   return w;
 }
 
-// 1/d for 1e-30 < d < 3e38 by Newton-Raphson refinement of an approximate
+// 1/d for 1e-300 < d < 1e300 (on the host, whose seed is single precision, 1e-30
+// to 3e38) by Newton-Raphson refinement of an approximate
 // seed (two steps, r <- r + r (1 - d r): 2^-20 -> 2^-40 -> rounding level,
 // within about an ulp of the correctly rounded quotient).  The seed is the
 // double-precision reciprocal approximation: 18 cycles, against 60 for a
@@ -231,12 +233,11 @@ CG_HD cplx weideman_map(double x, double y, double L, cplx* rden) {
 // b_k = c_k + r b_{k+1} - s b_{k+2}, and p(Z) = b_1 Z + c_0 - s b_2: two FMAs
 // per term instead of the four FP64 instructions of a complex Horner step.
 // A rounding of b_k acts on p as the same change of c_k times Z^k, and
-// |b_k| stays below 1e-9 down to k = 26, so the first kWeidemanTail steps run
-// in single precision and 28 of the 76 FP64 operations per point go to the FP32
-// pipe, which the kick leaves idle.  The NW
-// recurrences run side by side: each is one FMA latency per term.  For |z| < 30
-// in the first quadrant within 2e-15 of w relative to |w| (the form the
-// throughput kernels use).
+// |b_k| stays below 1e-10 down to k = 28, so the first kWeidemanTail steps run
+// in single precision and 24 of the 76 FP64 operations per point go to the FP32
+// pipe, which the kick leaves idle.  The NW recurrences run side by side: each
+// is one FMA latency per term.  For |z| < 30 in the first quadrant within 2e-15
+// of w relative to |w| (the form the throughput kernels use).
 template <int NW>
 CG_HD void w_weideman_fast(const double (&x)[NW], const double (&y)[NW], cplx (&w)[NW]) {
   const WeidemanTable& T = weideman_table();
