@@ -99,3 +99,35 @@ def test_turn_repeats_the_staged_calls(lr):
         (ca, sa), (cb, sb) = a.download(j), b.download(j)
         assert np.array_equal(ca, cb) and np.array_equal(sa, sb)
         assert a.moments()[j].transmission == t[j]
+
+
+def _bins(wl, z):
+    """First and last bin that a particle is in (MPBunch.cpp:2052, 2170)."""
+    r, t = wl.cfg.ring, wl.bbi_table
+    if wl.cfg.bbi.time_domain:
+        dz, lo = abs(t[1, 0] - t[0, 0]), -r.t0 * 299792458.0 / r.harmonics / 2
+    else:
+        dz = 1 / (2 * t[-1, 0]) * 299792458.0 * r.r_beta
+        lo = -dz * (len(t) - 1) - dz / 2
+    b = ((z - lo) / dz).astype(int)
+    return b.min(), b.max()
+
+
+@pytest.mark.parametrize("td,stretch,rows", CASES)
+def test_potentials_on_every_bin_between_the_particles(td, stretch, rows):
+    """The bins come from the particles, so that a bin or a plane left out
+    shows."""
+    wl, parts = _train(SIZES, stretch, td, rows)
+    g, o = pair(wl, parts)
+    for b in (g, o):
+        b.BBImpBeamInteraction()
+    for j, p in enumerate(parts):
+        first, last = _bins(wl, p[4])
+        a, have = g.bbi_profile(j)
+        have = have[1:, first - a:last + 1 - a]
+        want = o.bbi_profile(j)[1:, first:last + 1]
+        assert have.shape == want.shape == (5, last + 1 - first)
+        for q in range(5):
+            k = np.max(np.abs(want[q]))
+            assert k > 0 or p.shape[1] == 1  # one particle: its own wake can underflow
+            assert np.max(np.abs(have[q] - want[q])) <= 1e-11 * k
