@@ -86,3 +86,15 @@ def test_positions_on_the_edges_of_slices(flag, nz):
         for q in (1, 3):
             k = np.max(np.abs(want[q] - p[q]))
             assert np.max(np.abs(have[q] - want[q])) <= 1e-11 * k
+
+
+@pytest.mark.parametrize("flag", [1, 2])
+def test_chunks_of_more_tiles_than_one_round(flag):
+    """A bunch of more than 256 chunks of eight tiles, beside a small one,
+    against the oracle; tolerance as for the edges."""
+    wl, parts = _train(flag, (9, 8, 5), [531000, 700])
+    surv = [np.zeros(p.shape[1], dtype=np.uint8) for p in parts]
+    for p, want, have in zip(parts, *(_kick(wl, parts, surv, c) for c in (oracle.OracleBeam, MPBeam))):
+        for q in (1, 3):
+            k = np.max(np.abs(want[q] - p[q]))
+            assert np.max(np.abs(have[q] - want[q])) <= 1e-11 * k

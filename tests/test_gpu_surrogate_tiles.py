@@ -22,3 +22,16 @@ def test_gradients(n):
         assert np.linalg.norm(g[o:o + k] - gref[o:o + k]) <= 1e-4 * np.linalg.norm(gref[o:o + k])
     again = S.gradient(w, x, t)
     assert again[0] == loss and np.array_equal(again[1], g)
+
+
+def test_gradients_of_two_threads():
+    """Calls from two host threads share the pool of device memory: each gets
+    the gradient that it gets alone, bit for bit."""
+    from concurrent.futures import ThreadPoolExecutor
+    n = (128 * 9, 128)
+    args = [(mlp.init(9 + i), *S.dataset(11 + i, n[i])) for i in range(2)]
+    alone = [S.gradient(*a) for a in args]
+    with ThreadPoolExecutor(2) as ex:
+        both = list(ex.map(lambda i: (i, S.gradient(*args[i])), [0, 1] * 20))
+    for i, (loss, grad) in both:
+        assert loss == alone[i][0] and np.array_equal(grad, alone[i][1])

@@ -92,3 +92,29 @@ def test_turn_ends_with_the_marks(config, lost):
         assert np.array_equal(ca, cb) and np.array_equal(sa, sb)
         assert a.moments()[j].transmission == t[j]
     assert lost == "x" or t.max() < 1
+
+
+@pytest.mark.parametrize("config,scale", [("batched_uneven", 0.01), ("large_trapping", 0.005)])
+def test_last_map_joins_the_tail_before_the_feedback(config, scale):
+    """Turns with the feedback alone, whose last map is in the longitudinal
+    pass: equal to their staged calls bit for bit."""
+    wl = small(config, scale, flag_lr_wake=0, flag_sr_wake=0, flag_beam_ion=0, flag_fir=1)
+    parts = particles(wl, seed=12)
+    a, b = MPBeam(wl), MPBeam(wl)
+    for j, c in enumerate(parts):
+        a.upload(j, c)
+        b.upload(j, c)
+    a.Run(0, 3)
+    for turn in range(3):
+        for k in range(wl.cfg.n_sections):
+            b.BeamTransferPerInteractionPointDueToLatticeT(k)
+        b.BeamMomtumUpdateDueToRFTest()
+        b.BeamLongiPosTransferOneTurn()
+        b.BeamEnergyLossOneTurn()
+        b.BeamSynRadDamping(turn)
+        b.MPBeamRMSCal(0)
+        b.FIRBunchByBunchFeedback(turn)
+        b.MarkParticleLostInBunch()
+    for j in range(wl.n_bunches):
+        (ca, sa), (cb, sb) = a.download(j), b.download(j)
+        assert np.array_equal(ca, cb) and np.array_equal(sa, sb)
