@@ -96,6 +96,11 @@ CG_HD void matvec6_plain(const double* A, const double v[6], double out[6]) {
   out[5] = A[35] * v[5];
 }
 
+// z with what the zeros of the z row that matvec6_plain leaves out would bring
+// into it: nothing, or no number where a transverse coordinate is not finite (so
+// that the stages that look at z see a particle that has left the numbers).
+CG_HD double carry_nonfinite(double z, double x, double y) { return fma(0.0, x + y, z); }
+
 CG_HD void matvec6_section(const SectionDev& s, const double* A, const double v[6], double out[6]) {
   if (s.twiss_form == 2) matvec6_plain(A, v, out);
   else if (s.twiss_form) matvec6_twiss(A, v, out);
@@ -182,7 +187,7 @@ CG_HD void section_map_rotated(const SectionDev& s, const RingDev& r, const doub
   v2[1] = fma(-sx, v1[0], cx * v1[1]);
   v2[2] = fma(cy, v1[2], sy * v1[3]);
   v2[3] = fma(-sy, v1[2], cy * v1[3]);
-  v2[4] = v1[4];
+  v2[4] = s.twiss_form == 2 ? carry_nonfinite(v1[4], v2[0], v2[2]) : v1[4];
   v2[5] = v1[5];
 }
 
@@ -217,6 +222,7 @@ CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
     X[5] = fma(r.qe_coeff[2], g[5], X[5]);
   }
   matvec6_section(s0, s0.h1b1, X, v);
+  if (s0.twiss_form == 2) v[4] = carry_nonfinite(v[4], v[1], v[3]);
 }
 
 // Bunch::MarkLostParticle per particle (Bunch.cpp:179-191): returns the
