@@ -28,6 +28,7 @@
 // us: range 44 (one thread over the tiles) -> in the longitudinal pass,
 // histogram and lags 8 + 5 -> 6.4 together, potentials 7 -> 4.1 (a thread per
 // bin before), kick and loss check 5 + 7 -> 5.0 together.
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "turn_tail.cuh"
 
@@ -168,7 +169,7 @@ __device__ double rw_pseudo_fz(double u, double (*sw4)[8]) {
   return c1 * (c2 * (m025 - p075) + (-p025 + m075));
 }
 
-// One CTA per (bunch, lag): W_z(tau) summed over resonators, lag bin m = i - j.
+// A CTA: W_z(tau) summed over resonators, lag bin m = i - j of bunch b.
 __device__ __forceinline__ void sr_lag_cta(int b, int m, double dz, const SrResonator* __restrict__ res,
                                            const double* __restrict__ green, int n_res, int B,
                                            double sigmat, double rw_coeff, double* lag,
@@ -236,7 +237,7 @@ __device__ __forceinline__ void sr_lag_cta(int b, int m, double dz, const SrReso
   }
 }
 
-// CTAs [0, n_chunks): a chunk each; then one per (bunch, lag).
+// CTAs [0, n_chunks): a chunk each; then for each bunch CTAs of `per` lags.
 template <bool XY>
 __global__ void __launch_bounds__(kTile) k_sr_bins(const double* __restrict__ c, int64_t npad,
                                                    const uint8_t* __restrict__ surv,
@@ -247,12 +248,12 @@ __global__ void __launch_bounds__(kTile) k_sr_bins(const double* __restrict__ c,
                                                    const SrResonator* __restrict__ res,
                                                    const double* __restrict__ green, int n_res,
                                                    double sigmat, double rw_coeff, double* lag,
-                                                   const double* __restrict__ green_t) {
+                                                   const double* __restrict__ green_t, int per) {
   extern __shared__ unsigned char sm_raw[];
-  const int B = sr.B, lags = 2 * B - 1;
+  const int B = sr.B, lags = 2 * B - 1, shares = (lags + per - 1) / per;
   const bool hist = (int)blockIdx.x < n_chunks;
   const int q = (int)blockIdx.x - n_chunks;
-  const int4 l = hist ? chunk_loc[blockIdx.x] : make_int4(q / lags, 0, 0, 0);
+  const int4 l = hist ? chunk_loc[blockIdx.x] : make_int4(q / shares, 0, 0, 0);
   const int b = l.x, tile_off = bunch[b].tile_off;
   if (bunch[b].n_tiles == 0) return;  // held by another rank
   const SrGeom G = sr_geometry(sr.span[b], c[4 * npad + (int64_t)tile_off * kTile],
@@ -262,12 +263,13 @@ __global__ void __launch_bounds__(kTile) k_sr_bins(const double* __restrict__ c,
                       sr.sumx + (size_t)b * B, sr.sumy + (size_t)b * B, B, sm_raw);
     return;
   }
-  const int m = q % lags;
-  if (m == 0 && threadIdx.x == 0) {
+  const int m0 = q % shares * per;
+  if (m0 == 0 && threadIdx.x == 0) {
     geom[2 * b] = G.lo;
     geom[2 * b + 1] = G.dz;
   }
-  sr_lag_cta(b, m - (B - 1), G.dz, res, green, n_res, B, sigmat, rw_coeff, lag, XY ? green_t : nullptr);
+  for (int m = m0; m < min(m0 + per, lags); ++m)
+    sr_lag_cta(b, m - (B - 1), G.dz, res, green, n_res, B, sigmat, rw_coeff, lag, XY ? green_t : nullptr);
 }
 
 __global__ void __launch_bounds__(kTile) k_sr_pot(const BunchDev* __restrict__ bunch, SrDev sr,
@@ -349,10 +351,16 @@ cudaError_t launch_sr_wake(Handle& h, bool have_range, bool mark) {
   const double sigmat = 1.e-3 / kCLight;
   const bool xy = h.sr_xy && h.d.sr_potxy;
   const size_t sm = ((B * sizeof(int) + 15) & ~(size_t)15) + (xy ? 2 * B * sizeof(double) : 0);
-  (xy ? k_sr_bins<true> : k_sr_bins<false>)<<<h.n_chunks + h.M * (2 * B - 1), kTile, sm, h.stream>>>(
+  // lags per CTA: one while a few rounds of the 1184 CTAs that run at once hold
+  // them all; beyond, a CTA's start (three loads, one after the other) would
+  // cost as much as a lag (1000 bunches, 100 bins: a turn 2019 -> 1438 us)
+  const int lags = 2 * B - 1;
+  const int per = (int)std::min<int64_t>(lags, std::max<int64_t>(1, (int64_t)h.M * lags / (4 * 1184)));
+  const int shares = (lags + per - 1) / per;
+  (xy ? k_sr_bins<true> : k_sr_bins<false>)<<<h.n_chunks + h.M * shares, kTile, sm, h.stream>>>(
       h.d.c, h.npad, h.d.surv, h.d.chunk_loc, h.n_chunks, h.d.bunch, h.d.mom, sr, h.d.sr_geom,
       reinterpret_cast<const SrResonator*>(h.d.sr_green), h.d.sr_green + 3 * CG_MAX_RESONATORS,
-      h.cfg.sr_bbr.n, sigmat, h.sr_rw_coeff, h.d.sr_lag, h.d.sr_green_t);
+      h.cfg.sr_bbr.n, sigmat, h.sr_rw_coeff, h.d.sr_lag, h.d.sr_green_t, per);
   k_sr_pot<<<dim3((B + kTile / 32 - 1) / (kTile / 32), h.M), kTile, 0, h.stream>>>(
       h.d.bunch, sr, h.d.sr_lag, h.d.sr_pot, h.cfg.ring.electron_energy, xy ? h.d.sr_potxy : nullptr);
   (mark ? k_sr_kick<true> : k_sr_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(
