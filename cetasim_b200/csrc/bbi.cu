@@ -50,7 +50,6 @@ namespace cg {
 
 #define BBI_FULL 0xffffffffu
 constexpr int kBbiThreads = 256;
-constexpr int kBbiConvThreads = 1024;
 // Bins up to which a CTA counts in shared memory (20 bytes each); beyond, it
 // adds to the bunch's bins directly.
 constexpr int kBbiSharedBins = 1024;
@@ -151,12 +150,13 @@ __global__ void __launch_bounds__(kBbiThreads) k_bbi_hist(const double* __restri
 // over [s0, s1) equals the raw one; bins outside pass unchanged, every other
 // bin of the profile is zero and stays zero.  The raw profiles keep kBbiHalf
 // zeros on both sides, so that a tap away from s0 and s1 needs no check.
-__global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_bbi_conv(
     const BunchDev* __restrict__ bunch, const __grid_constant__ BbiParams p,
     const double* __restrict__ w, BbiSpan* span, int* cnt,
     unsigned long long* sxy, double* pot, int2* win) {
   extern __shared__ double sm[];
-  __shared__ double red[kBbiConvThreads / 32][6];
+  __shared__ double red[NT / 32][6];
   __shared__ double scale[3];
   const int b = blockIdx.x;
   const BunchDev& Bd = bunch[b];
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
   const double unit = p.td ? Bd.q_macro * kElectronCharge
                            : Bd.q_macro * kElectronCharge / p.dz * kCLight;
   const int smooth = p.td ? 1 : 3;  // profiles that are smoothed
-  for (int t = threadIdx.x; t < nr; t += kBbiConvThreads) {
+  for (int t = threadIdx.x; t < nr; t += NT) {
     const int j = a - kBbiHalf + t - l;
     double r0 = 0, r1 = 0, r2 = 0;
     if (j >= 0 && j < W) {
@@ -213,8 +213,8 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
   for (int q = 0; q < 3; ++q) {
     const double* raw = s_raw + q * nr + kBbiHalf;
     // the profiles one after the other over the threads
-    for (int t = ((int)threadIdx.x + kBbiConvThreads - q * n % kBbiConvThreads) % kBbiConvThreads;
-         t < n; t += kBbiConvThreads) {
+    for (int t = ((int)threadIdx.x + NT - q * n % NT) % NT;
+         t < n; t += NT) {
       const int i = a + t;
       double y = raw[t];
       if (q < smooth && i >= p.s0 && i < p.s1) {
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
   if (threadIdx.x < 32) {
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      double v = red[threadIdx.x][q];
+      double v = threadIdx.x < NT / 32 ? red[threadIdx.x][q] : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(BBI_FULL, v, o);
       sum[q] = v;
@@ -264,15 +264,15 @@ __global__ void __launch_bounds__(kBbiConvThreads, 1) k_bbi_conv(
     }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < smooth * n; t += kBbiConvThreads) {
+  for (int t = threadIdx.x; t < smooth * n; t += NT) {
     const int q = t >= 2 * n ? 2 : t >= n ? 1 : 0, i = a + t - q * n;
     if (i >= p.s0 && i < p.s1) s_p[t] *= scale[q];
   }
   __syncthreads();
   double* out = pot + (size_t)b * 6 * p.wcap;
-  for (int t = threadIdx.x; t < n; t += kBbiConvThreads) out[t] = s_p[t];
+  for (int t = threadIdx.x; t < n; t += NT) out[t] = s_p[t];
   const int N = p.nbins;
-  for (int task = threadIdx.x; task < 5 * n; task += kBbiConvThreads) {
+  for (int task = threadIdx.x; task < 5 * n; task += NT) {
     const int q = task / n, t = task - q * n, i = a + t;
     double v = 0;
     if (i >= l && i <= h && p.sim[q]) {
@@ -390,7 +390,12 @@ cudaError_t launch_bbi(Handle& h, bool have_range, bool mark) {
   k_bbi_hist<<<dim3(h.M, (big + tiles - 1) / tiles), kBbiThreads,
                5 * sizeof(unsigned) * std::min(p.wcap, kBbiSharedBins), h.stream>>>(
       h.d.c, h.npad, h.d.surv, h.d.bunch, tiles, p, span, h.d.status, h.d.bbi_cnt, h.d.bbi_sxy);
-  k_bbi_conv<<<h.M, kBbiConvThreads, bbi_conv_smem(p), h.stream>>>(
+  // a bunch's few thousand tasks want 1024 threads where each SM has a bunch or
+  // less; beyond, several CTAs of 256 share an SM
+  // (900 bunches of 270 particles, a kick 92 -> 75 us; 900 of 4000, a turn with the
+  // wake table 304 -> 285 us)
+  const bool few = h.M <= 148;
+  (few ? k_bbi_conv<1024> : k_bbi_conv<256>)<<<h.M, few ? 1024 : 256, bbi_conv_smem(p), h.stream>>>(
       h.d.bunch, p, h.d.bbi_w, span, h.d.bbi_cnt, h.d.bbi_sxy, h.d.bbi_pot, h.d.bbi_win);
   (mark ? k_bbi_kick<true> : k_bbi_kick<false>)<<<h.n_tiles, kTile, 0, h.stream>>>(
       h.d.c, h.npad, h.d.surv, h.d.tile_bunch, h.d.bunch, p, h.d.bbi_win, h.d.bbi_pot, f, aperture(h),
@@ -403,8 +408,10 @@ size_t bbi_conv_smem(const BbiParams& p) {
 }
 
 cudaError_t prepare_bbi(const BbiParams& p) {
-  return cudaFuncSetAttribute(k_bbi_conv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)bbi_conv_smem(p));
+  cudaError_t e = cudaFuncSetAttribute(k_bbi_conv<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)bbi_conv_smem(p));
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(k_bbi_conv<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)bbi_conv_smem(p));
 }
 
 // ---------------------------------------------------------------------------

@@ -131,3 +131,25 @@ def test_potentials_on_every_bin_between_the_particles(td, stretch, rows):
             k = np.max(np.abs(want[q]))
             assert k > 0 or p.shape[1] == 1  # one particle: its own wake can underflow
             assert np.max(np.abs(have[q] - want[q])) <= 1e-11 * k
+
+
+@pytest.mark.parametrize("td", [0, 1])
+@pytest.mark.parametrize("m", [148, 149])
+def test_potentials_of_trains_round_the_smaller_convolutions(m, td):
+    """More bunches than SMs take the convolution of 256 threads."""
+    wl = configs.make("batched_uneven", n_scale=0.004)
+    wl.n_macro, wl.harm, wl.ne = wl.n_macro[:m].copy(), wl.harm[:m].copy(), wl.ne[:m].copy()
+    c = wl.cfg
+    c.flag_beam_ion = c.flag_lr_wake = c.flag_fir = c.flag_sr_wake = 0
+    wl.set_bbi(bbicases.wake_table(400, 0.5e-3, 40) if td else bbicases.resonator_table(640, 300e9), td)
+    parts = particles(wl, seed=19)
+    g, o = pair(wl, parts)
+    for b in (g, o):
+        b.BBImpBeamInteraction()
+    for j, p in enumerate(parts):
+        first, last = _bins(wl, p[4])
+        a, have = g.bbi_profile(j)
+        have = have[:, first - a:last + 1 - a]
+        want = o.bbi_profile(j)[:, first:last + 1]
+        for q in range(6):
+            assert np.max(np.abs(have[q] - want[q])) <= 1e-11 * np.max(np.abs(want[q]))
