@@ -832,11 +832,13 @@ __global__ void k_lr_force(const BunchMomDev* __restrict__ mom, const BunchDev* 
     int nT = bunch[i].harm - hj - n * H;
     double tau = nT * tRF + (zj - hs[2 * M + i]) * inv_c_beta;
     double a = -tau / dt;
-    int idx = (int)floor(a);
-    if (tau > 0 || idx < 0 || idx + 1 >= np) {
+    // compared before the conversion, which saturates (or gives the smallest
+    // integer for a NaN)
+    if (tau > 0 || !(a >= 0 && a < np - 1)) {
       atomicOr(status, kStatusLrRange);
       continue;
     }
+    const int idx = (int)a;
     double v1 = a - idx, v0 = 1 - v1;
     double ne = bunch[i].ne;
     double w0 = tab[idx] * v0 + tab[idx + 1] * v1;
