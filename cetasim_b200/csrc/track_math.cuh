@@ -96,10 +96,11 @@ CG_HD void matvec6_plain(const double* A, const double v[6], double out[6]) {
   out[5] = A[35] * v[5];
 }
 
-// z with what the zeros of the z row that matvec6_plain leaves out would bring
-// into it: nothing, or no number where a transverse coordinate is not finite (so
-// that the stages that look at z see a particle that has left the numbers).
-CG_HD double carry_nonfinite(double z, double x, double y) { return fma(0.0, x + y, z); }
+// u with what the zeros that matvec6_plain leaves out of its row would bring into
+// it from the coordinates x and y: nothing, or no number where one of them is
+// not finite (so that the stages that look at u see a particle that has left the
+// numbers).
+CG_HD double carry_nonfinite(double u, double x, double y) { return fma(0.0, x + y, u); }
 
 CG_HD void matvec6_section(const SectionDev& s, const double* A, const double v[6], double out[6]) {
   if (s.twiss_form == 2) matvec6_plain(A, v, out);
@@ -209,6 +210,10 @@ CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
                            const double g[6], bool excite) {
   double X[6];
   matvec6_section(s0, s0.b1h1, v, X);
+  if (s0.twiss_form == 2) {  // and the transverse planes what the zeros bring from dp
+    X[0] = carry_nonfinite(X[0], v[5], 0.0);
+    X[2] = carry_nonfinite(X[2], v[5], 0.0);
+  }
   X[0] *= r.lambda[0];
   X[1] *= r.lambda[0];
   X[2] *= r.lambda[1];

@@ -42,3 +42,17 @@ def test_bunches_of_one_particle_in_an_ion_train_are_refused():
     b.generate(7)
     with pytest.raises(_abi.CgError):
         b.Run(0, 1)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_damping_with_a_momentum_that_is_not_finite(bad):
+    """The damping's zeros bring it into every coordinate."""
+    wl = small("plain_single", 0.003)
+    c = particles(wl, seed=4)[0]
+    c[5, 17] = bad
+    b = MPBeam(wl)
+    b.upload(0, c)
+    b.BeamSynRadDamping(0)
+    got = b.download(0)[0]
+    assert np.all(np.isnan(got[:5, 17])) and not np.isfinite(got[5, 17])
+    assert np.all(np.isfinite(np.delete(got, 17, axis=1)))
