@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_rf_prep(BlParams p, const Bunc
     const Affine all = affine_block_scan<kPrepThreads>(f, &ex, s_warp);
     if (k < nb && cv.excite != 0) {
       Affine pre = affine_then(carry, ex);
-      pre.a = rot(k);
+      if (k > 0) pre.a = rot(k);  // the head bin's is one, also where the range is infinite
       w.pre[bj * nb + k] = pre;
     }
     carry = affine_then(carry, all);

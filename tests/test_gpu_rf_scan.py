@@ -39,3 +39,22 @@ def test_rf_steps_match_the_sequential_recurrence(bunches, bins, excite):
         assert blcases.coord_rel_err(got, want, s == 0).max() <= 1e-12
     for x, y in zip(b.resonator(1), o.resonator(1)):
         assert abs(x - y) <= 1e-12 * (abs(y) + 1e-300)
+
+
+def test_one_bin_of_infinite_width():
+    """The head bin's voltage needs no rotation: the induced voltage of a bunch
+    with a particle infinitely far away is that of the same bunch without."""
+    with tempfile.TemporaryDirectory() as d:
+        wl, _, _ = blcases.build("ragged_harmonic", d)
+    wl.n_macro, wl.harm, wl.ne = (a[:1].copy() for a in (wl.n_macro, wl.harm, wl.ne))
+    wl.cfg.ring.rf_bunch_bins = 1
+    wl.cfg.ring.res_excite[1] = 1
+    parts = particles(wl, seed=3, spread=1.0)[0]
+    induced = []
+    for z in (parts[4, 1], np.inf):
+        parts[4, 1] = z
+        b = MPBeam(wl)
+        b.upload(0, parts)
+        b.BeamMomtumUpdateDueToRFTest()
+        induced.append(b.rf_info(0, 1)[2])
+    assert np.isfinite(induced[0]) and induced[0] == induced[1]
