@@ -45,7 +45,7 @@ constexpr int kWeidemanN = 40;
 // 0.7 % more in places).
 constexpr int kWeidemanTail = 12;
 
-struct WeidemanTable {
+struct alignas(128) WeidemanTable {  // whole lines of the constant cache
   double a[kWeidemanN];  // highest power first (Horner order)
   double L;
   float t[kWeidemanTail];  // the first of a in single precision

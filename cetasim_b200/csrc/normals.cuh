@@ -7,7 +7,9 @@
 
 namespace cg {
 
-struct NormalConst {
+// whole lines of the constant cache (8 bytes off one, the turn's tail takes 506 us
+// for 1.74e7 particles instead of 488)
+struct alignas(128) NormalConst {
   double atanh_c[7];  // (atanh(s) / s - 1) / s^2 in s^2 <= 0.0295
   double sin_c[6];    // (sin(y) / y - 1) / y^2 in y^2, |y| <= pi / 4
   double cos_c[6];    // (cos(y) - 1 + y^2 / 2) / y^4 in y^2
