@@ -86,21 +86,20 @@ CG_HD void matvec6_twiss(const double* A, const double v[6], double out[6]) {
   out[5] = A[35] * v[5];
 }
 
-// matvec6 for a matrix without dispersion terms: 8 operations.
-CG_HD void matvec6_plain(const double* A, const double v[6], double out[6]) {
-  out[0] = A[0] * v[0];
-  out[1] = fma(A[7], v[1], A[6] * v[0]);
-  out[2] = A[14] * v[2];
-  out[3] = fma(A[21], v[3], A[20] * v[2]);
-  out[4] = A[28] * v[4];
+// matvec6 for a matrix without dispersion terms: 8 operations.  What the zeros
+// that it leaves out would bring into a row is nothing, or no number where a
+// coordinate is not finite, and the stages that look at that row should see a
+// particle that has left the numbers.  So a caller adds 0 times such coordinates:
+// t to the transverse rows, tz to z's.
+CG_HD void matvec6_plain(const double* A, const double v[6], double out[6], double t = 0.0,
+                         double tz = 0.0) {
+  out[0] = fma(A[0], v[0], t);
+  out[1] = fma(A[7], v[1], fma(A[6], v[0], t));
+  out[2] = fma(A[14], v[2], t);
+  out[3] = fma(A[21], v[3], fma(A[20], v[2], t));
+  out[4] = fma(A[28], v[4], tz);
   out[5] = A[35] * v[5];
 }
-
-// u with what the zeros that matvec6_plain leaves out of its row would bring into
-// it from the coordinates x and y: nothing, or no number where one of them is
-// not finite (so that the stages that look at u see a particle that has left the
-// numbers).
-CG_HD double carry_nonfinite(double u, double x, double y) { return fma(0.0, x + y, u); }
 
 CG_HD void matvec6_section(const SectionDev& s, const double* A, const double v[6], double out[6]) {
   if (s.twiss_form == 2) matvec6_plain(A, v, out);
@@ -188,14 +187,16 @@ CG_HD void section_map_rotated(const SectionDev& s, const RingDev& r, const doub
   v2[1] = fma(-sx, v1[0], cx * v1[1]);
   v2[2] = fma(cy, v1[2], sy * v1[3]);
   v2[3] = fma(-sy, v1[2], cy * v1[3]);
-  v2[4] = s.twiss_form == 2 ? carry_nonfinite(v1[4], v2[0], v2[2]) : v1[4];
+  v2[4] = v1[4];
   v2[5] = v1[5];
 }
 
 CG_HD void section_map_particle(const SectionDev& s, const RingDev& r, double v[6]) {
   double v2[6];
   section_map_rotated(s, r, v, v2);
-  matvec6_section(s, s.h2b2, v2, v);
+  // the phases have brought dp into the transverse planes
+  if (s.twiss_form == 2) matvec6_plain(s.h2b2, v2, v, 0.0, 0.0 * (v2[0] + v2[2]));
+  else matvec6_section(s, s.h2b2, v2, v);
 }
 
 // Bunch::BunchLongPosTransferOneTurn (Bunch.cpp:499-500).
@@ -209,11 +210,9 @@ CG_HD double drift_z(const RingDev& r, double z, double dp) {
 CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
                            const double g[6], bool excite) {
   double X[6];
-  matvec6_section(s0, s0.b1h1, v, X);
-  if (s0.twiss_form == 2) {  // and the transverse planes what the zeros bring from dp
-    X[0] = carry_nonfinite(X[0], v[5], 0.0);
-    X[2] = carry_nonfinite(X[2], v[5], 0.0);
-  }
+  const bool plain = s0.twiss_form == 2;
+  if (plain) matvec6_plain(s0.b1h1, v, X, 0.0 * v[5]);
+  else matvec6_section(s0, s0.b1h1, v, X);
   X[0] *= r.lambda[0];
   X[1] *= r.lambda[0];
   X[2] *= r.lambda[1];
@@ -226,8 +225,8 @@ CG_HD void synrad_particle(const SectionDev& s0, const RingDev& r, double v[6],
     X[3] = fma(r.qe_coeff[1], g[3], X[3]);
     X[5] = fma(r.qe_coeff[2], g[5], X[5]);
   }
-  matvec6_section(s0, s0.h1b1, X, v);
-  if (s0.twiss_form == 2) v[4] = carry_nonfinite(v[4], v[1], v[3]);
+  if (plain) matvec6_plain(s0.h1b1, X, v, 0.0, 0.0 * (X[1] + X[3]));
+  else matvec6_section(s0, s0.h1b1, X, v);
 }
 
 // Bunch::MarkLostParticle per particle (Bunch.cpp:179-191): returns the
