@@ -1523,7 +1523,7 @@ static cudaError_t enqueue_turn(Handle& h) {
       if ((e = cudaStreamWaitEvent(h.stream, h.pipe_ev[kMaxPipeGroups], 0))) return e;
       if ((e = cudaEventRecord(h.kick_ev[kMaxPipeGroups], h.side2))) return e;
       if ((e = cudaStreamWaitEvent(h.stream, h.kick_ev[kMaxPipeGroups], 0))) return e;
-      if (fused && G > 1) {
+      if (fused) {
         if ((e = cudaEventRecord(h.side3_ev, h.side3))) return e;
         if ((e = cudaStreamWaitEvent(h.stream, h.side3_ev, 0))) return e;
       }

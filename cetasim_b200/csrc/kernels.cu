@@ -461,7 +461,8 @@ __global__ void __launch_bounds__(NT, MINB) k_ion_kick(double* __restrict__ c, i
 // The kick shapes of autotune choice v: threads per CTA and minimum CTAs per SM
 // (the register budget).  Three kernels; the numbers 1 and 4 to 7 once stood
 // for a 64-register shape, which spills, and for several tiles per CTA, which
-// the occupancy of these makes needless (359 us against 361 for 1.74e7 kicks).
+// the occupancy of these makes needless (359 us against 361 for 1.74e7 kicks;
+// 374 since two terms more of the series are in double precision).
 static const int kKickShapes[][2] = {{256, 3}, {256, 3}, {128, 4}, {128, 6},
                                      {256, 3}, {128, 6}, {128, 6}, {256, 3}};
 constexpr int kKickVariants = 8;
@@ -501,16 +502,19 @@ int kick_variant_first(int v) {
 // The particles' pass of one interaction point: the electron-side ion kick
 // (KICK), the map of section k and the moments the next stage reads (MOM: at
 // the twiss of section `mom_section`, MPBeam.cpp:1061/1069), each particle
-// read and written once.  A CTA takes one chunk, tile by tile, and issues the
-// next tile's loads before it works on the current one.  Results equal
-// k_ion_kick, k_map and k_moments in turn, bit for bit.
-// Bound by issue: 795 instructions a particle of which 327 on the FP64 pipe (48 %
+// read and written once.  A CTA takes one chunk, half a tile after the other;
+// other warps run while one's loads are under way.  Results equal k_ion_kick,
+// k_map and k_moments in turn, bit for bit.
+// Bound by issue: 805 instructions a particle of which 337 on the FP64 pipe (46 %
 // busy) at 16 warps an SM, the accumulators of the moments beside the two
-// series leaving no registers for more.  1.74e7 particles: 623 us (kick 359 and
-// map with moments 403 apart; 471 and 441 before); floors 316 us of FP64 and
-// 260 us of HBM.  Two particles at a time spill (810 us); the next tile's
-// loads in registers or by cp.async gain nothing (660 us); an unrolled loop
-// misses the instruction cache (729 us).
+// series leaving no registers for more: 128 a thread spill 44 bytes (one
+// instruction in fifty).  1.74e7 particles: 627 us (kick 374 and map with
+// moments 404 apart; 471 and 441 before); floors 326 us of FP64 and 260 us of
+// HBM.  Two particles at a time spill more (810 us); the next tile's loads in
+// registers or by cp.async gain nothing (660 us); an unrolled loop misses the
+// instruction cache (729 us).  Without the kick five CTAs per SM spill 140 bytes
+// at 96 registers; four that spill nothing took 4013 us for a turn of the 32 x 32
+// space charge instead of 3953.
 // MOM: 0 no moments, 1 moments without the z range (which only the turn's last
 // moments, the ones that callers can read, need), 2 all.
 template <int MOM, bool KICK>

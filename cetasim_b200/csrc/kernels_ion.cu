@@ -359,10 +359,12 @@ __device__ __forceinline__ void walk_window(const WalkStep* s_st, int flags, int
 // bunches of one segment while the next segment walks).
 // A train of few ions is bound by the chain of one ion (0.38 us a step alone,
 // of which the FP64 pipe issues 270 cycles), a large cloud by the FP64 pipe:
-// 219 FP64 operations per ion and step with one lane, 2 x 136 with two, 4 x
+// 227 FP64 operations per ion and step with one lane, 2 x 136 with two, 4 x
 // 165 in the form with four lanes per ion that this replaced.  200,000 ions
 // through 1000 bunches: 19.7 -> 3.5 ms per interaction point; the 900-bunch
-// train from empty clouds: 848 -> 521 us (prep to compaction).
+// train from empty clouds: 848 -> 521 us (prep to compaction).  The two forms and
+// the slow path in one kernel of 128 registers spill 200 to 280 bytes: one
+// instruction in thirty.
 template <int IONS>
 __global__ void __launch_bounds__(2 * IONS, 256 / IONS) k_ion_walk(ChainParams cp, IonWalk w,
                                                                  const CloudDev* __restrict__ clouds,

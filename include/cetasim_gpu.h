@@ -429,10 +429,10 @@ int cg_time_stage(cg_handle* h, int stage, int k, int reps, double* ms);
 /* FP64 FMA throughput of this device measured by a register-resident FMA
  * chain kernel, in FLOP/s (2 per FMA). */
 int cg_fp64_peak(double* flops);
-/* Latency of one bunch passage of the ion walk on this device, in us: one
- * quad of lanes advances an ion through a dependent chain of passages with
- * the walk's own step arithmetic (field arguments, w(z1) and w(z2) split over
- * lanes, the Gaussian factor, field, velocity and position update), without
+/* Latency of one bunch passage of the ion walk on this device, in us: two
+ * lanes advance an ion through a dependent chain of passages with the walk's
+ * own step arithmetic (field arguments, w(z1) and w(z2), one per lane, the
+ * Gaussian factor, field, velocity and position update), without
  * the walk's window stores, barriers and sums.  The floor of the sequential
  * ion chain, which needs one passage per bunch. */
 int cg_field_chain_latency(double* us_per_step);
