@@ -416,7 +416,7 @@ void cg_host_free(void* p);
  * turn graph launch runs on it (the turn graph's branches join it before the
  * turn ends). */
 void* cg_stream(cg_handle* h);
-/* Kernel launches one cg_run_turns turn issues. */
+/* Kernel launches one cg_run_turns turn issues (0 without a beam). */
 int cg_turn_launches(cg_handle* h, int* launches);
 /* Times `reps` back-to-back launches of one stage kernel with CUDA events on
  * h's stream; *ms = average per launch.  stage: 0 section map (k), 1 ion
