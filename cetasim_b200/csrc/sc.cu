@@ -39,7 +39,7 @@
 // the barriers round four small matrix products, the field models by the FP64
 // pipe.  A section of 80 bunches of 20,000, us: PIC 32 x 32 x 33 468 -> 196
 // (solve 80, map 47, kick 38, scatter 24, count 13, moments' merge 9, geom 4,
-// offsets 3); Bassetti-Erskine slices 373 -> 130.  Before, the transforms were
+// offsets 3); Bassetti-Erskine slices 373 -> 129.  Before, the transforms were
 // plain FP64 dot products, the deposit went through 64-bit shared atomics
 // (compare-and-swap loops) from the whole bunch's particles, and the kick
 // evaluated w(z) through the general path.  In the solve index arithmetic and
